@@ -114,16 +114,17 @@ struct sb_batch {
     };
     static constexpr int kLinGroups = 5;
     LinGroup lin_groups[kLinGroups];
-    // SimpleIterative solves: one launch per cluster size (1, 4, 8 CTAs, solve_cluster_size),
-    // a cluster per case; the job list is refilled every step from pinned memory, since it
+    // SimpleIterative solves: one launch per cluster size (1 to 16 CTAs, solve_cluster_size) and
+    // variant (rows per thread, components, kind of matrix), a cluster per case; the job list is refilled every step from pinned memory, since it
     // names the wake buffer of the step's parity
     struct SiGroup {
-        int cluster = 0, rows_per_thread = 1;
+        int cluster = 0, rows_per_thread = 1, comps = 2;
+        bool dynamic = false;  // with the precision, whether the matrix has lo parts off the diagonal
         std::vector<int> cases;
         long long off = 0;
     };
-    static constexpr int kSiGroups = 6;  // cluster size 1, 4, 8 x rows per thread 1, 4
-    SiGroup si_groups[kSiGroups];
+    std::vector<SiGroup> si_groups;
+    size_t si_smem_limit = kSiSmemShared;
     long long si_entries = 0;
     std::vector<char> si_batched;  // per case: its solve runs in a k_solve_si_jobs launch
     PinnedBuf<SolveJob> h_si_jobs;
@@ -295,16 +296,32 @@ struct sb_batch {
             if (!lj[g].empty()) lin_groups[g].jobs.upload(lj[g]);
         }
         si_batched.assign(cases.size(), 0);
+        auto si_case = [](const sb_sim& c) { return c.solver_kind == 0 && !c.solve.start_with_linearized; };
+        // the largest clusters with which all solves still run side by side, two CTAs to an SM
+        int crowding = 0;
+        for (; crowding < kMaxCrowding; ++crowding) {
+            long long ctas = 0;
+            for (const auto& c : cases) ctas += si_case(*c) ? solve_cluster_size(c->N, crowding) : 0;
+            if (ctas <= 2LL * sms) break;
+        }
         for (size_t i = 0; i < cases.size(); ++i) {
             const sb_sim& c = *cases[i];
-            if (c.solver_kind != 0 || c.solve.start_with_linearized) continue;
-            const int CS = solve_cluster_size(c.N);
+            if (!si_case(c)) continue;
+            const int CS = solve_cluster_size(c.N, crowding);
             if ((c.N + CS - 1) / CS > 1024) continue;  // too many rows per CTA: the single path reports it
-            const int rpt = si_rows_per_thread(c.N);
-            const int g = (CS == 1 ? 0 : (CS == 4 ? 1 : 2)) + (rpt == 1 ? 0 : 3);
-            si_groups[g].cluster = CS;
-            si_groups[g].rows_per_thread = rpt;
-            si_groups[g].cases.push_back(static_cast<int>(i));
+            const int rpt = si_plan(c.N, 0, 2, CS, si_smem_limit).rows_per_thread;
+            const int comps = c.split_basis() ? 2 : 3;
+            auto g = std::find_if(si_groups.begin(), si_groups.end(), [&](const SiGroup& q) {
+                return q.cluster == CS && q.rows_per_thread == rpt && q.comps == comps && q.dynamic == c.dynamic;
+            });
+            if (g == si_groups.end()) {
+                g = si_groups.insert(g, SiGroup());
+                g->cluster = CS;
+                g->rows_per_thread = rpt;
+                g->comps = comps;
+                g->dynamic = c.dynamic;
+            }
+            g->cases.push_back(static_cast<int>(i));
             si_batched[i] = 1;
         }
         for (auto& g : si_groups) {
@@ -591,11 +608,15 @@ struct sb_batch {
                     // shared memory of the group's largest case (its matrix slab depends on
                     // whether the matrix has lo parts off the diagonal, i.e. on the precision)
                     size_t smem = 0;
-                    for (int ci : g.cases)
-                        smem = std::max(smem, si_smem_bytes(cases[ci]->N, cases[ci]->solve_buffers().split_full,
-                                                              cases[ci]->solve_buffers().split_comps));
+                    for (int ci : g.cases) {
+                        const SolveBuffers sb = cases[ci]->solve_buffers();
+                        smem = std::max(smem, si_plan(cases[ci]->N, sb.split_full, sb.split_comps, g.cluster,
+                                                      si_smem_limit).smem);
+                    }
                     ck(launch_solve_simple_iterative_jobs(d_si_jobs.p + g.off, static_cast<int>(g.cases.size()), g.cluster,
-                                                          g.rows_per_thread, smem, n_launch > 1 ? pool[k++] : main),
+                                                          g.rows_per_thread, g.comps,
+                                                          cases[g.cases[0]]->solve_buffers().split_full, smem,
+                                                          n_launch > 1 ? pool[k++ % kPoolStreams] : main),
                        "batched simple iterative solve");
                 }
             if (n_launch > 1) join(1);
@@ -865,6 +886,9 @@ struct sb_batch {
                 j.m = c.dm;
                 j.st = c.solve;
                 j.b = c.solve_buffers();
+                const SiPlan p = si_plan(c.N, j.b.split_full, j.b.split_comps, g.cluster, si_smem_limit);
+                j.b.slab_rows = p.slab_rows;
+                j.b.lanes_log2 = p.lanes_log2;
                 j.b.second_margin = warm_margin;
             }
     }

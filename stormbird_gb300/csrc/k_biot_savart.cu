@@ -847,7 +847,7 @@ __global__ void __launch_bounds__(kBsReduceThreads) k_bs_reduce_jobs(const BsJob
 __device__ inline void store_factor(d3* factors, float* split, int N, const d3* basis, long long id, int c, int j, d3 u,
                                     bool fp32 = false) {
     if (factors) factors[id] = u;
-    if (split) {  // hi plane [N][C][stride], then the lo plane
+    if (split) {  // hi plane, then the lo plane: pairs (e1, e2) per column, or [N][3][stride]
         const int S = si_matrix_stride(N);
         const int C = basis ? 2 : 3;
         double comp[3] = {u.x, u.y, u.z};
@@ -862,12 +862,19 @@ __device__ inline void store_factor(d3* factors, float* split, int N, const d3* 
                 comp[1] = dot(u, e2);
             }
         }
-        float* r = split + static_cast<long long>(c) * C * S + j;
         const long long lo = static_cast<long long>(C) * N * S;
-        for (int q = 0; q < C; ++q) {
-            const float2 h = split_f64(comp[q]);
-            r[q * S] = h.x;
-            r[lo + q * S] = h.y;
+        if (C == 2) {
+            const float2 a = split_f64(comp[0]), b = split_f64(comp[1]);
+            float2* r = reinterpret_cast<float2*>(split + static_cast<long long>(c) * 2 * S) + j;
+            r[0] = make_float2(a.x, b.x);
+            *reinterpret_cast<float2*>(reinterpret_cast<float*>(r) + lo) = make_float2(a.y, b.y);
+        } else {
+            float* r = split + static_cast<long long>(c) * 3 * S + j;
+            for (int q = 0; q < 3; ++q) {
+                const float2 h = split_f64(comp[q]);
+                r[q * S] = h.x;
+                r[lo + q * S] = h.y;
+            }
         }
     }
 }

@@ -4,20 +4,21 @@
 // (stormbird/src/lifting_line/solvers/simple_iterative.rs:86-212) for one case on one
 // thread-block cluster. Every CTA of the cluster keeps the full circulation vector in
 // shared memory; CTA r owns a contiguous block of control points. Per iteration:
-//   1. induced velocity of its rows: fixed + M * Gamma (frozen_wake.rs:268-301), one warp
-//      per row, matrix rows read from L2 as (hi, lo) float pairs and the products summed
-//      in double-float arithmetic on the FP32 pipes (~2^-44 relative per product; this
-//      part's FP64 rate is 1/64 of its FP32 rate);
+//   1. induced velocity of its rows: fixed + M * Gamma (frozen_wake.rs:268-301), 8, 16 or 32
+//      lanes per row, the products summed in double-float arithmetic on the FP32 pipes
+//      (~2^-44 relative per product; this part's FP64 rate is 1/64 of its FP32 rate), while a
+//      ninth warp sums the residual terms of the iteration before (below);
 //   2. per row, in f64: total velocity (velocity_corrections.rs:28-100), span component
 //      removed (line_force_model/mod.rs:235-254), angle of attack
 //      (force_calculations.rs:79-107), Foil lift, circulation estimate
 //      (force_calculations.rs:271-292), residual term (force_calculations.rs:552-627) and
 //      the damped update; the thread's own f64 circulation stays in registers;
 //   3. new Gamma (as a float pair) and residual terms are stored into every CTA's shared
-//      memory through distributed shared memory, the per-CTA max |dGamma| likewise, one
-//      cluster barrier;
-//   4. every CTA sums the residual terms with one warp in a fixed order (the same value,
-//      hence the same stopping decision, in every CTA) and takes the max.
+//      memory through distributed shared memory, a residual term with its sign set where
+//      |dGamma| reaches the strength tolerance; one cluster barrier;
+//   4. every CTA's ninth warp sums the residual terms in a fixed order (the same value, hence
+//      the same stopping decision, in every CTA) during the next product, which a solve that
+//      stops there computes for nothing.
 // All waits are hardware cluster barriers; no spin loops.
 //
 // k_solve_lin / k_solve_lin_jobs: Linearized::solve (solvers/linearized.rs:54-222) with
@@ -29,11 +30,13 @@
 // common_utils/forces_and_moments.rs:163-245; flow_derivatives.rs:31-63).
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
 
 #include "sb_device.cuh"
+#include "sb_f64.cuh"
 #include "sb_kernels.h"
 #include "sb_ptx.cuh"
 
@@ -41,46 +44,23 @@ namespace cg = cooperative_groups;
 
 namespace sbgpu {
 
-constexpr int kSolveThreads = 256;
-constexpr int kSolveRowsPerThread = 4;  // most rows per thread (1024 per CTA)
-constexpr int kMaxCluster = 8;
-
-__host__ __device__ inline int si_cluster_size(int N) {
-    if (N <= 64) return 1;
-    if (N <= 256) return 4;
-    return 8;
-}
-int solve_cluster_size(int N) { return si_cluster_size(N); }
+constexpr int kSolveThreads = 256;                    // threads of the rows
+constexpr int kSolveCtaThreads = kSolveThreads + 32;  // and the warp that sums the residual
+constexpr int kSolveRowsPerThread = 4;                // most rows per thread (1024 per CTA)
+constexpr int kMaxCluster = 16;                       // above 8: a non-portable cluster size
 
 // Matrix slab of a CTA (its rows of the split matrix) in shared memory. Bytes of one row:
-// 2 or 3 components (SolveBuffers::split_comps) x stride floats, twice with the lo plane. When all of the CTA's rows fit
-// kSlabBudget they are copied once per solve and stay; else chunks of 4 to 8 rows (a row per
-// warp) stream through two buffers of half the budget each, every iteration. 0: not even 4
-// rows fit a buffer (N above about 900): the warps read their rows from global memory.
-constexpr long long kSlabBudget = 88 * 1024;
+// 2 or 3 components (SolveBuffers::split_comps) x stride floats, twice with the lo plane.
 __host__ __device__ inline long long si_row_bytes(int N, int full, int comps) {
     return 4LL * comps * si_matrix_stride(N) * (full ? 2 : 1);
 }
 // Shared memory before the slab, in doubles: circulation pairs 2 x stride, residual terms
-// 2 x N, maxima 2 x kMaxCluster, the CTA's M * Gamma pairs (3 doubles per row), the own
-// panels' lo parts (2 doubles per row), the own rows' in-plane bases (6 doubles per row),
-// rounded to 16 bytes.
-__host__ __device__ inline long long si_slab_offset(int N) {
-    const int CS = si_cluster_size(N);
-    const long long rp = (N + CS - 1) / CS;
-    const long long d = 2LL * si_matrix_stride(N) + 2LL * N + 2 * kMaxCluster + 3 * rp + 2 * rp + 6 * rp;
+// 2 x N, the f64 tables, the CTA's M * Gamma pairs (3 doubles per row), the own panels' lo
+// parts (2 doubles per row), rounded to 16 bytes.
+__host__ __device__ inline long long si_slab_offset(int N, int cluster) {
+    const long long rp = (N + cluster - 1) / cluster;
+    const long long d = 2LL * si_matrix_stride(N) + 2LL * N + kF64TableDoubles + 3 * rp + 2 * rp;
     return (d + 1) & ~1LL;
-}
-__host__ __device__ inline int si_slab_rows(int N, int full, int comps) {
-    const int CS = si_cluster_size(N);
-    const int rp = (N + CS - 1) / CS;
-    const long long rowb = si_row_bytes(N, full, comps);
-    // two CTAs of a cluster per SM: at most ~110 KB of shared memory each
-    const long long rest = 110 * 1024 - si_slab_offset(N) * 8;
-    const long long budget = rest < kSlabBudget ? rest : kSlabBudget;
-    if (rp * rowb <= budget) return rp;
-    const long long r = budget / (2 * rowb);
-    return r < 4 ? 0 : (r > 8 ? 8 : static_cast<int>(r));
 }
 
 struct RowGeom {
@@ -104,19 +84,6 @@ __device__ inline RowGeom row_geom(const DevModel& m, int i) {
     g.cl_gamma = (g.area == 0.0 || m.density == 0.0) ? 0.0 : 2.0 * len(span_rel) / g.area;
     g.wing = m.wing_of_line[i];
     return g;
-}
-
-// signed_angle_between(chord, u, span_dir) (vector_math.rs:65-95) with |chord| and |u| known:
-// cos = chord.u / (|chord| |u|) instead of / sqrt(|chord|^2 |u|^2) (the same to an ulp)
-__device__ inline double row_angle(const RowGeom& g, d3 u, double ul) {
-    const double triple = dot(g.chord, cross(u, g.span_dir));
-    double ang = 0.0;
-    if (!(g.chord_norm == 0.0 || ul == 0.0)) {
-        double c = dot(g.chord, u) / (g.chord_norm * ul);
-        c = fmin(fmax(c, -1.0), 1.0);
-        ang = acos(c);
-    }
-    return triple > 0.0 ? ang : -ang;
 }
 
 // velocity_corrections.rs:28-100 (returns freestream + induced, corrected)
@@ -150,61 +117,174 @@ __device__ inline double residual_from_cl(const DevModel& m, const RowGeom& g, d
 __device__ inline double residual_term(const DevModel& m, const RowGeom& g, const FoilP& f, double gam, d3 u, double aoa) {
     return residual_from_cl(m, g, gam, u, foil_cl_pre_stall(f, aoa));
 }
-// The same in the iterations, with |u| known. In the global output frame the line's span
-// vector is span_rel, to which u was made perpendicular (the projection before the angle),
-// so |u x span_rel| = |u| |span_rel| and the lift coefficient of the force is
-// -gam |u| |span_rel| rho / (area rho |u|^2 / 2) = -gam cl_gamma / |u|: one division for
-// the cross product, two square roots and the quotient of residual_from_cl. (Body-frame
-// output keeps that function: there the span vector is the body frame's.)
-__device__ inline double residual_of_row(const DevModel& m, const RowGeom& g, double gam, d3 u, double ul, double cl_pre) {
-    if (m.output_body) return residual_from_cl(m, g, gam, u, cl_pre);
-    const double clg = ul == 0.0 ? 0.0 : -gam * g.cl_gamma / ul;
-    return fabs(clg - cl_pre);
+// What an iteration needs of a line, fixed for the solve: the velocity without the induced
+// part of the first row of panels and the chord in the line's in-plane basis (e1 along the
+// chord's in-plane part, e2 = span x e1; line_basis), the foil's constants, and the stall
+// sigmoid's exponent as a straight line in |angle| (units of ln 2 / 512).
+struct SolveLine {
+    double a0, c0;           // (felt + fixed) . e1, . e2
+    double kappa, k2;        // in-plane part of the chord / |chord|; 1 - kappa^2 (0: chord in the plane)
+    double half_chord;       // -chord length / 2
+    double cl_gamma;         // 2 |span| / area (0 if the area or the density is 0)
+    double cl0, slope, cd_angle, exp_slope, exp_pos, exp_neg;
+    float fa0, fc0, fcd, fslope, fpos, fneg;  // a0, c0, cd_angle, exp_* in FP32
+    bool any;                // the line takes line_flow_any: see there
+    bool skew, even;         // k2 != 0; the same stall angle on both sides
+};
+
+__device__ __noinline__ void solve_line(const DevModel& m, int i, d3 fixed, SolveLine& out) {
+    SolveLine L;
+    const d3 e1 = m.solve_basis[2 * i], e2 = m.solve_basis[2 * i + 1];
+    const d3 base = m.felt_ctrl[i] + fixed;
+    L.a0 = dot(base, e1);
+    L.c0 = dot(base, e2);
+    const d3 span_rel = m.span_e[i] - m.span_s[i];
+    const d3 chord = m.chord_global[i];
+    const double cn = len(chord);
+    L.kappa = cn > 0.0 ? fmax(dot(chord, e1) / cn, 0.0) : -1.0;  // -1: no chord, no angle
+    const double along = cn > 0.0 ? dot(chord, normalize(span_rel)) / cn : 0.0;
+    // below 1e-24 the chord's part along the span changes no angle by more than 1e-12 rad at
+    // |angle| = 1e-12, far under the angle's own rounding in the lift
+    L.k2 = along * along > 1e-24 ? along * along : 0.0;
+    const double cl = m.chord_len[i], area = cl * m.span_len_local[i];
+    L.half_chord = -0.5 * cl;
+    L.cl_gamma = (area == 0.0 || m.density == 0.0) ? 0.0 : 2.0 * len(span_rel) / area;
+    const FoilP& f = m.foils[m.wing_of_line[i]];
+    L.cl0 = f.cl_zero_angle;
+    L.slope = f.cl_initial_slope;
+    L.cd_angle = f.angle_cd_min;
+    constexpr double kPerLn2 = 738.6598609351491;  // 512 / ln 2
+    L.exp_slope = -f.stall_slope * kPerLn2;
+    L.exp_pos = f.stall_slope * fabs(f.mean_positive_stall_angle) * kPerLn2;
+    L.exp_neg = f.stall_slope * fabs(f.mean_negative_stall_angle) * kPerLn2;
+    L.fa0 = static_cast<float>(L.a0);
+    L.fc0 = static_cast<float>(L.c0);
+    L.fcd = static_cast<float>(L.cd_angle);
+    L.fslope = static_cast<float>(L.exp_slope);
+    L.fpos = static_cast<float>(L.exp_pos);
+    L.fneg = static_cast<float>(L.exp_neg);
+    L.any = !(L.kappa > 0.0) || f.cl_high_order_power > 0.0;
+    L.skew = L.k2 != 0.0;
+    L.even = L.exp_pos == L.exp_neg;
+    out = L;
+}
+
+// Flow at a line with the in-plane velocity a e1 + c e2.
+struct LineFlow {
+    double ul, inv;  // |u|, 1 / |u| (inv = 0 where |u| is 0)
+    double cl_pre;   // the foil's pre-stall lift coefficient (foil.rs:166-190)
+    double cl_post;  // post-stall part (foil.rs:193-206), where asked for
+};
+
+// The same by CUDA's f64 functions, for what lies outside the ranges of line_flow's
+// arithmetic: |u| = 0, infinite or beyond 2^(+-50), a chord along the span or of no length, a
+// high-order lift term, a stall range so narrow that its exponential overflows.
+__device__ __noinline__ LineFlow line_flow_any(double kappa, const FoilP& f, double a, double c, bool post) {
+    LineFlow o;
+    o.ul = sqrt(a * a + c * c);
+    o.inv = o.ul == 0.0 ? 0.0 : 1.0 / o.ul;
+    double aoa = 0.0;
+    if (o.ul > kMinPositive && kappa >= 0.0) {
+        const double ang = acos(fmin(fmax(kappa * a / o.ul, -1.0), 1.0));
+        aoa = kappa * c > 0.0 ? ang : -ang;
+    }
+    o.cl_pre = foil_cl_pre_stall(f, aoa);
+    o.cl_post = post ? foil_cl_post_stall(f, aoa) : 0.0;
+    return o;
+}
+
+// Angle of attack (signed_angle_between(chord, u, span), vector_math.rs:65-95): its cosine is
+// kappa a / |u|, its sign that of kappa c, so the sine in the lift needs no angle, and the
+// angle in the stall sigmoid comes from both (better conditioned than acos of the cosine
+// near 0). fa, fc: a and c in FP32, from which the seeds, the table entries and the integer part of
+// the exponent are picked beside the FP64 chain. 29 FP64 instructions (CUDA's sqrt, division,
+// acos, sin and exp took about 150).
+__device__ __forceinline__ LineFlow line_flow(const SolveLine& L, const DevModel& m, int i, double a, double c, float fa,
+                                              float fc, bool post, const double* tab) {
+    // FP32: 1 / |u|, the angle, the exponent of the stall sigmoid in units of ln 2 / 512
+    const bool pos = f64_positive(c);
+    const float fq = fmaf(fa, fa, fc * fc), fi = rsqrt_seed(fq);
+    float fx = fa * fi, fy = fabsf(fc) * fi;
+    if (L.skew) {
+        fy = sqrtf(fmaf(static_cast<float>(L.k2) * fx, fx, fy * fy));
+        fx *= static_cast<float>(L.kappa);
+    }
+    float fang;
+    const double* e = angle_entry(fx, fy, tab, fang);
+    const float fe = (pos ? fang : -fang) + L.fcd;
+    const bool side = fe >= 0.f;  // which stall angle
+    // below 2^-64 the exponential leaves the stall at 1 (to rounding)
+    const float fw = fmaxf(fmaf(fabsf(fe), L.fslope, side ? L.fpos : L.fneg), -32768.f);
+    const int n = __float2int_rn(fminf(fw, 32768.f));
+    const double q = fma(a, a, c * c);
+    LineFlow o;
+    bool ok = !L.any && f64_seed_range(q) && fw < 32000.f;
+    ok = rsqrt_step(q, fi, o.inv) && ok;
+    o.ul = q * o.inv;
+    double y = fabs(c) * o.inv, d, x = 0.0;
+    if (L.skew) {  // a chord with a part along the span: cos = kappa a / |u|
+        x = a * o.inv;
+        const double y2 = fma(L.k2 * x, x, y * y);
+        ok = ok && f64_seed_range(y2);
+        y = y2 * rsqrt_f64(y2);
+        x *= L.kappa;
+        d = fma(y, e[0], -(x * e[1]));
+    } else {
+        d = fma(fabs(c), e[0], -(a * e[1])) * o.inv;
+    }
+    // |angle + angle_cd_min| = |th + sgn delta|, th the table angle with both signs in
+    const double del = arcsin_f64(d), th = (pos ? e[2] : -e[2]) + L.cd_angle;
+    const double ae = fabs(pos ? th + del : th - del);
+    // f: what the exponent has beyond its integer part n; beyond -32768 it is left out
+    double f = fma(ae, L.exp_slope, (side ? L.exp_pos : L.exp_neg) - f32_to_f64(static_cast<float>(n)));
+    if (fw <= -32768.f) f = 0.0;
+    const double v = 1.0 + exp2_512_f64(n, f, tab);
+    double stall;  // foil_amount_of_stall
+    ok = rcp_step(v, rcp_seed(1.f + exp2f(fw * (1.f / 512.f))), stall) && ok;
+    // (where the two stall angles differ, an angle so small that FP32 may see the other side too)
+    ok = ok && fabsf(f64_to_f32(f)) < 0.75f && (L.even || fabsf(fe) > 1e-6f);
+    if (!ok) return line_flow_any(L.kappa, m.foils[m.wing_of_line[i]], a, c, post);
+    const double sn = pos ? y : -y;
+    const double raw = fma(L.slope, sn, L.cl0);
+    o.cl_pre = fma(-raw, stall, raw);
+    if (post)  // sin 2a = 2 sin a cos a, |a| <= pi
+        o.cl_post = m.foils[m.wing_of_line[i]].cl_max_after_stall * (2.0 * sn * (L.skew ? x : a * o.inv)) * stall;
+    else
+        o.cl_post = 0.0;
+    return o;
+}
+
+// Residual term of a line (force_calculations.rs:552-627): |cl of the force - cl of the foil|.
+// In the global output frame the line's span vector is the one u was made perpendicular to, so
+// the lift coefficient of the force -gam |u| |span| rho / (area rho |u|^2 / 2) is
+// -gam cl_gamma / |u|. (Body-frame output keeps residual_from_cl: there the span vector is the
+// body frame's.)
+__device__ __noinline__ double residual_body(const DevModel& m, int i, double gam, double a, double c, double cl_pre) {
+    return residual_from_cl(m, row_geom(m, i), gam, m.solve_basis[2 * i] * a + m.solve_basis[2 * i + 1] * c, cl_pre);
+}
+__device__ __forceinline__ double residual_of_line(const DevModel& m, const SolveLine& L, int i, double gam, double a,
+                                                   double c, const LineFlow& o) {
+    if (m.output_body) return residual_body(m, i, gam, a, c, o.cl_pre);
+    return fabs(fma(-gam * L.cl_gamma, o.inv, -o.cl_pre));
 }
 
 // Double-float accumulation for the matrix-vector product: (S, C) += (xh + xl) * (gh + gl).
-// The product's head xh*gh is added to S by an error-free two-sum (Knuth); its rounding error
-// (an exact FMA) and the cross terms xh*gl + xl*gh go into C; xl*gl (~2^-48 of the product)
-// is dropped. The _rn intrinsics keep the compiler from fusing the steps.
-__device__ __forceinline__ void ff_mac(float& S, float& C, float2 x, float2 g) {
-    const float p = __fmul_rn(x.x, g.x);
-    float t = fmaf(x.x, g.x, -p);
-    t = fmaf(x.x, g.y, t);
-    t = fmaf(x.y, g.x, t);
+// The product's head xh*gh is added to S by an error-free two-sum (Knuth: exact for any
+// magnitudes; a Kahan-compensated sum, two operations cheaper, is exact only while the
+// running sum outweighs the new term and left the solve a residual floor near 1e-11); its
+// rounding error (an exact FMA) and the cross terms xh*gl + xl*gh go into C; xl*gl (~2^-48 of
+// the product) is dropped. The _rn intrinsics keep the compiler from fusing the steps.
+template <bool LO>
+__device__ __forceinline__ void ff_mac(float& S, float& C, float xh, float xl, float gh, float gl) {
+    const float p = __fmul_rn(xh, gh);
+    float t = fmaf(xh, gh, -p);
+    t = fmaf(xh, gl, t);
+    if (LO) t = fmaf(xl, gh, t);
     const float s = __fadd_rn(S, p);
     const float bv = __fsub_rn(s, S);
     const float err = __fadd_rn(__fsub_rn(S, __fsub_rn(s, bv)), __fsub_rn(p, bv));
     S = s;
     C = __fadd_rn(C, __fadd_rn(err, t));
-}
-// Four consecutive columns into one component's double-float sum (S, C): matrix entries
-// (a + al) (al = 0 without lo parts) against the circulation pairs (g01.x + g01.y),
-// (g01.z + g01.w), (g23.x + g23.y), (g23.z + g23.w), each by ff_mac (two-sum: exact for any
-// magnitudes; a Kahan-compensated sum, two operations cheaper, is exact only while the
-// running sum outweighs the new term and left the solve a residual floor near 1e-11).
-__device__ __forceinline__ void ff_mac4(float& S, float& C, float4 a, float4 al, float4 g01, float4 g23) {
-    ff_mac(S, C, make_float2(a.x, al.x), make_float2(g01.x, g01.y));
-    ff_mac(S, C, make_float2(a.y, al.y), make_float2(g01.z, g01.w));
-    ff_mac(S, C, make_float2(a.z, al.z), make_float2(g23.x, g23.y));
-    ff_mac(S, C, make_float2(a.w, al.w), make_float2(g23.z, g23.w));
-}
-
-// One lane's share of a row of the split matrix times the circulation: columns 4*lane + 128*t,
-// NC components (planes of S floats), hi plane fh and (full) lo plane fl.
-template <int NC>
-__device__ __forceinline__ void row_dot_lane(const float* fh, const float* fl, const float2* Gc, float (&acc)[6], int S,
-                                             int lane, int full) {
-#pragma unroll 2
-    for (int k = 4 * lane; k < S; k += 128) {
-        const float4 g01 = *reinterpret_cast<const float4*>(Gc + k);  // (hi, lo) of columns k, k + 1
-        const float4 g23 = *reinterpret_cast<const float4*>(Gc + k + 2);
-#pragma unroll
-        for (int q = 0; q < NC; ++q) {
-            const float4 a = *reinterpret_cast<const float4*>(fh + q * S + k);
-            const float4 al = full ? *reinterpret_cast<const float4*>(fl + q * S + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-            ff_mac4(acc[2 * q], acc[2 * q + 1], a, al, g01, g23);
-        }
-    }
 }
 // (S, C) += (h, l), another double-float partial sum
 __device__ __forceinline__ void ff_add(float& S, float& C, float h, float l) {
@@ -213,6 +293,89 @@ __device__ __forceinline__ void ff_add(float& S, float& C, float h, float l) {
     const float err = __fadd_rn(__fsub_rn(S, __fsub_rn(s, bv)), __fsub_rn(h, bv));
     S = s;
     C = __fadd_rn(C, __fadd_rn(err, l));
+}
+// The same for the two in-plane components at once, as the lanes of packed FP32 operations
+// (half the instructions: at two warps per SM sub-partition the product is bound by their issue and
+// latency): component x in .x, y in .y, the circulation as broadcast pairs. a - b is the packed
+// FMA (b * -1 + a), exact like the subtraction.
+__device__ __forceinline__ float2 f2_sub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+template <bool LO>
+__device__ __forceinline__ void ff_mac2(float2& S, float2& C, float2 xh, float2 xl, float2 gh, float2 gl) {
+    const float2 p = __fmul2_rn(xh, gh);
+    float2 t = __ffma2_rn(xh, gh, make_float2(-p.x, -p.y));
+    t = __ffma2_rn(xh, gl, t);
+    if (LO) t = __ffma2_rn(xl, gh, t);
+    const float2 s = __fadd2_rn(S, p);
+    const float2 bv = f2_sub(s, S);
+    const float2 err = __fadd2_rn(f2_sub(S, f2_sub(s, bv)), f2_sub(p, bv));
+    S = s;
+    C = __fadd2_rn(C, __fadd2_rn(err, t));
+}
+__device__ __forceinline__ void ff_add2(float2& S, float2& C, float2 h, float2 l) {
+    const float2 s = __fadd2_rn(S, h);
+    const float2 bv = f2_sub(s, S);
+    const float2 err = __fadd2_rn(f2_sub(S, f2_sub(s, bv)), f2_sub(h, bv));
+    S = s;
+    C = __fadd2_rn(C, __fadd2_rn(err, l));
+}
+__device__ __forceinline__ float2 shfl_xor2(float2 v, int o) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+
+// A row of the split matrix times the circulation Gc (pairs gh, gl), summed over the 1 << lp lanes
+// of a row (every one of them gets the sum): lane gl takes four consecutive columns 4 gl + (4 << lp) t.
+// out: (hi, lo) per component. Two components: pairs (x, y) per column; three: planes x, y, z of
+// S floats. fl: the lo plane (LO only).
+template <int NC, bool LO>
+__device__ __forceinline__ void row_dot(const float* fh, const float* fl, const float2* Gc, int S, int gl, int lp,
+                                        float (&out)[6]) {
+    if constexpr (NC == 2) {
+        float2 Sa = make_float2(0.f, 0.f), Ca = Sa, Sb = Sa, Cb = Sa;  // two chains, merged at the end
+#pragma unroll 1
+        for (int k = 4 * gl; k < S; k += 4 << lp) {
+            const float4 g0 = *reinterpret_cast<const float4*>(Gc + k), g1 = *reinterpret_cast<const float4*>(Gc + k + 2);
+            const float4 a0 = *reinterpret_cast<const float4*>(fh + 2 * k), a1 = *reinterpret_cast<const float4*>(fh + 2 * k + 4);
+            float4 l0 = make_float4(0.f, 0.f, 0.f, 0.f), l1 = l0;
+            if (LO) {
+                l0 = *reinterpret_cast<const float4*>(fl + 2 * k);
+                l1 = *reinterpret_cast<const float4*>(fl + 2 * k + 4);
+            }
+            ff_mac2<LO>(Sa, Ca, make_float2(a0.x, a0.y), make_float2(l0.x, l0.y), make_float2(g0.x, g0.x), make_float2(g0.y, g0.y));
+            ff_mac2<LO>(Sb, Cb, make_float2(a0.z, a0.w), make_float2(l0.z, l0.w), make_float2(g0.z, g0.z), make_float2(g0.w, g0.w));
+            ff_mac2<LO>(Sa, Ca, make_float2(a1.x, a1.y), make_float2(l1.x, l1.y), make_float2(g1.x, g1.x), make_float2(g1.y, g1.y));
+            ff_mac2<LO>(Sb, Cb, make_float2(a1.z, a1.w), make_float2(l1.z, l1.w), make_float2(g1.z, g1.z), make_float2(g1.w, g1.w));
+        }
+        ff_add2(Sa, Ca, Sb, Cb);
+#pragma unroll 1
+        for (int o = 1 << (lp - 1); o > 0; o >>= 1) ff_add2(Sa, Ca, shfl_xor2(Sa, o), shfl_xor2(Ca, o));
+        out[0] = Sa.x;
+        out[1] = Ca.x;
+        out[2] = Sa.y;
+        out[3] = Ca.y;
+    } else {
+        float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+        for (int k = 4 * gl; k < S; k += 4 << lp) {
+            const float4 g0 = *reinterpret_cast<const float4*>(Gc + k), g1 = *reinterpret_cast<const float4*>(Gc + k + 2);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const float4 a = *reinterpret_cast<const float4*>(fh + q * S + k);
+                const float4 l = LO ? *reinterpret_cast<const float4*>(fl + q * S + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                ff_mac<LO>(acc[2 * q], acc[2 * q + 1], a.x, l.x, g0.x, g0.y);
+                ff_mac<LO>(acc[2 * q], acc[2 * q + 1], a.y, l.y, g0.z, g0.w);
+                ff_mac<LO>(acc[2 * q], acc[2 * q + 1], a.z, l.z, g1.x, g1.y);
+                ff_mac<LO>(acc[2 * q], acc[2 * q + 1], a.w, l.w, g1.z, g1.w);
+            }
+        }
+#pragma unroll 1
+        for (int o = 1 << (lp - 1); o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                ff_add(acc[2 * q], acc[2 * q + 1], __shfl_xor_sync(0xffffffffu, acc[2 * q], o),
+                       __shfl_xor_sync(0xffffffffu, acc[2 * q + 1], o));
+#pragma unroll
+        for (int q = 0; q < 6; ++q) out[q] = acc[q];
+    }
 }
 
 // Sum / max over a warp in a fixed order (lane 0 gets the result): every CTA of a cluster
@@ -242,173 +405,198 @@ __device__ __forceinline__ unsigned long long warp_umax_to_lane0(unsigned long l
 // SimpleIterative::solve for one case on the calling thread-block cluster (see the top of
 // the file). Run by k_solve_si (one case) and k_solve_si_jobs (a cluster per case of a batch).
 // RPT = rows per thread: 1 while a CTA owns at most kSolveThreads rows (registers for two
-// CTAs per SM), else kSolveRowsPerThread.
-template <int RPT>
+// CTAs per SM), else kSolveRowsPerThread. NC = components of a matrix entry
+// (SolveBuffers::split_comps), LO: the lo plane is read (split_full). Each variant's loop is kept
+// small (rare branches out of line, one copy of the product and of the row math for the guard's
+// passes and the iterations alike): with every variant in one kernel the code was 325 KB, and a
+// loop that does not fit the instruction cache waits for its instructions.
+template <int RPT, int NC, bool LO>
 __device__ void si_solve(const DevModel& m, const SolveSettings& st, const SolveBuffers& b) {
     cg::cluster_group cl = cg::this_cluster();
     const int CS = static_cast<int>(cl.num_blocks());
     const int rank = static_cast<int>(cl.block_rank());
     const int N = m.N;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = kSolveThreads / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool sums = warp == kSolveThreads / 32;  // the warp that sums the residual and issues the copies
     extern __shared__ __align__(16) double smem[];
     // circulation of every line as (hi, lo) float pairs for the matrix-vector products, padded
     // with zeros to the matrix's row stride; the f64 circulation of the thread's own rows
     // stays in registers (gown)
     const int S = si_matrix_stride(N);
-    float2* G[2] = {reinterpret_cast<float2*>(smem), reinterpret_cast<float2*>(smem + S)};
-    double* RR[2] = {smem + 2 * S, smem + 2 * S + N};
-    double* MX[2] = {smem + 2 * S + 2 * N, smem + 2 * S + 2 * N + kMaxCluster};
     const int rp = (N + CS - 1) / CS;
     const int r0 = min(N, rank * rp), r1 = min(N, r0 + rp);
+    auto G = [&](int k) { return reinterpret_cast<float2*>(smem) + k * S; };
+    auto RR = [&](int k) { return smem + 2 * S + k * N; };
+    double* tab = smem + 2 * S + 2 * N;
+    // M * Gamma of the CTA's rows as double-float pairs (x hi, x lo, y hi, y lo, z hi, z lo);
+    // the row's owner adds them to the fixed part in f64
+    float* uff = reinterpret_cast<float*>(tab + kF64TableDoubles);
+    // lo parts of the own panels' entries (x, y, z), when the matrix has none elsewhere
+    float* diag_lo = reinterpret_cast<float*>(tab + kF64TableDoubles + 3 * rp);
+    float* slab = reinterpret_cast<float*>(smem + si_slab_offset(N, CS));
+    __shared__ double s_res;
+    __shared__ unsigned long long s_umax;
+    __shared__ int s_conv;
+    __shared__ __align__(8) uint64_t s_mbar[2];
+
+    auto barrier = [&]() {
+        if (CS > 1) cl.sync();
+        else __syncthreads();
+    };
     // The thread's k-th own row (offset from r0): consecutive rows on consecutive threads, so
     // that a CTA owning fewer than 256 rows fills as few warps as possible (this part's FP64
     // pipe costs the same per warp instruction however few lanes are active).
     auto own_row = [&](int k) { return tid + k * kSolveThreads; };
-    // M * Gamma of the CTA's rows as double-float pairs (x hi, x lo, y hi, y lo, z hi, z lo);
-    // the row's owner adds them to the fixed part in f64
-    float* uff = reinterpret_cast<float*>(smem + 2 * S + 2 * N + 2 * kMaxCluster);
-    const int rp_max = (N + CS - 1) / CS;
-    // lo parts of the own panels' entries (x, y, z), when the matrix has none elsewhere
-    float* diag_lo = reinterpret_cast<float*>(smem + 2 * S + 2 * N + 2 * kMaxCluster + 3 * rp_max);
-    d3* basis_sm = reinterpret_cast<d3*>(smem + 2 * S + 2 * N + 2 * kMaxCluster + 5 * rp_max);  // e1, e2 per own row
-    float* slab = reinterpret_cast<float*>(smem + si_slab_offset(N));
-    __shared__ double s_res;
-    __shared__ unsigned long long s_umax[kSolveThreads / 32];
-    __shared__ int s_conv;
-    __shared__ __align__(8) uint64_t s_mbar[2];
 
     const bool scale0 = fabs(st.correction_factor_initial - 1.0) > kMinPositive;
-    for (int i = tid; i < N; i += kSolveThreads) {
+    for (int i = tid; i < N; i += kSolveCtaThreads) {
         double g = b.gamma_prev[i];
         if (scale0) g *= st.correction_factor_initial;
-        G[0][i] = split_f64(g);
+        G(0)[i] = split_f64(g);
     }
-    for (int i = N + tid; i < S; i += kSolveThreads) G[0][i] = G[1][i] = make_float2(0.f, 0.f);
-    // per-thread rows
-    RowGeom rg[RPT];
-    d3 u_last[RPT];
-    double aoa_last[RPT], gown[RPT];
+    for (int i = N + tid; i < S; i += kSolveCtaThreads) G(0)[i] = G(1)[i] = make_float2(0.f, 0.f);
+    load_f64_tables(tab, tid, kSolveCtaThreads);
+    // per-thread rows: the in-plane velocity and the circulation estimate of the last iteration
+    SolveLine ln[RPT];
+    double a_last[RPT], c_last[RPT], est_last[RPT], gown[RPT];
     int nrows = 0;
     for (int k = 0; k < RPT; ++k) {
         int i = r0 + own_row(k);
-        if (i < r1) {
+        if (!sums && i < r1) {
             double g = b.gamma_prev[i];
             if (scale0) g *= st.correction_factor_initial;
             gown[k] = g;
-            rg[k] = row_geom(m, i);
-            u_last[k] = mk(0, 0, 0);
-            aoa_last[k] = 0.0;
+            SolveLine l;
+            solve_line(m, i, b.fixed[i], l);
+            ln[k] = l;
+            a_last[k] = c_last[k] = est_last[k] = 0.0;
             nrows = k + 1;
         }
     }
-    __syncthreads();
 
-    const int full = b.split_full;
-    const int C = b.split_comps;  // 2: in-plane components in the rows' bases, 3: x, y, z
-    const int slab_rows = si_slab_rows(N, full, C);
+    constexpr int C = NC;  // 2: in-plane components in the rows' bases, 3: x, y, z
+    const int slab_rows = b.slab_rows;
     const int nrows_cta = r1 - r0;
     const int nch = slab_rows > 0 ? (nrows_cta + slab_rows - 1) / slab_rows : 0;
-    const bool resident = slab_rows > 0 && slab_rows >= rp_max;  // copied once, kept
+    const bool resident = slab_rows > 0 && slab_rows >= rp;      // copied once, kept
     const long long rowf = static_cast<long long>(C) * S;         // floats of a row, one plane
-    const long long buf_floats = static_cast<long long>(slab_rows) * rowf * (full ? 2 : 1);
+    const long long buf_floats = static_cast<long long>(slab_rows) * rowf * (LO ? 2 : 1);
     const long long lo_plane = static_cast<long long>(C) * N * S;
-    if (tid == 0) {
+    const int lp = b.lanes_log2;  // log2 of the lanes per row of the product
+   if (tid == 0) {
         mbar_init(&s_mbar[0], 1);
         mbar_init(&s_mbar[1], 1);
         fence_mbar_init();
     }
-    for (int k = tid; k < nrows_cta; k += kSolveThreads) {
-        const long long row = r0 + k;
-        if (!full) {
+    if (!LO)
+        for (int k = tid; k < nrows_cta; k += kSolveCtaThreads) {
+            const long long row = r0 + k;
             const float* fl = b.factors_split + lo_plane + row * rowf;
-            for (int q = 0; q < C; ++q) diag_lo[3 * k + q] = fl[q * S + row];
+            for (int q = 0; q < C; ++q) diag_lo[3 * k + q] = fl[C == 2 ? 2 * row + q : q * S + row];
         }
-        if (C == 2) {
-            basis_sm[2 * k] = b.basis[2 * row];
-            basis_sm[2 * k + 1] = b.basis[2 * row + 1];
-        }
-    }
 
     // residual of the initial solution with zero velocity (simple_iterative.rs:180-184)
     double residual = 0.0;
     if (st.max_iterations == 0) {
         if (tid == 0) {
             double s = 0.0;
-            for (int i = 0; i < N; ++i) s += fabs(0.0 - foil_cl_pre_stall(m.foils[m.wing_of_line[i]], 0.0));
-            s_res = s / static_cast<double>(N);
+            for (int i = 0; i < N; ++i)
+                s += fabs(0.0 - line_flow_any(-1.0, m.foils[m.wing_of_line[i]], 0.0, 0.0, false).cl_pre);
+            s_res = s;
         }
         __syncthreads();
         residual = s_res;
     }
-    cl.sync();
+    barrier();
 
-    // induced velocity of own rows for the circulation Gc: fixed + M * Gc. One warp per row;
-    // double-float arithmetic on the FP32 pipes (this part's FP64 rate is 1/64 of its FP32
-    // rate), a lane taking four consecutive columns per 16-byte shared-memory load. The
-    // CTA's matrix rows come from its slab in shared memory: thread 0 copies them by bulk
-    // asynchronous copies (cp.async.bulk, completion on an mbarrier; bounded waits), kept for
-    // the whole solve when they fit, else streamed in chunks through two buffers (the copy
-    // of chunk c + 1 runs while the warps work on chunk c).
+    // induced velocity of own rows for the circulation Gc: fixed + M * Gc, in double-float
+    // arithmetic on the FP32 pipes (this part's FP64 rate is 1/64 of its FP32 rate). 8, 16 or 32
+    // lanes take a row, four consecutive columns per step, then a butterfly over them (row_dot). The CTA's matrix rows come from its slab in
+    // shared memory: one thread copies them by bulk asynchronous copies (cp.async.bulk,
+    // completion on an mbarrier; bounded waits), kept for the whole solve when they fit, else
+    // streamed in chunks through two buffers (the copy of chunk c + 1 runs while the warps
+    // work on chunk c).
     // A slab wait that runs out records kDevTimeout (the host raises SB_ERR_TIMEOUT after the
-    // launch); that thread then waits no more and thread 0 issues no more copies, and the
-    // solve runs its remaining (bounded) iterations on whatever the buffers hold, through the
+    // launch); that thread then waits no more and the copying thread issues no more copies, and
+    // the solve runs its remaining (bounded) iterations on whatever the buffers hold, through the
     // same barriers as the other CTAs of the cluster, so that none waits for it forever.
     uint32_t mph[2] = {0u, 0u};
-    bool pending[2] = {false, false};  // thread 0: a copy into the buffer not yet waited for
+    bool pending[2] = {false, false};  // copying thread: a copy into the buffer not yet waited for
     bool slab_loaded = false, dead = false;
-    auto issue = [&](int c, int bufi) {  // thread 0
+    const bool copier = tid == kSolveThreads;
+    auto issue = [&](int c, int bufi) {
         const long long row0 = r0 + static_cast<long long>(c) * slab_rows;
         const int nr = min(slab_rows, r1 - static_cast<int>(row0));
         const uint32_t bytes = static_cast<uint32_t>(nr * rowf * 4);
         float* dst = slab + bufi * buf_floats;
-        mbar_expect_tx(&s_mbar[bufi], full ? 2 * bytes : bytes);
+        mbar_expect_tx(&s_mbar[bufi], LO ? 2 * bytes : bytes);
         bulk_g2s(dst, b.factors_split + row0 * rowf, bytes, &s_mbar[bufi]);
-        if (full) bulk_g2s(dst + slab_rows * rowf, b.factors_split + lo_plane + row0 * rowf, bytes, &s_mbar[bufi]);
+        if (LO) bulk_g2s(dst + slab_rows * rowf, b.factors_split + lo_plane + row0 * rowf, bytes, &s_mbar[bufi]);
         pending[bufi] = true;
     };
-    // (S, C) += row . Gc over the lane's columns, from fh (hi) and fl (lo, full only)
-    auto row_dot = [&](const float* fh, const float* fl, const float2* Gc, float (&acc)[6]) {
-        if (C == 2) row_dot_lane<2>(fh, fl, Gc, acc, S, lane, full);
-        else row_dot_lane<3>(fh, fl, Gc, acc, S, lane, full);
+    // rows [row0, row0 + nr) of the matrix at `base` (lo plane at base + lo_off) times Gc. Every
+    // lane of a warp goes through the butterflies together: groups past the end repeat the last
+    // row and store nothing.
+    auto rows_times = [&](const float* base, long long lo_off, int row0, int nr, const float2* Gc) {
+        const int group = tid >> lp, gl = tid & ((1 << lp) - 1), groups = kSolveThreads >> lp;
+#pragma unroll 1
+        for (int w0 = 0; w0 < nr; w0 += groups) {
+            if (w0 + ((warp * 32) >> lp) >= nr) break;  // uniform in the warp
+            const int w = min(w0 + group, nr - 1);
+            const float* fh = base + w * rowf;
+            float acc[6];
+            row_dot<NC, LO>(fh, fh + lo_off, Gc, S, gl, lp, acc);
+            if (gl == 0 && w0 + group < nr) {
+                const int row = row0 + w;
+                if (!LO) {  // the own panel's entry is f64: its lo parts times Gamma hi
+                    const float g = Gc[row].x;
+                    const float* dl = diag_lo + 3 * (row - r0);
+#pragma unroll
+                    for (int q = 0; q < NC; ++q) ff_add(acc[2 * q], acc[2 * q + 1], __fmul_rn(dl[q], g), fmaf(dl[q], g, -__fmul_rn(dl[q], g)));
+                }
+                float* o = uff + 6 * (row - r0);
+#pragma unroll
+                for (int q = 0; q < 2 * NC; ++q) o[q] = acc[q];
+            }
+        }
     };
-    auto finish_row = [&](int row, float (&acc)[6], const float2* Gc) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-                if (q < C)
-                    ff_add(acc[2 * q], acc[2 * q + 1], __shfl_down_sync(0xffffffffu, acc[2 * q], o),
-                           __shfl_down_sync(0xffffffffu, acc[2 * q + 1], o));
+    // The sum of the residual over all lines from the terms in R and whether the solve stops there
+    // (the summing warp): lanes over lines lane, lane + 32, ..., then a fixed-order tree. The mean
+    // is compared with its tolerance as the sum with N times it (a division is 9 FP64
+    // instructions); the mean itself is the last sum over N.
+    const bool want_max = st.strength_tolerance > 0.0;
+    const double sum_tolerance = st.residual_tolerance * static_cast<double>(N);
+    auto decide = [&](const double* R) {
+        double s = 0.0;
+        bool big = false;  // some |dGamma| at or above the strength tolerance (the term's sign)
+#pragma unroll 1
+        for (int i = lane; i < N; i += 32) {
+            const double v = R[i];
+            s += fabs(v);
+            big = big || __double2hiint(v) < 0;
+        }
+        s = warp_sum_to_lane0(s);
+        big = __any_sync(0xffffffffu, big) != 0;
         if (lane == 0) {
-            if (!full) {  // the own panel's entry is f64: its lo parts times Gamma hi
-                const float2 g = Gc[row];
-                const float* dl = diag_lo + 3 * (row - r0);
-#pragma unroll
-                for (int q = 0; q < 3; ++q)
-                    if (q < C) ff_mac(acc[2 * q], acc[2 * q + 1], make_float2(0.f, dl[q]), g);
-            }
-            float* o = uff + 6 * (row - r0);
-#pragma unroll
-            for (int q = 0; q < 6; ++q) o[q] = acc[q];
+            s_res = s;
+            s_conv = s < sum_tolerance || (want_max && !big);
         }
     };
-    auto induced_rows = [&](const float2* Gc) {
-        if (slab_rows == 0) {  // rows from global memory
-            for (int row = r0 + warp; row < r1; row += nwarps) {
-                const float* fh = b.factors_split + static_cast<long long>(row) * rowf;
-                float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                row_dot(fh, fh + lo_plane, Gc, acc);
-                finish_row(row, acc, Gc);
-            }
-            __syncthreads();
-            return;
-        }
-        const bool copy = !(resident && slab_loaded);
-        if (copy && tid == 0 && !dead) {
+    // M * Gc of the CTA's rows (none: Gc == nullptr) beside the sum of the residual terms R of the
+    // iteration before (none: R == nullptr)
+    auto induced_rows = [&](const float2* Gc, const double* R) {
+        const bool copy = nch > 0 && !(resident && slab_loaded) && Gc;  // nch: 0 also for a CTA without rows
+        if (copy && copier && !dead) {
             issue(0, 0);
             if (nch > 1) issue(1, 1);
         }
-        for (int c = 0; c < nch; ++c) {
+        if (sums) {
+            __syncwarp();
+            if (R) decide(R);
+        }
+        const int chunks = !Gc ? 0 : (slab_rows > 0 ? nch : (nrows_cta > 0 ? 1 : 0));
+#pragma unroll 1
+        for (int c = 0; c < chunks; ++c) {
             const int bufi = c & 1;
             if (copy) {
                 if (!dead) {
@@ -418,37 +606,43 @@ __device__ void si_solve(const DevModel& m, const SolveSettings& st, const Solve
                 mph[bufi] ^= 1u;
             }
             const int row0 = r0 + c * slab_rows;
-            const int nr = min(slab_rows, r1 - row0);
-            const float* base = slab + bufi * buf_floats;
-            for (int w = warp; w < nr; w += nwarps) {
-                float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                row_dot(base + w * rowf, base + (slab_rows + w) * rowf, Gc, acc);
-                finish_row(row0 + w, acc, Gc);
-            }
+            const int nr = slab_rows > 0 ? min(slab_rows, r1 - row0) : nrows_cta;  // 0: rows from global memory
+            const float* base = slab_rows > 0 ? slab + bufi * buf_floats : b.factors_split + static_cast<long long>(r0) * rowf;
+            if (!sums) rows_times(base, slab_rows > 0 ? slab_rows * rowf : lo_plane, row0, nr, Gc);
             __syncthreads();  // every warp is done with this buffer
-            if (copy && !resident && tid == 0 && !dead && c + 2 < nch) issue(c + 2, bufi);
+            if (copy && !resident && copier && !dead && c + 2 < nch) issue(c + 2, bufi);
         }
-        slab_loaded = true;
+        if (chunks == 0) __syncthreads();
+        else slab_loaded = true;
     };
-    // Velocity of own row i with its span component taken out (project(u, span_rel) before
-    // the angle): freestream + fixed + M * Gamma. With two components the products are already
-    // the in-plane coordinates along the row's basis (e1, e2), and the velocity correction is
-    // off (the only mode the two-component matrix is built for).
-    auto row_velocity = [&](int i, const RowGeom& g) {
+    // In-plane velocity (a, c) of own row i: freestream + fixed + M * Gamma with the span
+    // component taken out (project(u, span_rel) before the angle). With two components the
+    // products are already the in-plane coordinates along the row's basis (e1, e2), and the
+    // velocity correction is off (the only mode the two-component matrix is built for).
+    auto row_velocity = [&](int i, const SolveLine& L, double& a, double& c, float& fa, float& fc) {
         const float* o = uff + 6 * (i - r0);
-        const d3 fx = b.fixed[i];
         if (C == 2) {
-            const d3 e1 = basis_sm[2 * (i - r0)], e2 = basis_sm[2 * (i - r0) + 1];
-            const d3 base = g.felt + fx;
-            const double a = dot(base, e1) + (static_cast<double>(o[0]) + static_cast<double>(o[1]));
-            const double c = dot(base, e2) + (static_cast<double>(o[2]) + static_cast<double>(o[3]));
-            return e1 * a + e2 * c;
+            fa = L.fa0 + o[0];
+            fc = L.fc0 + o[2];
+            a = L.a0 + (f32_to_f64_any(o[0]) + f32_to_f64_any(o[1]));
+            c = L.c0 + (f32_to_f64_any(o[2]) + f32_to_f64_any(o[3]));
+            return;
         }
+        const d3 fx = b.fixed[i];
         const d3 ind = mk(fx.x + (static_cast<double>(o[0]) + static_cast<double>(o[1])),
                           fx.y + (static_cast<double>(o[2]) + static_cast<double>(o[3])),
                           fx.z + (static_cast<double>(o[4]) + static_cast<double>(o[5])));
-        const d3 u = total_velocity(st, g.felt, ind);
-        return u - g.span_dir * dot(u, g.span_dir);
+        const d3 u = total_velocity(st, m.felt_ctrl[i], ind);
+        a = dot(u, m.solve_basis[2 * i]);
+        c = dot(u, m.solve_basis[2 * i + 1]);
+        fa = static_cast<float>(a);
+        fc = static_cast<float>(c);
+    };
+    // v into slot i of an array of every CTA of the cluster
+    auto store_all = [&](auto* arr, int i, auto v) {
+        if (CS == 1) arr[i] = v;
+        else
+            for (int q = 0; q < CS; ++q) cl.map_shared_rank(arr, q)[i] = v;
     };
 
     // Guarded warm start: residual (simple_iterative.rs:160-176) of the plain start G[0]
@@ -460,239 +654,270 @@ __device__ void si_solve(const DevModel& m, const SolveSettings& st, const Solve
     // default) on both measures: its per-line error is noise-like, and a start that is only slightly
     // better by the initial residual took more iterations than the extrapolation (566 of
     // 2,560 solves of the uneven-case batch: 108 iterations against 107 from the plain start).
-    if (b.candidate[0] || b.candidate[1]) {
-        double best = 0.0, best_max = 0.0;
-        int taken = 0;
-        for (int v = 0; v < 3; ++v) {
-            const double* src = v == 0 ? nullptr : b.candidate[v - 1];
-            if (v > 0 && !src) continue;
-            float2* Gv = v == 0 ? G[0] : G[1];
-            if (v > 0) {
-                for (int i = tid; i < N; i += kSolveThreads) G[1][i] = split_f64(src[i]);
-                __syncthreads();
-            }
-            induced_rows(Gv);
-            for (int k = 0; k < nrows; ++k) {
-                int i = r0 + own_row(k);
-                const RowGeom& g = rg[k];
-                const FoilP f = m.foils[g.wing];
-                const d3 u = row_velocity(i, g);
-                double aoa = len(u) > kMinPositive ? signed_angle_between(g.chord, u, g.span_dir) : 0.0;
-                double r = residual_term(m, g, f, v == 0 ? gown[k] : src[i], u, aoa);
-                for (int q = 0; q < CS; ++q) cl.map_shared_rank(RR[0], q)[i] = r;
-            }
-            cl.sync();
-            if (warp == 0) {
-                double s = 0.0;
-                unsigned long long mx = 0;
-                for (int i = lane; i < N; i += 32) {
-                    s += RR[0][i];
-                    const unsigned long long bi = mag_bits(RR[0][i]);
-                    mx = bi > mx ? bi : mx;
-                }
-                s = warp_sum_to_lane0(s);
-                mx = warp_umax_to_lane0(mx);
-                if (lane == 0) {
-                    s_res = s;
-                    s_umax[0] = mx;
-                }
-            }
-            __syncthreads();
-            const double rv = s_res, rmax = bits_value(s_umax[0]);
-            if (v == 0) {
-                best = rv;
-                best_max = rmax;
-            } else if (isfinite(rv) && rv < (v == 2 ? b.second_margin : 1.0) * best &&
-                       rmax < (v == 2 ? b.second_margin : 1.0) * best_max) {  // same decision in every CTA
-                best = rv;
-                best_max = rmax;
-                taken = v;
-                for (int i = tid; i < N; i += kSolveThreads) G[0][i] = G[1][i];
-                for (int k = 0; k < nrows; ++k) gown[k] = src[r0 + own_row(k)];
-            }
-            cl.sync();  // RR[0] and G[1] are written again by the next pass or the first iteration
-        }
-        if (rank == 0 && tid == 0) b.scalars[4] = static_cast<double>(taken);
-    } else if (rank == 0 && tid == 0) {
-        b.scalars[4] = -1.0;
-    }
-
+    // Passes start = 0 (plain), 1, 2 (candidates) run the iteration's own product and row math;
+    // 3: the iterations.
+    const bool guarded = b.candidate[0] || b.candidate[1];
+    int start = guarded ? 0 : 3;
+    double best = 0.0, best_max = 0.0;
+    int taken = guarded ? 0 : -1;
     int it = 0, cur = 0;
     bool conv = false;
-    const bool want_max = st.strength_tolerance > 0.0;
-    while (it < st.max_iterations && !conv) {
-        it += 1;
-        const float2* Gc = G[cur];
-        // 1. induced velocity of own rows
-        induced_rows(Gc);
-        // 2. row updates
-        unsigned long long lmax = 0;  // max |dGamma| of the thread's rows (mag_bits)
-        for (int k = 0; k < nrows; ++k) {
-            int i = r0 + own_row(k);
-            const RowGeom& g = rg[k];
-            const FoilP f = m.foils[g.wing];
-            const d3 u = row_velocity(i, g);
-            const double ul = len(u);
-            double aoa = ul > kMinPositive ? row_angle(g, u, ul) : 0.0;
-            // the pre-stall lift coefficient serves the estimate and the residual alike
-            const double clp = foil_cl_pre_stall(f, aoa);
-            const double clc = m.include_viscous_lift ? clp + foil_cl_post_stall(f, aoa) : clp;  // circulation_cl
-            double est = -0.5 * g.chord_len * ul * clc;
-            double gold = gown[k];
-            double r = residual_of_row(m, g, gold, u, ul, clp);
-            double d = est - gold;
-            if (want_max) {
-                const unsigned long long db = mag_bits(d);
-                lmax = db > lmax ? db : lmax;
+#pragma unroll 1
+    while (true) {
+        const double* src = nullptr;
+        if (start == 1 || start == 2) {
+            src = b.candidate[start - 1];
+            if (!src) {
+                ++start;
+                continue;
             }
-            double gnew = gold + st.damping * d;
-            gown[k] = gnew;
-            u_last[k] = u;
-            aoa_last[k] = aoa;
-            const float2 gs = split_f64(gnew);
-            for (int q = 0; q < CS; ++q) {
-                float2* Gr = cl.map_shared_rank(G[cur ^ 1], q);
-                double* Rr = cl.map_shared_rank(RR[cur], q);
-                Gr[i] = gs;
-                Rr[i] = r;
-            }
-        }
-        // block max of |dGamma|, only where a strength tolerance can stop the solve (with a
-        // tolerance <= 0 the test `max < tolerance` never holds)
-        if (want_max) {
-            lmax = warp_umax_to_lane0(lmax);
-            if (lane == 0) s_umax[warp] = lmax;
+            for (int i = tid; i < N; i += kSolveCtaThreads) G(1)[i] = split_f64(src[i]);
             __syncthreads();
-            if (tid == 0) {
-                unsigned long long v = 0;
-                for (int w = 0; w < nwarps; ++w) v = s_umax[w] > v ? s_umax[w] : v;
-                for (int q = 0; q < CS; ++q) cl.map_shared_rank(MX[cur], q)[rank] = bits_value(v);
-            }
         }
-        cl.sync();
+        const bool more = start < 3 || it < st.max_iterations;
+        // 1. induced velocity of own rows; the last iteration's residual and decision
+        induced_rows(more ? G(start < 3 ? start > 0 : cur) : nullptr, it > 0 ? RR((it - 1) & 1) : nullptr);
+        if (it > 0) {
+            residual = s_res;
+            conv = s_conv != 0;
+        }
+        if (conv || !more) break;
+        // 2. row updates
+#pragma unroll 1
+        for (int k = 0; k < (RPT == 1 ? min(nrows, 1) : nrows); ++k) {
+            const int i = r0 + own_row(k);
+            const SolveLine& L = ln[RPT == 1 ? 0 : k];
+            double a, c;
+            float fa, fc;
+            row_velocity(i, L, a, c, fa, fc);
+            const LineFlow o = line_flow(L, m, i, a, c, fa, fc, m.include_viscous_lift != 0, tab);
+            const double gold = src ? src[i] : gown[RPT == 1 ? 0 : k];
+            double r = residual_of_line(m, L, i, gold, a, c, o);
+            if (start == 3) {
+                // circulation_cl: the pre-stall lift serves the estimate and the residual alike
+                const double est = L.half_chord * o.ul * (m.include_viscous_lift ? o.cl_pre + o.cl_post : o.cl_pre);
+                const double d = est - gold;
+                const double gnew = fma(st.damping, d, gold);
+                store_all(G(cur ^ 1), i, split_f64_int(gnew));
+                // |d| >= tolerance, as integers (the FP64 pipe takes a compare like an add); not for a NaN
+                const long long db = __double_as_longlong(d) & 0x7FFFFFFFFFFFFFFFll;
+                if (want_max && db >= __double_as_longlong(st.strength_tolerance) && db <= 0x7FF0000000000000ll) r = -r;
+                const int kk = RPT == 1 ? 0 : k;
+                gown[kk] = gnew;
+                a_last[kk] = a;
+                c_last[kk] = c;
+                est_last[kk] = est;
+            }
+            store_all(RR(it & 1), i, r);
+        }
+        if (start == 3) {
+            it += 1;
+            cur ^= 1;
+            barrier();
+            continue;
+        }
+        barrier();
         if (warp == 0) {
             double s = 0.0;
-            for (int i = lane; i < N; i += 32) s += RR[cur][i];
+            unsigned long long mx = 0;
+#pragma unroll 1
+            for (int i = lane; i < N; i += 32) {
+                s += RR(0)[i];
+                const unsigned long long bi = mag_bits(RR(0)[i]);
+                mx = bi > mx ? bi : mx;
+            }
             s = warp_sum_to_lane0(s);
+            mx = warp_umax_to_lane0(mx);
             if (lane == 0) {
-                double res = s / static_cast<double>(N);
-                unsigned long long mb = 0;
-                if (want_max)
-                    for (int q = 0; q < CS; ++q) {
-                        const unsigned long long bq = static_cast<unsigned long long>(__double_as_longlong(MX[cur][q]));
-                        mb = bq > mb ? bq : mb;
-                    }
-                const double mx = bits_value(mb);
-                s_res = res;
-                s_conv = (res < st.residual_tolerance) || (want_max && mx < st.strength_tolerance);
+                s_res = s;
+                s_umax = mx;
             }
         }
         __syncthreads();
-        residual = s_res;
-        conv = s_conv != 0;
-        cur ^= 1;
+        const double rv = s_res, rmax = bits_value(s_umax), margin = start == 2 ? b.second_margin : 1.0;
+        if (start == 0) {
+            best = rv;
+            best_max = rmax;
+        } else if (isfinite(rv) && rv < margin * best && rmax < margin * best_max) {  // same decision in every CTA
+            best = rv;
+            best_max = rmax;
+            taken = start;
+            for (int i = tid; i < N; i += kSolveCtaThreads) G(0)[i] = G(1)[i];
+            for (int k = 0; k < nrows; ++k) gown[k] = src[r0 + own_row(k)];
+        }
+        barrier();  // RR[0] and G[1] are written again by the next pass or the first iteration
+        ++start;
     }
 
     // final circulation from the last velocities (simple_iterative.rs:200-203)
     for (int k = 0; k < nrows; ++k) {
-        int i = r0 + own_row(k);
-        const RowGeom& g = rg[k];
-        double gam = -0.5 * g.chord_len * len(u_last[k]) * circulation_cl(m, m.foils[g.wing], aoa_last[k]);
+        const int i = r0 + own_row(k);
+        const double gam = est_last[k];
         b.gamma_prev[i] = gam;
-        b.vel_out[i] = u_last[k];
+        b.vel_out[i] = m.solve_basis[2 * i] * a_last[k] + m.solve_basis[2 * i + 1] * c_last[k];
         if (b.wake_str_row0) b.wake_str_row0[i] = gam;
         if (b.rec32_row0) b.rec32_row0[i].v[kRec32Gamma] = static_cast<float>(gam);
         if (b.rec64_row0) b.rec64_row0[i].v[kRec64Gamma] = gam;
     }
     if (rank == 0 && tid == 0) {
-        b.scalars[0] = residual;
+        b.scalars[0] = residual / static_cast<double>(N);
         b.scalars[1] = static_cast<double>(it);
         b.scalars[2] = conv ? 1.0 : 0.0;
+        b.scalars[4] = static_cast<double>(taken);
     }
     // a copy whose wait ran out may still be in flight: wait for it (bounded) before leaving
-    if (tid == 0)
+    if (copier)
         for (int q = 0; q < 2; ++q)
             if (pending[q]) mbar_wait_bounded(&s_mbar[q], mph[q] ^ 1u, b.err);
-    cl.sync();  // no CTA leaves while others may still write into its shared memory
+    barrier();  // no CTA leaves while others may still write into its shared memory
 }
 
-template <int RPT>
-__global__ void __launch_bounds__(kSolveThreads, RPT == 1 ? 2 : 1) k_solve_si(DevModel m, SolveSettings st, SolveBuffers b) {
-    si_solve<RPT>(m, st, b);
+template <int RPT, int NC, bool LO>
+__global__ void __launch_bounds__(kSolveCtaThreads, 1) k_solve_si(DevModel m, SolveSettings st, SolveBuffers b) {
+    si_solve<RPT, NC, LO>(m, st, b);
 }
 
-// Every case of a batch whose cluster size (and rows per thread) is this launch's: cluster i
-// solves jobs[i].
-template <int RPT>
-__global__ void __launch_bounds__(kSolveThreads, RPT == 1 ? 2 : 1) k_solve_si_jobs(const SolveJob* jobs) {
+// Every case of a batch whose cluster size and variant are this launch's: cluster i solves jobs[i].
+template <int RPT, int NC, bool LO>
+__global__ void __launch_bounds__(kSolveCtaThreads, RPT == 1 ? 2 : 1) k_solve_si_jobs(const SolveJob* jobs) {
     cg::cluster_group cl = cg::this_cluster();
     const SolveJob& j = jobs[blockIdx.x / cl.num_blocks()];
-    si_solve<RPT>(j.m, j.st, j.b);
+    si_solve<RPT, NC, LO>(j.m, j.st, j.b);
 }
 
-// rows per thread of a solve of N span lines
-int si_rows_per_thread(int N) {
-    const int CS = solve_cluster_size(N);
-    const int rp = (N + CS - 1) / CS;
-    return rp <= kSolveThreads ? 1 : kSolveRowsPerThread;
-}
+namespace {
 
-size_t si_smem_bytes(int N, int full, int comps) {
-    const int CS = si_cluster_size(N);
-    const int rp = (N + CS - 1) / CS;
-    const int sr = si_slab_rows(N, full, comps);
-    const long long bufs = sr == 0 ? 0 : (sr >= rp ? 1 : 2);
-    return static_cast<size_t>(si_slab_offset(N) * 8 + bufs * sr * si_row_bytes(N, full, comps));
-}
+using SiKernel = void (*)(DevModel, SolveSettings, SolveBuffers);
+using SiJobsKernel = void (*)(const SolveJob*);
 
-cudaError_t launch_solve_simple_iterative_jobs(const SolveJob* jobs, int n, int cluster, int rows_per_thread,
-                                               size_t smem, cudaStream_t s) {
-    if (n <= 0) return cudaSuccess;
-    if (cluster != 1 && cluster != 4 && cluster != 8) return cudaErrorInvalidValue;
-    if (rows_per_thread != 1 && rows_per_thread != kSolveRowsPerThread) return cudaErrorInvalidValue;
-    auto kernel = rows_per_thread == 1 ? k_solve_si_jobs<1> : k_solve_si_jobs<kSolveRowsPerThread>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
+// f(kernel pair) of the variant (rows per thread, components, lo plane)
+template <int RPT, int NC, bool LO>
+struct SiVariant {
+    static SiKernel one() { return k_solve_si<RPT, NC, LO>; }
+    static SiJobsKernel jobs() { return k_solve_si_jobs<RPT, NC, LO>; }
+};
+template <class F>
+auto si_variant(int rpt, int comps, int full, F&& f) {
+    if (rpt == 1) {
+        if (comps == 2) return full ? f(SiVariant<1, 2, true>()) : f(SiVariant<1, 2, false>());
+        return full ? f(SiVariant<1, 3, true>()) : f(SiVariant<1, 3, false>());
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(n * cluster), 1, 1);
-    cfg.blockDim = dim3(kSolveThreads, 1, 1);
+    if (comps == 2) return full ? f(SiVariant<kSolveRowsPerThread, 2, true>()) : f(SiVariant<kSolveRowsPerThread, 2, false>());
+    return full ? f(SiVariant<kSolveRowsPerThread, 3, true>()) : f(SiVariant<kSolveRowsPerThread, 3, false>());
+}
+
+void si_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, int clusters, int CS, size_t smem, cudaStream_t s) {
+    cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(clusters * CS), 1, 1);
+    cfg.blockDim = dim3(kSolveCtaThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(CS);
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, jobs);
+}
+
+// Raises the kernels' shared-memory limit and allows clusters of 16, once per device; the
+// largest cluster size the device can hold with kSiSmemSingle bytes per CTA.
+int si_largest_cluster() {
+    static std::mutex mu;
+    static std::map<int, int> largest;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 8;
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = largest.find(dev);
+    if (it != largest.end()) return it->second;
+    auto prepare = [](auto kernel) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSiSmemSingle)) ==
+                   cudaSuccess &&
+               cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    };
+    bool ok = true;
+    for (int rpt : {1, kSolveRowsPerThread})
+        for (int comps : {2, 3})
+            for (int full : {0, 1})
+                ok = ok && si_variant(rpt, comps, full, [&](auto v) { return prepare(v.one()) && prepare(v.jobs()); });
+    int c = ok ? kMaxCluster : 8;
+    for (; c > 8; c /= 2) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr;
+        si_config(cfg, attr, 1, c, kSiSmemSingle, nullptr);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_solve_si<1, 2, true>, &cfg) == cudaSuccess && n > 0) break;
+    }
+    (void)cudaGetLastError();  // a refused shape is not an error of the caller
+    largest[dev] = c;
+    return c;
+}
+
+}  // namespace
+
+// One case alone: the cluster that ends its iterations soonest. Measured per iteration (us, the
+// dynamic two-component matrix; clusters of 1, 4, 8, 16): N = 32: 4.19 / 4.47 / 4.53 / 4.75,
+// 60: 4.93 / 4.65 / 4.61 / 4.81, 128: 7.49 / 5.03 / 4.83 / 5.02, 183: 18.2 / 6.22 / 5.35 / 5.19,
+// 256: 25.9 / 7.07 / 5.71 / 5.37, 1024: 263 / 80.1 / 41.4 / 22.6. Each crowding level halves it, down to
+// the size whose CTAs keep their matrix slab in shared memory two to an SM: with more cases than
+// SMs their sum of CTA time counts (N = 128: 4 CTAs x 5.03 us against 8 x 4.83).
+int solve_cluster_size(int N, int crowding) {
+    const int alone = N <= 48 ? 1 : (N <= 160 ? 8 : 16), least = N <= 64 ? 1 : (N <= 256 ? 4 : 8);
+    return std::min(std::max(alone >> crowding, least), si_largest_cluster());
+}
+
+SiPlan si_plan(int N, int full, int comps, int cluster, size_t smem_limit) {
+    SiPlan p;
+    p.cluster = cluster;
+    const int rp = (N + cluster - 1) / cluster;
+    p.rows_per_thread = rp <= kSolveThreads ? 1 : kSolveRowsPerThread;
+    const long long off = si_slab_offset(N, cluster) * 8, rowb = si_row_bytes(N, full, comps);
+    const long long budget = static_cast<long long>(smem_limit) - off;
+    const long long r = budget / (2 * rowb);
+    if (rp * rowb <= budget) {
+        p.slab_rows = rp;
+        p.smem = static_cast<size_t>(off + rp * rowb);
+    } else {
+        p.slab_rows = r < 4 ? 0 : static_cast<int>(std::min<long long>(r, 16));
+        p.smem = static_cast<size_t>(off + 2 * p.slab_rows * rowb);
+    }
+    // Lanes per row: the fewest instructions of a warp over a chunk's rows, a step of four columns
+    // being about 22 per component and a row's butterfly 14 per level
+    const int at_once = p.slab_rows > 0 ? std::min(p.slab_rows, rp) : rp;
+    long long best = 0;
+    for (int l = 3; l <= 5; ++l) {
+        const long long rows = kSolveThreads >> l, passes = (at_once + rows - 1) / rows;
+        const long long cost = passes * ((si_matrix_stride(N) + (4 << l) - 1) / (4 << l) * 22 * comps + 14 * l + 60);
+        if (l == 3 || cost < best) {
+            best = cost;
+            p.lanes_log2 = l;
+        }
+    }
+    return p;
+}
+
+cudaError_t launch_solve_simple_iterative_jobs(const SolveJob* jobs, int n, int cluster, int rows_per_thread, int comps,
+                                               int full, size_t smem, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    if (cluster < 1 || cluster > si_largest_cluster() || smem > kSiSmemSingle) return cudaErrorInvalidValue;
+    if (rows_per_thread != 1 && rows_per_thread != kSolveRowsPerThread) return cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    si_config(cfg, attr, n, cluster, smem, s);
+    return cudaLaunchKernelEx(&cfg, si_variant(rows_per_thread, comps, full, [](auto v) { return v.jobs(); }), jobs);
 }
 
 cudaError_t launch_solve_simple_iterative(const DevModel& m, const SolveSettings& st, const SolveBuffers& b, cudaStream_t s) {
-    const int CS = solve_cluster_size(m.N);
-    const int rp = (m.N + CS - 1) / CS;
-    if (rp > kSolveThreads * kSolveRowsPerThread) return cudaErrorInvalidValue;
-    size_t smem = si_smem_bytes(m.N, b.split_full, b.split_comps);
-    auto kernel = si_rows_per_thread(m.N) == 1 ? k_solve_si<1> : k_solve_si<kSolveRowsPerThread>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(CS, 1, 1);
-    cfg.blockDim = dim3(kSolveThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = CS;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, m, st, b);
+    const SiPlan p = si_plan(m.N, b.split_full, b.split_comps, solve_cluster_size(m.N, 0), kSiSmemSingle);
+    if ((m.N + p.cluster - 1) / p.cluster > kSolveThreads * kSolveRowsPerThread) return cudaErrorInvalidValue;
+    SolveBuffers sb = b;
+    sb.slab_rows = p.slab_rows;
+    sb.lanes_log2 = p.lanes_log2;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    si_config(cfg, attr, 1, p.cluster, p.smem, s);
+    return cudaLaunchKernelEx(&cfg, si_variant(p.rows_per_thread, b.split_comps, b.split_full, [](auto v) { return v.one(); }),
+                              m, st, sb);
 }
 
 // ---------------------------------------------------------------------------------------

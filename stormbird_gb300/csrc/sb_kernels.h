@@ -97,8 +97,8 @@ cudaError_t launch_bs_reduce(const double* partial, int n_chunks, long long M, l
 // ceil(M_total / kBsReduceThreads), job k starting at its block_begin.
 cudaError_t launch_bs_reduce_jobs(const BsJob* jobs, int n_jobs, long long blocks, cudaStream_t s);
 // The influence matrices are written in f64 (`factors`, [N][N] d3, for the Linearized
-// solver) and/or as f32 (hi, lo) pairs (`split`: the hi plane [N][3][si_matrix_stride(N)]
-// floats, row c, component, column, then the lo plane; hi = the nearest float, lo = the
+// solver) and/or as f32 (hi, lo) pairs (`split`: the hi plane, then the lo plane, in the layout of
+// SolveBuffers::factors_split; hi = the nearest float, lo = the
 // nearest float of the remainder, for the SimpleIterative solver's matrix-vector products;
 // the padding columns are left untouched). Either pointer may be null.
 // Frozen-wake unit matrix of the first wake row: from the FP32 row-0 records when row0_32 is
@@ -222,8 +222,9 @@ __host__ __device__ inline int si_matrix_stride(int N) { return (N + 3) & ~3; }
 struct SolveBuffers {
     const d3* fixed = nullptr;      // [N]
     const d3* factors = nullptr;    // [N][N] (Linearized)
-    // SimpleIterative matrix as floats: hi plane [N][split_comps][stride] (row, component, column;
-    // stride = si_matrix_stride(N)), then the lo plane (the nearest float of the remainder);
+    // SimpleIterative matrix as floats: hi plane, then the lo plane (the nearest float of the
+    // remainder), each [N][stride][2] (row, column, component) with two components, [N][3][stride]
+    // (row, component, column) with three; stride = si_matrix_stride(N);
     // split_full = 0 when only the diagonal carries lo parts (the FP32 unit matrix: every
     // other entry is an FP32 value, lo = 0)
     const float* factors_split = nullptr;
@@ -248,9 +249,16 @@ struct SolveBuffers {
     // best start's before it (the warm-start guard, see si_solve)
     double second_margin = 0.5;
     int* err = nullptr;
+    // rows of the matrix a CTA of the SimpleIterative solve keeps (>= its rows) or streams at a
+    // time in shared memory (SiPlan); 0: rows from global memory
+    int slab_rows = 0;
+    int lanes_log2 = 3;  // lanes of a row of its matrix-vector product: 8, 16 or 32 (SiPlan)
 };
 
-int solve_cluster_size(int N);
+// Thread-block cluster (CTAs) of a SimpleIterative solve of N lines on the current device.
+// crowding: 0 for a case alone, up to kMaxCrowding where many cases share the GPU.
+constexpr int kMaxCrowding = 4;
+int solve_cluster_size(int N, int crowding);
 cudaError_t launch_solve_simple_iterative(const DevModel& m, const SolveSettings& st, const SolveBuffers& b, cudaStream_t s);
 cudaError_t launch_solve_linearized(const DevModel& m, const SolveSettings& st, const SolveBuffers& b, cudaStream_t s);
 
@@ -273,12 +281,20 @@ LinPlan linearized_plan(int N);
 // n solves of one plan shape in one launch (smem: the largest of the jobs' plans).
 cudaError_t launch_solve_linearized_jobs(const SolveJob* jobs, int n, const LinPlan& plan, cudaStream_t s);
 // SimpleIterative solves of a batch: n cases of one cluster size (solve_cluster_size of
-// their N) in one launch, a cluster per case; smem = the largest si_smem_bytes of the jobs.
-// full: the matrix's lo plane is read (SolveBuffers::split_full); comps: SolveBuffers::split_comps
-size_t si_smem_bytes(int N, int full, int comps);
-int si_rows_per_thread(int N);  // 1 or 4: a launch holds one kind (rows_per_thread below)
-cudaError_t launch_solve_simple_iterative_jobs(const SolveJob* jobs, int n, int cluster, int rows_per_thread,
-                                               size_t smem, cudaStream_t s);
+// their N) in one launch, a cluster per case; smem = the largest of the jobs' plans.
+// How such a solve runs: rows per thread (1 or 4: a launch holds one kind), rows of the matrix
+// slab and dynamic shared memory per CTA (at most smem_limit). full: the matrix's lo plane is read
+// (SolveBuffers::split_full); comps: SolveBuffers::split_comps.
+constexpr size_t kSiSmemSingle = 220 * 1024;  // one CTA per SM
+constexpr size_t kSiSmemShared = 110 * 1024;  // two CTAs per SM
+struct SiPlan {
+    int cluster = 1, rows_per_thread = 1, slab_rows = 0, lanes_log2 = 3;
+    size_t smem = 0;
+};
+SiPlan si_plan(int N, int full, int comps, int cluster, size_t smem_limit);
+// comps, full: the jobs' SolveBuffers::split_comps and split_full.
+cudaError_t launch_solve_simple_iterative_jobs(const SolveJob* jobs, int n, int cluster, int rows_per_thread, int comps,
+                                               int full, size_t smem, cudaStream_t s);
 
 struct ForceArgs {
     const double* gamma = nullptr;  // [N]

@@ -25,54 +25,87 @@
 #include <math_constants.h>
 
 #include "sb_device.cuh"
+#include "sb_f64.cuh"
 #include "sb_kernels.h"
 #include "sb_ptx.cuh"
 
 namespace sbgpu {
 
 // ---------------------------------------------------------------------------------------
-// FP64 element functions (literal restatement, used by k_unit_matrix and the FP64 sweep)
+// FP64 element functions (used by the unit matrices, the horseshoe matrix and the FP64 sweep)
 // ---------------------------------------------------------------------------------------
-// vortex_line.rs:18-106
-__device__ inline d3 line_unit_f64(d3 a, d3 b, d3 x, double rc) {
-    d3 r1 = x - a, r2 = x - b;
-    double r1sq = len2(r1), r2sq = len2(r2);
-    double l1 = sqrt(r1sq), l2 = sqrt(r2sq);
-    double r1r2 = l1 * l2;
-    double den = r1r2 * (r1r2 + dot(r1, r2));
-    if (fabs(den) > 1.0e-10) {
-        double core = 1.0;
-        if (rc != 0.0) {
-            d3 rl = b - a;
-            double ll = sqrt(len2(rl));
-            d3 dir = rl / ll;
-            double t = dot(r1, dir);
-            double d2 = t < 0.0 ? r1sq : (t > ll ? r2sq : len2(r1) - t * t);
-            double rc2 = rc * rc;
-            double cden = sqrt(rc2 * rc2 + d2 * d2);
-            core = cden > 0.0 ? d2 / cden : 0.0;
-        }
-        double k = (l1 + l2) / den;
-        return (core * cross(r1, r2)) * (k * kFourPiInv);
-    }
-    return mk(0, 0, 0);
+// vortex_line.rs:18-106 for the line from a to b at x, unit strength, given r1 = x - a, r2 = x - b
+// and their squares: 4 pi velocity = line_scale x (r1 x r2). With il2 = 1 / |b - a|^2:
+//   l1 l2 = sqrt(|r1|^2 |r2|^2),  l1 + l2 = sqrt(|r1|^2 + |r2|^2 + 2 l1 l2),
+//   den = l1 l2 (l1 l2 + r1.r2),  tt = r1.(b - a) = |r1|^2 - r1.r2 (past the end: r1.r2 > |r2|^2),
+//   d2 = |r1|^2 - tt^2 il2 inside, the end-point distance outside,
+//   core k = d2 (l1 + l2) / sqrt(den^2 (d2^2 + rc^4))   (den > 0 wherever it counts),
+// three reciprocal square roots of 4 FP64 instructions for the reference's four square roots and
+// four divisions of 9 to 22. A zero core leaves its factor out, as there. |den| <= 1e-10 gives 0,
+// and so does a degenerate line (il2 infinite; there by its core factor).
+__device__ __forceinline__ double line_scale(d3 r1, double s1, d3 r2, double s2, double il2, double rc4) {
+    const double r12 = dot(r1, r2);
+    const double p = sqrt_any(s1 * s2);
+    const double b = p + r12, den = p * b;
+    if (!(fabs(den) > 1.0e-10) || __double2hiint(il2) == 0x7FF00000) return 0.0;
+    const double sum = sqrt_any(fma(2.0, p, s1 + s2));
+    const double tt = s1 - r12;
+    double d2 = fma(-tt * tt, il2, s1);
+    if (__double2hiint(r12 - s2) >= 0) d2 = s2;  // r1.r2 >= |r2|^2
+    if (__double2hiint(tt) < 0) d2 = s1;
+    if (__double_as_longlong(rc4) == 0) return copysign(sum * rcp_any(den), den);
+    const double k = d2 * sum * rsqrt_any(den * den * fma(d2, d2, rc4));
+    return den < 0.0 ? -k : k;
+}
+__device__ __forceinline__ d3 line_unit_f64(d3 a, d3 b, d3 x, double il2, double rc4) {
+    const d3 r1 = x - a, r2 = x - b;
+    return (line_scale(r1, len2(r1), r2, len2(r2), il2, rc4) * kFourPiInv) * cross(r1, r2);
 }
 
-// panel.rs:61-118 (record layout of PanelRec<double>: [25] holds the core length itself)
-__device__ inline d3 panel_unit_f64(const double* v, d3 x) {
-    d3 c = mk(v[16], v[17], v[18]);
-    d3 t = x - c;
-    double d2 = len2(t);
-    if (d2 <= v[19]) {
-        d3 p[4] = {mk(v[0], v[1], v[2]), mk(v[3], v[4], v[5]), mk(v[6], v[7], v[8]), mk(v[9], v[10], v[11])};
-        d3 u = mk(0, 0, 0);
-        for (int i = 0; i < 4; ++i) u = u + line_unit_f64(p[i], p[(i + 1) & 3], x, v[25]);
-        return u;
+// Vortex ring of a PanelRec<double> at x, times 4 pi (panel.rs:99-118). Out of line: the sweep's far
+// pairs run past a few instructions, not past four unrolled lines.
+__device__ __noinline__ d3 ring_f64(const double* v, d3 x) {
+    d3 u = mk(0, 0, 0);
+    d3 r1 = x - mk(v[0], v[1], v[2]);
+    double s1 = len2(r1);
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+        const double* p = v + 3 * ((k + 1) & 3);
+        const d3 r2 = x - mk(p[0], p[1], p[2]);
+        const double s2 = len2(r2);
+        const double g = line_scale(r1, s1, r2, s2, v[12 + k], v[27]);
+        const d3 c = cross(r1, r2);
+        u.x = fma(g, c.x, u.x);
+        u.y = fma(g, c.y, u.y);
+        u.z = fma(g, c.z, u.z);
+        r1 = r2;
+        s1 = s2;
     }
-    d3 n = mk(v[20], v[21], v[22]);
-    double d5 = d2 * d2 * sqrt(d2);
-    double h = dot(t, n);
-    return (v[23] * ((3.0 * h) * t - d2 * n)) / d5;
+    return u;
+}
+// panel.rs:61-118 for strength g, added to u
+__device__ __forceinline__ void add_panel_f64(const double* v, d3 x, double g, d3& u) {
+    const d3 t = x - mk(v[16], v[17], v[18]);
+    const double d2 = len2(t);
+    if (d2 <= v[19]) {
+        const d3 w = ring_f64(v, x);
+        const double f = g * kFourPiInv;
+        u.x = fma(f, w.x, u.x);
+        u.y = fma(f, w.y, u.y);
+        u.z = fma(f, w.z, u.z);
+        return;
+    }
+    // point doublet: g area / (4 pi) (3 (t.n) t / |t|^5 - n / |t|^3)
+    const d3 n = mk(v[20], v[21], v[22]);
+    const double r = rsqrt_any(d2), r2 = r * r, c = g * v[23] * (r * r2), h = 3.0 * dot(t, n) * r2;
+    u.x = fma(c, fma(h, t.x, -n.x), u.x);
+    u.y = fma(c, fma(h, t.y, -n.y), u.y);
+    u.z = fma(c, fma(h, t.z, -n.z), u.z);
+}
+__device__ __noinline__ d3 panel_unit_f64(const double* v, d3 x) {
+    d3 u = mk(0, 0, 0);
+    add_panel_f64(v, x, 1.0, u);
+    return u;
 }
 
 __device__ inline d3 mirror(int sym, d3 p) {
@@ -692,10 +725,11 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
 #pragma unroll
                         for (int t = 0; t < TT; ++t) {
                             if (!valid[t] || (NEGLECT && tw[t] == pw)) continue;
-                            d3 u = panel_unit_f64(v, mk(xh[t], yh[t], zh[t]));
-                            tx[t] += gam * u.x;
-                            ty[t] += gam * u.y;
-                            tz[t] += gam * u.z;
+                            d3 u = mk(tx[t], ty[t], tz[t]);
+                            add_panel_f64(v, mk(xh[t], yh[t], zh[t]), gam, u);
+                            tx[t] = u.x;
+                            ty[t] = u.y;
+                            tz[t] = u.z;
                         }
                     }
 #pragma unroll
@@ -939,8 +973,7 @@ __device__ __forceinline__ void panel_unit2(const float* v, float2 X2h, float2 Y
     }
 }
 
-__device__ inline void unit_matrix_f32_elem(const PanelRec<float>* row0_32, const PanelRec<double>* row0, const d3* ctrl,
-                                            int N, int sym, int neglect, const int* wing_of_line, d3* factors,
+__device__ inline void unit_matrix_f32_elem(const PanelRec<float>* row0_32, const d3* ctrl, int N, int sym, int neglect, const int* wing_of_line, d3* factors,
                                             float* split, const d3* basis, long long id) {
     const int pairs = (N + 1) / 2;
     if (id >= static_cast<long long>(pairs) * N) return;
@@ -980,28 +1013,66 @@ __device__ inline void unit_matrix_f32_elem(const PanelRec<float>* row0_32, cons
     for (int l = 0; l < 2; ++l) {
         const int c = l == 0 ? c0 : c1;
         if (l == 1 && c1 == c0) break;
+        if (c == p) continue;  // own_panel_elem
         d3 u = mk(uxa[l], uya[l], uza[l]);
-        bool fp32 = true;
-        if (neglect && wing_of_line[c] == wing_of_line[p]) {
-            u = mk(0, 0, 0);
-        } else if (c == p) {
-            const d3 x = ctrl[c];
-            u = panel_unit_f64(row0[p].v, x);
-            if (sym) u = sym_correct(sym, u, panel_unit_f64(row0[p].v, mirror(sym, x)));
-            fp32 = false;
-        }
-        store_factor(factors, split, N, basis, static_cast<long long>(c) * N + p, c, p, u, fp32);
+        if (neglect && wing_of_line[c] == wing_of_line[p]) u = mk(0, 0, 0);
+        store_factor(factors, split, N, basis, static_cast<long long>(c) * N + p, c, p, u, true);
     }
+}
+
+// The control points' own panels in FP64: thread t takes ring segment t mod 4 of line t / 4, so that
+// the FP64 chain of an entry (the longest in the kernel) is one line's and not four's. Every lane
+// of a warp calls it (lines past the end repeat the last one and store nothing).
+__device__ inline void own_panel_elem(const PanelRec<double>* row0, const d3* ctrl, int N, int sym, int neglect, d3* factors,
+                                      float* split, const d3* basis, long long t) {
+    const int c = static_cast<int>(min(t / 4, static_cast<long long>(N - 1))), k = static_cast<int>(t & 3);
+    const double* v = row0[c].v;
+    const d3 x = ctrl[c];
+    d3 u = mk(0, 0, 0);
+#pragma unroll 1
+    for (int q = 0; q < (sym ? 2 : 1); ++q) {
+        const d3 y = q ? mirror(sym, x) : x;
+        const d3 e = y - mk(v[16], v[17], v[18]);
+        d3 w = mk(0, 0, 0);
+        if (len2(e) <= v[19]) {  // the same for the four lanes of a line
+            const int k1 = 3 * ((k + 1) & 3);
+            w = line_unit_f64(mk(v[3 * k], v[3 * k + 1], v[3 * k + 2]), mk(v[k1], v[k1 + 1], v[k1 + 2]), y, v[12 + k], v[27]);
+        } else if (k == 0) {
+            w = panel_unit_f64(v, y);
+        }
+#pragma unroll 1
+        for (int o = 1; o < 4; o <<= 1) {
+            w.x += __shfl_xor_sync(0xffffffffu, w.x, o);
+            w.y += __shfl_xor_sync(0xffffffffu, w.y, o);
+            w.z += __shfl_xor_sync(0xffffffffu, w.z, o);
+        }
+        u = q ? sym_correct(sym, u, w) : w;
+    }
+    if (neglect) u = mk(0, 0, 0);
+    if (k == 0 && t / 4 < N) store_factor(factors, split, N, basis, static_cast<long long>(c) * N + c, c, c, u);
+}
+
+constexpr int kUnitMatrixThreads = 128;
+
+// blocks of own_panel_elem (first: they take longest), then those of unit_matrix_f32_elem
+__host__ __device__ inline long long own_panel_blocks(int N) { return (4LL * N + kUnitMatrixThreads - 1) / kUnitMatrixThreads; }
+
+__device__ inline void unit_matrix_f32_block(const PanelRec<float>* row0_32, const PanelRec<double>* row0, const d3* ctrl,
+                                             int N, int sym, int neglect, const int* wing_of_line, d3* factors,
+                                             float* split, const d3* basis, long long block) {
+    const long long own = own_panel_blocks(N);
+    if (block < own)
+        own_panel_elem(row0, ctrl, N, sym, neglect, factors, split, basis, block * kUnitMatrixThreads + threadIdx.x);
+    else
+        unit_matrix_f32_elem(row0_32, ctrl, N, sym, neglect, wing_of_line, factors, split, basis,
+                             (block - own) * kUnitMatrixThreads + threadIdx.x);
 }
 
 __global__ void k_unit_matrix_f32(const PanelRec<float>* row0_32, const PanelRec<double>* row0, const d3* ctrl, int N,
                                   int sym, int neglect, const int* wing_of_line, d3* factors, float* split,
                                   const d3* basis) {
-    unit_matrix_f32_elem(row0_32, row0, ctrl, N, sym, neglect, wing_of_line, factors, split, basis,
-                         blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x);
+    unit_matrix_f32_block(row0_32, row0, ctrl, N, sym, neglect, wing_of_line, factors, split, basis, blockIdx.x);
 }
-
-constexpr int kUnitMatrixThreads = 128;
 
 // The unit-strength matrices of every case of a batch in one launch (block -> case by a
 // binary search over the cases' first blocks, as the other job-list kernels).
@@ -1013,19 +1084,19 @@ __global__ void k_unit_matrix_jobs(const CaseStepJob* jobs, int n) {
         else hi = mid - 1;
     }
     const CaseStepJob& J = jobs[lo];
-    const long long id = (blockIdx.x - J.blk_matrix) * static_cast<long long>(kUnitMatrixThreads) + threadIdx.x;
+    const long long block = blockIdx.x - J.blk_matrix;
     const DevModel& m = J.m;
     if (J.row0_32)
-        unit_matrix_f32_elem(J.row0_32, J.w.row0_64, m.ctrl, m.N, m.symmetry, m.neglect_self, m.wing_of_line, J.factors,
-                             J.split, J.basis, id);
+        unit_matrix_f32_block(J.row0_32, J.w.row0_64, m.ctrl, m.N, m.symmetry, m.neglect_self, m.wing_of_line, J.factors,
+                              J.split, J.basis, block);
     else
         unit_matrix_elem(J.w.row0_64, m.ctrl, m.N, m.symmetry, m.neglect_self, m.wing_of_line, J.factors, J.split,
-                         J.basis, id);
+                         J.basis, block * kUnitMatrixThreads + threadIdx.x);
 }
 
 long long unit_matrix_blocks(int N, bool fp32) {
     const long long tot = fp32 ? static_cast<long long>((N + 1) / 2) * N : static_cast<long long>(N) * N;
-    return (tot + kUnitMatrixThreads - 1) / kUnitMatrixThreads;
+    return (tot + kUnitMatrixThreads - 1) / kUnitMatrixThreads + (fp32 ? own_panel_blocks(N) : 0);
 }
 
 cudaError_t launch_unit_matrix_jobs(const CaseStepJob* jobs, int n, long long blocks, cudaStream_t s) {
@@ -1034,69 +1105,91 @@ cudaError_t launch_unit_matrix_jobs(const CaseStepJob* jobs, int n, long long bl
     return cudaGetLastError();
 }
 
-// Quasi-steady wake: core length and wake vectors (frozen_wake.rs:74-100). One CTA: the
-// span line lengths and the wake vectors in parallel (FP64 square roots and divisions are
-// slow on this part, so a serial loop over them costs microseconds per line), the mean
-// length summed in line order by one thread.
+// Quasi-steady wake: relative core length (frozen_wake.rs:74-100), the mean span line length.
 constexpr int kQsPrepThreads = 256;
-__global__ void __launch_bounds__(kQsPrepThreads) k_qs_prep(DevModel m, int core_kind, double core_value,
-                                                            double wake_length, d3* wake_vec, double* rc_out) {
-    const int tid = threadIdx.x;
-    for (int k = tid; k < m.Np; k += kQsPrepThreads) wake_vec[k] = normalize(m.felt_span[k]) * wake_length;
-    if (core_kind != 0) {
-        if (tid == 0) *rc_out = core_kind == 1 ? core_value : 0.0;
-        return;
-    }
-    extern __shared__ double lens[];  // [N]
-    for (int i = tid; i < m.N; i += kQsPrepThreads) lens[i] = len(m.span_e[i] - m.span_s[i]);
+__global__ void __launch_bounds__(kQsPrepThreads) k_qs_prep(DevModel m, double core_value, double* rc_out) {
+    __shared__ double part[kQsPrepThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31;
+    double s = 0.0;
+    for (int i = tid; i < m.N; i += kQsPrepThreads) s += sqrt_any(len2(m.span_e[i] - m.span_s[i]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) part[tid >> 5] = s;
     __syncthreads();
     if (tid == 0) {
-        double s = 0.0;
-        for (int i = 0; i < m.N; ++i) s += lens[i];
+        for (int w = 1; w < kQsPrepThreads / 32; ++w) s += part[w];
         *rc_out = core_value * (s / static_cast<double>(m.N));
     }
 }
 
 // Horseshoe influence matrix (frozen_wake.rs:102-128, horseshoe_vortex.rs:23-103):
 // factors[c][j] = unit velocity of horseshoe j (bound + start trailing + end trailing) at
-// control point c. Horseshoe j of wing w uses wake vectors j + w and j + w + 1.
-__global__ void k_horseshoe_matrix(DevModel m, const d3* wake_vec, const double* rc_dev, int sym, d3* factors,
-                                   float* split, const d3* basis) {
-    long long id = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    const int N = m.N;
-    if (id >= static_cast<long long>(N) * N) return;
-    int c = static_cast<int>(id / N), j = static_cast<int>(id % N);
-    const double rc = *rc_dev;
-    const int k = j + m.wing_of_line[j];
-    d3 s = m.span_s[j], e = m.span_e[j];
-    d3 st0 = s + wake_vec[k], en1 = e + wake_vec[k + 1];
-    auto hs = [&](d3 x) {
-        d3 u = mk(0, 0, 0);
-        u = u + line_unit_f64(s, e, x, rc);
-        u = u + line_unit_f64(st0, s, x, rc);
-        u = u + line_unit_f64(e, en1, x, rc);
-        return u;
-    };
-    d3 x = m.ctrl[c];
-    d3 u = hs(x);
-    if (sym) u = sym_correct(sym, u, hs(mirror(sym, x)));
-    store_factor(factors, split, N, basis, id, c, j, u);
+// control point c. Horseshoe j of wing w uses wake vectors j + w and j + w + 1: its end trailing
+// line and the next horseshoe's start trailing line are the same line run the other way, so a thread
+// evaluates the trailing line of one span point and the bound line that starts there, and takes
+// the neighbour's trailing line from shared memory (two lines per entry instead of three). Block: one
+// control point, 128 span points of which the last only serves its neighbour. FP64-bound: about 65
+// instructions per line.
+constexpr int kHorseshoePoints = 128;
+__global__ void __launch_bounds__(kHorseshoePoints) k_horseshoe_matrix(DevModel m, double wake_length, double rc_value,
+                                                                       const double* rc_dev, int sym, int tiles,
+                                                                       d3* factors, float* split, const d3* basis) {
+    __shared__ d3 trail[kHorseshoePoints];
+    const int N = m.N, tid = threadIdx.x;
+    const int c = blockIdx.x / tiles;
+    const int k0 = (blockIdx.x % tiles) * (kHorseshoePoints - 1), k = k0 + tid;
+    const bool have = k < m.Np;
+    const int j = have ? m.sp_line[k] : 0;
+    const bool line = have && !m.sp_end[k];  // a line starts at this point
+    const double rc = rc_dev ? *rc_dev : rc_value, rc4 = (rc * rc) * (rc * rc);
+    const d3 s = have ? m.span_pts[k] : mk(0, 0, 0), e = have ? m.span_e[j] : mk(0, 0, 0);
+    d3 far = s;
+    double il_far = 0.0, il_bound = 0.0;
+    if (have) {
+        const d3 f = m.felt_span[k];
+        const double l = len2(f);
+        d3 w = mk(0, 0, 0);  // normalize(f) wake_length
+        if (l > 0.0) w = f * (wake_length * rsqrt_any(l));
+        far = s + w;
+        il_far = rcp_any(len2(w));
+        il_bound = rcp_any(len2(e - s));
+    }
+    d3 u = mk(0, 0, 0);
+#pragma unroll 1
+    for (int q = 0; q < (sym ? 2 : 1); ++q) {
+        const d3 y = q ? mirror(sym, m.ctrl[c]) : m.ctrl[c];
+        d3 own = mk(0, 0, 0), b = mk(0, 0, 0);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {  // the trailing line away from the point, then the bound line
+            if (!have || (h && !line)) break;
+            const d3 w = line_unit_f64(s, h ? e : far, y, h ? il_bound : il_far, rc4);
+            if (h) b = w;
+            else own = w;
+        }
+        trail[tid] = own;
+        __syncthreads();
+        if (line && tid + 1 < kHorseshoePoints) {
+            const d3 v = b - own + trail[tid + 1];
+            u = q ? sym_correct(sym, u, v) : v;
+        }
+        __syncthreads();
+    }
+    if (line && tid + 1 < kHorseshoePoints)
+        store_factor(factors, split, N, basis, static_cast<long long>(c) * N + j, c, j, u);
 }
 
-cudaError_t launch_horseshoe_matrix(const DevModel& m, int core_kind, double core_value, double wake_length, d3* wake_vec,
+cudaError_t launch_horseshoe_matrix(const DevModel& m, int core_kind, double core_value, double wake_length,
                                     double* rc_dev, int sym, d3* factors, float* split, const d3* basis,
                                     cudaStream_t s) {
-    const size_t smem = static_cast<size_t>(m.N) * sizeof(double);
-    if (smem > 48 * 1024) {
-        cudaError_t a = cudaFuncSetAttribute(k_qs_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (a != cudaSuccess) return a;
+    if (core_kind == 0) {
+        k_qs_prep<<<1, kQsPrepThreads, 0, s>>>(m, core_value, rc_dev);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
     }
-    k_qs_prep<<<1, kQsPrepThreads, smem, s>>>(m, core_kind, core_value, wake_length, wake_vec, rc_dev);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    long long tot = static_cast<long long>(m.N) * m.N;
-    k_horseshoe_matrix<<<static_cast<unsigned>((tot + 127) / 128), 128, 0, s>>>(m, wake_vec, rc_dev, sym, factors, split,
-                                                                               basis);
+    const int tiles = (m.Np - 1 + kHorseshoePoints - 2) / (kHorseshoePoints - 1);
+    k_horseshoe_matrix<<<static_cast<unsigned>(static_cast<long long>(m.N) * tiles), kHorseshoePoints, 0, s>>>(
+        m, wake_length, core_kind == 1 ? core_value : 0.0, core_kind == 0 ? rc_dev : nullptr, sym, tiles, factors, split,
+        basis);
     return cudaGetLastError();
 }
 

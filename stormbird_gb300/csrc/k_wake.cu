@@ -286,7 +286,7 @@ __device__ void write_panel_records(const d3 (&pp)[4], double rc, double g, doub
             q.v[3 * k] = pp[k].x;
             q.v[3 * k + 1] = pp[k].y;
             q.v[3 * k + 2] = pp[k].z;
-            q.v[12 + k] = 0.0;
+            q.v[12 + k] = 1.0 / l2[k];
         }
         q.v[16] = c.x;
         q.v[17] = c.y;
@@ -299,7 +299,7 @@ __device__ void write_panel_records(const d3 (&pp)[4], double rc, double g, doub
         q.v[kRec64Gamma] = g;
         q.v[25] = rc;
         q.v[26] = static_cast<double>(wing);
-        q.v[27] = 0.0;
+        q.v[27] = rc2 * rc2;
         *r64 = q;
     } else {
         float lf[4];

@@ -199,8 +199,9 @@ __device__ inline double foil_cd(const FoilP& f, double a) {
 //   [47] near/far band: a bound on |fl32 |x_hi - c_hi|^2 - |x - c|^2| for targets x at the
 //        far-field radius (0 when hi is infinite)
 // FP64 record (PanelRec<double>, 28 doubles = 224 B):
-//   [0..11] corners, [16..18] centre, [19] far-field length squared, [20..22] normal,
-//   [23] area / (4 pi), [24] Gamma, [25] core length, [26] wing index.
+//   [0..11] corners, [12..15] 1/|d_k|^2 of the ring's segments (infinite for a degenerate one),
+//   [16..18] centre, [19] far-field length squared, [20..22] normal,
+//   [23] area / (4 pi), [24] Gamma, [25] core length, [26] wing index, [27] core length^4.
 template <class R>
 struct PanelRecSize;
 template <>

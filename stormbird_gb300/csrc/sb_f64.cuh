@@ -107,6 +107,23 @@ __device__ __forceinline__ double rsqrt_f64(double q) {
     return r;
 }
 
+// The same for any positive normal argument (the exponent is taken out of the seed and the step), by
+// CUDA's functions for the others: out of line, so that the loops they appear in stay small.
+static __device__ __noinline__ double sqrt_slow(double q) { return sqrt(q); }
+static __device__ __noinline__ double rsqrt_slow(double q) { return 1.0 / sqrt(q); }
+static __device__ __noinline__ double rcp_slow(double d) { return 1.0 / d; }
+__device__ __forceinline__ bool f64_normal_positive(double v) {
+    return static_cast<unsigned>(__double2hiint(v)) - 0x00100000u < 0x7FE00000u;
+}
+__device__ __forceinline__ double rsqrt_any(double q) {
+    if (!f64_normal_positive(q)) return rsqrt_slow(q);
+    const int hi = __double2hiint(q), e = ((hi >> 20) - 1023) >> 1;
+    const double r = rsqrt_f64(__hiloint2double(hi - (e << 21), __double2loint(q)));  // [1, 4)
+    return __hiloint2double(__double2hiint(r) - (e << 20), __double2loint(r));
+}
+__device__ __forceinline__ double sqrt_any(double q) { return f64_normal_positive(q) ? q * rsqrt_any(q) : sqrt_slow(q); }
+__device__ __forceinline__ double rcp_any(double d) { return f64_seed_range(fabs(d)) ? copysign(rcp_f64(fabs(d)), d) : rcp_slow(d); }
+
 // Entry (cos, sin, angle) of the angle table nearest to the angle of (x, y >= 0), in [0, pi].
 __device__ __forceinline__ const double* angle_entry(float x, float y, const double* t, float& angle) {
     angle = atan2f(y, x);

@@ -108,8 +108,8 @@ cudaError_t launch_bs_reduce_jobs(const BsJob* jobs, int n_jobs, long long block
 cudaError_t launch_unit_matrix(const PanelRec<double>* row0, const PanelRec<float>* row0_32, const d3* ctrl, int N,
                                int sym, int neglect, const int* wing_of_line, d3* factors, float* split, const d3* basis,
                                cudaStream_t s);
-// Quasi-steady horseshoe matrix; core_kind 0 relative, 1 absolute, 2 none.
-cudaError_t launch_horseshoe_matrix(const DevModel& m, int core_kind, double core_value, double wake_length, d3* wake_vec,
+// Quasi-steady horseshoe matrix; core_kind 0 relative (rc_dev: device scratch), 1 absolute, 2 none.
+cudaError_t launch_horseshoe_matrix(const DevModel& m, int core_kind, double core_value, double wake_length,
                                     double* rc_dev, int sym, d3* factors, float* split, const d3* basis,
                                     cudaStream_t s);
 

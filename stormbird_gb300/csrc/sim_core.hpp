@@ -340,7 +340,7 @@ struct sb_sim {
     DevBuf<PanelRec<double>> rec64, row0_64;
     int cur = 0;
     // frozen wake and sweeps
-    DevBuf<d3> fixed, factors, qs_wake_vec;
+    DevBuf<d3> fixed, factors;
     DevBuf<float> factors_split;  // the SimpleIterative solver's matrix: hi plane, then lo plane
     DevBuf<double> qs_rc, partial;
     DevBuf<unsigned long long> counters;
@@ -579,7 +579,6 @@ struct sb_sim {
             rec32.alloc(P_pan);
             row0_64.alloc(N);
         } else {
-            qs_wake_vec.alloc(Np);
             qs_rc.alloc(1);
         }
     }
@@ -948,10 +947,10 @@ struct sb_sim {
             const auto& q = setup.quasi_steady_wake;
             double wl = q.wake_length_factor * dm.rep_chord;
             ck(launch_horseshoe_matrix(dm, static_cast<int>(q.viscous_core_length.kind), q.viscous_core_length.value, wl,
-                                       qs_wake_vec.p, qs_rc.p, static_cast<int>(q.symmetry_condition), factors.p,
+                                       qs_rc.p, static_cast<int>(q.symmetry_condition), factors.p,
                                        factors_split.p, split_basis(), stream),
                "horseshoe matrix");
-            launches += 2;
+            launches += q.viscous_core_length.kind == sbsetup::CoreKind::Relative ? 2 : 1;
             record(3);
         }
         record(4);

@@ -114,6 +114,7 @@ struct sb_batch {
     };
     static constexpr int kLinGroups = 5;
     LinGroup lin_groups[kLinGroups];
+    LinGroup lin_refined[kLinGroups];  // the same cases by the cluster of their refined solve, launched first
     // SimpleIterative solves: one launch per cluster size (1 to 16 CTAs, solve_cluster_size) and
     // variant (rows per thread, components, kind of matrix), a cluster per case; the job list is refilled every step from pinned memory, since it
     // names the wake buffer of the step's parity
@@ -281,9 +282,23 @@ struct sb_batch {
             gj.push_back(g);
         }
         gather_jobs.upload(gj);
-        std::vector<SolveJob> lj[kLinGroups];
+        std::vector<SolveJob> lj[kLinGroups], rj[kLinGroups];
+        int lin_crowding = 0;  // the largest clusters that all run side by side, a CTA to an SM
+        for (; lin_crowding < kMaxCrowding; ++lin_crowding) {
+            long long ctas = 0;
+            for (const auto& c : cases) ctas += c->linearized_quasi_steady() ? linearized_refined_plan(c->N, lin_crowding).cluster : 0;
+            if (ctas <= sms) break;
+        }
         for (size_t i = 0; i < cases.size(); ++i)
             if (cases[i]->linearized_quasi_steady()) {
+                const LinPlan rp = linearized_refined_plan(cases[i]->N, lin_crowding);
+                if (rp.cluster > 0) {
+                    int q = 0;
+                    while ((1 << q) < rp.cluster) ++q;
+                    lin_refined[q].plan.cluster = rp.cluster;
+                    lin_refined[q].plan.smem = std::max(lin_refined[q].plan.smem, rp.smem);
+                    rj[q].push_back(cases[i]->linearized_job());
+                }
                 const LinPlan p = linearized_plan(cases[i]->N);
                 int g = 0;
                 while ((1 << g) < p.cluster) ++g;
@@ -294,6 +309,8 @@ struct sb_batch {
         for (int g = 0; g < kLinGroups; ++g) {
             lin_groups[g].n = static_cast<int>(lj[g].size());
             if (!lj[g].empty()) lin_groups[g].jobs.upload(lj[g]);
+            lin_refined[g].n = static_cast<int>(rj[g].size());
+            if (!rj[g].empty()) lin_refined[g].jobs.upload(rj[g]);
         }
         si_batched.assign(cases.size(), 0);
         auto si_case = [](const sb_sim& c) { return c.solver_kind == 0 && !c.solve.start_with_linearized; };
@@ -593,6 +610,17 @@ struct sb_batch {
         join(1);
         // the batched solves: a launch per Linearized plan shape and per SimpleIterative
         // cluster size, side by side on the pool streams
+        int n_refined = 0;
+        for (const auto& g : lin_refined) n_refined += g.n > 0 ? 1 : 0;
+        if (n_refined > 1) fork(1);
+        {
+            int k = 0;
+            for (const auto& g : lin_refined)
+                if (g.n > 0)
+                    ck(launch_solve_linearized_refined_jobs(g.jobs.p, g.n, g.plan, n_refined > 1 ? pool[k++] : main),
+                       "batched linearized solve");
+        }
+        if (n_refined > 1) join(1);
         int n_launch = 0;
         for (const auto& g : lin_groups) n_launch += g.n > 0 ? 1 : 0;
         for (const auto& g : si_groups) n_launch += g.cases.empty() ? 0 : 1;

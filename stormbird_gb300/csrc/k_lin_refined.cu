@@ -1,0 +1,563 @@
+// Linearized solver (sm_103a): Linearized::solve (stormbird/src/lifting_line/solvers/linearized.rs:
+// 54-222) by an FP32 inverse and f64 refinement, on one thread-block cluster per case.
+//
+// The reference eliminates the N x N system in f64 (stormath/src/matrix/linalg.rs:41-103). This part's
+// FP64 rate is 1/64 of its FP32 rate and a pivoted elimination takes a cluster barrier per column, so
+// here:
+//   1. each CTA builds its rows of the matrix in f64 (kept in global memory) and their FP32 copy in
+//      shared memory (linearized.rs:61-136);
+//   2. the FP32 copy is inverted in place by block Gauss-Jordan, blocks of 16 rows dealt round-robin:
+//      the owner of block k inverts its diagonal block, scales its 16 rows and leaves them in
+//      global memory, one cluster barrier, every CTA subtracts their multiples from its rows (a rank-16
+//      update from shared memory). N / 16 barriers instead of N; the owner of block k + 1 updates those
+//      rows first and publishes them before the rest of its rows, beside the others' updates;
+//   3. x = x + X32 (b - A x) with the residual in f64 until the correction is rounding (two or three
+//      digits short of full precision are left after the first, each further one gains as many as
+//      the FP32 inverse is good for);
+//   4. induced velocities, viscous correction, residual and outputs (linearized.rs:141-213), each CTA
+//      its rows.
+// No pivoting across blocks: the diagonal dominates (2 / (c u) plus the line's own trailing pair
+// against its neighbours'), and a system where that fails shows in step 3. Where a pivot is below
+// 1e-6 (the reference calls 1e-12 singular), a correction does not shrink or a value is not finite,
+// scalars[5] stays 0 and the elimination kernels of k_solve.cu, launched after this one, solve the case
+// as before (they return at once where scalars[5] is 1).
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+
+#include "sb_device.cuh"
+#include "sb_kernels.h"
+#include "sb_line.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace sbgpu {
+
+namespace {
+
+constexpr int kThreads = 512;
+constexpr int kBlk = 16;  // rows of a block
+constexpr int kMaxRefine = 20;
+
+__host__ __device__ inline int padded(int N) { return (N + kBlk - 1) / kBlk * kBlk; }
+__host__ __device__ inline int local_rows(int N, int C) { return (padded(N) / kBlk + C - 1) / C * kBlk; }
+
+// Shared memory of a CTA, in order (all multiples of 16 bytes)
+struct Layout {
+    size_t A, P, M, x, g, rv, dx, vel, w, rhs, tab, total;
+    __host__ __device__ static Layout make(int N, int C) {
+        const size_t n = padded(N), R = local_rows(N, C);
+        Layout l{};
+        size_t at = 0;
+        l.A = at; at += R * n * 4;         // own rows, FP32
+        l.P = at; at += kBlk * n * 4;      // scaled pivot rows
+        l.M = at; at += kBlk * R * 4;      // multipliers, [16][R]
+        l.x = at; at += n * 8;             // solution
+        l.g = at; at += n * 8;             // corrected circulation, then residual terms (CTA 0)
+        l.rv = at; at += n * 4;            // residual
+        l.dx = at; at += n * 4;            // correction
+        l.vel = at; at += R * sizeof(d3);  // velocity of the own rows
+        l.w = at; at += R * sizeof(d3);    // row vectors of the matrix
+        l.rhs = at; at += 2 * R * 8;       // right-hand side, diagonal term
+        l.tab = at; at += (kF64TableDoubles + 1) / 2 * 16;
+        l.total = at;
+        return l;
+    }
+};
+
+__device__ __forceinline__ d3 fast_normalize(d3 a) {
+    const double q = len2(a);
+    return q > 0.0 ? a * rsqrt_any(q) : mk(0, 0, 0);
+}
+
+// velocity_corrections.rs:28-100 (returns freestream + induced, corrected)
+__device__ __noinline__ d3 corrected_velocity(const SolveSettings& st, d3 fs, d3 ind) {
+    if (st.velocity_correction == 1) {
+        const double im = len(ind), mx = st.velocity_correction_ratio * len(fs);
+        return fs + (im > mx ? normalize(ind) * mx : ind);
+    }
+    return normalize(fs + ind) * len(fs);
+}
+
+// |cl of the force - cl of the foil| (force_calculations.rs:552-607)
+__device__ __forceinline__ double residual_of(const DevModel& m, int i, double gam, d3 u, double cl_pre) {
+    const double area = m.chord_len[i] * m.span_len_local[i], q = len2(u);
+    const double ff = 0.5 * area * m.density * q;
+    const d3 s = m.output_body ? m.span_e_local[i] - m.span_s_local[i] : m.span_e[i] - m.span_s[i];
+    double clg = 0.0;
+    if (ff != 0.0) {
+        const double force = q == 0.0 ? 0.0 : sqrt_any(len2(cross(u, s))) * fabs(gam * m.density);
+        clg = -signum(gam) * (force * rcp_any(ff));
+    }
+    return fabs(clg - cl_pre);
+}
+
+__device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuffers& b, unsigned char* dyn) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = static_cast<int>(cl.num_blocks()), rank = static_cast<int>(cl.block_rank());
+    const int N = m.N, n = padded(N), R = local_rows(N, C), blocks = n / kBlk;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int kWarps = kThreads / 32;
+    const Layout L = Layout::make(N, C);
+    float* A = reinterpret_cast<float*>(dyn + L.A);
+    float* P = reinterpret_cast<float*>(dyn + L.P);
+    float* M = reinterpret_cast<float*>(dyn + L.M);
+    double* x = reinterpret_cast<double*>(dyn + L.x);
+    double* g = reinterpret_cast<double*>(dyn + L.g);
+    float* rv = reinterpret_cast<float*>(dyn + L.rv);
+    float* dx = reinterpret_cast<float*>(dyn + L.dx);
+    d3* vel = reinterpret_cast<d3*>(dyn + L.vel);
+    d3* roww = reinterpret_cast<d3*>(dyn + L.w);
+    double* rhs = reinterpret_cast<double*>(dyn + L.rhs);
+    double* diag = rhs + R;
+    double* tab = reinterpret_cast<double*>(dyn + L.tab);
+    float* Pg = reinterpret_cast<float*>(b.lin_work);          // [2][16][n] (lin_work_doubles)
+    double* A64 = b.lin_work + static_cast<size_t>(kBlk) * n;  // [N][N]
+    __shared__ __align__(16) float s_inv[kBlk][kBlk];
+    __shared__ float s_red[kWarps][2];
+    __shared__ int s_bad;
+
+    // row l of the CTA is row (rank + (l / 16) C) 16 + l % 16 of the system
+    auto row_of = [&](int l) { return (rank + l / kBlk * C) * kBlk + l % kBlk; };
+    auto barrier = [&]() {
+        if (C > 1) cl.sync();
+        else __syncthreads();
+    };
+
+    load_f64_tables(tab, tid, kThreads);
+    if (tid == 0) s_bad = 0;
+    __syncthreads();
+    // 1. the system (linearized.rs:61-136): row i is dot(factors[i][c], w_i) + diagonal, with
+    // w_i = -cl slope / u_t x the normal of the row's in-plane velocity
+    for (int l = tid; l < R; l += kThreads) {
+        const int i = row_of(l);
+        roww[l] = mk(0, 0, 0);
+        rhs[l] = 0.0;
+        diag[l] = 1.0;  // rows past the end: the identity
+        if (i < N) {
+            const d3 sd = fast_normalize(m.span_e[i] - m.span_s[i]);
+            d3 v = m.felt_ctrl[i] + b.fixed[i];
+            v = v - sd * dot(v, sd);
+            const d3 un = fast_normalize(v);
+            const double iut = rcp_any(dot(v, un));
+            const FoilP& f = m.foils[m.wing_of_line[i]];
+            roww[l] = cross(un, sd) * (-f.cl_initial_slope * iut);
+            rhs[l] = -line_lift(f, m.chord_global[i], v, sd, tab).cl_linear;
+            diag[l] = 2.0 * iut * rcp_any(m.chord_len[i]);
+        }
+    }
+    __syncthreads();
+    for (int l = warp; l < R; l += kWarps) {
+        const int i = row_of(l);
+        const d3 w = roww[l];
+        const double dg = diag[l];
+        for (int c = lane; c < n; c += 32) {
+            float a = i == c && i >= N ? 1.f : 0.f;
+            if (i < N && c < N) {
+                double v = dot(b.factors[static_cast<long long>(i) * N + c], w);
+                if (i == c) v += dg;
+                A64[static_cast<long long>(i) * N + c] = v;
+                a = static_cast<float>(v);
+            }
+            A[static_cast<long long>(l) * n + c] = a;
+        }
+    }
+    __syncthreads();
+
+    // 2. FP32 inverse in place
+    // The diagonal block of rows lk.. (columns k 16..) inverted by warp 0 (row = lane mod 16, eight
+    // columns a lane), its rows scaled into P and the global buffer: outside the block's
+    // columns inverse x row, inside the inverse.
+    auto publish = [&](int k, int lk) {
+        float* Pk = Pg + (k & 1) * kBlk * n;
+        if (warp == 0) {
+            const int row = lane & 15, half = lane >> 4;
+            float* a = A + static_cast<long long>(lk + row) * n + k * kBlk + 8 * half;
+            float v[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) v[c] = a[c];
+            float least = 3e38f;
+#pragma unroll
+            for (int q = 0; q < kBlk; ++q) {
+                const int holder = q & 8 ? 16 : 0;  // lanes holding column q
+                const float f = __shfl_sync(0xffffffffu, v[q & 7], holder + row);  // column q of the own row
+                const float p = __shfl_sync(0xffffffffu, v[q & 7], holder + q);    // the pivot
+                const float ip = rcp_seed(p);
+                least = fminf(least, fabsf(p));
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const float t = __shfl_sync(0xffffffffu, v[c], 16 * half + q) * ip;  // scaled pivot row
+                    const bool pc = 8 * half + c == q;  // the pivot's column: of the identity
+                    v[c] = row == q ? (pc ? ip : t) : (pc ? -f * ip : fmaf(-f, t, v[c]));
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 8; ++c) s_inv[8 * half + c][row] = v[c];  // transposed
+            if (lane == 0 && !(least > 1e-6f)) s_bad = 1;
+        }
+        __syncthreads();
+        for (int t = tid; t < n / 2; t += kThreads) {
+            const int j = t % (n / 4) * 4, r0 = t / (n / 4) * 8;
+            float4 o[8];
+            if (j / kBlk == k) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    o[q] = make_float4(s_inv[j % kBlk][r0 + q], s_inv[j % kBlk + 1][r0 + q], s_inv[j % kBlk + 2][r0 + q],
+                                       s_inv[j % kBlk + 3][r0 + q]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) o[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+                for (int e = 0; e < kBlk; ++e) {
+                    const float4 a = *reinterpret_cast<const float4*>(A + static_cast<long long>(lk + e) * n + j);
+                    const float4 f0 = *reinterpret_cast<const float4*>(&s_inv[e][r0]);
+                    const float4 f1 = *reinterpret_cast<const float4*>(&s_inv[e][r0 + 4]);
+                    const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        o[q].x = fmaf(f[q], a.x, o[q].x);
+                        o[q].y = fmaf(f[q], a.y, o[q].y);
+                        o[q].z = fmaf(f[q], a.z, o[q].z);
+                        o[q].w = fmaf(f[q], a.w, o[q].w);
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) __stcg(reinterpret_cast<float4*>(Pk + (r0 + q) * n + j), o[q]);
+        }
+    };
+    // rows [l0, l1) of the CTA less their multiples of P, 8 x 4 elements a thread; rows [own, own + 16)
+    // become P itself
+    auto update = [&](int l0, int l1, int own) {
+        const int quads = n / 4;
+        for (int t = tid; t < (l1 - l0) / 8 * quads; t += kThreads) {
+            const int l = l0 + t / quads * 8, j = t % quads * 4;
+            float* a = A + static_cast<long long>(l) * n + j;
+            float4 o[8];
+            if (l >= own && l < own + kBlk) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) o[q] = *reinterpret_cast<const float4*>(P + (l - own + q) * n + j);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) o[q] = *reinterpret_cast<const float4*>(a + static_cast<long long>(q) * n);
+#pragma unroll 2
+                for (int e = 0; e < kBlk; ++e) {
+                    const float4 p = *reinterpret_cast<const float4*>(P + e * n + j);
+                    const float4 m0 = *reinterpret_cast<const float4*>(M + e * R + l);
+                    const float4 m1 = *reinterpret_cast<const float4*>(M + e * R + l + 4);
+                    const float f[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        o[q].x = fmaf(-f[q], p.x, o[q].x);
+                        o[q].y = fmaf(-f[q], p.y, o[q].y);
+                        o[q].z = fmaf(-f[q], p.z, o[q].z);
+                        o[q].w = fmaf(-f[q], p.w, o[q].w);
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) *reinterpret_cast<float4*>(a + static_cast<long long>(q) * n) = o[q];
+        }
+    };
+    if (rank == 0) publish(0, 0);
+    // split cluster barrier: a CTA arrives when it has read the last block's rows (and published the
+    // next block's, where it owns it) and waits after updating its own rows
+    auto arrive = [&]() {
+        if (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        else __syncthreads();
+    };
+    auto wait = [&]() {
+        if (C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    };
+    __syncthreads();
+    arrive();
+#pragma unroll 1
+    for (int k = 0; k < blocks; ++k) {
+        const float* Pk = Pg + (k & 1) * kBlk * n;
+        const int lk = k % C == rank ? k / C * kBlk : -kBlk;  // the block's first row where it is this CTA's
+        const int nx = (k + 1 < blocks && (k + 1) % C == rank) ? (k + 1) / C * kBlk : -1;  // the next block's
+        // the rows of block k are published; the buffer of block k - 1, which the owner of block k + 1
+        // writes next, has been read by every CTA
+        wait();
+#pragma unroll 4
+        for (int t = tid; t < kBlk * n / 4; t += kThreads)
+            reinterpret_cast<float4*>(P)[t] = __ldcg(reinterpret_cast<const float4*>(Pk) + t);
+        // multipliers of the own rows; the block's columns then start from 0
+        for (int t = tid; t < R * kBlk; t += kThreads) {
+            const int l = t >> 4, e = t & (kBlk - 1);
+            float* a = A + static_cast<long long>(l) * n + k * kBlk + e;
+            M[e * R + l] = *a;
+            *a = 0.f;
+        }
+        __syncthreads();
+        if (nx >= 0) {
+            update(nx, nx + kBlk, lk);
+            __syncthreads();
+            publish(k + 1, nx);
+        }
+        __syncwarp();
+        if (k + 1 < blocks) arrive();
+        if (nx >= 0) {
+            update(0, nx, lk);
+            update(nx + kBlk, R, lk);
+        } else {
+            update(0, R, lk);
+        }
+        __syncthreads();
+    }
+
+    // value v of row i into every CTA's array
+    auto store_all = [&](auto* arr, int i, auto v) {
+        if (C == 1) arr[i] = v;
+        else
+            for (int q = 0; q < C; ++q) cl.map_shared_rank(arr, q)[i] = v;
+    };
+    // 3. refinement. A bad pivot of any CTA makes its first residual NaN, so that all of them stop.
+    for (int i = tid; i < n; i += kThreads) x[i] = 0.0;
+    const float poison = s_bad ? __int_as_float(0x7FC00000) : 0.f;
+    barrier();
+    bool ok = false;
+    float last = 0.f;
+#pragma unroll 1
+    for (int it = 0; it < kMaxRefine; ++it) {
+        // residual of the own rows, to every CTA: eight lanes a row (the FP64 pipe takes a warp
+        // instruction as long for one row's tree as for four rows')
+        for (int l = 4 * warp + (lane >> 3); l < R; l += 4 * kWarps) {
+            const int i = row_of(l);
+            double s = 0.0;
+            if (it > 0 && i < N)
+                for (int c = lane & 7; c < N; c += 8) s = fma(-__ldcg(A64 + static_cast<long long>(i) * N + c), x[c], s);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            const float f = static_cast<float>(rhs[l] + s) + poison;
+            if (C == 1) {
+                if ((lane & 7) == 0) rv[i] = f;
+            } else {
+                for (int q = lane & 7; q < C; q += 8) cl.map_shared_rank(rv, q)[i] = f;
+            }
+        }
+        barrier();
+        // correction of the own rows, to every CTA
+        for (int l = warp; l < R; l += kWarps) {
+            const int i = row_of(l);
+            float s = 0.f;
+            for (int c = 4 * lane; c < n; c += 128) {
+                const float4 a = *reinterpret_cast<const float4*>(A + static_cast<long long>(l) * n + c);
+                const float4 r = *reinterpret_cast<const float4*>(rv + c);
+                s = fmaf(a.x, r.x, fmaf(a.y, r.y, fmaf(a.z, r.z, fmaf(a.w, r.w, s))));
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (C == 1) {
+                if (lane == 0) dx[i] = s;
+            } else if (lane < C) {
+                cl.map_shared_rank(dx, lane)[i] = s;
+            }
+        }
+        barrier();
+        float d = 0.f, y = 0.f;  // largest |dx| and |x|; a NaN stays
+        bool fin = true;
+        for (int i = tid; i < N; i += kThreads) {
+            x[i] += static_cast<double>(dx[i]);
+            const float a = fabsf(dx[i]);
+            fin = fin && a < 3e38f;
+            d = fmaxf(d, a);
+            y = fmaxf(y, fabsf(static_cast<float>(x[i])));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            d = fmaxf(d, __shfl_xor_sync(0xffffffffu, d, o));
+            y = fmaxf(y, __shfl_xor_sync(0xffffffffu, y, o));
+        }
+        if (lane == 0) {
+            s_red[warp][0] = d;
+            s_red[warp][1] = y;
+        }
+        fin = __syncthreads_and(fin);
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            d = fmaxf(d, s_red[w][0]);
+            y = fmaxf(y, s_red[w][1]);
+        }
+        // the same numbers, so the same decision in every CTA
+        if (!fin) break;
+        // what is left is at most the ratio of the last two corrections times the last
+        if (d <= 0x1p-50f * y || (it > 0 && d < 0.1f * last && d * (d / last) <= 0x1p-53f * y)) {
+            ok = true;
+            break;
+        }
+        if (it > 0 && d > 0.5f * last) {  // no longer shrinking: rounding, or an inverse that is none
+            ok = d <= 1e-10f * y;
+            break;
+        }
+        last = d;
+        __syncthreads();  // s_red is written again
+    }
+    if (!ok) {  // the elimination kernels take the case
+        if (rank == 0 && tid == 0) b.scalars[5] = 0.0;
+        barrier();
+        return;
+    }
+
+    // 4. induced velocity, total velocity, viscous correction (linearized.rs:141-202)
+    auto total_velocities = [&](const double* gam) {
+        for (int l = 4 * warp + (lane >> 3); l < R; l += 4 * kWarps) {
+            const int i = row_of(l);
+            d3 s = mk(0, 0, 0);
+            if (i < N)
+                for (int c = lane & 7; c < N; c += 8) {
+                    const d3 f = b.factors[static_cast<long long>(i) * N + c];
+                    s.x = fma(f.x, gam[c], s.x);
+                    s.y = fma(f.y, gam[c], s.y);
+                    s.z = fma(f.z, gam[c], s.z);
+                }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+                s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+                s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
+            }
+            if ((lane & 7) == 0 && i < N) {
+                const d3 ind = b.fixed[i] + s, fs = m.felt_ctrl[i];
+                vel[l] = st.velocity_correction == 0 ? fs + ind : corrected_velocity(st, fs, ind);
+            }
+        }
+        __syncthreads();
+    };
+    total_velocities(x);
+    double* gam = x;
+    if (!st.disable_viscous_corrections) {
+        for (int l = tid; l < R; l += kThreads) {
+            const int i = row_of(l);
+            if (i >= N) break;
+            const LineLift o = line_lift(m.foils[m.wing_of_line[i]], m.chord_global[i], vel[l],
+                                         fast_normalize(m.span_e[i] - m.span_s[i]), tab);
+            store_all(g, i, fabs(o.cl_linear) > kMinPositive ? x[i] * (o.cl_pre / o.cl_linear) : x[i]);
+        }
+        barrier();
+        gam = g;
+        if (st.full_induced_correction) total_velocities(g);
+    }
+    // residual terms (linearized.rs:204-213) to CTA 0 (into x, no longer needed there unless it is
+    // the circulation: then into g) and the outputs
+    double* terms = gam == x ? g : x;
+    barrier();
+    for (int l = tid; l < R; l += kThreads) {
+        const int i = row_of(l);
+        if (i >= N) break;
+        const double gi = gam[i];
+        const d3 v = vel[l];
+        const LineLift o = line_lift(m.foils[m.wing_of_line[i]], m.chord_global[i], v,
+                                     fast_normalize(m.span_e[i] - m.span_s[i]), tab);
+        *(cl.map_shared_rank(terms, 0) + i) = residual_of(m, i, gi, v, o.cl_pre);
+        b.gamma_prev[i] = gi;
+        b.vel_out[i] = v;
+        if (b.wake_str_row0) b.wake_str_row0[i] = gi;
+        if (b.rec32_row0) b.rec32_row0[i].v[kRec32Gamma] = static_cast<float>(gi);
+        if (b.rec64_row0) b.rec64_row0[i].v[kRec64Gamma] = gi;
+    }
+    barrier();
+    if (rank == 0 && warp == 0) {
+        double s = 0.0;
+        for (int i = lane; i < N; i += 32) s += terms[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0) {
+            b.scalars[0] = s / static_cast<double>(N);
+            b.scalars[1] = 1.0;
+            b.scalars[2] = 1.0;
+            b.scalars[5] = 1.0;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads, 1) k_lin_refined(DevModel m, SolveSettings st, SolveBuffers b) {
+    extern __shared__ __align__(16) unsigned char refined_dyn[];
+    solve(m, st, b, refined_dyn);
+}
+
+// Every case of a batch whose cluster size is this launch's: cluster i solves jobs[i].
+__global__ void __launch_bounds__(kThreads, 1) k_lin_refined_jobs(const SolveJob* jobs) {
+    extern __shared__ __align__(16) unsigned char refined_dyn[];
+    const SolveJob& j = jobs[blockIdx.x / cg::this_cluster().num_blocks()];
+    solve(j.m, j.st, j.b, refined_dyn);
+}
+
+void config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, int clusters, int C, size_t smem, cudaStream_t s) {
+    cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(clusters * C), 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(C);
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+}
+
+constexpr size_t kSmemLimit = 224 * 1024;
+
+// Raises the kernels' limits, once per device; the largest cluster the device holds at kSmemLimit.
+int largest_cluster() {
+    static std::mutex mu;
+    static std::map<int, int> largest;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 8;
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = largest.find(dev);
+    if (it != largest.end()) return it->second;
+    auto prepare = [](auto kernel) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit)) ==
+                   cudaSuccess &&
+               cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    };
+    int c = prepare(k_lin_refined) && prepare(k_lin_refined_jobs) ? 16 : 0;
+    for (; c > 8; c /= 2) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr;
+        config(cfg, attr, 1, c, kSmemLimit, nullptr);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_lin_refined, &cfg) == cudaSuccess && n > 0) break;
+    }
+    (void)cudaGetLastError();  // a refused shape is not an error of the caller
+    largest[dev] = c;
+    return c;
+}
+
+}  // namespace
+
+size_t lin_work_doubles(int N) {
+    // the elimination's [N][N + 1], or the f64 matrix [N][N] and two buffers of scaled rows [16][padded] floats
+    return std::max(static_cast<size_t>(N) * (N + 1), static_cast<size_t>(N) * N + static_cast<size_t>(kBlk) * padded(N));
+}
+
+LinPlan linearized_refined_plan(int N, int crowding) {
+    int C = largest_cluster();
+    while (C > 1 && C > padded(N) / kBlk) C /= 2;
+    if (C < 1 || Layout::make(N, C).total > kSmemLimit) return {0, 0};
+    for (; crowding > 0 && C > 1 && Layout::make(N, C / 2).total <= kSmemLimit; --crowding) C /= 2;
+    return {C, Layout::make(N, C).total};
+}
+
+cudaError_t launch_solve_linearized_refined(const DevModel& m, const SolveSettings& st, const SolveBuffers& b,
+                                            const LinPlan& p, cudaStream_t s) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    config(cfg, attr, 1, p.cluster, p.smem, s);
+    return cudaLaunchKernelEx(&cfg, k_lin_refined, m, st, b);
+}
+
+cudaError_t launch_solve_linearized_refined_jobs(const SolveJob* jobs, int n, const LinPlan& p, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    if (p.cluster < 1 || p.smem > kSmemLimit) return cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    config(cfg, attr, n, p.cluster, p.smem, s);
+    return cudaLaunchKernelEx(&cfg, k_lin_refined_jobs, jobs);
+}
+
+}  // namespace sbgpu

@@ -1044,6 +1044,7 @@ __device__ void lin_solve_case(const DevModel& m, const SolveSettings& st, const
     double* gam = reinterpret_cast<double*>(ind + N);     // [N]
     double* A = lin_vec_bytes(N) + lin_mat_bytes(N) <= dyn_bytes ? gam + N : b.lin_work;  // [N][N+1]
     __shared__ int s_piv;
+    if (b.scalars[5] != 0.0) return;  // solved by k_lin_refined
 
     for (int i = tid; i < N; i += nt) lin_build_row(m, b, i, A + static_cast<long long>(i) * W1);
     __syncthreads();
@@ -1155,6 +1156,7 @@ __device__ void lin_solve_cluster(const DevModel& m, const SolveSettings& st, co
     double* A = reinterpret_cast<double*>(pos + N);    // [R][N + 1] rows rank, rank + C, ...
     __shared__ double s_cand_v[2];
     __shared__ int s_cand_p[2], s_piv;
+    if (b.scalars[5] != 0.0) return;  // solved by k_lin_refined (the same value in every CTA)
 
     // the candidate of this CTA for column k: first largest |A[r][k]| over its rows at
     // positions >= k (lowest position among equal values), into slot k & 1
@@ -1347,6 +1349,11 @@ LinPlan linearized_plan(int N) {
 }
 
 cudaError_t launch_solve_linearized(const DevModel& m, const SolveSettings& st, const SolveBuffers& b, cudaStream_t s) {
+    const LinPlan refined = linearized_refined_plan(m.N, 0);
+    if (refined.cluster > 0) {
+        const cudaError_t e = launch_solve_linearized_refined(m, st, b, refined, s);
+        if (e != cudaSuccess) return e;
+    }
     const LinPlan p = linearized_plan(m.N);
     if (p.cluster == 1) {
         if (p.smem > 48 * 1024) {

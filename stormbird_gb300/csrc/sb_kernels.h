@@ -235,8 +235,9 @@ struct SolveBuffers {
     const d3* basis = nullptr;
     double* gamma_prev = nullptr;   // [N] in: initial solution, out: solution
     d3* vel_out = nullptr;          // [N] output control-point velocity
-    double* scalars = nullptr;      // [8]: residual, iterations, converged, singular, start (below)
-    double* lin_work = nullptr;     // [N*(N+1)] Gaussian elimination scratch (linearized)
+    double* scalars = nullptr;      // [8]: residual, iterations, converged, singular, start (below),
+                                    // solved by the refined inverse (linearized)
+    double* lin_work = nullptr;     // [lin_work_doubles(N)] scratch of the linearized solves
     double* wake_str_row0 = nullptr;        // strengths row 0 (dynamic) or nullptr
     PanelRec<float>* rec32_row0 = nullptr;  // FP32 record row 0 (dynamic) or nullptr
     PanelRec<double>* rec64_row0 = nullptr; // FP64 record row 0 in the FP64 sweep mode
@@ -278,8 +279,17 @@ struct LinPlan {
     size_t smem = 0;
 };
 LinPlan linearized_plan(int N);
+// The FP32 inverse with f64 refinement (k_lin_refined.cu), launched before the elimination, which
+// solves only what it leaves (SolveBuffers::scalars[5] = 0). cluster = 0: too large for it.
+// crowding halves the cluster that many times, as far as shared memory allows: for batches whose
+// clusters would not all run side by side.
+LinPlan linearized_refined_plan(int N, int crowding);
+size_t lin_work_doubles(int N);  // SolveBuffers::lin_work
+cudaError_t launch_solve_linearized_refined(const DevModel& m, const SolveSettings& st, const SolveBuffers& b,
+                                            const LinPlan& plan, cudaStream_t s);
 // n solves of one plan shape in one launch (smem: the largest of the jobs' plans).
 cudaError_t launch_solve_linearized_jobs(const SolveJob* jobs, int n, const LinPlan& plan, cudaStream_t s);
+cudaError_t launch_solve_linearized_refined_jobs(const SolveJob* jobs, int n, const LinPlan& plan, cudaStream_t s);
 // SimpleIterative solves of a batch: n cases of one cluster size (solve_cluster_size of
 // their N) in one launch, a cluster per case; smem = the largest of the jobs' plans.
 // How such a solve runs: rows per thread (1 or 4: a launch holds one kind), rows of the matrix

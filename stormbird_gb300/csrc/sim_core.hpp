@@ -561,7 +561,7 @@ struct sb_sim {
         ck(cudaMemset(gamma_prev.p, 0, N * sizeof(double)), "memset");
         gamma_p = gamma_prev.p;
         ck(cudaMemset(scalars.p, 0, 8 * sizeof(double)), "memset");
-        if (solver_kind == 1 || solve.start_with_linearized) lin_work.alloc(static_cast<size_t>(N) * (N + 1));
+        if (solver_kind == 1 || solve.start_with_linearized) lin_work.alloc(lin_work_doubles(N));
         vel_out.alloc(N); hist0.alloc(N); hist1.alloc(N);
         ck(cudaMemset(hist0.p, 0, N * sizeof(d3)), "memset");
         ck(cudaMemset(hist1.p, 0, N * sizeof(d3)), "memset");

@@ -133,6 +133,7 @@ struct sb_batch {
     // forces of every case, one launch (refilled each step: step parameters can change)
     PinnedBuf<ForceJob> h_force_jobs;
     DevBuf<ForceJob> d_force_jobs;
+    int force_blocks = 0;  // wings of all cases
     // geometry, wake update, unit-strength matrix and chain records of the dynamic cases past
     // their first step: one launch per kind for all of them (refilled each step: the jobs
     // name the step's wake buffers and time step)
@@ -140,7 +141,7 @@ struct sb_batch {
     PinnedBuf<CaseStepJob> h_case_jobs;
     DevBuf<CaseStepJob> d_case_jobs;
     int n_case_jobs = 0;
-    long long blk_advect = 0, blk_panels = 0, blk_matrix = 0, blk_chain = 0;
+    long long blk_geometry = 0, blk_advect = 0, blk_panels = 0, blk_matrix = 0, blk_chain = 0;
 
     // Sweep work lists: group = (sweep kind, symmetry, neglect); one launch each.
     struct Group {
@@ -589,7 +590,7 @@ struct sb_batch {
         }
         join(0);
         if (n_case_jobs > 0) {  // geometry, then wake advection and panels, of the batched cases
-            ck(launch_prep_geometry_jobs(d_case_jobs.p, n_case_jobs, main), "batched geometry");
+            ck(launch_prep_geometry_jobs(d_case_jobs.p, n_case_jobs, blk_geometry, main), "batched geometry");
             ck(launch_wake_jobs(d_case_jobs.p, n_case_jobs, blk_advect, blk_panels, main), "batched wake update");
         }
         if (warm_mode != 0) warm_start_before_solve();
@@ -667,7 +668,7 @@ struct sb_batch {
         fill_force_jobs();
         ck(cudaMemcpyAsync(d_force_jobs.p, h_force_jobs.p, cases.size() * sizeof(ForceJob), cudaMemcpyHostToDevice, main),
            "H2D force jobs");
-        ck(launch_forces_jobs(d_force_jobs.p, static_cast<int>(cases.size()), main), "batched forces");
+        ck(launch_forces_jobs(d_force_jobs.p, static_cast<int>(cases.size()), force_blocks, main), "batched forces");
         for (auto& c : cases) c->after_forces();
         k_gather<<<static_cast<unsigned>(cases.size()), 128, 0, main>>>(gather_jobs.p);
         ck(cudaGetLastError(), "gather");
@@ -874,16 +875,18 @@ struct sb_batch {
     // The job of every dynamic case past its first step (state before the step).
     void fill_case_jobs(double time, double dt) {
         n_case_jobs = 0;
-        blk_advect = blk_panels = blk_matrix = blk_chain = 0;
+        blk_geometry = blk_advect = blk_panels = blk_matrix = blk_chain = 0;
         for (size_t i = 0; i < cases.size(); ++i) {
             const sb_sim& c = *cases[i];
             case_batched[i] = c.batch_kernels_ok() ? 1 : 0;
             if (!case_batched[i]) continue;
             CaseStepJob j = c.step_job(time, dt);
+            j.blk_geometry = blk_geometry;
             j.blk_advect = blk_advect;
             j.blk_panels = blk_panels;
             j.blk_matrix = blk_matrix;
             j.blk_chain = blk_chain;
+            blk_geometry += prep_geometry_blocks(c.dm);
             blk_advect += wake_advect_blocks(c.dm);
             blk_panels += wake_panels_blocks(c.dm);
             blk_matrix += unit_matrix_blocks(c.N, j.row0_32 != nullptr);
@@ -901,7 +904,12 @@ struct sb_batch {
 
     // The forces job of every case (read by the graph's copy node at launch when replayed).
     void fill_force_jobs() {
-        for (size_t i = 0; i < cases.size(); ++i) h_force_jobs.p[i] = cases[i]->force_job();
+        force_blocks = 0;
+        for (size_t i = 0; i < cases.size(); ++i) {
+            h_force_jobs.p[i] = cases[i]->force_job();
+            h_force_jobs.p[i].block_begin = force_blocks;
+            force_blocks += cases[i]->S;
+        }
     }
 
     // The SimpleIterative jobs of the step (each case's model, settings and buffers, with the

@@ -67,11 +67,6 @@ struct Layout {
     }
 };
 
-__device__ __forceinline__ d3 fast_normalize(d3 a) {
-    const double q = len2(a);
-    return q > 0.0 ? a * rsqrt_any(q) : mk(0, 0, 0);
-}
-
 // velocity_corrections.rs:28-100 (returns freestream + induced, corrected)
 __device__ __noinline__ d3 corrected_velocity(const SolveSettings& st, d3 fs, d3 ind) {
     if (st.velocity_correction == 1) {
@@ -137,10 +132,10 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
         rhs[l] = 0.0;
         diag[l] = 1.0;  // rows past the end: the identity
         if (i < N) {
-            const d3 sd = fast_normalize(m.span_e[i] - m.span_s[i]);
+            const d3 sd = normalize(m.span_e[i] - m.span_s[i]);
             d3 v = m.felt_ctrl[i] + b.fixed[i];
             v = v - sd * dot(v, sd);
-            const d3 un = fast_normalize(v);
+            const d3 un = normalize(v);
             const double iut = rcp_any(dot(v, un));
             const FoilP& f = m.foils[m.wing_of_line[i]];
             roww[l] = cross(un, sd) * (-f.cl_initial_slope * iut);
@@ -433,7 +428,7 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
             const int i = row_of(l);
             if (i >= N) break;
             const LineLift o = line_lift(m.foils[m.wing_of_line[i]], m.chord_global[i], vel[l],
-                                         fast_normalize(m.span_e[i] - m.span_s[i]), tab);
+                                         normalize(m.span_e[i] - m.span_s[i]), tab);
             store_all(g, i, fabs(o.cl_linear) > kMinPositive ? x[i] * (o.cl_pre / o.cl_linear) : x[i]);
         }
         barrier();
@@ -450,7 +445,7 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
         const double gi = gam[i];
         const d3 v = vel[l];
         const LineLift o = line_lift(m.foils[m.wing_of_line[i]], m.chord_global[i], v,
-                                     fast_normalize(m.span_e[i] - m.span_s[i]), tab);
+                                     normalize(m.span_e[i] - m.span_s[i]), tab);
         *(cl.map_shared_rank(terms, 0) + i) = residual_of(m, i, gi, v, o.cl_pre);
         b.gamma_prev[i] = gi;
         b.vel_out[i] = v;

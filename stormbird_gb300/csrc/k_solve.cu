@@ -1,4 +1,4 @@
-// Circulation solvers and force output (sm_103a), f64.
+// Circulation solvers (sm_103a), f64.
 //
 // k_solve_si: the damped fixed-point solve SimpleIterative::solve
 // (stormbird/src/lifting_line/solvers/simple_iterative.rs:86-212) for one case on one
@@ -25,9 +25,6 @@
 // the Gaussian elimination with partial pivoting of stormath/src/matrix/linalg.rs:41-103,
 // one CTA per case: one case, or all linearized quasi-steady cases of a batch in one
 // launch.
-//
-// k_forces: SimulationResult of one step (force_calculations.rs:322-452, 669-698;
-// common_utils/forces_and_moments.rs:163-245; flow_derivatives.rs:31-63).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -1390,128 +1387,6 @@ cudaError_t launch_solve_linearized_jobs(const SolveJob* jobs, int n, const LinP
     cudaLaunchAttribute attr;
     cluster_config(cfg, attr, n, plan.cluster, plan.smem, s);
     return cudaLaunchKernelEx(&cfg, k_solve_lin_cluster_jobs, jobs);
-}
-
-// ---------------------------------------------------------------------------------------
-// Forces, one CTA
-// ---------------------------------------------------------------------------------------
-constexpr int kForceThreads = 256;
-
-// One case's forces on the calling CTA (k_forces: one case; k_forces_jobs: a CTA per case
-// of a batch, all cases side by side instead of one SM per case on a few streams).
-__device__ void forces_case(const DevModel& m, const StepParams& p, const ForceArgs& f) {
-    const int N = m.N, S = m.S, tid = threadIdx.x, nt = blockDim.x;
-    const OutLayout L = OutLayout::make(N, S);
-    double* o = f.out;
-    const bool body = m.output_body != 0;
-    for (int i = tid; i < N; i += nt) {
-        double g = f.gamma[i];
-        d3 v = f.vel[i];
-        d3 sr = m.span_e[i] - m.span_s[i];
-        double aoa = len(v) > kMinPositive ? signed_angle_between(m.chord_global[i], v, normalize(sr)) : 0.0;
-        d3 acc = mk(0, 0, 0);
-        if (f.fd_count >= 2) acc = (v * 3.0 - f.hist1[i] * 4.0 + f.hist0[i]) / (2.0 * p.dt);
-        f.hist0[i] = f.hist1[i];
-        f.hist1[i] = v;
-        d3 fv = body ? to_body(v, p.rotation) : v;
-        d3 fa = body ? to_body(acc, p.rotation) : acc;
-        d3 sl_local = m.span_e_local[i] - m.span_s_local[i];
-        d3 sl_out = body ? sl_local : sr;
-        d3 cv_out = body ? m.chord_local[i] : m.chord_global[i];
-        const FoilP fo = m.foils[m.wing_of_line[i]];
-        double area = m.chord_len[i] * m.span_len_local[i];
-        double ff = 0.5 * area * m.density * len2(fv);
-        d3 circ = len(fv) == 0.0 ? mk(0, 0, 0) : (g * cross(fv, sl_out)) * m.density;
-        d3 visc = mk(0, 0, 0);
-        if (!m.include_viscous_lift) visc = normalize(cross(sl_local, fv)) * foil_cl_post_stall(fo, aoa) * ff;
-        d3 drag = normalize(fv) * foil_cd(fo, aoa) * ff;
-        double strip = m.chord_len[i] * len(sl_out);
-        d3 ra = fa - project(fa, normalize(sl_out));
-        ra = ra - project(ra, cv_out);
-        d3 am = mk(0, 0, 0);
-        if (len(ra) != 0.0) am = (fo.added_mass_factor * len(ra)) * m.density * strip * normalize(ra);
-        d3 gy = mk(0, 0, 0);
-        d3 tot = circ;
-        tot = tot + visc;
-        tot = tot + drag;
-        tot = tot + am;
-        tot = tot + gy;
-        d3 comps[6] = {circ, visc, drag, am, gy, tot};
-        o[L.gamma + i] = g;
-        d3 ctrl = m.ctrl[i];
-        d3 felt = m.felt_ctrl[i];
-        const d3* src[6] = {&v, &felt, &fv, &fa, &ctrl, nullptr};
-        long long offs[5] = {L.vel, L.felt, L.fvel, L.acc, L.ctrl};
-        for (int q = 0; q < 5; ++q) {
-            o[offs[q] + 3 * i] = src[q]->x;
-            o[offs[q] + 3 * i + 1] = src[q]->y;
-            o[offs[q] + 3 * i + 2] = src[q]->z;
-        }
-        o[L.aoa + i] = aoa;
-        for (int c = 0; c < 6; ++c) {
-            long long base = L.sect + (static_cast<long long>(c) * N + i) * 3;
-            o[base] = comps[c].x;
-            o[base + 1] = comps[c].y;
-            o[base + 2] = comps[c].z;
-        }
-    }
-    __syncthreads();
-    // integrated force and moment of each (wing, component), summed in line order
-    for (int t = tid; t < S * 6; t += nt) {
-        const int w = t / 6, c = t % 6;
-        d3 fs = mk(0, 0, 0), ms = mk(0, 0, 0);
-        for (int i = m.wing_start[w]; i < m.wing_end[w]; ++i) {
-            if (m.is_virtual[i]) continue;
-            d3 cp = body ? 0.5 * (m.span_s_local[i] + m.span_e_local[i]) : 0.5 * (m.span_s[i] + m.span_e[i]);
-            long long base = L.sect + (static_cast<long long>(c) * N + i) * 3;
-            d3 sf = mk(o[base], o[base + 1], o[base + 2]);
-            fs = fs + sf;
-            ms = ms + cross(cp, sf);
-        }
-        long long bf = L.intf + (static_cast<long long>(w) * 6 + c) * 3, bm = L.intm + (static_cast<long long>(w) * 6 + c) * 3;
-        o[bf] = fs.x;
-        o[bf + 1] = fs.y;
-        o[bf + 2] = fs.z;
-        o[bm] = ms.x;
-        o[bm + 1] = ms.y;
-        o[bm + 2] = ms.z;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        d3 fsum = mk(0, 0, 0), msum = mk(0, 0, 0);
-        for (int w = 0; w < S; ++w) {
-            long long bf = L.intf + (static_cast<long long>(w) * 6 + 5) * 3, bm = L.intm + (static_cast<long long>(w) * 6 + 5) * 3;
-            fsum = fsum + mk(o[bf], o[bf + 1], o[bf + 2]);
-            msum = msum + mk(o[bm], o[bm + 1], o[bm + 2]);
-        }
-        o[L.fsum] = fsum.x;
-        o[L.fsum + 1] = fsum.y;
-        o[L.fsum + 2] = fsum.z;
-        o[L.msum] = msum.x;
-        o[L.msum + 1] = msum.y;
-        o[L.msum + 2] = msum.z;
-        o[L.residual] = f.scalars[0];
-        o[L.iterations] = f.scalars[1];
-        o[L.converged] = f.scalars[2];
-    }
-}
-
-__global__ void __launch_bounds__(kForceThreads) k_forces(DevModel m, StepParams p, ForceArgs f) { forces_case(m, p, f); }
-
-__global__ void __launch_bounds__(kForceThreads) k_forces_jobs(const ForceJob* jobs) {
-    const ForceJob& j = jobs[blockIdx.x];
-    forces_case(j.m, j.p, j.f);
-}
-
-cudaError_t launch_forces(const DevModel& m, const StepParams& p, const ForceArgs& f, cudaStream_t s) {
-    k_forces<<<1, kForceThreads, 0, s>>>(m, p, f);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_forces_jobs(const ForceJob* jobs, int n, cudaStream_t s) {
-    if (n <= 0) return cudaSuccess;
-    k_forces_jobs<<<static_cast<unsigned>(n), kForceThreads, 0, s>>>(jobs);
-    return cudaGetLastError();
 }
 
 }  // namespace sbgpu

@@ -16,64 +16,138 @@
 namespace sbgpu {
 
 // ---------------------------------------------------------------------------------------
-// Geometry of the line force model for one step. One CTA: O(N) work.
+// Geometry of the line force model for one step: about 150 FP64 instructions a line. A block takes 62
+// lines (64 threads, a line before and one after them for the span points' means), so that a model's
+// lines spread over SMs; the sines and cosines (a wing's angle, the body's rotation) are a few
+// threads' work per block. One CTA with CUDA's sin, cos and normalisations per line took 18 us at
+// 21 lines and 62 us at 570 (cold instruction cache); this takes 10 and 11 us.
 // ---------------------------------------------------------------------------------------
-__device__ void prep_geometry_block(const DevModel& m, const StepParams& p, const d3* fs_ctrl, d3* mean_out) {
-    const int tid = threadIdx.x, nt = blockDim.x;
-    for (int i = tid; i < m.N; i += nt) {
-        int w = m.wing_of_line[i];
-        int ws = m.wing_start[w];
-        d3 axis = m.span_e_local[ws] - m.span_s_local[ws];  // data_access.rs:256-258
-        d3 cl = rotate_around_axis(m.chord_not_rotated[i], p.local_wing_angles[w], axis);
-        m.chord_local[i] = cl;
-        m.chord_global[i] = rotate_xyz(cl, p.rotation);
-        d3 s = rotate_xyz(m.span_s_local[i], p.rotation) + p.translation;
-        d3 e = rotate_xyz(m.span_e_local[i], p.rotation) + p.translation;
-        m.span_s[i] = s;
-        m.span_e[i] = e;
-        d3 c = 0.5 * (s + e);
-        m.ctrl[i] = c;
-        if (m.solve_basis) line_basis(m.chord_global[i], s, e, m.solve_basis[2 * i], m.solve_basis[2 * i + 1]);
-        if (fs_ctrl) {
-            // rigid_body_motion.rs:53-60
-            d3 mv = p.velocity_linear + cross(p.velocity_angular, c - p.translation);
-            m.felt_ctrl[i] = fs_ctrl[i] - mv;
+constexpr int kGeometryThreads = 64;
+constexpr int kGeometryLines = kGeometryThreads - 2;
+
+__device__ __noinline__ void sin_cos(double a, double& s, double& c) { sincos(a, &s, &c); }
+
+// rotate_xyz (transformations.rs:182-207) with the sines and cosines at hand (an angle of 0 is left out,
+// as there)
+struct Rotation {
+    double s[3], c[3];
+    d3 r;
+};
+__device__ __forceinline__ d3 rotate(d3 v, const Rotation& R) {
+    if (R.r.x != 0.0) v = mk(v.x, v.y * R.c[0] - v.z * R.s[0], v.y * R.s[0] + v.z * R.c[0]);
+    if (R.r.y != 0.0) v = mk(v.x * R.c[1] + v.z * R.s[1], v.y, -v.x * R.s[1] + v.z * R.c[1]);
+    if (R.r.z != 0.0) v = mk(v.x * R.c[2] - v.y * R.s[2], v.x * R.s[2] + v.y * R.c[2], v.z);
+    return v;
+}
+
+__device__ void prep_geometry_block(const DevModel& m, const StepParams& p, const d3* fs_ctrl, d3* mean_out, int block) {
+    const int tid = threadIdx.x;
+    __shared__ Rotation s_rot;
+    __shared__ d3 s_axis[kMaxWings];            // of the wings met in this block, by wing - first wing
+    __shared__ double s_sin[kMaxWings], s_cos[kMaxWings];
+    __shared__ d3 s_chord[kGeometryThreads], s_felt[kGeometryThreads];
+    const int first = block * kGeometryLines;
+    const int i = first - 1 + tid;              // line of the thread, the neighbours' included
+    const int w0 = m.wing_of_line[max(first - 1, 0)], w1 = m.wing_of_line[min(first + kGeometryLines, m.N - 1)];
+    for (int t = tid; t < w1 - w0 + 1 + 3; t += kGeometryThreads) {
+        const int q = t - (w1 - w0 + 1);
+        double sn, cs;
+        sin_cos(q < 0 ? p.local_wing_angles[w0 + t] : q == 0 ? p.rotation.x : q == 1 ? p.rotation.y : p.rotation.z, sn, cs);
+        if (q < 0) {
+            const int ws = m.wing_start[w0 + t];
+            s_axis[t] = normalize(m.span_e_local[ws] - m.span_s_local[ws]);  // data_access.rs:256-258
+            s_sin[t] = sn;
+            s_cos[t] = cs;
+        } else {
+            s_rot.s[q] = sn;
+            s_rot.c[q] = cs;
+            if (q == 0) s_rot.r = p.rotation;
         }
     }
     __syncthreads();
-    for (int k = tid; k < m.Np; k += nt) {
-        int l = m.sp_line[k];
-        m.span_pts[k] = m.sp_end[k] ? m.span_e[l] : m.span_s[l];
-        int a = m.sp_val_a[k], b = m.sp_val_b[k];
-        m.chord_span_pts[k] = (a == b) ? m.chord_global[a] : (m.chord_global[a] + m.chord_global[b]) * 0.5;
-        if (fs_ctrl) m.felt_span[k] = (a == b) ? m.felt_ctrl[a] : (m.felt_ctrl[a] + m.felt_ctrl[b]) * 0.5;
+    const bool have = i >= 0 && i < m.N, own = have && tid >= 1 && tid <= kGeometryLines;
+    d3 chord = mk(0, 0, 0), felt = mk(0, 0, 0), s = chord, e = chord;
+    int w = 0;
+    if (have) {
+        w = m.wing_of_line[i];
+        // Rodrigues rotation of the chord about the wing's axis (transformations.rs:139-150)
+        const d3 v = m.chord_not_rotated[i], n = s_axis[w - w0];
+        const double c = s_cos[w - w0], sn = s_sin[w - w0];
+        const d3 cl = v * c + cross(n, v) * sn + n * dot(n, v) * (1.0 - c);
+        chord = rotate(cl, s_rot);
+        s = rotate(m.span_s_local[i], s_rot) + p.translation;
+        e = rotate(m.span_e_local[i], s_rot) + p.translation;
+        const d3 ctrl = 0.5 * (s + e);
+        if (fs_ctrl)  // rigid_body_motion.rs:53-60
+            felt = fs_ctrl[i] - (p.velocity_linear + cross(p.velocity_angular, ctrl - p.translation));
+        if (own) {
+            m.chord_local[i] = cl;
+            m.chord_global[i] = chord;
+            m.span_s[i] = s;
+            m.span_e[i] = e;
+            m.ctrl[i] = ctrl;
+            if (m.solve_basis) line_basis(chord, s, e, m.solve_basis[2 * i], m.solve_basis[2 * i + 1]);
+            if (fs_ctrl) m.felt_ctrl[i] = felt;
+        }
     }
-    if (mean_out && tid == 0) {
+    s_chord[tid] = chord;
+    s_felt[tid] = felt;
+    __syncthreads();
+    if (own) {
+        // the span point where the line starts (value_mapping.rs:87-137: the mean of the lines on both
+        // sides, the line's own value at a wing's end), and the wing's last point
+        const int k = i + w;
+        const bool tip = i == m.wing_start[w], last = i == m.wing_end[w] - 1;
+        m.span_pts[k] = s;
+        m.chord_span_pts[k] = tip ? chord : (s_chord[tid - 1] + chord) * 0.5;
+        if (fs_ctrl) m.felt_span[k] = tip ? felt : (s_felt[tid - 1] + felt) * 0.5;
+        if (last) {
+            m.span_pts[k + 1] = e;
+            m.chord_span_pts[k + 1] = chord;
+            if (fs_ctrl) m.felt_span[k + 1] = felt;
+        }
+    }
+    if (mean_out && block == 0 && tid == 0) {
         // simulation.rs:74-75: sum in order, then divide
-        d3 s = mk(0, 0, 0);
-        for (int i = 0; i < m.N; ++i) s = s + fs_ctrl[i];
-        *mean_out = s / static_cast<double>(m.N);
+        d3 sum = mk(0, 0, 0);
+        for (int l = 0; l < m.N; ++l) sum = sum + fs_ctrl[l];
+        *mean_out = sum / static_cast<double>(m.N);
     }
 }
 
-__global__ void k_prep_geometry(DevModel m, StepParams p, const d3* fs_ctrl, d3* mean_out) {
-    prep_geometry_block(m, p, fs_ctrl, mean_out);
+__global__ void __launch_bounds__(kGeometryThreads) k_prep_geometry(DevModel m, StepParams p, const d3* fs_ctrl, d3* mean_out) {
+    prep_geometry_block(m, p, fs_ctrl, mean_out, blockIdx.x);
 }
 
-// The geometry of every case of a batch: one CTA per case.
-__global__ void k_prep_geometry_jobs(const CaseStepJob* jobs) {
-    const CaseStepJob& J = jobs[blockIdx.x];
-    prep_geometry_block(J.m, J.p, J.fs_ctrl, nullptr);
+// Job that block b belongs to: the last one whose first block of the kind is at or before it (jobs [n]
+// ascending in each kind's first block).
+template <long long CaseStepJob::*First>
+__device__ inline int job_of_block(const CaseStepJob* jobs, int n, long long b) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (jobs[mid].*First <= b) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
 }
+
+// The geometry of every case of a batch.
+__global__ void __launch_bounds__(kGeometryThreads) k_prep_geometry_jobs(const CaseStepJob* jobs, int n) {
+    const CaseStepJob& J = jobs[job_of_block<&CaseStepJob::blk_geometry>(jobs, n, blockIdx.x)];
+    prep_geometry_block(J.m, J.p, J.fs_ctrl, nullptr, static_cast<int>(blockIdx.x - J.blk_geometry));
+}
+
+long long prep_geometry_blocks(const DevModel& m) { return (m.N + kGeometryLines - 1) / kGeometryLines; }
 
 cudaError_t launch_prep_geometry(const DevModel& m, const StepParams& p, const d3* fs_ctrl, d3* mean_out, cudaStream_t s) {
-    k_prep_geometry<<<1, 512, 0, s>>>(m, p, fs_ctrl, mean_out);
+    k_prep_geometry<<<static_cast<unsigned>(prep_geometry_blocks(m)), kGeometryThreads, 0, s>>>(m, p, fs_ctrl, mean_out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_prep_geometry_jobs(const CaseStepJob* jobs, int n, cudaStream_t s) {
-    if (n <= 0) return cudaSuccess;
-    k_prep_geometry_jobs<<<n, 512, 0, s>>>(jobs);
+cudaError_t launch_prep_geometry_jobs(const CaseStepJob* jobs, int n, long long blocks, cudaStream_t s) {
+    if (n <= 0 || blocks <= 0) return cudaSuccess;
+    k_prep_geometry_jobs<<<static_cast<unsigned>(blocks), kGeometryThreads, 0, s>>>(jobs, n);
     return cudaGetLastError();
 }
 
@@ -269,13 +343,15 @@ __device__ void write_panel_records(const d3 (&pp)[4], double rc, double g, doub
     r.v[41] = static_cast<float>(wing);
     for (int k = kRec32DD + 4; k < 48; ++k) r.v[k] = 0.f;
     if (r64) {
-        const double la = sqrt(l2[0]), lb = sqrt(l2[1]), lc = sqrt(l2[2]), ld = sqrt(l2[3]);
+        const double la = sqrt_any(l2[0]), lb = sqrt_any(l2[1]), lc = sqrt_any(l2[2]), ld = sqrt_any(l2[3]);
         const double sp = (la + lb + lc + ld) * 0.5;
-        const double area = sqrt((sp - la) * (sp - lb) * (sp - lc) * (sp - ld));
+        const double area = sqrt_any((sp - la) * (sp - lb) * (sp - lc) * (sp - ld));
         const d3 n = normalize(cross(pp[2] - pp[0], pp[3] - pp[1]));
         const double t = fmax(la, lb) * far_field_ratio;
         const double ff2 = t * t;
-        for (int k = 0; k < 4; ++k) r.v[24 + k] = l2[k] > 0.0 ? static_cast<float>(1.0 / l2[k]) : 0.f;
+        double il2[4];
+        for (int k = 0; k < 4; ++k) il2[k] = rcp_any(l2[k]);
+        for (int k = 0; k < 4; ++k) r.v[24 + k] = l2[k] > 0.0 ? static_cast<float>(il2[k]) : 0.f;
         far_field_fields(ff2, c, &r.v[31], &r.v[kRec32FF2Lo], &r.v[kRec32FF2Band]);
         r.v[35] = static_cast<float>(area * kFourPiInv * kInv3Sqrt3);
         r.v[36] = static_cast<float>(n.x);
@@ -286,7 +362,7 @@ __device__ void write_panel_records(const d3 (&pp)[4], double rc, double g, doub
             q.v[3 * k] = pp[k].x;
             q.v[3 * k + 1] = pp[k].y;
             q.v[3 * k + 2] = pp[k].z;
-            q.v[12 + k] = 1.0 / l2[k];
+            q.v[12 + k] = il2[k];
         }
         q.v[16] = c.x;
         q.v[17] = c.y;
@@ -490,17 +566,6 @@ cudaError_t launch_wake_panels(const DevModel& m, const WakeBuffers& w, int shif
 // to the last job whose first block of that kind is at or before b (jobs [n] ascending in
 // each kind's first block), and runs that job's element at b's offset within it.
 // ---------------------------------------------------------------------------------------
-template <long long CaseStepJob::*First>
-__device__ inline int job_of_block(const CaseStepJob* jobs, int n, long long b) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].*First <= b) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
 __global__ void k_wake_advect_jobs(const CaseStepJob* jobs, int n) {
     const CaseStepJob& J = jobs[job_of_block<&CaseStepJob::blk_advect>(jobs, n, blockIdx.x)];
     const long long id = (blockIdx.x - J.blk_advect) * static_cast<long long>(kAdvectThreads) + threadIdx.x;

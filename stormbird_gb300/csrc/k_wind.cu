@@ -19,13 +19,15 @@ namespace sbgpu {
 
 namespace {
 
-__device__ double spectrum_value(const double* s, int n, double time) {
+// (out of line: with pow, log, atan and sin inlined wherever they are used the kernel was 195 KB of
+// code that each of its blocks fetched past)
+__device__ __noinline__ double spectrum_value(const double* s, int n, double time) {
     double out = 0.0;
     for (int i = 0; i < n; ++i) out += s[n + i] * sin(kTau * s[i] * time + s[2 * n + i]);
     return out;
 }
 
-__device__ double velocity_at_height(const WindDevice& w, double h) {
+__device__ __noinline__ double velocity_at_height(const WindDevice& w, double h) {
     if (w.vv_kind == 0) return w.vv_constant;
     if (w.vv_kind == 1) {
         const double f = w.power_factor > 0.0 ? pow(h / w.reference_height, w.power_factor) : 1.0;
@@ -67,8 +69,11 @@ __device__ T interpolate(double x, const double* xd, int n, Y&& y) {
     return two(xd[lo], xd[lo + 1], y(lo), y(lo + 1));
 }
 
+__device__ __noinline__ d3 turned(d3 v, double angle, d3 axis) { return rotate_around_axis(v, angle, axis); }
+__device__ __noinline__ double angle_between(d3 a, d3 b, d3 axis) { return signed_angle_between(a, b, axis); }
+
 __device__ d3 true_wind_direction(const WindDevice& w) {
-    return rotate_around_axis(w.zero, w.direction_coming_from, w.axis);
+    return turned(w.zero, w.direction_coming_from, w.axis);
 }
 
 __global__ void k_wind_freestream(WindDevice w, const d3* ctrl, const int* wing_of_line, int N, const d3* wake,
@@ -90,7 +95,7 @@ __global__ void k_wind_freestream(WindDevice w, const d3* ctrl, const int* wing_
         // apparent wind direction of the steady wind at 10 m
         const d3 location = 10.0 * w.up;
         const double vh = velocity_at_height(w, fmax(dot(location, w.up) - w.water_plane_height, 0.0));
-        const double direction = signed_angle_between(w.zero, vh * pdir + linear, w.axis);
+        const double direction = angle_between(w.zero, vh * pdir + linear, w.axis);
         const int wing = wing_of_line[i];
         const double hc = dot(p, w.up);
         const d3 vel = u;
@@ -105,7 +110,7 @@ __global__ void k_wind_freestream(WindDevice w, const d3* ctrl, const int* wing_
             const int m = static_cast<int>(r1 - r0);
             const double mag = interpolate<double>(hc, hs, m, [&](int k) { return ms[k]; });
             const double ang = interpolate<double>(hc, hs, m, [&](int k) { return as[k]; });
-            return mag * rotate_around_axis(vel, ang, w.up);
+            return mag * turned(vel, ang, w.up);
         };
         u = interpolate<d3>(direction, w.dirs, w.n_dirs, corrected);
     }
@@ -125,11 +130,11 @@ __global__ void k_controller_input(DevModel m, StepParams p, const d3* v, double
         const d3 u = v[i];
         const d3 span_dir = normalize(m.span_e[i] - m.span_s[i]);
         out[i] = len(u);
-        out[N + i] = len(u) > kMinPositive ? signed_angle_between(m.chord_global[i], u, span_dir) : 0.0;
+        out[N + i] = len(u) > kMinPositive ? angle_between(m.chord_global[i], u, span_dir) : 0.0;
         const int ws = m.wing_start[m.wing_of_line[i]];
         const d3 axis = normalize(m.span_e[ws] - m.span_s[ws]);
         const d3 chord_first = rotate_xyz(m.chord_not_rotated[ws], p.rotation);
-        out[2 * N + i] = signed_angle_between(chord_first, u, axis);
+        out[2 * N + i] = angle_between(chord_first, u, axis);
     }
 }
 

@@ -20,6 +20,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "sb_f64.cuh"
+
 namespace sbgpu {
 
 constexpr int kMaxWings = 64;
@@ -43,27 +45,37 @@ __host__ __device__ inline d3 operator*(double s, d3 a) { return {s * a.x, s * a
 __host__ __device__ inline d3 operator/(d3 a, double s) { return {a.x / s, a.y / s, a.z / s}; }
 __host__ __device__ inline double dot(d3 a, d3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __host__ __device__ inline double len2(d3 a) { return a.x * a.x + a.y * a.y + a.z * a.z; }
-__host__ __device__ inline double len(d3 a) { return sqrt(len2(a)); }
+// On the device by sb_f64.cuh: a square root there is 5 FP64 instructions and its out-of-line fallback, where
+// CUDA's inlines 9 and its own
+__host__ __device__ inline double len(d3 a) {
+#ifdef __CUDA_ARCH__
+    return sqrt_any(len2(a));
+#else
+    return sqrt(len2(a));
+#endif
+}
 __host__ __device__ inline d3 cross(d3 a, d3 b) {
     return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
 __host__ __device__ inline d3 normalize(d3 a) {
+#ifdef __CUDA_ARCH__
+    const double q = len2(a);
+    if (q > 0.0) {
+        const double r = rsqrt_any(q);
+        return {a.x * r, a.y * r, a.z * r};
+    }
+    return {0.0, 0.0, 0.0};
+#else
     double l = len(a);
     if (l > 0.0) return {a.x / l, a.y / l, a.z / l};
     return {0.0, 0.0, 0.0};
+#endif
 }
 __host__ __device__ inline d3 project(d3 a, d3 onto) {
     d3 n = normalize(onto);
     return n * dot(a, n);
 }
 __host__ __device__ inline double signum(double v) { return copysign(1.0, v); }
-
-// f64 value as a pair of floats: hi = the nearest float, lo = the nearest float of v - hi
-// (hi + lo carries about 48 significant bits)
-__device__ inline float2 split_f64(double v) {
-    const float h = __double2float_rn(v);
-    return make_float2(h, __double2float_rn(v - static_cast<double>(h)));
-}
 
 // Angle between two vectors, signed by the right-hand rule about `axis`
 // (stormath/src/spatial_vector/vector_math.rs:65-95).

@@ -21,7 +21,8 @@
 // Arguments outside the stated ranges are the caller's to keep on CUDA's functions.
 #pragma once
 
-#include "sb_device.cuh"
+#include <cstdint>
+#include <cuda_runtime.h>
 
 namespace sbgpu {
 
@@ -57,6 +58,12 @@ __device__ __forceinline__ double f32_to_f64(float v) {
 __device__ __forceinline__ double f32_to_f64_any(float v) {
     if ((__float_as_uint(v) & 0x7F800000u) == 0x7F800000u) return static_cast<double>(v);
     return f32_to_f64(v);
+}
+// f64 value as a pair of floats: hi = the nearest float, lo = the nearest float of v - hi
+// (hi + lo carries about 48 significant bits)
+__device__ inline float2 split_f64(double v) {
+    const float h = __double2float_rn(v);
+    return make_float2(h, __double2float_rn(v - static_cast<double>(h)));
 }
 // split_f64 with the conversions on the integer pipe where v allows
 __device__ __forceinline__ float2 split_f64_int(double v) {

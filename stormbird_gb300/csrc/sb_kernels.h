@@ -179,15 +179,16 @@ struct CaseStepJob {
     const d3* basis = nullptr;                // two-component split matrix (nullptr: three)
     ChainArgs chain;                          // chain records (chain_n = 0: none)
     long long chain_n = 0;
-    long long blk_advect = 0, blk_panels = 0, blk_matrix = 0, blk_chain = 0;
+    long long blk_geometry = 0, blk_advect = 0, blk_panels = 0, blk_matrix = 0, blk_chain = 0;
 };
 // Blocks a job needs per kind.
+long long prep_geometry_blocks(const DevModel& m);
 long long wake_advect_blocks(const DevModel& m);
 long long wake_panels_blocks(const DevModel& m);
 long long chain_records_blocks(long long n_build);
 long long unit_matrix_blocks(int N, bool fp32);
-// One CTA per job: the geometry of every case (k_prep_geometry).
-cudaError_t launch_prep_geometry_jobs(const CaseStepJob* jobs, int n, cudaStream_t s);
+// The geometry of every case (k_prep_geometry).
+cudaError_t launch_prep_geometry_jobs(const CaseStepJob* jobs, int n, long long blocks, cudaStream_t s);
 // Wake advection (with the last row) of every case, then its panel records with the strength
 // shift (k_wake_advect, k_wake_panels).
 cudaError_t launch_wake_jobs(const CaseStepJob* jobs, int n, long long advect_blocks, long long panel_blocks,
@@ -200,7 +201,7 @@ cudaError_t launch_panels_from_corners(const double* corners, const double* stre
                                        double far_field_ratio, PanelRec<float>* r32, PanelRec<double>* r64,
                                        cudaStream_t s);
 
-// ---- solver and forces (k_solve.cu) ----------------------------------------------------
+// ---- solvers (k_solve.cu, k_lin_refined.cu) ----------------------------------------------------
 struct SolveSettings {
     int max_iterations = 40;
     double damping = 0.05;
@@ -314,6 +315,7 @@ struct ForceArgs {
     int fd_count = 0;               // updates done so far
     double* out = nullptr;          // output block
     const double* scalars = nullptr;
+    unsigned* counter = nullptr;    // wings done in this launch: zero before, left zero
 };
 
 // Output block layout (doubles), N span lines, S wings.
@@ -382,15 +384,17 @@ void report_error(int code, const std::string& message);
 double measure_fp32_peak(int device, int reps);
 double measure_fp64_peak(int device, int reps);
 
+// ---- forces (k_forces.cu) --------------------------------------------------------------
 // Sectional and integrated forces (force_calculations.rs:322-452, 669-698;
 // forces_and_moments.rs:163-245; flow_derivatives.rs:31-63).
 cudaError_t launch_forces(const DevModel& m, const StepParams& p, const ForceArgs& f, cudaStream_t s);
-// The forces of every case of a batch in one launch (one CTA per case).
+// The forces of every case of a batch in one launch (one CTA per wing of each case).
 struct ForceJob {
     DevModel m;
     StepParams p;
     ForceArgs f;
+    int block_begin = 0;  // first CTA (wing) of the case in the launch
 };
-cudaError_t launch_forces_jobs(const ForceJob* jobs, int n, cudaStream_t s);
+cudaError_t launch_forces_jobs(const ForceJob* jobs, int n, int blocks, cudaStream_t s);
 
 }  // namespace sbgpu

@@ -556,6 +556,7 @@ struct sb_sim {
         }
         ck(cudaMemset(fixed.p, 0, N * sizeof(d3)), "memset");
         counters.alloc(4); err.alloc(4);
+        ck(cudaMemset(counters.p, 0, 4 * sizeof(unsigned long long)), "memset");
         ck(cudaMemset(err.p, 0, 4 * sizeof(int)), "memset");
         gamma_prev.alloc(N); gamma_tmp.alloc(N); scalars.alloc(8);
         ck(cudaMemset(gamma_prev.p, 0, N * sizeof(double)), "memset");
@@ -1040,6 +1041,7 @@ struct sb_sim {
         j.f.fd_count = fd_count;
         j.f.out = out.p;
         j.f.scalars = scalars.p;
+        j.f.counter = reinterpret_cast<unsigned*>(counters.p + 3);  // slots 0..2: the sweeps
         return j;
     }
 

@@ -702,7 +702,6 @@ struct sb_batch {
             h_feat.alloc(cases.size());
             d_feat.alloc(cases.size());
         }
-        if (mode == 1) mlp_reserve(m, N_total);
         mlp = mode == 1 ? m : nullptr;
         warm_mode = mode;
         warm_hist.assign(cases.size(), 0);

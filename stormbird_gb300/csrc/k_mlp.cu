@@ -19,12 +19,16 @@
 // bounded: a wait that runs out records kDevTimeout, skips the epilogue, waits (bounded)
 // for the copies and MMAs in flight and frees the tensor memory.
 //
+// k_mlp_forward: the whole network for inference, layers fused (see there).
+//
 // The rest are CUDA-core kernels: the width->1 output layer with the MSE loss, input
 // packing, deterministic fixed-order reductions, Adam, weight casts, and the batch-side
 // feature / candidate / target kernels of the warm start.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
+
+#include <algorithm>
 
 #include "sb_mlp.h"
 #include "sb_ptx.cuh"
@@ -256,6 +260,228 @@ __global__ void __launch_bounds__(kGemmThreads) k_mlp_gemm(const __grid_constant
     if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 
+// ---------------------------------------------------------------------------------------
+// Inference: the whole network for 128-row tiles in one persistent kernel, two tiles at a time on an SM.
+// The activations never leave it: a layer's epilogue writes the next layer's A operand (BF16,
+// 128-byte-swizzled K-major) over the one the tensor cores have just finished with. Roles (18
+// warps): one thread streams the weights by TMA in 128 x 64 half slabs through a ring of five, one
+// issues the MMAs, eight warps a tile drain its accumulator (tensor memory: two tiles x 256 FP32
+// columns); the two tiles take turns, so that one's MMAs and weights run under the other's epilogue.
+// With no more tiles than SMs all sixteen warps drain the one.
+// The epilogue is what bounds it: 1,024 GELUs a row with erff, 32 issued instructions each (98,307 rows: 85 us
+// at one per cycle and SM sub-partition), against 8,192 tensor-core FMAs a cycle. Results are those of
+// the layer-by-layer kernels bit for bit (the same K order in the accumulator, the same roundings,
+// the output layer's sums in k_mlp_head's order).
+// 98,307 rows: layer by layer (pack, four GEMMs, output layer; activations through L2 and HBM, each CTA's
+// epilogue after its main loop) 290 us a call, both tiles in step 187, in turn 174 us.
+constexpr int kFwdWarps = 16;
+constexpr int kFwdThreads = 32 * (kFwdWarps + 2);
+constexpr int kFwdRing = 5;
+constexpr uint32_t kFwdSub = 128 * kKStep * 2;   // a 128 x 64 BF16 sub-tile (A quarter or half slab)
+constexpr uint32_t kFwdTile = 4 * kFwdSub;       // activations of a tile
+constexpr int kFwdPartLd = 33;                   // row pitch of the output layer's partial sums
+constexpr uint32_t kFwdSmem = 2 * kFwdTile + kFwdRing * kFwdSub + (kMlpHidden * kMlpWidth + kMlpWidth + 4) * 4 + 1024;
+static_assert(128 * kFwdPartLd * 4 <= kFwdTile, "partial sums fit a tile's activations");
+
+struct FwdMaps {
+    CUtensorMap w[kMlpHidden];
+};
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+__global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const __grid_constant__ FwdMaps maps, FwdArgs g) {
+    extern __shared__ unsigned char dyn[];
+    unsigned char* act = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
+    unsigned char* ring = act + 2 * kFwdTile;
+    float* bias = reinterpret_cast<float*>(ring + kFwdRing * kFwdSub);  // [4][256]
+    float* wout = bias + kMlpHidden * kMlpWidth;                        // [257]
+    __shared__ __align__(8) uint64_t full[kFwdRing], empty[kFwdRing], acc_full[2], act_ready[2];
+    __shared__ uint32_t s_tmem;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+    const int tiles = (g.rows + 127) / 128, G = gridDim.x;
+    const bool wide = tiles <= G;  // one tile at a time
+    // tile k of slot q: the first slots of all CTAs, then the second ones
+    auto tile_of = [&](int k, int q) { return wide ? (q == 0 && k == 0 ? static_cast<int>(blockIdx.x) : tiles)
+                                                   : (2 * k + q) * G + static_cast<int>(blockIdx.x); };
+    if (warp == 0) tmem_alloc(&s_tmem, 512);
+    if (tid == 0) {
+        for (int s = 0; s < kFwdRing; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int q = 0; q < 2; ++q) {
+            mbar_init(&acc_full[q], 1);
+            mbar_init(&act_ready[q], wide ? kFwdWarps : kFwdWarps / 2);
+        }
+        fence_mbar_init();
+    }
+    for (int i = tid; i < kMlpHidden * kMlpWidth; i += kFwdThreads) bias[i] = g.bias[i / kMlpWidth][i % kMlpWidth];
+    for (int i = tid; i <= kMlpWidth; i += kFwdThreads) wout[i] = g.w_out[i];
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem;
+    // half slabs of layer l: 128 outputs x 64 inputs, the two halves of a slab after one another
+    auto halves = [](int l) { return l == 0 ? 2 * (kMlpInPad / kKStep) : 2 * (kMlpWidth / kKStep); };
+
+    if (warp == kFwdWarps) {
+        if (lane == 0) {  // weights
+            int n = 0;
+            bool ok = true;
+            for (int k = 0; tile_of(k, 0) < tiles && ok; ++k)
+                for (int l = 0; l < kMlpHidden && ok; ++l)
+                    for (int q = 0; q < 2 && tile_of(k, q) < tiles && ok; ++q)
+                        for (int h = 0; h < halves(l); ++h, ++n) {
+                            const int s = n % kFwdRing;
+                            if (n >= kFwdRing && !mbar_wait_bounded(&empty[s], (n / kFwdRing - 1) & 1, g.err)) {
+                                ok = false;
+                                break;
+                            }
+                            mbar_expect_tx(&full[s], kFwdSub);
+                            tma_load_2d(ring + s * kFwdSub, &maps.w[l], (h >> 1) * kKStep, (h & 1) * 128, &full[s]);
+                        }
+            // every copy has landed before the CTA leaves (those of a finished pass were waited for)
+            if (!ok)
+                for (int k = n - kFwdRing > 0 ? n - kFwdRing : 0; k < n; ++k)
+                    mbar_wait_bounded(&full[k % kFwdRing], (k / kFwdRing) & 1, g.err);
+        }
+    } else if (warp == kFwdWarps + 1) {
+        if (lane == 0) {  // MMAs
+            const uint32_t idesc = idesc_bf16(128, 128);
+            int n = 0, layer[2] = {0, 0};
+            bool ok = true;
+            for (int k = 0; tile_of(k, 0) < tiles && ok; ++k)
+                for (int l = 0; l < kMlpHidden && ok; ++l)
+                    for (int q = 0; q < 2 && tile_of(k, q) < tiles && ok; ++q) {
+                        if (!mbar_wait_bounded(&act_ready[q], layer[q] & 1, g.err)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        for (int h = 0; h < halves(l); ++h, ++n) {
+                            const int s = n % kFwdRing;
+                            if (!mbar_wait_bounded(&full[s], (n / kFwdRing) & 1, g.err)) {
+                                ok = false;
+                                break;
+                            }
+                            tc_fence_after();
+                            const uint32_t b = smem_u32(ring + s * kFwdSub);
+                            const uint32_t a = smem_u32(act + q * kFwdTile + (h >> 1) * kFwdSub);
+#pragma unroll
+                            for (int j = 0; j < kKStep / 16; ++j)
+                                mma_bf16(tmem + q * 256 + (h & 1) * 128, smem_desc_sw128(a + j * 32), smem_desc_sw128(b + j * 32),
+                                         idesc, (h > 1 || j > 0) ? 1u : 0u);
+                            mma_commit(&empty[s]);
+                        }
+                        mma_commit(&acc_full[q]);  // after a wait that ran out: of what was issued
+                        ++layer[q];
+                    }
+            // a commit arrives when every MMA before it is done: the last of both slots
+            for (int q = 0; q < 2; ++q)
+                if (layer[q] > 0) mbar_wait_bounded(&acc_full[q], (layer[q] - 1) & 1, g.err);
+        }
+    } else {
+        const int quad = warp & 3;          // tensor-memory lanes
+        const int row = quad * 32 + lane;   // of a tile
+        const int q = wide ? 0 : warp >> 3;                           // slot
+        const int part = wide ? warp >> 2 : (warp >> 2) & 1, parts = wide ? 4 : 2;  // of the tile's columns
+        const int width = kMlpWidth / parts;
+        const int meet = wide ? 32 * kFwdWarps : 16 * kFwdWarps;      // threads of the slot
+        const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quad * 32) << 16);
+        int layer = 0;
+        // a warp whose wait ran out works no more, but arrives and meets the others' barriers
+        bool ok = true;
+        for (int k = 0; tile_of(k, q) < tiles; ++k) {
+            unsigned char* a = act + q * kFwdTile;
+            const long long r = tile_of(k, q) * 128LL + row;
+            // A element (row, column): 64-column sub-tiles, rows of 128 bytes, 16-byte chunks XOR-ed with row mod 8
+            auto chunk = [&](int col) { return a + (col >> 6) * kFwdSub + row * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4); };
+            {  // inputs, BF16, zeros past n_in and past the last row
+                const float* x = g.x + r * g.n_in;
+                for (int c = part * (kMlpInPad / parts); c < (part + 1) * (kMlpInPad / parts); c += 8) {
+                    float v[8];
+                    if (g.vec_x && r < g.rows && c + 8 <= g.n_in) {
+                        const float4 u0 = *reinterpret_cast<const float4*>(x + c), u1 = *reinterpret_cast<const float4*>(x + c + 4);
+                        v[0] = u0.x; v[1] = u0.y; v[2] = u0.z; v[3] = u0.w;
+                        v[4] = u1.x; v[5] = u1.y; v[6] = u1.z; v[7] = u1.w;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) v[j] = (r < g.rows && c + j < g.n_in) ? x[c + j] : 0.f;
+                    }
+                    __nv_bfloat162 p[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) p[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                    *reinterpret_cast<uint4*>(chunk(c)) = *reinterpret_cast<uint4*>(p);
+                }
+            }
+#pragma unroll 1
+            for (int l = 0; l < kMlpHidden; ++l, ++layer) {
+                // the operand is written (and the accumulator read): the tensor cores may start
+                tc_fence_before();
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&act_ready[q]);
+                if (ok && !mbar_wait_bounded(&acc_full[q], layer & 1, g.err)) ok = false;
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) continue;
+                tc_fence_after();
+                const float* bl = bias + l * kMlpWidth;
+#pragma unroll 1
+                for (int c0 = part * width; c0 < (part + 1) * width; c0 += 32) {
+                    float v[32];
+                    tmem_ld32(lane_addr + static_cast<uint32_t>(q * 256 + c0), v);
+#pragma unroll
+                    for (int j = 0; j < 32; j += 4) {
+                        const float4 b4 = *reinterpret_cast<const float4*>(bl + c0 + j);
+                        v[j] = gelu(v[j] + b4.x);
+                        v[j + 1] = gelu(v[j + 1] + b4.y);
+                        v[j + 2] = gelu(v[j + 2] + b4.z);
+                        v[j + 3] = gelu(v[j + 3] + b4.w);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; j += 8) {
+                        __nv_bfloat162 p[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(v[j + 2 * i], v[j + 2 * i + 1]);
+                        if (l + 1 < kMlpHidden) {
+                            *reinterpret_cast<uint4*>(chunk(c0 + j)) = *reinterpret_cast<uint4*>(p);
+                        } else {  // output layer: the partial sum of these 8 columns
+                            float s = 0.f;
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const float2 f = __bfloat1622float2(p[i]);
+                                s = fmaf(f.x, wout[c0 + j + 2 * i], s);
+                                s = fmaf(f.y, wout[c0 + j + 2 * i + 1], s);
+                            }
+                            reinterpret_cast<float*>(a)[row * kFwdPartLd + ((c0 + j) >> 3)] = s;
+                        }
+                    }
+                }
+            }
+            // a row's 32 partial sums in the order of a butterfly over 32 lanes
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + q), "r"(meet) : "memory");
+            if (ok && part == 0 && r < g.rows) {
+                const float* p = reinterpret_cast<const float*>(a) + row * kFwdPartLd;
+                float s[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) s[i] = p[i] + p[i + 16];
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < o; ++i) s[i] += s[i + o];
+                g.y[r] = s[0] + wout[kMlpWidth];
+            }
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + q), "r"(meet) : "memory");
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
 __global__ void __launch_bounds__(32 * kHeadRowsPerCta) k_mlp_head(HeadArgs a) {
     __shared__ float wacc[kHeadRowsPerCta][kMlpWidth + 2];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -278,10 +504,6 @@ __global__ void __launch_bounds__(32 * kHeadRowsPerCta) k_mlp_head(HeadArgs a) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     const float y = s + a.w[kMlpWidth];
-    if (!a.target) {
-        if (lane == 0 && r < a.rows) a.y[r] = y;
-        return;
-    }
     const float res = r < a.rows ? y - a.target[r] : 0.f;
     const float dy = 2.f * res * a.inv_n;
     const float4* zp = reinterpret_cast<const float4*>(a.z + static_cast<long long>(r) * kMlpWidth + f0);
@@ -455,6 +677,9 @@ unsigned blocks_for(long long n, int t) { return static_cast<unsigned>((n + t - 
 size_t mlp_gemm_smem_bytes() { return kStages * static_cast<size_t>(kStage) + 1024; }
 
 cudaError_t configure_mlp_gemm() {
+    const cudaError_t e = cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(kFwdSmem));
+    if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(k_mlp_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(mlp_gemm_smem_bytes()));
 }
@@ -502,6 +727,20 @@ cudaError_t launch_mlp_gemm(const GemmArgs& g, cudaStream_t s) {
         return cudaErrorInvalidValue;
     const int splits = (g.K + g.k_split - 1) / g.k_split;
     k_mlp_gemm<<<dim3(g.M / kMlpRowTile, splits), kGemmThreads, mlp_gemm_smem_bytes(), s>>>(ma, mb, g);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_mlp_forward(const FwdArgs& args, cudaStream_t s) {
+    if (args.rows <= 0) return cudaSuccess;
+    FwdArgs g = args;
+    g.vec_x = g.n_in % 4 == 0 && reinterpret_cast<uintptr_t>(g.x) % 16 == 0 ? 1 : 0;
+    FwdMaps maps;
+    for (int l = 0; l < kMlpHidden; ++l) {
+        const int in = l == 0 ? kMlpInPad : kMlpWidth;
+        if (!encode_bf16_map(&maps.w[l], g.w[l], kMlpWidth, in, in, 128)) return cudaErrorInvalidValue;
+    }
+    const int tiles = (g.rows + 127) / 128;
+    k_mlp_forward<<<std::min(tiles, std::max(1, g.sms)), kFwdThreads, kFwdSmem, s>>>(maps, g);
     return cudaGetLastError();
 }
 

@@ -26,11 +26,10 @@ struct sb_mlp {
     int in_dim[kMlpHidden] = {0};
     DevBuf<float> params, grads, adam_m, adam_v;
     DevBuf<bf16> Wb[kMlpHidden], WbT[kMlpHidden];
-    int cap = 0;   // rows the activation buffers hold (multiple of 128)
-    bool cap_train = false;
+    int cap = 0;   // rows the training buffers hold (multiple of 128)
+    int sms = 1;
     DevBuf<bf16> X0, X0T, H[kMlpHidden], HT[kMlpHidden], DZ[kMlpHidden], DZT[kMlpHidden];
     DevBuf<float> Z[kMlpHidden], part, head_part, loss;
-    DevBuf<float> y_tmp, t_tmp;
     DevBuf<int> err;
     PinnedBuf<float> h_loss;
     PinnedBuf<int> h_err;
@@ -46,6 +45,7 @@ struct sb_mlp {
         device = dev;
         n_in = n_inputs;
         ck(cudaSetDevice(device), "cudaSetDevice");
+        sms = num_sms(device);
         ck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
         long long at = 0;
         for (int l = 0; l < kMlpHidden; ++l) {
@@ -113,28 +113,25 @@ struct sb_mlp {
         return static_cast<int>(((rows + kMlpRowTile - 1) / kMlpRowTile) * kMlpRowTile);
     }
 
-    // Activation buffers for `rows` rows (allocation: call outside any stream capture).
-    void ensure(long long rows, bool train) {
+    // Buffers of a training step of `rows` rows (inference keeps its activations on the SMs).
+    void ensure(long long rows) {
         const int need = pad_rows(std::max<long long>(rows, 1));
-        if (need <= cap && (!train || cap_train)) return;
-        const int c = std::max(need, cap);
-        const size_t w = static_cast<size_t>(c) * kMlpWidth;
-        X0.alloc(static_cast<size_t>(c) * kMlpInPad);
+        if (need <= cap) return;
+        const size_t w = static_cast<size_t>(need) * kMlpWidth;
+        X0.alloc(static_cast<size_t>(need) * kMlpInPad);
+        X0T.alloc(static_cast<size_t>(need) * kMlpInPad);
         for (int l = 0; l < kMlpHidden; ++l) {
             H[l].alloc(w);
-            Z[l].alloc(train ? w : 0);
-            HT[l].alloc(train ? w : 0);
-            DZ[l].alloc(train ? w : 0);
-            DZT[l].alloc(train ? w : 0);
+            Z[l].alloc(w);
+            HT[l].alloc(w);
+            DZ[l].alloc(w);
+            DZT[l].alloc(w);
         }
-        X0T.alloc(train ? static_cast<size_t>(c) * kMlpInPad : 0);
-        head_part.alloc(train ? static_cast<size_t>(c / kHeadRowsPerCta) * (kMlpWidth + 2) : 0);
+        head_part.alloc(static_cast<size_t>(need / kHeadRowsPerCta) * (kMlpWidth + 2));
         // split-K over the batch rows for the weight gradients: about one wave of CTAs
-        splits = std::max(1, std::min(c / 64, 76));
-        part.alloc(train ? static_cast<size_t>(splits) * kMlpWidth * kMlpWidth : 0);
-        y_tmp.alloc(static_cast<size_t>(c));
-        cap = c;
-        cap_train = train;
+        splits = std::max(1, std::min(need / 64, 76));
+        part.alloc(static_cast<size_t>(splits) * kMlpWidth * kMlpWidth);
+        cap = need;
     }
 
     GemmArgs gemm(const bf16* A, long long lda, const bf16* B, long long ldb, int M, int N, int K, int mode) const {
@@ -152,20 +149,39 @@ struct sb_mlp {
         return g;
     }
 
-    // Forward pass over rows of x [rows][n_in] (device). Inference writes y [rows]; training
-    // (target != nullptr) keeps what the backward pass needs.
-    void forward(const float* x, long long rows, float* y, const float* target, cudaStream_t s) {
-        const bool train = target != nullptr;
+    // Inference over rows of x [rows][n_in] (device) into y [rows].
+    void forward(const float* x, long long rows, float* y, cudaStream_t s) {
+        FwdArgs g;
+        g.x = x;
+        g.n_in = n_in;
+        for (int l = 0; l < kMlpHidden; ++l) {
+            g.w[l] = Wb[l].p;
+            g.bias[l] = params.p + off_b[l];
+        }
+        g.w_out = params.p + off_out;
+        g.sms = sms;
+        g.err = err.p;
+        constexpr long long kPass = 1 << 30;  // rows per launch (row numbers of a launch are int)
+        for (long long r0 = 0; r0 < rows; r0 += kPass) {
+            g.x = x + r0 * n_in;
+            g.y = y + r0;
+            g.rows = static_cast<int>(std::min(kPass, rows - r0));
+            ck(launch_mlp_forward(g, s), "network");
+        }
+    }
+
+    // Forward pass of a training step: keeps what the backward pass needs.
+    void forward_train(const float* x, long long rows, const float* target, cudaStream_t s) {
         const int R = pad_rows(rows);
-        ck(launch_mlp_pack(x, static_cast<int>(rows), n_in, R, X0.p, train ? X0T.p : nullptr, s), "pack inputs");
+        ck(launch_mlp_pack(x, static_cast<int>(rows), n_in, R, X0.p, X0T.p, s), "pack inputs");
         const bf16* in = X0.p;
         long long ld = kMlpInPad;
         for (int l = 0; l < kMlpHidden; ++l) {
             GemmArgs g = gemm(in, ld, Wb[l].p, in_dim[l], R, kMlpWidth, in_dim[l], kGemmForward);
             g.bias = params.p + off_b[l];
-            g.z_out = train ? Z[l].p : nullptr;
+            g.z_out = Z[l].p;
             g.h_out = H[l].p;
-            g.hT_out = train ? HT[l].p : nullptr;
+            g.hT_out = HT[l].p;
             g.ldt = R;
             ck(launch_mlp_gemm(g, s), "forward GEMM");
             in = H[l].p;
@@ -173,15 +189,14 @@ struct sb_mlp {
         }
         HeadArgs h;
         h.h = H[kMlpHidden - 1].p;
-        h.z = train ? Z[kMlpHidden - 1].p : nullptr;
+        h.z = Z[kMlpHidden - 1].p;
         h.w = params.p + off_out;
         h.target = target;
         h.rows = static_cast<int>(rows);
         h.rows_pad = R;
-        h.y = y;
-        h.dz = train ? DZ[kMlpHidden - 1].p : nullptr;
-        h.dzT = train ? DZT[kMlpHidden - 1].p : nullptr;
-        h.part = train ? head_part.p : nullptr;
+        h.dz = DZ[kMlpHidden - 1].p;
+        h.dzT = DZT[kMlpHidden - 1].p;
+        h.part = head_part.p;
         h.inv_n = 1.f / static_cast<float>(std::max<long long>(rows, 1));
         ck(launch_mlp_head(h, s), "output layer");
     }
@@ -247,9 +262,8 @@ struct sb_mlp {
 
 namespace sbhost {
 int mlp_inputs(const sb_mlp* m) { return m->n_in; }
-void mlp_reserve(sb_mlp* m, long long rows) { m->ensure(rows, m->cap_train); }
 void mlp_forward_async(sb_mlp* m, const float* x, long long rows, float* y, cudaStream_t s) {
-    m->forward(x, rows, y, nullptr, s);
+    m->forward(x, rows, y, s);
 }
 void mlp_check(sb_mlp* m) {
     ck(cudaDeviceSynchronize(), "network");
@@ -308,9 +322,8 @@ int sb_mlp_forward(sb_mlp* m, const float* x_dev, size_t rows, float* y_dev) {
     if (!m || (rows && (!x_dev || !y_dev))) return null_arg();
     if (rows == 0) return SB_OK;
     return guard([&] {
-        m->ensure(static_cast<long long>(rows), m->cap_train);
         order_after_caller(m->stream);
-        m->forward(x_dev, static_cast<long long>(rows), y_dev, nullptr, m->stream);
+        m->forward(x_dev, static_cast<long long>(rows), y_dev, m->stream);
         m->check_err(m->stream);
     });
 }
@@ -323,9 +336,9 @@ int sb_mlp_gradients(sb_mlp* m, const float* x_dev, const float* target_dev, siz
         return SB_ERR_SIZE;
     }
     return guard([&] {
-        m->ensure(static_cast<long long>(rows), true);
+        m->ensure(static_cast<long long>(rows));
         order_after_caller(m->stream);
-        m->forward(x_dev, static_cast<long long>(rows), m->y_tmp.p, target_dev, m->stream);
+        m->forward_train(x_dev, static_cast<long long>(rows), target_dev, m->stream);
         m->backward(static_cast<long long>(rows), m->stream);
         ck(cudaMemcpyAsync(grads_host, m->grads.p, m->n_params * sizeof(float), cudaMemcpyDeviceToHost, m->stream),
            "D2H gradients");
@@ -342,9 +355,9 @@ int sb_mlp_train_step(sb_mlp* m, const float* x_dev, const float* target_dev, si
         return SB_ERR_SIZE;
     }
     return guard([&] {
-        m->ensure(static_cast<long long>(rows), true);
+        m->ensure(static_cast<long long>(rows));
         order_after_caller(m->stream);
-        m->forward(x_dev, static_cast<long long>(rows), m->y_tmp.p, target_dev, m->stream);
+        m->forward_train(x_dev, static_cast<long long>(rows), target_dev, m->stream);
         m->backward(static_cast<long long>(rows), m->stream);
         m->adam(learning_rate, m->stream);
         // the inputs are read by the time the call returns (the caller may reuse them)

@@ -47,8 +47,20 @@ size_t mlp_gemm_smem_bytes();
 cudaError_t configure_mlp_gemm();
 cudaError_t launch_mlp_gemm(const GemmArgs& g, cudaStream_t s);
 
-// Output layer (width -> 1) on the CUDA cores. Inference: y[r] = h[r] . w + w[width].
-// Training (target != nullptr): MSE residuals, dz of the last hidden layer (row-major and
+// Inference: y[r] = the network at row r of x [rows][n_in] (k_mlp_forward).
+struct FwdArgs {
+    const float* x = nullptr;
+    int rows = 0, n_in = 0, vec_x = 0;        // vec_x: set by the launch
+    const bf16* w[kMlpHidden] = {nullptr};    // [256][64], then [256][256]
+    const float* bias[kMlpHidden] = {nullptr};
+    const float* w_out = nullptr;             // [257]
+    float* y = nullptr;
+    int sms = 1;
+    int* err = nullptr;
+};
+cudaError_t launch_mlp_forward(const FwdArgs& g, cudaStream_t s);
+
+// Output layer (width -> 1) of a training pass on the CUDA cores: MSE residuals, dz of the last hidden layer (row-major and
 // transposed) and per-CTA partials [grid][width + 2] of (dw, db, sum of squared residuals).
 struct HeadArgs {
     const bf16* h = nullptr;
@@ -56,7 +68,6 @@ struct HeadArgs {
     const float* w = nullptr;   // [width + 1]
     const float* target = nullptr;
     int rows = 0, rows_pad = 0;
-    float* y = nullptr;
     bf16* dz = nullptr;
     bf16* dzT = nullptr;
     float* part = nullptr;
@@ -117,8 +128,6 @@ cudaError_t launch_batch_targets(const double* gamma_new, const double* q, const
 struct sb_mlp;
 namespace sbhost {
 int mlp_inputs(const sb_mlp* m);
-// Buffers for `rows` inference rows (allocates: call outside any stream capture).
-void mlp_reserve(sb_mlp* m, long long rows);
 // y [rows] = network(x [rows][inputs]) enqueued on s (no synchronisation).
 void mlp_forward_async(sb_mlp* m, const float* x, long long rows, float* y, cudaStream_t s);
 // Throws when a bounded wait in the network's kernels ran out (synchronises the device).

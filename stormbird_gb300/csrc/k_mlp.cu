@@ -45,6 +45,7 @@ constexpr uint32_t kStageA = kMlpRowTile * kKStep * 2;
 constexpr uint32_t kStageB = kMlpWidth * kKStep * 2;
 constexpr uint32_t kStage = kStageA + kStageB;
 constexpr uint32_t kTmemCols = 256;
+constexpr int kTurnLd = 36;  // floats of a row of a warp's 32 x 32 turning tile
 static_assert(kStageA % 1024 == 0 && kStage % 1024 == 0, "stages keep the 1024-byte swizzle alignment");
 
 // tcgen05 shared-memory matrix descriptor of a K-major 128-byte-swizzled tile: start
@@ -115,17 +116,6 @@ __device__ __forceinline__ float gelu_grad(float z) {
     return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
-__device__ __forceinline__ void store_bf16x32(bf16* dst, const float (&v)[32]) {
-    uint4* d = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        __nv_bfloat162 p[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) p[j] = __floats2bfloat162_rn(v[q * 8 + 2 * j], v[q * 8 + 2 * j + 1]);
-        d[q] = *reinterpret_cast<uint4*>(p);
-    }
-}
-
 __global__ void __launch_bounds__(kGemmThreads) k_mlp_gemm(const __grid_constant__ CUtensorMap map_a,
                                                            const __grid_constant__ CUtensorMap map_b, GemmArgs g) {
     extern __shared__ unsigned char dyn[];
@@ -137,6 +127,10 @@ __global__ void __launch_bounds__(kGemmThreads) k_mlp_gemm(const __grid_constant
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * kMlpRowTile;
     const int split = blockIdx.y;
+    // gridDim.z CTAs share a row tile's columns (two while there are no more tiles than SMs, as with the 128
+    // tiles of 16,384 training rows: the epilogue takes most of the time, and two CTAs of an SM overlap the one's
+    // with the other's main loop: forward 20 us at one, 18 at two)
+    const int cols = g.N / gridDim.z, n0 = blockIdx.z * cols;
     const int k_begin = split * g.k_split;
     const int k_end = min(g.K, k_begin + g.k_split);
     const int nk = (k_end - k_begin) / kKStep;
@@ -155,14 +149,14 @@ __global__ void __launch_bounds__(kGemmThreads) k_mlp_gemm(const __grid_constant
     const uint32_t tmem = s_tmem;
 
     if (tid == 0) {
-        const uint32_t idesc = idesc_bf16(kMlpRowTile, g.N);
-        const uint32_t tx = kStageA + static_cast<uint32_t>(g.N) * kKStep * 2;
+        const uint32_t idesc = idesc_bf16(kMlpRowTile, cols);
+        const uint32_t tx = kStageA + static_cast<uint32_t>(cols) * kKStep * 2;
         auto load = [&](int kt) {
             const int s = kt % kStages;
             unsigned char* sa = base + s * kStage;
             mbar_expect_tx(&full[s], tx);
             tma_load_2d(sa, &map_a, k_begin + kt * kKStep, m0, &full[s]);
-            tma_load_2d(sa + kStageA, &map_b, k_begin + kt * kKStep, 0, &full[s]);
+            tma_load_2d(sa + kStageA, &map_b, k_begin + kt * kKStep, n0, &full[s]);
         };
         int loaded = 0;  // K steps whose copies were issued
         for (; loaded < min(nk, kStages); ++loaded) load(loaded);
@@ -217,42 +211,91 @@ __global__ void __launch_bounds__(kGemmThreads) k_mlp_gemm(const __grid_constant
         const int quad = warp & 3, half = warp >> 2;
         const int row = m0 + quad * 32 + lane;
         const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quad * 32) << 16);
-        const int c_end = (half + 1) * (g.N / 2);
-        for (int c0 = half * (g.N / 2); c0 < c_end; c0 += 32) {
-            float v[32];
-            tmem_ld32(lane_addr + static_cast<uint32_t>(c0), v);
-            if (g.mode == kGemmPartial) {
-                float4* o = reinterpret_cast<float4*>(g.part_out + (static_cast<long long>(split) * g.M + row) * g.N + c0);
+        const int c_end = n0 + (half + 1) * (cols / 2);
+        // The operands are done with: their shared memory turns rows per lane into rows per warp, so that
+        // a store (or load) instruction covers whole 64- or 128-byte pieces of rows (at 16,384 x 256, a lane
+        // storing its own row and 2-byte columns: forward 20.7 us, backward 21.3; now 16.3 and 17.6, bound by
+        // the error function's instructions). FP32: 32 x 32 values,
+        // rows padded to 36; BF16: 64-byte rows of four 16-byte chunks, XOR-ed so that rows written by
+        // lanes, rows read four lanes to one and columns read by ldmatrix all hit distinct banks.
+        float* tf = reinterpret_cast<float*>(base) + warp * (32 * kTurnLd + 32 * 16);
+        unsigned char* tb = reinterpret_cast<unsigned char*>(tf + 32 * kTurnLd);
+        auto chunk = [&](int r, int c) { return tb + r * 64 + ((c ^ ((r >> 1) & 3) ^ ((r >> 3) & 3)) << 4); };
+        const int r8 = lane >> 3, c8 = (lane & 7) * 4;
+        for (int c0 = n0 + half * (cols / 2); c0 < c_end; c0 += 32) {
+            // element (row r8 + 4 q, column c8) of the FP32 tile in memory
+            const long long at = static_cast<long long>(m0 + quad * 32 + r8) * g.N + c0 + c8;
+            if (g.mode == kGemmBackward) {
+                float4 z[8];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                continue;
+                for (int q = 0; q < 8; ++q) z[q] = *reinterpret_cast<const float4*>(g.z_in + at + 4 * q * g.N);
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 8; ++q) *reinterpret_cast<float4*>(tf + (r8 + 4 * q) * kTurnLd + c8) = z[q];
+                __syncwarp();
             }
-            if (g.mode == kGemmForward) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] += g.bias[c0 + j];
-                if (g.z_out) {
-                    float4* o = reinterpret_cast<float4*>(g.z_out + static_cast<long long>(row) * g.N + c0);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                }
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = gelu(v[j]);
-            } else {  // backward through the GELU of the layer below
-                const float4* zi = reinterpret_cast<const float4*>(g.z_in + static_cast<long long>(row) * g.N + c0);
+            float v[32];
+            tmem_ld32(lane_addr + static_cast<uint32_t>(c0 - n0), v);
+            float* mine = tf + lane * kTurnLd;
+            if (g.mode == kGemmBackward) {  // through the GELU of the layer below
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    const float4 z = zi[q];
+                    const float4 z = *reinterpret_cast<const float4*>(mine + 4 * q);
                     v[4 * q] *= gelu_grad(z.x);
                     v[4 * q + 1] *= gelu_grad(z.y);
                     v[4 * q + 2] *= gelu_grad(z.z);
                     v[4 * q + 3] *= gelu_grad(z.w);
                 }
-            }
-            if (g.h_out) store_bf16x32(g.h_out + static_cast<long long>(row) * g.N + c0, v);
-            if (g.hT_out) {
+            } else {
+                if (g.mode == kGemmForward) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) g.hT_out[static_cast<long long>(c0 + j) * g.ldt + row] = __float2bfloat16_rn(v[j]);
+                    for (int j = 0; j < 32; j += 4) {
+                        const float4 b4 = *reinterpret_cast<const float4*>(g.bias + c0 + j);
+                        v[j] += b4.x;
+                        v[j + 1] += b4.y;
+                        v[j + 2] += b4.z;
+                        v[j + 3] += b4.w;
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    *reinterpret_cast<float4*>(mine + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                __syncwarp();
+                float* o = g.mode == kGemmPartial ? g.part_out + static_cast<long long>(split) * g.M * g.N : g.z_out;
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    *reinterpret_cast<float4*>(o + at + 4 * q * g.N) = *reinterpret_cast<const float4*>(tf + (r8 + 4 * q) * kTurnLd + c8);
+                if (g.mode == kGemmPartial) continue;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = gelu(v[j]);
             }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                __nv_bfloat162 p[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) p[j] = __floats2bfloat162_rn(v[q * 8 + 2 * j], v[q * 8 + 2 * j + 1]);
+                *reinterpret_cast<uint4*>(chunk(lane, q)) = *reinterpret_cast<uint4*>(p);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int rr = 8 * q + (lane >> 2);
+                *reinterpret_cast<uint4*>(g.h_out + static_cast<long long>(m0 + quad * 32 + rr) * g.N + c0 + (lane & 3) * 8) =
+                    *reinterpret_cast<const uint4*>(chunk(rr, lane & 3));
+            }
+            // transposed: with row 8 t + 2 m + e as row 2 t + e of matrix m, lane 4 c + t of a transposed
+            // ldmatrix gets rows 8 t .. 8 t + 7 of column c, 16 bytes of a row of the transpose
+            const int lr = 8 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                uint4 w;
+                asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(smem_u32(chunk(lr, q))) : "memory");
+                *reinterpret_cast<uint4*>(g.hT_out + static_cast<long long>(c0 + 8 * q + (lane >> 2)) * g.ldt + m0 + quad * 32 +
+                                          (lane & 3) * 8) = w;
+            }
+            __syncwarp();
         }
     }
     tc_fence_before();
@@ -482,78 +525,167 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const __grid_con
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
+// A CTA takes kHeadGroups groups of kHeadRowsPerCta rows, a warp per row of a group; each group has its own
+// partial sums (the sums over groups then add them in group order, k_mlp_head_sums). dz goes out
+// transposed through shared memory: 64 bytes of a column's rows at a time (with 8 rows a CTA its
+// 2-byte stores made the kernel 43 us at 16,384 rows).
 __global__ void __launch_bounds__(32 * kHeadRowsPerCta) k_mlp_head(HeadArgs a) {
+    constexpr int kRows = kHeadGroups * kHeadRowsPerCta;
     __shared__ float wacc[kHeadRowsPerCta][kMlpWidth + 2];
+    __shared__ __align__(16) bf16 dzs[kRows][kMlpWidth + 8];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int r = blockIdx.x * kHeadRowsPerCta + warp;  // < rows_pad
     const int f0 = lane * 8;
-    float hv[8];
-    {
-        const uint4 raw = *reinterpret_cast<const uint4*>(a.h + static_cast<long long>(r) * kMlpWidth + f0);
-        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    float w8[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 f = __bfloat1622float2(p[j]);
-            hv[2 * j] = f.x;
-            hv[2 * j + 1] = f.y;
+    for (int j = 0; j < 8; ++j) w8[j] = a.w[f0 + j];
+#pragma unroll 1
+    for (int gr = 0; gr < kHeadGroups; ++gr) {
+        const int lr = gr * kHeadRowsPerCta + warp;
+        const int r = blockIdx.x * kRows + lr;  // < rows_pad
+        float hv[8];
+        {
+            const uint4 raw = *reinterpret_cast<const uint4*>(a.h + static_cast<long long>(r) * kMlpWidth + f0);
+            const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 f = __bfloat1622float2(p[j]);
+                hv[2 * j] = f.x;
+                hv[2 * j + 1] = f.y;
+            }
+        }
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s = fmaf(hv[j], w8[j], s);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const float y = s + a.w[kMlpWidth];
+        const float res = r < a.rows ? y - a.target[r] : 0.f;
+        const float dy = 2.f * res * a.inv_n;
+        const float4* zp = reinterpret_cast<const float4*>(a.z + static_cast<long long>(r) * kMlpWidth + f0);
+        const float4 z0 = zp[0], z1 = zp[1];
+        const float zz[8] = {z0.x, z0.y, z0.z, z0.w, z1.x, z1.y, z1.z, z1.w};
+        float dz[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) dz[j] = dy * w8[j] * gelu_grad(zz[j]);
+        __nv_bfloat162 pk[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) pk[j] = __floats2bfloat162_rn(dz[2 * j], dz[2 * j + 1]);
+        *reinterpret_cast<uint4*>(a.dz + static_cast<long long>(r) * kMlpWidth + f0) = *reinterpret_cast<uint4*>(pk);
+        *reinterpret_cast<uint4*>(&dzs[lr][f0]) = *reinterpret_cast<uint4*>(pk);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) wacc[warp][f0 + j] = dy * hv[j];
+        if (lane == 0) {
+            wacc[warp][kMlpWidth] = dy;
+            wacc[warp][kMlpWidth + 1] = res * res;
+        }
+        __syncthreads();
+        for (int i = tid; i < kMlpWidth + 2; i += blockDim.x) {
+            float t = 0.f;
+            for (int w = 0; w < kHeadRowsPerCta; ++w) t += wacc[w][i];
+            a.part[(static_cast<long long>(blockIdx.x) * kHeadGroups + gr) * (kMlpWidth + 2) + i] = t;
+        }
+        __syncthreads();
+    }
+    // column c = tid of the tile's rows, 16 bytes (8 rows) a store
+    for (int c = tid; c < kMlpWidth; c += blockDim.x) {
+        bf16* o = a.dzT + static_cast<long long>(c) * a.rows_pad + blockIdx.x * kRows;
+#pragma unroll
+        for (int k = 0; k < kRows; k += 8) {
+            __align__(16) bf16 v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = dzs[k + j][c];
+            *reinterpret_cast<uint4*>(o + k) = *reinterpret_cast<uint4*>(v);
         }
     }
-    float s = 0.f;
+}
+
+// Output layer's gradient and the loss: the groups' partial sums added in group order (one chain per
+// column), 32 columns a CTA. Eight warps copy the next 128 groups into shared memory while the first
+// adds the present ones (one thread per column with a global load per addition took 143 us at 2,048 groups).
+constexpr int kSumRows = 128;
+__global__ void __launch_bounds__(256) k_mlp_head_sums(const float* part, int groups, float* grad, float* loss) {
+    constexpr int kCols = kMlpWidth + 2;
+    __shared__ float buf[2][kSumRows][32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int col = blockIdx.x * 32 + lane;
+    float v[kSumRows / 8];
+    auto fetch = [&](int g0) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s = fmaf(hv[j], a.w[f0 + j], s);
+        for (int q = 0; q < kSumRows / 8; ++q) {
+            const int g = g0 + warp + 8 * q;
+            v[q] = g < groups && col < kCols ? part[static_cast<long long>(g) * kCols + col] : 0.f;
+        }
+    };
+    auto put = [&](int b) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const float y = s + a.w[kMlpWidth];
-    const float res = r < a.rows ? y - a.target[r] : 0.f;
-    const float dy = 2.f * res * a.inv_n;
-    const float4* zp = reinterpret_cast<const float4*>(a.z + static_cast<long long>(r) * kMlpWidth + f0);
-    const float4 z0 = zp[0], z1 = zp[1];
-    const float zz[8] = {z0.x, z0.y, z0.z, z0.w, z1.x, z1.y, z1.z, z1.w};
-    float dz[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) dz[j] = dy * a.w[f0 + j] * gelu_grad(zz[j]);
-    __nv_bfloat162 pk[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) pk[j] = __floats2bfloat162_rn(dz[2 * j], dz[2 * j + 1]);
-    *reinterpret_cast<uint4*>(a.dz + static_cast<long long>(r) * kMlpWidth + f0) = *reinterpret_cast<uint4*>(pk);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) a.dzT[static_cast<long long>(f0 + j) * a.rows_pad + r] = __float2bfloat16_rn(dz[j]);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) wacc[warp][f0 + j] = dy * hv[j];
-    if (lane == 0) {
-        wacc[warp][kMlpWidth] = dy;
-        wacc[warp][kMlpWidth + 1] = res * res;
-    }
+        for (int q = 0; q < kSumRows / 8; ++q) buf[b][warp + 8 * q][lane] = v[q];
+    };
+    fetch(0);
+    put(0);
     __syncthreads();
-    for (int i = tid; i < kMlpWidth + 2; i += blockDim.x) {
-        float t = 0.f;
-        for (int w = 0; w < kHeadRowsPerCta; ++w) t += wacc[w][i];
-        a.part[static_cast<long long>(blockIdx.x) * (kMlpWidth + 2) + i] = t;
+    float t = 0.f;
+    int b = 0;
+    for (int g0 = 0; g0 < groups; g0 += kSumRows, b ^= 1) {
+        fetch(g0 + kSumRows);
+        if (warp == 0) {
+            const int n = min(kSumRows, groups - g0);
+#pragma unroll 16
+            for (int q = 0; q < n; ++q) t += buf[b][q][lane];
+        }
+        put(b ^ 1);
+        __syncthreads();
+    }
+    if (warp == 0) {
+        if (col <= kMlpWidth) grad[col] = t;
+        else if (col == kMlpWidth + 1) *loss = t;
     }
 }
 
-__global__ void k_mlp_pack(const float* x, int rows, int n_in, int rows_pad, bf16* X, bf16* XT) {
-    const long long id = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (id >= static_cast<long long>(rows_pad) * kMlpInPad) return;
-    const int r = static_cast<int>(id / kMlpInPad), c = static_cast<int>(id % kMlpInPad);
-    const float v = (r < rows && c < n_in) ? x[static_cast<long long>(r) * n_in + c] : 0.f;
-    const bf16 b = __float2bfloat16_rn(v);
-    X[id] = b;
-    if (XT) XT[static_cast<long long>(c) * rows_pad + r] = b;
+// Inputs in BF16, zero-padded, row-major and transposed: 64 rows a CTA, turned in shared memory (a thread
+// per element with 2-byte stores took 12 us at 16,384 rows).
+constexpr int kPackRows = 64;
+__global__ void __launch_bounds__(256) k_mlp_pack(const float* x, int rows, int n_in, int rows_pad, bf16* X, bf16* XT) {
+    static_assert(256 % kMlpInPad == 0 && 256 / kMlpInPad == 4, "four rows a pass");
+    __shared__ __align__(16) bf16 t[kPackRows][kMlpInPad + 8];
+    const int r0 = blockIdx.x * kPackRows, tid = threadIdx.x;
+    const int c0 = tid % kMlpInPad;
+    float v[kPackRows / 4];
+#pragma unroll
+    for (int k = 0; k < kPackRows / 4; ++k) {
+        const int r = r0 + tid / kMlpInPad + 4 * k;
+        v[k] = r < rows && c0 < n_in ? x[static_cast<long long>(r) * n_in + c0] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < kPackRows / 4; ++k) t[tid / kMlpInPad + 4 * k][c0] = __float2bfloat16_rn(v[k]);
+    __syncthreads();
+    for (int i = tid; i < kPackRows * kMlpInPad / 8; i += 256) {
+        const int r = i / (kMlpInPad / 8), c = i % (kMlpInPad / 8) * 8;
+        *reinterpret_cast<uint4*>(X + static_cast<long long>(r0 + r) * kMlpInPad + c) = *reinterpret_cast<const uint4*>(&t[r][c]);
+        __align__(16) bf16 w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] = t[c + j][r];  // here r is a column and c a row
+        *reinterpret_cast<uint4*>(XT + static_cast<long long>(r) * rows_pad + r0 + c) = *reinterpret_cast<const uint4*>(w);
+    }
 }
 
-__global__ void k_mlp_sum_partials(const float* part, int splits, long long n, long long stride, float* out) {
-    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (i >= n) return;
-    float t = 0.f;
-    for (int s = 0; s < splits; ++s) t += part[static_cast<long long>(s) * stride + i];
-    out[i] = t;
-}
-
-__global__ void __launch_bounds__(256) k_mlp_colsum(const bf16* XT, int rows_pad, float* out) {
+// Weight gradients from the partial products of `splits` row ranges, added in their order, and the bias
+// gradients, the column sums of dZ (kMlpWidth CTAs, the last ones).
+__global__ void __launch_bounds__(256) k_mlp_grads(const float* part, int splits, int n, float* gw, const bf16* dzT, int rows_pad,
+                                                   float* gb) {
     __shared__ float red[256];
-    const bf16* row = XT + static_cast<long long>(blockIdx.x) * rows_pad;
+    const int nb = gridDim.x - kMlpWidth;
     float t = 0.f;
+    if (static_cast<int>(blockIdx.x) < nb) {
+        const int i = blockIdx.x * 256 + threadIdx.x;
+        if (i >= n) return;
+#pragma unroll 32
+        for (int s = 0; s < splits; ++s) t += part[static_cast<long long>(s) * n + i];
+        gw[i] = t;
+        return;
+    }
+    const int col = blockIdx.x - nb;
+    const bf16* row = dzT + static_cast<long long>(col) * rows_pad;
+#pragma unroll 16
     for (int r = threadIdx.x; r < rows_pad; r += 256) t += __bfloat162float(row[r]);
     red[threadIdx.x] = t;
     __syncthreads();
@@ -561,28 +693,32 @@ __global__ void __launch_bounds__(256) k_mlp_colsum(const bf16* XT, int rows_pad
         if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[blockIdx.x] = red[0];
+    if (threadIdx.x == 0) gb[col] = red[0];
 }
 
-__global__ void k_mlp_adam(float* p, const float* g, float* m, float* v, long long n, float lr_t, float b1, float b2,
-                           float eps) {
+// Adam, and the updated weights' BF16 copies (row-major and transposed)
+__global__ void k_mlp_adam(AdamArgs a) {
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr_t * mi / (sqrtf(vi) + eps);
-}
-
-__global__ void k_mlp_cast(const float* W, int out, int in, bf16* Wb, bf16* WbT) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= out * in) return;
-    const int o = id / in, i = id % in;
-    const bf16 b = __float2bfloat16_rn(W[id]);
-    Wb[id] = b;
-    if (WbT) WbT[static_cast<long long>(i) * out + o] = b;
+    if (i >= a.n) return;
+    float p = a.p[i];
+    if (a.g) {
+        const float gi = a.g[i];
+        const float mi = fmaf(1.f - a.b1, gi, a.b1 * a.m[i]);
+        const float vi = fmaf((1.f - a.b2) * gi, gi, a.b2 * a.v[i]);
+        a.m[i] = mi;
+        a.v[i] = vi;
+        p -= a.lr_t * mi / (sqrtf(vi) + a.eps);
+        a.p[i] = p;
+    }
+    const bf16 b = __float2bfloat16_rn(p);
+#pragma unroll
+    for (int l = 0; l < kMlpHidden; ++l) {
+        const int in = l == 0 ? kMlpInPad : kMlpWidth;
+        const long long k = i - a.off_W[l];
+        if (k < 0 || k >= static_cast<long long>(kMlpWidth) * in) continue;
+        a.Wb[l][k] = b;
+        if (a.WbT[l]) a.WbT[l][k % in * kMlpWidth + k / in] = b;
+    }
 }
 
 // ---- batch side ------------------------------------------------------------------------
@@ -723,10 +859,11 @@ cudaError_t launch_mlp_gemm(const GemmArgs& g, cudaStream_t s) {
         reinterpret_cast<uintptr_t>(g.A) % 16 || reinterpret_cast<uintptr_t>(g.B) % 16)
         return cudaErrorInvalidValue;
     CUtensorMap ma, mb;
-    if (!encode_bf16_map(&ma, g.A, g.M, g.K, g.lda, kMlpRowTile) || !encode_bf16_map(&mb, g.B, g.N, g.K, g.ldb, g.N))
+    const int splits = (g.K + g.k_split - 1) / g.k_split, tiles = g.M / kMlpRowTile;
+    const int z = g.N >= 128 && tiles * splits <= g.sms ? 2 : 1;
+    if (!encode_bf16_map(&ma, g.A, g.M, g.K, g.lda, kMlpRowTile) || !encode_bf16_map(&mb, g.B, g.N, g.K, g.ldb, g.N / z))
         return cudaErrorInvalidValue;
-    const int splits = (g.K + g.k_split - 1) / g.k_split;
-    k_mlp_gemm<<<dim3(g.M / kMlpRowTile, splits), kGemmThreads, mlp_gemm_smem_bytes(), s>>>(ma, mb, g);
+    k_mlp_gemm<<<dim3(tiles, splits, z), kGemmThreads, mlp_gemm_smem_bytes(), s>>>(ma, mb, g);
     return cudaGetLastError();
 }
 
@@ -745,36 +882,30 @@ cudaError_t launch_mlp_forward(const FwdArgs& args, cudaStream_t s) {
 }
 
 cudaError_t launch_mlp_head(const HeadArgs& a, cudaStream_t s) {
-    if (a.rows_pad % kHeadRowsPerCta) return cudaErrorInvalidValue;
-    k_mlp_head<<<a.rows_pad / kHeadRowsPerCta, 32 * kHeadRowsPerCta, 0, s>>>(a);
+    constexpr int kRows = kHeadGroups * kHeadRowsPerCta;
+    if (a.rows_pad % kRows) return cudaErrorInvalidValue;
+    k_mlp_head<<<a.rows_pad / kRows, 32 * kHeadRowsPerCta, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_mlp_pack(const float* x, int rows, int n_in, int rows_pad, bf16* X, bf16* XT, cudaStream_t s) {
-    const long long n = static_cast<long long>(rows_pad) * kMlpInPad;
-    k_mlp_pack<<<blocks_for(n, 256), 256, 0, s>>>(x, rows, n_in, rows_pad, X, XT);
+    if (rows_pad % kPackRows) return cudaErrorInvalidValue;
+    k_mlp_pack<<<rows_pad / kPackRows, 256, 0, s>>>(x, rows, n_in, rows_pad, X, XT);
     return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_sum_partials(const float* part, int splits, long long n, long long stride, float* out,
-                                    cudaStream_t s) {
-    k_mlp_sum_partials<<<blocks_for(n, 256), 256, 0, s>>>(part, splits, n, stride, out);
+cudaError_t launch_mlp_grads(const float* part, int splits, int n, float* gw, const bf16* dzT, int rows_pad, float* gb, cudaStream_t s) {
+    k_mlp_grads<<<(n + 255) / 256 + kMlpWidth, 256, 0, s>>>(part, splits, n, gw, dzT, rows_pad, gb);
     return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_colsum(const bf16* XT, int n_out, int rows_pad, float* out, cudaStream_t s) {
-    k_mlp_colsum<<<n_out, 256, 0, s>>>(XT, rows_pad, out);
+cudaError_t launch_mlp_head_sums(const float* part, int groups, float* grad, float* loss, cudaStream_t s) {
+    k_mlp_head_sums<<<(kMlpWidth + 2 + 31) / 32, 256, 0, s>>>(part, groups, grad, loss);
     return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_adam(float* p, const float* g, float* m, float* v, long long n, float lr_t, float b1, float b2,
-                            float eps, cudaStream_t s) {
-    k_mlp_adam<<<blocks_for(n, 256), 256, 0, s>>>(p, g, m, v, n, lr_t, b1, b2, eps);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_mlp_cast(const float* W, int out, int in, bf16* Wb, bf16* WbT, cudaStream_t s) {
-    k_mlp_cast<<<blocks_for(static_cast<long long>(out) * in, 256), 256, 0, s>>>(W, out, in, Wb, WbT);
+cudaError_t launch_mlp_adam(const AdamArgs& a, cudaStream_t s) {
+    k_mlp_adam<<<blocks_for(a.n, 256), 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 

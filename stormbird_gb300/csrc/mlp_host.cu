@@ -22,6 +22,9 @@ struct sb_mlp {
     int device = 0;
     int n_in = 0;
     cudaStream_t stream = nullptr;
+    // Beside the chain of input gradients: weight and bias gradients; the output layer's.
+    cudaStream_t side[2] = {nullptr, nullptr};
+    cudaEvent_t ev_dz[kMlpHidden] = {nullptr}, ev_side[2] = {nullptr, nullptr};
     long long off_W[kMlpHidden] = {0}, off_b[kMlpHidden] = {0}, off_out = 0, n_params = 0;
     int in_dim[kMlpHidden] = {0};
     DevBuf<float> params, grads, adam_m, adam_v;
@@ -37,6 +40,9 @@ struct sb_mlp {
     int splits = 1;
 
     ~sb_mlp() {
+        for (auto& e : ev_dz) if (e) cudaEventDestroy(e);
+        for (auto& e : ev_side) if (e) cudaEventDestroy(e);
+        for (auto& q : side) if (q) cudaStreamDestroy(q);
         if (stream) cudaStreamDestroy(stream);
     }
 
@@ -47,6 +53,9 @@ struct sb_mlp {
         ck(cudaSetDevice(device), "cudaSetDevice");
         sms = num_sms(device);
         ck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
+        for (auto& q : side) ck(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking), "cudaStreamCreate");
+        for (auto& e : ev_dz) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+        for (auto& e : ev_side) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         long long at = 0;
         for (int l = 0; l < kMlpHidden; ++l) {
             in_dim[l] = l == 0 ? kMlpInPad : kMlpWidth;
@@ -103,11 +112,18 @@ struct sb_mlp {
         ck(cudaStreamSynchronize(stream), "mlp build");
     }
 
-    void cast_weights(cudaStream_t s) {
-        for (int l = 0; l < kMlpHidden; ++l)
-            ck(launch_mlp_cast(params.p + off_W[l], kMlpWidth, in_dim[l], Wb[l].p, l > 0 ? WbT[l].p : nullptr, s),
-               "weight cast");
+    AdamArgs adam_args() const {
+        AdamArgs a;
+        a.p = params.p;
+        a.n = n_params;
+        for (int l = 0; l < kMlpHidden; ++l) {
+            a.off_W[l] = off_W[l];
+            a.Wb[l] = Wb[l].p;
+            a.WbT[l] = l > 0 ? WbT[l].p : nullptr;
+        }
+        return a;
     }
+    void cast_weights(cudaStream_t s) { ck(launch_mlp_adam(adam_args(), s), "weight cast"); }
 
     static int pad_rows(long long rows) {
         return static_cast<int>(((rows + kMlpRowTile - 1) / kMlpRowTile) * kMlpRowTile);
@@ -145,6 +161,7 @@ struct sb_mlp {
         g.K = K;
         g.k_split = K;
         g.mode = mode;
+        g.sms = sms;
         g.err = err.p;
         return g;
     }
@@ -205,23 +222,13 @@ struct sb_mlp {
     void backward(long long rows, cudaStream_t s) {
         const int R = pad_rows(rows);
         const int nh = R / kHeadRowsPerCta;
-        // output layer: dw_out, db_out and the loss from the per-CTA partials
-        ck(launch_mlp_sum_partials(head_part.p, nh, kMlpWidth + 1, kMlpWidth + 2, grads.p + off_out, s),
-           "head gradient");
-        ck(launch_mlp_sum_partials(head_part.p + kMlpWidth + 1, nh, 1, kMlpWidth + 2, loss.p, s), "loss");
+        // Weight and bias gradients of layer l need dZ_l alone: they run on a side stream while the
+        // main one goes on with dZ_{l-1}. (They share `part`, one after the other.)
+        ck(cudaEventRecord(ev_dz[kMlpHidden - 1], s), "event");
+        ck(cudaStreamWaitEvent(side[1], ev_dz[kMlpHidden - 1], 0), "side stream");
+        // output layer: dw_out, db_out and the loss from the groups' partials
+        ck(launch_mlp_head_sums(head_part.p, nh, grads.p + off_out, loss.p, side[1]), "head gradient");
         for (int l = kMlpHidden - 1; l >= 0; --l) {
-            // dW_l = dZ_l^T X_{l-1}: M = 256 outputs, N = inputs, K = rows (split)
-            const bf16* XT = l == 0 ? X0T.p : HT[l - 1].p;
-            GemmArgs g = gemm(DZT[l].p, R, XT, R, kMlpWidth, in_dim[l], R, kGemmPartial);
-            int ks = ((R / splits + 63) / 64) * 64;
-            if (ks < 64) ks = 64;
-            g.k_split = ks;
-            g.part_out = part.p;
-            ck(launch_mlp_gemm(g, s), "weight-gradient GEMM");
-            const int ns = (R + ks - 1) / ks;
-            const long long nw = static_cast<long long>(kMlpWidth) * in_dim[l];
-            ck(launch_mlp_sum_partials(part.p, ns, nw, nw, grads.p + off_W[l], s), "weight-gradient reduce");
-            ck(launch_mlp_colsum(DZT[l].p, kMlpWidth, R, grads.p + off_b[l], s), "bias gradient");
             if (l > 0) {
                 // dZ_{l-1} = (dZ_l W_l) * gelu'(Z_{l-1})
                 GemmArgs b = gemm(DZ[l].p, kMlpWidth, WbT[l].p, kMlpWidth, R, kMlpWidth, kMlpWidth, kGemmBackward);
@@ -230,7 +237,24 @@ struct sb_mlp {
                 b.hT_out = DZT[l - 1].p;
                 b.ldt = R;
                 ck(launch_mlp_gemm(b, s), "input-gradient GEMM");
+                ck(cudaEventRecord(ev_dz[l - 1], s), "event");
             }
+            // dW_l = dZ_l^T X_{l-1}: M = 256 outputs, N = inputs, K = rows (split)
+            const bf16* XT = l == 0 ? X0T.p : HT[l - 1].p;
+            GemmArgs g = gemm(DZT[l].p, R, XT, R, kMlpWidth, in_dim[l], R, kGemmPartial);
+            int ks = ((R / splits + 63) / 64) * 64;
+            if (ks < 64) ks = 64;
+            g.k_split = ks;
+            g.part_out = part.p;
+            ck(cudaStreamWaitEvent(side[0], ev_dz[l], 0), "side stream");
+            ck(launch_mlp_gemm(g, side[0]), "weight-gradient GEMM");
+            ck(launch_mlp_grads(part.p, (R + ks - 1) / ks, kMlpWidth * in_dim[l], grads.p + off_W[l], DZT[l].p, R, grads.p + off_b[l],
+                                side[0]),
+               "weight-gradient sums");
+        }
+        for (int q = 0; q < 2; ++q) {
+            ck(cudaEventRecord(ev_side[q], side[q]), "event");
+            ck(cudaStreamWaitEvent(s, ev_side[q], 0), "side stream");
         }
     }
 
@@ -253,10 +277,15 @@ struct sb_mlp {
         adam_step += 1;
         const double b1 = 0.9, b2 = 0.999;
         const double lr_t = lr * std::sqrt(1.0 - std::pow(b2, adam_step)) / (1.0 - std::pow(b1, adam_step));
-        ck(launch_mlp_adam(params.p, grads.p, adam_m.p, adam_v.p, n_params, static_cast<float>(lr_t),
-                           static_cast<float>(b1), static_cast<float>(b2), 1e-8f, s),
-           "adam");
-        cast_weights(s);
+        AdamArgs a = adam_args();
+        a.g = grads.p;
+        a.m = adam_m.p;
+        a.v = adam_v.p;
+        a.lr_t = static_cast<float>(lr_t);
+        a.b1 = static_cast<float>(b1);
+        a.b2 = static_cast<float>(b2);
+        a.eps = 1e-8f;
+        ck(launch_mlp_adam(a, s), "adam");
     }
 };
 

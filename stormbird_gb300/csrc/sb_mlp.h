@@ -40,6 +40,7 @@ struct GemmArgs {
     long long ldt = 0;
     const float* z_in = nullptr;
     float* part_out = nullptr;
+    int sms = 1;
     int* err = nullptr;
 };
 size_t mlp_gemm_smem_bytes();
@@ -61,7 +62,7 @@ struct FwdArgs {
 cudaError_t launch_mlp_forward(const FwdArgs& g, cudaStream_t s);
 
 // Output layer (width -> 1) of a training pass on the CUDA cores: MSE residuals, dz of the last hidden layer (row-major and
-// transposed) and per-CTA partials [grid][width + 2] of (dw, db, sum of squared residuals).
+// transposed) and partials [rows_pad / kHeadRowsPerCta][width + 2] of (dw, db, sum of squared residuals).
 struct HeadArgs {
     const bf16* h = nullptr;
     const float* z = nullptr;
@@ -73,22 +74,31 @@ struct HeadArgs {
     float* part = nullptr;
     float inv_n = 0.f;
 };
-constexpr int kHeadRowsPerCta = 8;
+constexpr int kHeadRowsPerCta = 8;  // rows of a partial sum
+constexpr int kHeadGroups = 4;      // partial sums a CTA makes
+// The partials added up: grad [width + 1] and the sum of squared residuals.
+cudaError_t launch_mlp_head_sums(const float* part, int groups, float* grad, float* loss, cudaStream_t s);
 cudaError_t launch_mlp_head(const HeadArgs& a, cudaStream_t s);
 
-// Input packing: x [rows][n_in] f32 -> X [rows_pad][64] BF16 (zero padded) and, when XT is
-// not null, its transpose [64][rows_pad].
+// Input packing: x [rows][n_in] f32 -> X [rows_pad][64] BF16 (zero padded) and its transpose XT [64][rows_pad].
 cudaError_t launch_mlp_pack(const float* x, int rows, int n_in, int rows_pad, bf16* X, bf16* XT, cudaStream_t s);
-// out[i] = sum over s < splits of part[s * stride + i], i < n, in split order.
-cudaError_t launch_mlp_sum_partials(const float* part, int splits, long long n, long long stride, float* out,
-                                    cudaStream_t s);
-// out[o] = sum over r < rows_pad of XT[o][r] (bias gradients from a transposed dz), o < n_out.
-cudaError_t launch_mlp_colsum(const bf16* XT, int n_out, int rows_pad, float* out, cudaStream_t s);
-// Adam update of n parameters (bias-corrected step sizes precomputed on the host).
-cudaError_t launch_mlp_adam(float* p, const float* g, float* m, float* v, long long n, float lr_t, float b1, float b2,
-                            float eps, cudaStream_t s);
-// W [out][in] f32 -> Wb [out][in] BF16 and, when WbT is not null, WbT [in][out].
-cudaError_t launch_mlp_cast(const float* W, int out, int in, bf16* Wb, bf16* WbT, cudaStream_t s);
+// gw[i] = sum over s < splits of part[s * n + i] in split order; gb[o] = sum over r < rows_pad of dzT[o][r].
+cudaError_t launch_mlp_grads(const float* part, int splits, int n, float* gw, const bf16* dzT, int rows_pad, float* gb, cudaStream_t s);
+// Adam update of n parameters (bias-corrected step sizes precomputed on the host) and the BF16 copies of
+// the weights [out][in] at off_W[l], row-major (Wb) and, when WbT is not null, transposed; g null:
+// the copies alone.
+struct AdamArgs {
+    float* p = nullptr;
+    const float* g = nullptr;
+    float* m = nullptr;
+    float* v = nullptr;
+    long long n = 0;
+    float lr_t = 0.f, b1 = 0.f, b2 = 0.f, eps = 0.f;
+    long long off_W[kMlpHidden] = {0};
+    bf16* Wb[kMlpHidden] = {nullptr};
+    bf16* WbT[kMlpHidden] = {nullptr};
+};
+cudaError_t launch_mlp_adam(const AdamArgs& a, cudaStream_t s);
 
 // ---- batch side ----------------------------------------------------------------------
 // One case of a batch, for the per-panel features of the warm start.

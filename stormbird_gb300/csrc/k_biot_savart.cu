@@ -129,6 +129,8 @@ struct TileSize<float> { static constexpr int value = 64; };
 template <>
 struct TileSize<double> { static constexpr int value = 32; };
 
+constexpr int kFarRun = 8;  // panels of a run of the far-field fast path
+
 template <class R>
 __device__ __forceinline__ void two_sum_acc(R& s, R& c, R t) {
     R sum = s + t;
@@ -374,7 +376,8 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
     __shared__ int s_chunk;
     __shared__ int s_timed_out;  // a tile wait of this CTA ran out
     // far-field fast path (FP32 panel sweeps): bounding box of each warp's targets (hi parts)
-    __shared__ float s_wbox[kBsThreads / 32][6];
+    // and the largest magnitude per axis
+    __shared__ float s_wbox[kBsThreads / 32][9];
     constexpr bool FAST_FAR = F32 && !CHAIN && !NEGLECT;
     __shared__ BsJob s_job;  // the current item's sweep (one copy per item, by thread 0)
 
@@ -493,7 +496,10 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
                 }
             if ((tid & 31) == 0)
 #pragma unroll
-                for (int q = 0; q < 6; ++q) s_wbox[tid >> 5][q] = b6[q];
+                for (int q = 0; q < 6; ++q) {
+                    s_wbox[tid >> 5][q] = b6[q];
+                    if (q < 3) s_wbox[tid >> 5][6 + q] = fmaxf(fabsf(b6[q]), fabsf(b6[q + 3]));
+                }
             __syncwarp();
         }
 
@@ -532,113 +538,9 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
             {
                 if constexpr (F32) {
                     float2 TX = bc(0.f), TY = bc(0.f), TZ = bc(0.f);
-                    // Far-field fast path, per quarter of the tile (a sub-tile of TILE / 4 panels):
-                    // when the box of the sub-tile's panel centres lies farther from the box of the
-                    // warp's targets than the sub-tile's largest far-field radius (with a margin well
-                    // beyond the FP32 rounding of the per-pair distance), every pair of it is a point
-                    // doublet (panel.rs:53-57, 82-96) and the per-pair test below would decide so for
-                    // every lane: the warp evaluates the doublets alone, without the test and the
-                    // votes. Quarters keep the boxes compact where a tile holds the end of one wing's
-                    // row of panels and the start of the next.
-                    unsigned far_mask = 0;   // bit q: sub-tile q is all far
-                    unsigned zero_mask = 0;  // bit q: sub-tile q holds a zero-strength panel
-                    if constexpr (FAST_FAR) {
-                        static_assert(TILE % 32 == 0, "the fast path's sub-tiles are 8 lanes x TILE / 32 panels");
-                        constexpr int PPL = TILE / 32;  // panels per lane; sub-tile q = lanes 8q .. 8q + 7
-                        float c7[7] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F,
-                                       0.f};
-                        bool zero = false;  // a zero-strength panel: skipped, so not in the box
-#pragma unroll
-                        for (int j = 0; j < PPL; ++j) {
-                            const int q = PPL * lane + j;
-                            if (q < np && tile[buf][q].v[kRec32Gamma] == 0.f) zero = true;
-                            else if (q < np) {
-                                const float4 c = *reinterpret_cast<const float4*>(&tile[buf][q].v[28]);  // centre hi, ff2
-                                c7[0] = fminf(c7[0], c.x);
-                                c7[1] = fminf(c7[1], c.y);
-                                c7[2] = fminf(c7[2], c.z);
-                                c7[3] = fmaxf(c7[3], c.x);
-                                c7[4] = fmaxf(c7[4], c.y);
-                                c7[5] = fmaxf(c7[5], c.z);
-                                c7[6] = fmaxf(c7[6], c.w);
-                            }
-                        }
-#pragma unroll
-                        for (int o = 4; o > 0; o >>= 1)
-#pragma unroll
-                            for (int q = 0; q < 7; ++q) {
-                                const float w = __shfl_xor_sync(0xffffffffu, c7[q], o);
-                                c7[q] = q < 3 ? fminf(c7[q], w) : fmaxf(c7[q], w);
-                            }
-                        const float* wb = s_wbox[tid >> 5];
-                        // the boxes are of hi parts, each within 2^-24 |x| of its point: the gaps
-                        // shrink by both sides' bound before the test (an empty sub-tile's box
-                        // gives a gap of 0: not far, and no panels to take)
-                        auto gap = [&](int q) {
-                            const float m = fmaxf(fmaxf(fabsf(c7[q]), fabsf(c7[q + 3])), fmaxf(fabsf(wb[q]), fabsf(wb[q + 3])));
-                            return fmaxf(0.f, fmaxf(c7[q] - wb[q + 3], wb[q] - c7[q + 3]) - 0x1p-23f * m);
-                        };
-                        const float gx = gap(0), gy = gap(1), gz = gap(2);
-                        const unsigned b =
-                            __ballot_sync(0xffffffffu, c7[6] < CUDART_INF_F && gx * gx + gy * gy + gz * gz > 1.001f * c7[6]);
-                        far_mask = (b & 1u) | ((b >> 7) & 2u) | ((b >> 14) & 4u) | ((b >> 21) & 8u);
-                        const unsigned z = __ballot_sync(0xffffffffu, zero);
-                        zero_mask = ((z & 0xffu) ? 1u : 0u) | ((z & 0xff00u) ? 2u : 0u) | ((z & 0xff0000u) ? 4u : 0u) |
-                                    ((z & 0xff000000u) ? 8u : 0u);
-                    }
-                    constexpr int NSUB = FAST_FAR ? 4 : 1;
-                    constexpr int SUB = TILE / NSUB;
-#pragma unroll 1
-                    for (int sq = 0; sq < NSUB; ++sq) {
-                    const int pa = sq * SUB, pz = min(np, pa + SUB);
-                    if ((far_mask >> sq) & 1u) {
-                        // lanes of targets past the end compute values that are never stored; four
-                        // panels per trip give the scheduler independent chains to interleave, which
-                        // it can only do without a branch per panel: a sub-tile with no
-                        // zero-strength panel takes every panel
-                        if (!((zero_mask >> sq) & 1u)) {
-#pragma unroll 4
-                            for (int p = pa; p < pz; ++p) {
-                                const float* v = reinterpret_cast<const float*>(tile[buf][p].v);
-                                const float2 ex = sub2s(X2h, v[28]);
-                                const float2 ey = sub2s(Y2h, v[29]);
-                                const float2 ez = sub2s(Z2h, v[30]);
-                                const float2 e2s = fma2(ex, ex, fma2(ey, ey, mul2(ez, ez)));
-                                doublet2(bc(v[35] * v[kRec32Gamma]), v, ex, ey, ez, e2s, TX, TY, TZ);
-                            }
-                            continue;
-                        }
-                        // a zero-strength panel must be skipped: only its strength slot is written
-                        // (its other fields may hold anything, and 0 times NaN is NaN)
-#pragma unroll 4
-                        for (int p = pa; p < pz; ++p) {
-                            const float* v = reinterpret_cast<const float*>(tile[buf][p].v);
-                            const float gam = v[kRec32Gamma];
-                            if (gam == 0.f) continue;  // uniform across the CTA
-                            const float2 ex = sub2s(X2h, v[28]);
-                            const float2 ey = sub2s(Y2h, v[29]);
-                            const float2 ez = sub2s(Z2h, v[30]);
-                            const float2 e2s = fma2(ex, ex, fma2(ey, ey, mul2(ez, ez)));
-                            doublet2(bc(v[35] * gam), v, ex, ey, ez, e2s, TX, TY, TZ);
-                        }
-                        continue;
-                    }
-                    for (int p = pa; p < pz; ++p) {
-                        const float* v = reinterpret_cast<const float*>(tile[buf][p].v);
-                        if constexpr (CHAIN) {  // every pair near-field: the chain's segments
-                            if (v[kChainAny] == 0.f) continue;  // uniform across the CTA
-                            const float2 ex = add2(sub2s(X2h, v[0]), sub2s(X2l, v[3]));
-                            const float2 ey = add2(sub2s(Y2h, v[1]), sub2s(Y2l, v[4]));
-                            const float2 ez = add2(sub2s(Z2h, v[2]), sub2s(Z2l, v[5]));
-                            float2 ax, ay, az;
-                            chain2(v, ex, ey, ez, ax, ay, az);
-                            TX = add2(TX, ax);
-                            TY = add2(TY, ay);
-                            TZ = add2(TZ, az);
-                            continue;
-                        }
+                    // one panel at the thread's two targets, by the per-pair near/far test
+                    auto panel2 = [&](const float* v) {
                         const float gam = v[kRec32Gamma];
-                        if (gam == 0.f) continue;  // uniform across the CTA
                         // target - centre from the hi parts: the near/far test's first look and the
                         // far-field doublet's (at least ff_ratio panel sizes away), as in the fast
                         // path above; the ring below adds the lo parts
@@ -678,7 +580,83 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
                             TY = fma2(gm, ay, TY);
                             TZ = fma2(gm, az, TZ);
                         }
-                    }
+                    };
+                    // the doublet alone; lanes of targets past the end compute values never stored
+                    auto far2 = [&](const float* v) {
+                        const float2 ex = sub2s(X2h, v[28]);
+                        const float2 ey = sub2s(Y2h, v[29]);
+                        const float2 ez = sub2s(Z2h, v[30]);
+                        const float2 e2s = fma2(ex, ex, fma2(ey, ey, mul2(ez, ez)));
+                        doublet2(bc(v[35] * v[kRec32Gamma]), v, ex, ey, ez, e2s, TX, TY, TZ);
+                    };
+                    if constexpr (FAST_FAR) {
+                        // Far-field fast path: a panel whose centre lies farther from the box of the warp's
+                        // targets than its far-field radius (with a margin well beyond the FP32 rounding of
+                        // the per-pair distance) is a point doublet (panel.rs:53-57, 82-96) at all of them,
+                        // as the per-pair test would decide for every lane: the warp evaluates the doublet
+                        // alone, without the test and its votes. Each lane tests a panel of 32 and a ballot
+                        // hands the answers round. (A box per 16 panels, reduced over 8 lanes by 21 shuffles,
+                        // took a sixth of the sweep, and one near panel sent all 16 to the per-pair test:
+                        // 413,832 targets x 409,600 panels 136.6 ms, now 129.4; in runs of 4 132.3. What is
+                        // left runs at 56 cycles a panel and warp, 41 of them the FMA pipe's 20 packed
+                        // operations at half rate.)
+                        const float* wb = s_wbox[tid >> 5];
+#pragma unroll 1
+                        for (int p0 = 0; p0 < np; p0 += 32) {
+                            bool far = false, any = false;  // any: of non-zero strength
+                            if (p0 + lane < np) {
+                                const float* v = reinterpret_cast<const float*>(tile[buf][p0 + lane].v);
+                                const float4 c = *reinterpret_cast<const float4*>(v + 28);  // centre hi, ff2
+                                any = v[kRec32Gamma] != 0.f;  // the other fields of a zero panel may hold anything
+                                // the box and the centre are hi parts, each within 2^-24 |x| of its point:
+                                // the gaps shrink by both sides' bound before the test
+                                auto gap = [&](float x, int q) {
+                                    return fmaxf(0.f, fmaxf(x - wb[q + 3], wb[q] - x) - 0x1p-23f * fmaxf(fabsf(x), wb[q + 6]));
+                                };
+                                const float gx = gap(c.x, 0), gy = gap(c.y, 1), gz = gap(c.z, 2);
+                                far = any && c.w < CUDART_INF_F && gx * gx + gy * gy + gz * gz > 1.001f * c.w;
+                            }
+                            const unsigned live = __ballot_sync(0xffffffffu, any);
+                            const unsigned fast = __ballot_sync(0xffffffffu, far);
+                            const PanelRec<R>* t0 = &tile[buf][p0];
+#pragma unroll 1
+                            for (int q = 0; q < 32; q += kFarRun) {
+                                constexpr unsigned kAll = (1u << kFarRun) - 1u;
+                                // a run of far panels, with no branch between them: independent chains for
+                                // the scheduler to interleave
+                                if (((fast >> q) & kAll) == kAll) {
+#pragma unroll
+                                    for (int j = 0; j < kFarRun; ++j) far2(reinterpret_cast<const float*>(t0[q + j].v));
+                                    continue;
+                                }
+                                // one by one (uniform branches); zero-strength panels and those past the end
+                                // are left out
+                                for (unsigned w = (live >> q) & kAll; w != 0; w &= w - 1) {
+                                    const int p = q + __ffs(w) - 1;
+                                    const float* v = reinterpret_cast<const float*>(t0[p].v);
+                                    if ((fast >> p) & 1u) far2(v);
+                                    else panel2(v);
+                                }
+                            }
+                        }
+                    } else {
+                        for (int p = 0; p < np; ++p) {
+                            const float* v = reinterpret_cast<const float*>(tile[buf][p].v);
+                            if constexpr (CHAIN) {  // every pair near-field: the chain's segments
+                                if (v[kChainAny] == 0.f) continue;  // uniform across the CTA
+                                const float2 ex = add2(sub2s(X2h, v[0]), sub2s(X2l, v[3]));
+                                const float2 ey = add2(sub2s(Y2h, v[1]), sub2s(Y2l, v[4]));
+                                const float2 ez = add2(sub2s(Z2h, v[2]), sub2s(Z2l, v[5]));
+                                float2 ax, ay, az;
+                                chain2(v, ex, ey, ez, ax, ay, az);
+                                TX = add2(TX, ax);
+                                TY = add2(TY, ay);
+                                TZ = add2(TZ, az);
+                            } else {
+                                if (v[kRec32Gamma] == 0.f) continue;  // uniform across the CTA
+                                panel2(v);
+                            }
+                        }
                     }
                     const float txa[2] = {TX.x, TX.y}, tya[2] = {TY.x, TY.y}, tza[2] = {TZ.x, TZ.y};
 #pragma unroll

@@ -137,7 +137,14 @@ struct sb_batch {
     // geometry, wake update, unit-strength matrix and chain records of the dynamic cases past
     // their first step: one launch per kind for all of them (refilled each step: the jobs
     // name the step's wake buffers and time step)
-    std::vector<char> case_batched;  // per case, in the current step
+    std::vector<char> case_batched;  // per case, in the current step: by CaseStepJob or QsStepJob
+    PinnedBuf<QsStepJob> h_qs_jobs;
+    DevBuf<QsStepJob> d_qs_jobs;
+    int n_qs_jobs = 0;
+    long long blk_qs_geometry = 0, blk_qs_matrix = 0;
+    PinnedBuf<WindJob> h_wind_jobs;  // every case (with set_wind)
+    DevBuf<WindJob> d_wind_jobs;
+    long long blk_wind_geometry = 0, blk_wind = 0, blk_ctrl = 0;
     PinnedBuf<CaseStepJob> h_case_jobs;
     DevBuf<CaseStepJob> d_case_jobs;
     int n_case_jobs = 0;
@@ -355,6 +362,8 @@ struct sb_batch {
         case_batched.assign(cases.size(), 0);
         h_case_jobs.alloc(cases.size());
         d_case_jobs.alloc(cases.size());
+        h_qs_jobs.alloc(cases.size());
+        d_qs_jobs.alloc(cases.size());
         counters.alloc(16);
         err.alloc(1);
         ck(cudaMemset(err.p, 0, sizeof(int)), "memset");
@@ -535,12 +544,14 @@ struct sb_batch {
     }
 
     // ------------------------------------------------------------------ one step
-    void fork(int slot) {
+    // The first n pool streams wait for main; main for them. (All 16 cost the host some 50 us a pair.)
+    void fork(int slot, int n = kPoolStreams) {
+        if (n <= 0) return;
         ck(cudaEventRecord(ev_fork[slot], main), "fork");
-        for (auto& s : pool) ck(cudaStreamWaitEvent(s, ev_fork[slot], 0), "fork");
+        for (int k = 0; k < std::min(n, kPoolStreams); ++k) ck(cudaStreamWaitEvent(pool[k], ev_fork[slot], 0), "fork");
     }
-    void join(int slot) {
-        for (int k = 0; k < kPoolStreams; ++k) {
+    void join(int slot, int n = kPoolStreams) {
+        for (int k = 0; k < std::min(n, kPoolStreams); ++k) {
             ck(cudaEventRecord(ev_join[slot][k], pool[k]), "join");
             ck(cudaStreamWaitEvent(main, ev_join[slot][k], 0), "join");
         }
@@ -581,14 +592,25 @@ struct sb_batch {
             ck(cudaMemcpyAsync(d_case_jobs.p, h_case_jobs.p, n_case_jobs * sizeof(CaseStepJob), cudaMemcpyHostToDevice,
                                main),
                "H2D case jobs");
-        fork(0);
+        if (wind) {  // complete_sail_model/mod.rs:213-257
+            ck(cudaMemcpyAsync(d_wind_jobs.p, h_wind_jobs.p, cases.size() * sizeof(WindJob), cudaMemcpyHostToDevice, main),
+               "H2D wind jobs");
+            launch_wind_jobs();
+        }
+        if (n_qs_jobs > 0) {
+            ck(cudaMemcpyAsync(d_qs_jobs.p, h_qs_jobs.p, n_qs_jobs * sizeof(QsStepJob), cudaMemcpyHostToDevice, main),
+               "H2D case jobs");
+            ck(launch_prep_geometry_jobs(d_qs_jobs.p, n_qs_jobs, blk_qs_geometry, main), "batched geometry");
+        }
+        // cases are spread over the pool's streams: forks and joins only where one has launches of its own
+        const int own_begin = n_case_jobs + n_qs_jobs < static_cast<int>(cases.size()) ? kPoolStreams : 0;
+        fork(0, own_begin);
         for (size_t i = 0; i < cases.size(); ++i) {
             sb_sim& c = *cases[i];
-            if (wind) c.enqueue_wind_freestream();  // complete_sail_model/mod.rs:213-257
             if (case_batched[i]) c.step_begin_host(time, dt);
             else c.step_begin(time, dt);
         }
-        join(0);
+        join(0, own_begin);
         if (n_case_jobs > 0) {  // geometry, then wake advection and panels, of the batched cases
             ck(launch_prep_geometry_jobs(d_case_jobs.p, n_case_jobs, blk_geometry, main), "batched geometry");
             ck(launch_wake_jobs(d_case_jobs.p, n_case_jobs, blk_advect, blk_panels, main), "batched wake update");
@@ -597,23 +619,28 @@ struct sb_batch {
         sweeps(0);
         for (auto& c : cases) if (c->dynamic) c->after_fixed_sweep();
         if (n_case_jobs > 0) ck(launch_unit_matrix_jobs(d_case_jobs.p, n_case_jobs, blk_matrix, main), "batched unit matrix");
-        fork(1);
+        if (n_qs_jobs > 0)
+            ck(launch_horseshoe_matrix_jobs(d_qs_jobs.p, n_qs_jobs, blk_qs_matrix, main), "batched horseshoe matrix");
+        int own_solve = 0;
+        for (size_t i = 0; i < cases.size(); ++i)
+            if (!case_batched[i] || !(si_batched[i] || cases[i]->linearized_quasi_steady())) own_solve = kPoolStreams;
+        fork(1, own_solve);
         for (size_t i = 0; i < cases.size(); ++i) {
             sb_sim& c = *cases[i];
-            if (case_batched[i]) {
-                if (!si_batched[i]) c.step_solve();  // matrix and chain records come from the batch
+            if (case_batched[i]) {  // matrix and chain records come from the batch
+                if (!si_batched[i] && !c.linearized_quasi_steady()) c.step_solve();
             } else if (c.linearized_quasi_steady() || si_batched[i]) {
                 c.step_matrix();
             } else {
                 c.step_matrix_and_solve();
             }
         }
-        join(1);
+        join(1, own_solve);
         // the batched solves: a launch per Linearized plan shape and per SimpleIterative
         // cluster size, side by side on the pool streams
         int n_refined = 0;
         for (const auto& g : lin_refined) n_refined += g.n > 0 ? 1 : 0;
-        if (n_refined > 1) fork(1);
+        if (n_refined > 1) fork(1, n_refined);
         {
             int k = 0;
             for (const auto& g : lin_refined)
@@ -621,12 +648,12 @@ struct sb_batch {
                     ck(launch_solve_linearized_refined_jobs(g.jobs.p, g.n, g.plan, n_refined > 1 ? pool[k++] : main),
                        "batched linearized solve");
         }
-        if (n_refined > 1) join(1);
+        if (n_refined > 1) join(1, n_refined);
         int n_launch = 0;
         for (const auto& g : lin_groups) n_launch += g.n > 0 ? 1 : 0;
         for (const auto& g : si_groups) n_launch += g.cases.empty() ? 0 : 1;
         if (n_launch > 0) {
-            if (n_launch > 1) fork(1);
+            if (n_launch > 1) fork(1, n_launch);
             int k = 0;
             for (const auto& g : lin_groups)
                 if (g.n > 0)
@@ -648,7 +675,7 @@ struct sb_batch {
                                                           n_launch > 1 ? pool[k++ % kPoolStreams] : main),
                        "batched simple iterative solve");
                 }
-            if (n_launch > 1) join(1);
+            if (n_launch > 1) join(1, n_launch);
         }
         // what follows a solve in its case (chain records of the wake), after the batched solves
         bool after = false;
@@ -794,6 +821,7 @@ struct sb_batch {
         const int parity = any_dynamic ? first_dynamic().cur : (steps & 1);
         ck(cudaEventRecord(ev_t0, main), "event");
         fill_case_jobs(time, dt);
+        if (wind) fill_wind_jobs(nullptr);
         if (use_graph && steady()) {
             // job lists of this step, read by the graph's copy node at launch
             fill_jobs_after_begin();
@@ -869,16 +897,47 @@ struct sb_batch {
         return *cases[0];
     }
 
+    // Geometry and freestream of every case's wind (jobs on the device).
+    void launch_wind_jobs() {
+        const int n = static_cast<int>(cases.size());
+        ck(launch_prep_geometry_jobs(d_wind_jobs.p, n, blk_wind_geometry, main), "batched wind geometry");
+        ck(launch_wind_freestream_jobs(d_wind_jobs.p, n, blk_wind, main), "batched wind freestream");
+    }
+
+    void fill_wind_jobs(double* ctrl) {
+        blk_wind_geometry = blk_wind = blk_ctrl = 0;
+        for (size_t i = 0; i < cases.size(); ++i) {
+            WindJob& j = h_wind_jobs.p[i];
+            j = cases[i]->wind_job(ctrl ? ctrl + 3 * line_off[i] : nullptr);
+            j.blk_geometry = blk_wind_geometry;
+            j.blk_wind = blk_wind;
+            j.blk_ctrl = blk_ctrl;
+            blk_wind_geometry += prep_geometry_blocks(j.m);
+            blk_wind += wind_blocks(j.m.N, j.n_wake);
+            blk_ctrl += controller_input_blocks(j.m.N);
+        }
+    }
+
     // The work lists describe the sweeps as they will be after step_begin (which swaps the
     // wake buffers): compute them with the parity flipped for the duration.
-    // The job of every dynamic case past its first step (state before the step).
+    // The job of every case past its first step (state before the step).
     void fill_case_jobs(double time, double dt) {
-        n_case_jobs = 0;
+        n_case_jobs = n_qs_jobs = 0;
+        blk_qs_geometry = blk_qs_matrix = 0;
         blk_geometry = blk_advect = blk_panels = blk_matrix = blk_chain = 0;
         for (size_t i = 0; i < cases.size(); ++i) {
             const sb_sim& c = *cases[i];
-            case_batched[i] = c.batch_kernels_ok() ? 1 : 0;
+            case_batched[i] = c.batch_kernels_ok() || c.batch_qs_kernels_ok() ? 1 : 0;
             if (!case_batched[i]) continue;
+            if (!c.dynamic) {
+                QsStepJob& j = h_qs_jobs.p[n_qs_jobs++];
+                j = c.qs_step_job(time, dt);
+                j.blk_geometry = blk_qs_geometry;
+                j.blk_matrix = blk_qs_matrix;
+                blk_qs_geometry += prep_geometry_blocks(c.dm);
+                blk_qs_matrix += horseshoe_blocks(c.dm);
+                continue;
+            }
             CaseStepJob j = c.step_job(time, dt);
             j.blk_geometry = blk_geometry;
             j.blk_advect = blk_advect;
@@ -943,6 +1002,8 @@ struct sb_batch {
         ck(cudaStreamSynchronize(main), "sync");
         drop_graphs();
         if (wind_steps.n == 0) {
+            h_wind_jobs.alloc(cases.size());
+            d_wind_jobs.alloc(cases.size());
             wind_steps.alloc(cases.size() * 2);
             h_wind_steps.alloc(cases.size() * 2);
         }
@@ -986,17 +1047,13 @@ struct sb_batch {
         }
         ck(cudaMemcpyAsync(wind_steps.p, h_wind_steps.p, cases.size() * 2 * sizeof(double), cudaMemcpyHostToDevice, main),
            "H2D wind steps");
-        fork(0);
-        for (size_t i = 0; i < cases.size(); ++i) {
-            sb_sim& c = *cases[i];
-            c.enqueue_wind_freestream();
-            double* d = ctrl_in.p + 3 * line_off[i];
-            ck(launch_controller_input(c.dm, c.params, c.fs_p, d, c.stream), "controller input");
-            ck(cudaMemcpyAsync(h_ctrl_in.p + 3 * line_off[i], d, 3 * c.N * sizeof(double), cudaMemcpyDeviceToHost,
-                               c.stream),
-               "D2H controller input");
-        }
-        join(0);
+        fill_wind_jobs(ctrl_in.p);
+        ck(cudaMemcpyAsync(d_wind_jobs.p, h_wind_jobs.p, cases.size() * sizeof(WindJob), cudaMemcpyHostToDevice, main),
+           "H2D wind jobs");
+        launch_wind_jobs();
+        ck(launch_controller_input_jobs(d_wind_jobs.p, static_cast<int>(cases.size()), blk_ctrl, main), "controller input");
+        ck(cudaMemcpyAsync(h_ctrl_in.p, ctrl_in.p, static_cast<size_t>(N_total) * 3 * sizeof(double), cudaMemcpyDeviceToHost, main),
+           "D2H controller input");
         ck(cudaStreamSynchronize(main), "controller input");
         return h_ctrl_in.p;
     }

@@ -1085,7 +1085,7 @@ cudaError_t launch_unit_matrix_jobs(const CaseStepJob* jobs, int n, long long bl
 
 // Quasi-steady wake: relative core length (frozen_wake.rs:74-100), the mean span line length.
 constexpr int kQsPrepThreads = 256;
-__global__ void __launch_bounds__(kQsPrepThreads) k_qs_prep(DevModel m, double core_value, double* rc_out) {
+__device__ __forceinline__ void qs_prep_block(const DevModel& m, double core_value, double* rc_out) {
     __shared__ double part[kQsPrepThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31;
     double s = 0.0;
@@ -1109,17 +1109,16 @@ __global__ void __launch_bounds__(kQsPrepThreads) k_qs_prep(DevModel m, double c
 // control point, 128 span points of which the last only serves its neighbour. FP64-bound: about 65
 // instructions per line.
 constexpr int kHorseshoePoints = 128;
-__global__ void __launch_bounds__(kHorseshoePoints) k_horseshoe_matrix(DevModel m, double wake_length, double rc_value,
-                                                                       const double* rc_dev, int sym, int tiles,
-                                                                       d3* factors, float* split, const d3* basis) {
+__device__ __forceinline__ int horseshoe_tiles(const DevModel& m) { return (m.Np - 1 + kHorseshoePoints - 2) / (kHorseshoePoints - 1); }
+__device__ __forceinline__ void horseshoe_block(const DevModel& m, const HorseshoeArgs& h, long long block) {
     __shared__ d3 trail[kHorseshoePoints];
-    const int N = m.N, tid = threadIdx.x;
-    const int c = blockIdx.x / tiles;
-    const int k0 = (blockIdx.x % tiles) * (kHorseshoePoints - 1), k = k0 + tid;
+    const int N = m.N, tid = threadIdx.x, tiles = horseshoe_tiles(m), sym = h.sym;
+    const int c = static_cast<int>(block / tiles);
+    const int k0 = static_cast<int>(block % tiles) * (kHorseshoePoints - 1), k = k0 + tid;
     const bool have = k < m.Np;
     const int j = have ? m.sp_line[k] : 0;
     const bool line = have && !m.sp_end[k];  // a line starts at this point
-    const double rc = rc_dev ? *rc_dev : rc_value, rc4 = (rc * rc) * (rc * rc);
+    const double rc = h.core_kind == 0 ? *h.rc_dev : h.core_kind == 1 ? h.core_value : 0.0, rc4 = (rc * rc) * (rc * rc);
     const d3 s = have ? m.span_pts[k] : mk(0, 0, 0), e = have ? m.span_e[j] : mk(0, 0, 0);
     d3 far = s;
     double il_far = 0.0, il_bound = 0.0;
@@ -1127,7 +1126,7 @@ __global__ void __launch_bounds__(kHorseshoePoints) k_horseshoe_matrix(DevModel 
         const d3 f = m.felt_span[k];
         const double l = len2(f);
         d3 w = mk(0, 0, 0);  // normalize(f) wake_length
-        if (l > 0.0) w = f * (wake_length * rsqrt_any(l));
+        if (l > 0.0) w = f * (h.wake_length * rsqrt_any(l));
         far = s + w;
         il_far = rcp_any(len2(w));
         il_bound = rcp_any(len2(e - s));
@@ -1138,10 +1137,10 @@ __global__ void __launch_bounds__(kHorseshoePoints) k_horseshoe_matrix(DevModel 
         const d3 y = q ? mirror(sym, m.ctrl[c]) : m.ctrl[c];
         d3 own = mk(0, 0, 0), b = mk(0, 0, 0);
 #pragma unroll 1
-        for (int h = 0; h < 2; ++h) {  // the trailing line away from the point, then the bound line
-            if (!have || (h && !line)) break;
-            const d3 w = line_unit_f64(s, h ? e : far, y, h ? il_bound : il_far, rc4);
-            if (h) b = w;
+        for (int t = 0; t < 2; ++t) {  // the trailing line away from the point, then the bound line
+            if (!have || (t && !line)) break;
+            const d3 w = line_unit_f64(s, t ? e : far, y, t ? il_bound : il_far, rc4);
+            if (t) b = w;
             else own = w;
         }
         trail[tid] = own;
@@ -1153,21 +1152,41 @@ __global__ void __launch_bounds__(kHorseshoePoints) k_horseshoe_matrix(DevModel 
         __syncthreads();
     }
     if (line && tid + 1 < kHorseshoePoints)
-        store_factor(factors, split, N, basis, static_cast<long long>(c) * N + j, c, j, u);
+        store_factor(h.factors, h.split, N, h.basis, static_cast<long long>(c) * N + j, c, j, u);
 }
 
-cudaError_t launch_horseshoe_matrix(const DevModel& m, int core_kind, double core_value, double wake_length,
-                                    double* rc_dev, int sym, d3* factors, float* split, const d3* basis,
-                                    cudaStream_t s) {
-    if (core_kind == 0) {
-        k_qs_prep<<<1, kQsPrepThreads, 0, s>>>(m, core_value, rc_dev);
+__global__ void __launch_bounds__(kQsPrepThreads) k_qs_prep(DevModel m, HorseshoeArgs h) { qs_prep_block(m, h.core_value, h.rc_dev); }
+__global__ void __launch_bounds__(kHorseshoePoints) k_horseshoe_matrix(DevModel m, HorseshoeArgs h) { horseshoe_block(m, h, blockIdx.x); }
+// Every quasi-steady case of a batch (36 cases of 72 lines: 36 launches of each took the host longer than the GPU).
+__global__ void __launch_bounds__(kQsPrepThreads) k_qs_prep_jobs(const QsStepJob* jobs) {
+    const QsStepJob& J = jobs[blockIdx.x];
+    if (J.h.core_kind == 0) qs_prep_block(J.m, J.h.core_value, J.h.rc_dev);
+}
+__global__ void __launch_bounds__(kHorseshoePoints) k_horseshoe_matrix_jobs(const QsStepJob* jobs, int n) {
+    const QsStepJob& J = jobs[job_of_block<QsStepJob, &QsStepJob::blk_matrix>(jobs, n, blockIdx.x)];
+    horseshoe_block(J.m, J.h, blockIdx.x - J.blk_matrix);
+}
+
+long long horseshoe_blocks(const DevModel& m) {
+    return static_cast<long long>(m.N) * ((m.Np - 1 + kHorseshoePoints - 2) / (kHorseshoePoints - 1));
+}
+
+cudaError_t launch_horseshoe_matrix(const DevModel& m, const HorseshoeArgs& h, cudaStream_t s) {
+    if (h.core_kind == 0) {
+        k_qs_prep<<<1, kQsPrepThreads, 0, s>>>(m, h);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    const int tiles = (m.Np - 1 + kHorseshoePoints - 2) / (kHorseshoePoints - 1);
-    k_horseshoe_matrix<<<static_cast<unsigned>(static_cast<long long>(m.N) * tiles), kHorseshoePoints, 0, s>>>(
-        m, wake_length, core_kind == 1 ? core_value : 0.0, core_kind == 0 ? rc_dev : nullptr, sym, tiles, factors, split,
-        basis);
+    k_horseshoe_matrix<<<static_cast<unsigned>(horseshoe_blocks(m)), kHorseshoePoints, 0, s>>>(m, h);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_horseshoe_matrix_jobs(const QsStepJob* jobs, int n, long long blocks, cudaStream_t s) {
+    if (n <= 0 || blocks <= 0) return cudaSuccess;
+    k_qs_prep_jobs<<<n, kQsPrepThreads, 0, s>>>(jobs);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_horseshoe_matrix_jobs<<<static_cast<unsigned>(blocks), kHorseshoePoints, 0, s>>>(jobs, n);
     return cudaGetLastError();
 }
 

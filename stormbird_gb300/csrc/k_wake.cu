@@ -10,6 +10,8 @@
 // (new row i = old row i-1 + dt * velocity) becomes one independent update per point.
 // Positions are integrated in f64; the panel records for the sweep are written in FP32
 // (and f64 for the first row and in the FP64 precision mode).
+#include <type_traits>
+
 #include "sb_device.cuh"
 #include "sb_kernels.h"
 
@@ -119,23 +121,13 @@ __global__ void __launch_bounds__(kGeometryThreads) k_prep_geometry(DevModel m, 
     prep_geometry_block(m, p, fs_ctrl, mean_out, blockIdx.x);
 }
 
-// Job that block b belongs to: the last one whose first block of the kind is at or before it (jobs [n]
-// ascending in each kind's first block).
-template <long long CaseStepJob::*First>
-__device__ inline int job_of_block(const CaseStepJob* jobs, int n, long long b) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].*First <= b) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// The geometry of every case of a batch.
-__global__ void __launch_bounds__(kGeometryThreads) k_prep_geometry_jobs(const CaseStepJob* jobs, int n) {
-    const CaseStepJob& J = jobs[job_of_block<&CaseStepJob::blk_geometry>(jobs, n, blockIdx.x)];
-    prep_geometry_block(J.m, J.p, J.fs_ctrl, nullptr, static_cast<int>(blockIdx.x - J.blk_geometry));
+// The geometry of every case of a list.
+template <class Job>
+__global__ void __launch_bounds__(kGeometryThreads) k_prep_geometry_jobs(const Job* jobs, int n) {
+    const Job& J = jobs[job_of_block<Job, &Job::blk_geometry>(jobs, n, blockIdx.x)];
+    const d3* fs = nullptr;
+    if constexpr (!std::is_same<Job, WindJob>::value) fs = J.fs_ctrl;
+    prep_geometry_block(J.m, J.p, fs, nullptr, static_cast<int>(blockIdx.x - J.blk_geometry));
 }
 
 long long prep_geometry_blocks(const DevModel& m) { return (m.N + kGeometryLines - 1) / kGeometryLines; }
@@ -145,10 +137,20 @@ cudaError_t launch_prep_geometry(const DevModel& m, const StepParams& p, const d
     return cudaGetLastError();
 }
 
-cudaError_t launch_prep_geometry_jobs(const CaseStepJob* jobs, int n, long long blocks, cudaStream_t s) {
+template <class Job>
+static cudaError_t launch_geometry_list(const Job* jobs, int n, long long blocks, cudaStream_t s) {
     if (n <= 0 || blocks <= 0) return cudaSuccess;
     k_prep_geometry_jobs<<<static_cast<unsigned>(blocks), kGeometryThreads, 0, s>>>(jobs, n);
     return cudaGetLastError();
+}
+cudaError_t launch_prep_geometry_jobs(const CaseStepJob* jobs, int n, long long blocks, cudaStream_t s) {
+    return launch_geometry_list(jobs, n, blocks, s);
+}
+cudaError_t launch_prep_geometry_jobs(const QsStepJob* jobs, int n, long long blocks, cudaStream_t s) {
+    return launch_geometry_list(jobs, n, blocks, s);
+}
+cudaError_t launch_prep_geometry_jobs(const WindJob* jobs, int n, long long blocks, cudaStream_t s) {
+    return launch_geometry_list(jobs, n, blocks, s);
 }
 
 // Direction of the first free wake row (update_data.rs:152-199).
@@ -567,19 +569,19 @@ cudaError_t launch_wake_panels(const DevModel& m, const WakeBuffers& w, int shif
 // each kind's first block), and runs that job's element at b's offset within it.
 // ---------------------------------------------------------------------------------------
 __global__ void k_wake_advect_jobs(const CaseStepJob* jobs, int n) {
-    const CaseStepJob& J = jobs[job_of_block<&CaseStepJob::blk_advect>(jobs, n, blockIdx.x)];
+    const CaseStepJob& J = jobs[job_of_block<CaseStepJob, &CaseStepJob::blk_advect>(jobs, n, blockIdx.x)];
     const long long id = (blockIdx.x - J.blk_advect) * static_cast<long long>(kAdvectThreads) + threadIdx.x;
     wake_advect_elem(J.m, J.w, J.p.dt, J.steps_done, id);
 }
 
 __global__ void k_wake_panels_jobs(const CaseStepJob* jobs, int n) {
-    const CaseStepJob& J = jobs[job_of_block<&CaseStepJob::blk_panels>(jobs, n, blockIdx.x)];
+    const CaseStepJob& J = jobs[job_of_block<CaseStepJob, &CaseStepJob::blk_panels>(jobs, n, blockIdx.x)];
     const long long id = (blockIdx.x - J.blk_panels) * static_cast<long long>(kPanelThreads) + threadIdx.x;
     wake_panel_elem(J.m, J.w, 1, id);
 }
 
 __global__ void k_chain_records_jobs(const CaseStepJob* jobs, int n) {
-    const CaseStepJob& J = jobs[job_of_block<&CaseStepJob::blk_chain>(jobs, n, blockIdx.x)];
+    const CaseStepJob& J = jobs[job_of_block<CaseStepJob, &CaseStepJob::blk_chain>(jobs, n, blockIdx.x)];
     const long long id = (blockIdx.x - J.blk_chain) * static_cast<long long>(kChainThreads) + threadIdx.x;
     chain_record_elem(J.chain, J.chain_n, id);
 }

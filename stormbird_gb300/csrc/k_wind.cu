@@ -76,10 +76,9 @@ __device__ d3 true_wind_direction(const WindDevice& w) {
     return turned(w.zero, w.direction_coming_from, w.axis);
 }
 
-__global__ void k_wind_freestream(WindDevice w, const d3* ctrl, const int* wing_of_line, int N, const d3* wake,
-                                  long long n_wake, d3* out) {
-    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (i >= N + n_wake) return;
+constexpr int kWindThreads = 128;
+
+__device__ void wind_point(const WindDevice& w, const d3* ctrl, const int* wing_of_line, int N, const d3* wake, d3* out, long long i) {
     const double time = w.step[0];
     const d3 linear = w.zero * w.step[1];
     const d3 p = i < N ? ctrl[i] : wake[i - N];
@@ -117,6 +116,19 @@ __global__ void k_wind_freestream(WindDevice w, const d3* ctrl, const int* wing_
     out[i] = u;
 }
 
+__global__ void k_wind_freestream(WindDevice w, const d3* ctrl, const int* wing_of_line, int N, const d3* wake,
+                                  long long n_wake, d3* out) {
+    const long long i = blockIdx.x * static_cast<long long>(kWindThreads) + threadIdx.x;
+    if (i < N + n_wake) wind_point(w, ctrl, wing_of_line, N, wake, out, i);
+}
+
+// Every case of a batch.
+__global__ void k_wind_freestream_jobs(const WindJob* jobs, int n) {
+    const WindJob& J = jobs[job_of_block<WindJob, &WindJob::blk_wind>(jobs, n, blockIdx.x)];
+    const long long i = (blockIdx.x - J.blk_wind) * kWindThreads + threadIdx.x;
+    if (i < J.m.N + J.n_wake) wind_point(J.w, J.m.ctrl, J.m.wing_of_line, J.m.N, J.wake, J.out, i);
+}
+
 // ControllerInput::new_from_velocity (controller/input.rs:99-157) per line, on the geometry
 // k_prep_geometry left for the current wing angles and motion: out[i] = |v_i|,
 // out[N + i] = the angle of attack (force_calculations.rs:79-107: signed angle from the global
@@ -124,33 +136,56 @@ __global__ void k_wind_freestream(WindDevice w, const d3* ctrl, const int* wing_
 // apparent wind direction (environment.rs:315-345: signed angle from the unrotated chord of
 // the wing's first strip, moved by the rigid body's rotation, to v about that strip's global
 // span direction).
-__global__ void k_controller_input(DevModel m, StepParams p, const d3* v, double* out) {
+__device__ void controller_line(const DevModel& m, const StepParams& p, const d3* v, double* out, int i) {
     const int N = m.N;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        const d3 u = v[i];
-        const d3 span_dir = normalize(m.span_e[i] - m.span_s[i]);
-        out[i] = len(u);
-        out[N + i] = len(u) > kMinPositive ? angle_between(m.chord_global[i], u, span_dir) : 0.0;
-        const int ws = m.wing_start[m.wing_of_line[i]];
-        const d3 axis = normalize(m.span_e[ws] - m.span_s[ws]);
-        const d3 chord_first = rotate_xyz(m.chord_not_rotated[ws], p.rotation);
-        out[2 * N + i] = angle_between(chord_first, u, axis);
-    }
+    const d3 u = v[i];
+    const d3 span_dir = normalize(m.span_e[i] - m.span_s[i]);
+    out[i] = len(u);
+    out[N + i] = len(u) > kMinPositive ? angle_between(m.chord_global[i], u, span_dir) : 0.0;
+    const int ws = m.wing_start[m.wing_of_line[i]];
+    const d3 axis = normalize(m.span_e[ws] - m.span_s[ws]);
+    const d3 chord_first = rotate_xyz(m.chord_not_rotated[ws], p.rotation);
+    out[2 * N + i] = angle_between(chord_first, u, axis);
+}
+
+__global__ void k_controller_input(DevModel m, StepParams p, const d3* v, double* out) {
+    const int i = blockIdx.x * kWindThreads + threadIdx.x;
+    if (i < m.N) controller_line(m, p, v, out, i);
+}
+
+__global__ void k_controller_input_jobs(const WindJob* jobs, int n) {
+    const WindJob& J = jobs[job_of_block<WindJob, &WindJob::blk_ctrl>(jobs, n, blockIdx.x)];
+    const int i = static_cast<int>(blockIdx.x - J.blk_ctrl) * kWindThreads + threadIdx.x;
+    if (i < J.m.N) controller_line(J.m, J.p, J.out, J.ctrl_out, i);
 }
 
 }  // namespace
 
+long long wind_blocks(int N, long long n_wake) { return (N + n_wake + kWindThreads - 1) / kWindThreads; }
+long long controller_input_blocks(int N) { return (N + kWindThreads - 1) / kWindThreads; }
+
+cudaError_t launch_wind_freestream_jobs(const WindJob* jobs, int n, long long blocks, cudaStream_t s) {
+    if (n <= 0 || blocks <= 0) return cudaSuccess;
+    k_wind_freestream_jobs<<<static_cast<unsigned>(blocks), kWindThreads, 0, s>>>(jobs, n);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_controller_input_jobs(const WindJob* jobs, int n, long long blocks, cudaStream_t s) {
+    if (n <= 0 || blocks <= 0) return cudaSuccess;
+    k_controller_input_jobs<<<static_cast<unsigned>(blocks), kWindThreads, 0, s>>>(jobs, n);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_controller_input(const DevModel& m, const StepParams& p, const d3* v, double* out, cudaStream_t s) {
     if (m.N <= 0) return cudaSuccess;
-    k_controller_input<<<(m.N + 127) / 128, 128, 0, s>>>(m, p, v, out);
+    k_controller_input<<<static_cast<unsigned>(controller_input_blocks(m.N)), kWindThreads, 0, s>>>(m, p, v, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_wind_freestream(const WindDevice& w, const d3* ctrl, const int* wing_of_line, int N, const d3* wake,
                                    long long n_wake, d3* out, cudaStream_t s) {
-    const long long n = N + n_wake;
-    if (n <= 0) return cudaSuccess;
-    k_wind_freestream<<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(w, ctrl, wing_of_line, N, wake, n_wake, out);
+    if (N + n_wake <= 0) return cudaSuccess;
+    k_wind_freestream<<<static_cast<unsigned>(wind_blocks(N, n_wake)), kWindThreads, 0, s>>>(w, ctrl, wing_of_line, N, wake, n_wake, out);
     return cudaGetLastError();
 }
 

@@ -190,6 +190,19 @@ __device__ inline double foil_cd(const FoilP& f, double a) {
     return raw + during;
 }
 
+// Job that block b of a launch over a job list belongs to: the last one whose first block of the kind is
+// at or before it (jobs [n] ascending in each kind's first block).
+template <class Job, long long Job::*First>
+__device__ inline int job_of_block(const Job* jobs, int n, long long b) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (jobs[mid].*First <= b) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
 // ---------------------------------------------------------------------------------------
 // Panel records
 // ---------------------------------------------------------------------------------------

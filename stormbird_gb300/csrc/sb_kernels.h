@@ -109,9 +109,16 @@ cudaError_t launch_unit_matrix(const PanelRec<double>* row0, const PanelRec<floa
                                int sym, int neglect, const int* wing_of_line, d3* factors, float* split, const d3* basis,
                                cudaStream_t s);
 // Quasi-steady horseshoe matrix; core_kind 0 relative (rc_dev: device scratch), 1 absolute, 2 none.
-cudaError_t launch_horseshoe_matrix(const DevModel& m, int core_kind, double core_value, double wake_length,
-                                    double* rc_dev, int sym, d3* factors, float* split, const d3* basis,
-                                    cudaStream_t s);
+struct HorseshoeArgs {
+    int core_kind = 0;  // 0: core_value of the mean line length, into rc_dev; 1: core_value; 2: none
+    double core_value = 0.0, wake_length = 0.0;
+    double* rc_dev = nullptr;
+    int sym = 0;
+    d3* factors = nullptr;
+    float* split = nullptr;
+    const d3* basis = nullptr;
+};
+cudaError_t launch_horseshoe_matrix(const DevModel& m, const HorseshoeArgs& h, cudaStream_t s);
 
 // ---- wake and geometry (k_wake.cu) ------------------------------------------------------
 struct WakeBuffers {
@@ -195,6 +202,18 @@ cudaError_t launch_wake_jobs(const CaseStepJob* jobs, int n, long long advect_bl
                              cudaStream_t s);
 cudaError_t launch_unit_matrix_jobs(const CaseStepJob* jobs, int n, long long blocks, cudaStream_t s);
 cudaError_t launch_chain_records_jobs(const CaseStepJob* jobs, int n, long long blocks, cudaStream_t s);
+
+// One quasi-steady case of a batched step, past its first: its geometry, core length and horseshoe matrix.
+struct QsStepJob {
+    DevModel m;
+    StepParams p;
+    const d3* fs_ctrl = nullptr;
+    HorseshoeArgs h;
+    long long blk_geometry = 0, blk_matrix = 0;
+};
+long long horseshoe_blocks(const DevModel& m);
+cudaError_t launch_prep_geometry_jobs(const QsStepJob* jobs, int n, long long blocks, cudaStream_t s);
+cudaError_t launch_horseshoe_matrix_jobs(const QsStepJob* jobs, int n, long long blocks, cudaStream_t s);
 
 // Records of caller-given panels for the standalone sweep (corners [P][4][3] in ring order).
 cudaError_t launch_panels_from_corners(const double* corners, const double* strengths, const double* cores, long long P,
@@ -370,6 +389,23 @@ struct WindDevice {
     const long long* ranges = nullptr;
     const double* step = nullptr;
 };
+// The wind of one case of a batch: geometry of the current angles and motion, freestream at the control
+// points and the wake points into out; controller measurements [3][N] into ctrl_out from out.
+struct WindJob {
+    DevModel m;
+    StepParams p;
+    WindDevice w;
+    const d3* wake = nullptr;
+    long long n_wake = 0;
+    d3* out = nullptr;
+    double* ctrl_out = nullptr;
+    long long blk_geometry = 0, blk_wind = 0, blk_ctrl = 0;
+};
+long long wind_blocks(int N, long long n_wake);
+long long controller_input_blocks(int N);
+cudaError_t launch_prep_geometry_jobs(const WindJob* jobs, int n, long long blocks, cudaStream_t s);
+cudaError_t launch_wind_freestream_jobs(const WindJob* jobs, int n, long long blocks, cudaStream_t s);
+cudaError_t launch_controller_input_jobs(const WindJob* jobs, int n, long long blocks, cudaStream_t s);
 // Freestream at the control points [N] then the wake points [n_wake] into out.
 cudaError_t launch_wind_freestream(const WindDevice& w, const d3* ctrl, const int* wing_of_line, int N, const d3* wake,
                                    long long n_wake, d3* out, cudaStream_t s);

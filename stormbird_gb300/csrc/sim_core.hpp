@@ -900,6 +900,31 @@ struct sb_sim {
     // chain records come from the batch's job-list launches (CaseStepJob).
     bool batch_kernels_ok() const { return dynamic && first_step_completed; }
 
+    // A quasi-steady case past its first step: geometry and horseshoe matrix come from QsStepJob lists.
+    bool batch_qs_kernels_ok() const { return !dynamic && first_step_completed; }
+    QsStepJob qs_step_job(double time, double dt) const {
+        QsStepJob j;
+        j.m = dm;
+        j.p = params;
+        j.p.time = time;
+        j.p.dt = dt;
+        j.fs_ctrl = fs_p;
+        j.h = horseshoe_args();
+        return j;
+    }
+    // The case's wind at the current state (the geometry of enqueue_wind_freestream, then the freestream).
+    WindJob wind_job(double* ctrl_out) const {
+        WindJob j;
+        j.m = dm;
+        j.p = params;
+        j.w = wind;
+        j.wake = dynamic ? pts[cur].p : nullptr;
+        j.n_wake = dynamic ? P_pts : 0;
+        j.out = fs_p;
+        j.ctrl_out = ctrl_out;
+        return j;
+    }
+
     // The case's job for a step, from the state before the step.
     CaseStepJob step_job(double time, double dt) const {
         CaseStepJob j;
@@ -927,7 +952,7 @@ struct sb_sim {
         params.dt = dt;
         launches = 0;
         swept[0] = swept[1] = false;
-        cur ^= 1;
+        if (dynamic) cur ^= 1;
     }
 
     // Influence matrix (unit matrix of the first wake row, or horseshoes) and the solve.
@@ -935,6 +960,20 @@ struct sb_sim {
     // In-plane bases for a two-component SimpleIterative matrix (no velocity correction: the
     // solve uses the velocity's in-plane part only), else nullptr (three components).
     const d3* split_basis() const { return solve.velocity_correction == 0 ? dm.solve_basis : nullptr; }
+
+    HorseshoeArgs horseshoe_args() const {
+        const auto& q = setup.quasi_steady_wake;
+        HorseshoeArgs h;
+        h.core_kind = static_cast<int>(q.viscous_core_length.kind);
+        h.core_value = q.viscous_core_length.value;
+        h.wake_length = q.wake_length_factor * dm.rep_chord;
+        h.rc_dev = qs_rc.p;
+        h.sym = static_cast<int>(q.symmetry_condition);
+        h.factors = factors.p;
+        h.split = factors_split.p;
+        h.basis = split_basis();
+        return h;
+    }
 
     void step_matrix() {
         if (dynamic) {
@@ -945,13 +984,9 @@ struct sb_sim {
                "unit matrix");
             launches += 1;
         } else {
-            const auto& q = setup.quasi_steady_wake;
-            double wl = q.wake_length_factor * dm.rep_chord;
-            ck(launch_horseshoe_matrix(dm, static_cast<int>(q.viscous_core_length.kind), q.viscous_core_length.value, wl,
-                                       qs_rc.p, static_cast<int>(q.symmetry_condition), factors.p,
-                                       factors_split.p, split_basis(), stream),
-               "horseshoe matrix");
-            launches += q.viscous_core_length.kind == sbsetup::CoreKind::Relative ? 2 : 1;
+            const HorseshoeArgs h = horseshoe_args();
+            ck(launch_horseshoe_matrix(dm, h, stream), "horseshoe matrix");
+            launches += h.core_kind == 0 ? 2 : 1;
             record(3);
         }
         record(4);

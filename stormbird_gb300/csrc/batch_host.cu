@@ -51,6 +51,8 @@ struct GatherJob {
     const double* scalars = nullptr;  // solver scalars ([4]: start taken)
     double* gamma_dst = nullptr;
     double* summary_dst = nullptr;
+    long long intf = 0, intm = 0, total_dst = 0;  // per-wing forces and moments in out; their place among the batch's
+    int n_int = 0;                                // values of each (k_gather_totals)
 };
 
 // One CTA per case: circulation and SB_BATCH_SUMMARY summary values into the compact buffer.
@@ -68,6 +70,16 @@ __global__ void k_gather(const GatherJob* jobs) {
         s[8] = g.out[g.converged];
         s[9] = static_cast<double>(*g.err);
         s[10] = g.scalars[4];
+    }
+}
+
+// One CTA per case: its per-wing integrated forces, then moments, into the batch's buffer.
+__global__ void k_gather_totals(const GatherJob* jobs, double* totals) {
+    const GatherJob& g = jobs[blockIdx.x];
+    double* d = totals + g.total_dst;
+    for (int i = threadIdx.x; i < g.n_int; i += blockDim.x) {
+        d[i] = g.out[g.intf + i];
+        d[g.n_int + i] = g.out[g.intm + i];
     }
 }
 
@@ -142,6 +154,7 @@ struct sb_batch {
     DevBuf<QsStepJob> d_qs_jobs;
     int n_qs_jobs = 0;
     long long blk_qs_geometry = 0, blk_qs_matrix = 0;
+    WindArena wind_arena;
     PinnedBuf<WindJob> h_wind_jobs;  // every case (with set_wind)
     DevBuf<WindJob> d_wind_jobs;
     long long blk_wind_geometry = 0, blk_wind = 0, blk_ctrl = 0;
@@ -199,6 +212,7 @@ struct sb_batch {
     DevBuf<double> ctrl_in;
     PinnedBuf<double> h_ctrl_in;
     PinnedBuf<double> h_wing_totals;
+    DevBuf<double> wing_totals_dev;
 
     bool use_graph = true;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -270,6 +284,7 @@ struct sb_batch {
         h_compact.alloc(ncomp);
         std::memset(h_compact.p, 0, ncomp * sizeof(double));
         std::vector<GatherJob> gj;
+        long long totals = 0;
         for (size_t i = 0; i < cases.size(); ++i) {
             sb_sim& c = *cases[i];
             c.fs_p = fs_all.p + fs_off[i];
@@ -287,6 +302,11 @@ struct sb_batch {
             g.scalars = c.scalars.p;
             g.gamma_dst = compact.p + line_off[i];
             g.summary_dst = compact.p + N_total + static_cast<long long>(i) * SB_BATCH_SUMMARY;
+            g.intf = c.L.intf;
+            g.intm = c.L.intm;
+            g.n_int = c.S * 18;
+            g.total_dst = totals;
+            totals += 2 * g.n_int;
             gj.push_back(g);
         }
         gather_jobs.upload(gj);
@@ -1007,15 +1027,22 @@ struct sb_batch {
             wind_steps.alloc(cases.size() * 2);
             h_wind_steps.alloc(cases.size() * 2);
         }
+        std::vector<WindPack> packs;
+        packs.reserve(cases.size());
+        sbsetup::WindEnvironment env;
         for (size_t i = 0; i < cases.size(); ++i) {
             if (!cond_jsons[i]) raise(SB_ERR_NULL_ARG, "wind condition of case " + std::to_string(i) + " is NULL");
             try {
-                cases[i]->set_wind(env_json, cond_jsons[i]);
+                if (i == 0) env = sbsetup::parse_wind_environment(env_json);
+                packs.push_back(cases[i]->pack_wind(env, sbsetup::parse_wind_condition(cond_jsons[i])));
+            } catch (const sbsetup::SetupError& e) {
+                raise(SB_ERR_BAD_JSON, "case " + std::to_string(i) + ": " + e.what());
             } catch (const SbFail& e) {
                 raise(e.code, "case " + std::to_string(i) + ": " + e.msg);
             }
-            cases[i]->wind.step = wind_steps.p + 2 * i;
         }
+        wind_arena.upload(packs, main);
+        for (size_t i = 0; i < cases.size(); ++i) cases[i]->use_wind(packs[i].w, wind_steps.p + 2 * i);
         has_wind = true;
     }
 
@@ -1063,18 +1090,14 @@ struct sb_batch {
     const double* wing_totals() {
         size_t total = 0;
         for (const auto& c : cases) total += static_cast<size_t>(c->S) * 36;
-        if (h_wing_totals.n < total) h_wing_totals.alloc(total);
-        size_t off = 0;
-        for (const auto& c : cases) {
-            const size_t n = static_cast<size_t>(c->S) * 18;
-            ck(cudaMemcpyAsync(h_wing_totals.p + off, c->out.p + c->L.intf, n * sizeof(double), cudaMemcpyDeviceToHost,
-                               main),
-               "D2H wing forces");
-            ck(cudaMemcpyAsync(h_wing_totals.p + off + n, c->out.p + c->L.intm, n * sizeof(double),
-                               cudaMemcpyDeviceToHost, main),
-               "D2H wing moments");
-            off += 2 * n;
+        if (h_wing_totals.n < total) {
+            h_wing_totals.alloc(total);
+            wing_totals_dev.alloc(total);
         }
+        k_gather_totals<<<static_cast<unsigned>(cases.size()), 128, 0, main>>>(gather_jobs.p, wing_totals_dev.p);
+        ck(cudaGetLastError(), "wing totals");
+        ck(cudaMemcpyAsync(h_wing_totals.p, wing_totals_dev.p, total * sizeof(double), cudaMemcpyDeviceToHost, main),
+           "D2H wing totals");
         ck(cudaStreamSynchronize(main), "wing totals");
         return h_wing_totals.p;
     }

@@ -107,6 +107,60 @@ struct PinnedBuf {
     }
 };
 
+// Wind model of one condition: the device struct, and on the host the tables it points to (w.spec_off
+// within data; dirs and the corrections within data, ints and ranges).
+struct WindPack {
+    WindDevice w;
+    std::vector<double> data;
+    std::vector<int> ints;
+    std::vector<long long> ranges;
+    size_t dirs_off = 0, corr_base = 0;
+};
+
+// The tables of one or many wind models in one device buffer, kept from one condition to the next and
+// written by one copy (three allocations and blocking copies per model took 36 us, 1.3 ms for a sweep of 36
+// wind directions).
+struct WindArena {
+    DevBuf<double> dev;
+    PinnedBuf<double> host;
+    // Uploads the packs' tables and points each pack's device struct at them. Everything enqueued on s
+    // before has read the old tables by the time this returns.
+    void upload(std::vector<WindPack>& packs, cudaStream_t s) {
+        static_assert(sizeof(long long) == sizeof(double) && 2 * sizeof(int) == sizeof(double), "8-byte slots");
+        size_t n = 0;
+        for (const auto& p : packs) n += p.data.size() + p.ranges.size() + (p.ints.size() + 1) / 2;
+        n = std::max<size_t>(n, 1);
+        ck(cudaStreamSynchronize(s), "wind tables");
+        if (dev.n < n) {
+            dev.alloc(n);
+            host.alloc(n);
+        }
+        size_t at = 0;
+        for (auto& p : packs) {
+            WindDevice& w = p.w;
+            auto put = [&](const void* src, size_t bytes, size_t slots) {
+                if (bytes) std::memcpy(host.p + at, src, bytes);
+                const double* d = dev.p + at;
+                at += slots;
+                return d;
+            };
+            const double* data = put(p.data.data(), p.data.size() * sizeof(double), p.data.size());
+            w.spectra = data;
+            const double* ranges = put(p.ranges.data(), p.ranges.size() * sizeof(long long), p.ranges.size());
+            const double* ints = put(p.ints.data(), p.ints.size() * sizeof(int), (p.ints.size() + 1) / 2);
+            if (w.n_dirs > 0) {
+                w.dirs = data + p.dirs_off;
+                w.corr = data + p.corr_base;
+                w.corr_off = reinterpret_cast<const int*>(ints);
+                w.corr_len = w.corr_off + w.n_dirs;
+                w.ranges = reinterpret_cast<const long long*>(ranges);
+            }
+        }
+        if (at > 0) ck(cudaMemcpyAsync(dev.p, host.p, at * sizeof(double), cudaMemcpyHostToDevice, s), "H2D wind tables");
+        ck(cudaStreamSynchronize(s), "wind tables");
+    }
+};
+
 inline FoilP to_dev(const sbsetup::Foil& f) {
     FoilP o;
     o.stall_slope = 4.5951212 / f.stall_range;
@@ -369,9 +423,8 @@ struct sb_sim {
     // time and ship velocity (device memory; a batch points `wind.step` at its own array).
     bool has_wind = false;
     WindDevice wind;
-    DevBuf<double> wind_data, wind_step_own;
-    DevBuf<int> wind_ints;
-    DevBuf<long long> wind_ranges;
+    DevBuf<double> wind_step_own;
+    WindArena wind_arena;
     PinnedBuf<double> h_wind_step;
     int chain_SP = 0;
     long long chain_Bq = 0, chain_Q = 0;
@@ -1320,16 +1373,10 @@ struct sb_sim {
     }
 
     // ---------------------------------------------------------------- wind model
-    void set_wind(const char* env_json, const char* cond_json) {
-        sbsetup::WindEnvironment env;
-        sbsetup::WindCondition cond;
-        try {
-            env = sbsetup::parse_wind_environment(env_json);
-            cond = sbsetup::parse_wind_condition(cond_json);
-        } catch (const sbsetup::SetupError& e) {
-            raise(SB_ERR_BAD_JSON, e.what());
-        }
-        WindDevice w;
+    // The wind model of one condition, its tables still on the host.
+    WindPack pack_wind(const sbsetup::WindEnvironment& env, const sbsetup::WindCondition& cond) const {
+        WindPack k;
+        WindDevice& w = k.w;
         auto d3of = [](const sbsetup::Vec3& v) { return mk(v.x, v.y, v.z); };
         w.up = d3of(env.up_direction);
         w.axis = d3of(env.wind_rotation_axis);
@@ -1349,20 +1396,21 @@ struct sb_sim {
         w.von_karman = v.von_karman_constant;
         w.stable_coefficient = v.stable_coefficient;
         w.unstable_coefficient = v.unstable_coefficient;
-        std::vector<double> data;
+        std::vector<double>& data = k.data;
         const sbsetup::Spectrum* gusts[3] = {&cond.parallel_gust, &cond.perpendicular_gust, &cond.vertical_gust};
-        for (int k = 0; k < 3; ++k) {
-            if (!gusts[k]->present) continue;
-            w.spec_off[k] = static_cast<int>(data.size());
-            w.spec_n[k] = static_cast<int>(gusts[k]->frequencies.size());
-            data.insert(data.end(), gusts[k]->frequencies.begin(), gusts[k]->frequencies.end());
-            data.insert(data.end(), gusts[k]->amplitudes.begin(), gusts[k]->amplitudes.end());
-            data.insert(data.end(), gusts[k]->phases.begin(), gusts[k]->phases.end());
+        for (int q = 0; q < 3; ++q) {
+            if (!gusts[q]->present) continue;
+            w.spec_off[q] = static_cast<int>(data.size());
+            w.spec_n[q] = static_cast<int>(gusts[q]->frequencies.size());
+            data.insert(data.end(), gusts[q]->frequencies.begin(), gusts[q]->frequencies.end());
+            data.insert(data.end(), gusts[q]->amplitudes.begin(), gusts[q]->amplitudes.end());
+            data.insert(data.end(), gusts[q]->phases.begin(), gusts[q]->phases.end());
         }
-        std::vector<int> ints;
-        std::vector<long long> ranges;
+        std::vector<int>& ints = k.ints;
+        std::vector<long long>& ranges = k.ranges;
         const auto& ic = env.inflow_corrections;
-        size_t dirs_off = data.size(), corr_base = 0;
+        size_t& corr_base = k.corr_base;
+        k.dirs_off = data.size();
         if (ic.present) {
             // the reference indexes each direction's wing ranges by wing (inflow_corrections.rs:28)
             for (const auto& c : ic.corrections)
@@ -1387,24 +1435,29 @@ struct sb_sim {
             ints = offs;
             ints.insert(ints.end(), lens.begin(), lens.end());
         }
-        wind_data.upload(data.empty() ? std::vector<double>{0.0} : data);
-        wind_ints.upload(ints.empty() ? std::vector<int>{0} : ints);
-        wind_ranges.upload(ranges.empty() ? std::vector<long long>{0} : ranges);
-        w.spectra = wind_data.p;
-        if (ic.present) {
-            w.dirs = wind_data.p + dirs_off;
-            w.corr = wind_data.p + corr_base;
-            w.corr_off = wind_ints.p;
-            w.corr_len = wind_ints.p + w.n_dirs;
-            w.ranges = wind_ranges.p;
+        return k;
+    }
+    // Takes a wind model whose tables lie on the device.
+    void use_wind(const WindDevice& w, const double* step) {
+        wind = w;
+        wind.step = step;
+        has_wind = true;
+    }
+
+    void set_wind(const char* env_json, const char* cond_json) {
+        std::vector<WindPack> packs;
+        try {
+            const sbsetup::WindEnvironment env = sbsetup::parse_wind_environment(env_json);
+            packs.push_back(pack_wind(env, sbsetup::parse_wind_condition(cond_json)));
+        } catch (const sbsetup::SetupError& e) {
+            raise(SB_ERR_BAD_JSON, e.what());
         }
         if (wind_step_own.n == 0) {
             wind_step_own.alloc(2);
             h_wind_step.alloc(2);
         }
-        w.step = has_wind && wind.step ? wind.step : wind_step_own.p;
-        wind = w;
-        has_wind = true;
+        wind_arena.upload(packs, stream);
+        use_wind(packs[0].w, has_wind && wind.step ? wind.step : wind_step_own.p);
     }
 
     void set_wind_step(double time, double ship_velocity) {

@@ -429,20 +429,24 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
         __syncthreads();
         if (s_item >= n_items) break;
         const BsJob& J = s_job;
-        const long long ttile = s_ttile;
 
         // targets: float-float pairs (FP32) or doubles (FP64 path, lo parts 0)
         R xh[TT], yh[TT], zh[TT], xl[TT], yl[TT], zl[TT];
         bool valid[TT];
         int tw[TT];
+        // with the far-field fast path a warp's targets are consecutive points (a compact box), T adjacent ones
+        // to a thread; else a thread's targets are T rows of the tile apart
+        const int wt = FAST_FAR && J.warp_targets > 0 ? J.warp_targets : 32 * T;
+        const bool mine = lane * T < wt;
+        auto target_slot = [&](int t) {
+            return FAST_FAR ? (s_ttile * kWarps + (tid >> 5)) * wt + lane * T + t
+                            : s_ttile * TM + static_cast<long long>(t) * kBsThreads + tid;
+        };
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-            // with the far-field fast path a thread's targets are adjacent (a warp's 64 targets
-            // are consecutive points, a compact box); else T rows of the tile apart
-            const long long slot = ttile * TM + (FAST_FAR ? static_cast<long long>(tid) * T + t
-                                                          : static_cast<long long>(t) * kBsThreads + tid);
+            const long long slot = target_slot(t);
             const long long idx = FAST_FAR ? bs_slot_target(J, slot) : slot;
-            valid[t] = slot < bs_slots(J) && idx < J.M;
+            valid[t] = mine && slot < bs_slots(J) && idx < J.M;
             d3 p = valid[t] ? J.targets[idx] : mk(0, 0, 0);
             tw[t] = (NEGLECT && valid[t]) ? J.target_wing[idx] : -1;
             d3 q[2] = {p, SYM ? mirror(SYM, p) : p};
@@ -459,6 +463,10 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
                 tw[u] = tw[t];
             }
         }
+        bool some = false;
+#pragma unroll
+        for (int t = 0; t < T; ++t) some = some || valid[t];
+        const bool busy = __any_sync(0xffffffffu, some);
         // running sums and compensations; for FP32 lane j of a float2 is target j (s_acc)
         R sx[TT], sy[TT], sz[TT], cx[TT], cy[TT], cz[TT];
         if constexpr (SMEM_ACC) {
@@ -534,7 +542,9 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
                 if (lane == 0) s_timed_out = 1;
                 break;
             }
-            const int np = tile_panels(k);
+            // a warp without targets (a last or only target tile) goes past the panels: on 32 targets its three
+            // per-pair tests of every panel against nothing took twice as long as the one working warp
+            const int np = busy ? tile_panels(k) : 0;
             {
                 if constexpr (F32) {
                     float2 TX = bc(0.f), TY = bc(0.f), TZ = bc(0.f);
@@ -730,7 +740,6 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
             }
         }
 
-        const long long ttile_out = s_ttile;
         const int chunk = s_chunk;
         if constexpr (SMEM_ACC) {
 #pragma unroll
@@ -745,10 +754,9 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
         }
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-            const long long slot = ttile_out * TM + (FAST_FAR ? static_cast<long long>(tid) * T + t
-                                                              : static_cast<long long>(t) * kBsThreads + tid);
+            const long long slot = target_slot(t);
             const long long idx = FAST_FAR ? bs_slot_target(J, slot) : slot;
-            if (slot < bs_slots(J) && idx < J.M) {
+            if (mine && slot < bs_slots(J) && idx < J.M) {
                 d3 u = mk(static_cast<double>(sx[t]) + static_cast<double>(cx[t]),
                           static_cast<double>(sy[t]) + static_cast<double>(cy[t]),
                           static_cast<double>(sz[t]) + static_cast<double>(cz[t]));

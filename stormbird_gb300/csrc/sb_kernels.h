@@ -23,7 +23,8 @@ struct BsJob {
     long long M = 0;
     int chunk_panels = 0;              // panels per source chunk (multiple of the tile)
     int n_chunks = 1;
-    long long n_ttiles = 0;            // target tiles of kBsThreads * T targets
+    long long n_ttiles = 0;            // target tiles of kBsThreads * T targets, or of 4 warps x warp_targets
+    int warp_targets = 0;              // targets of a warp, a multiple of T (FP32 far-field sweeps; 0: 32 T)
     double* partial = nullptr;         // [n_chunks][M][3]
     long long item_begin = 0;          // first item of this sweep in a batched launch
     // reduction (batched launches): out[i] = base[i] + sum over chunks, base only for i >= M

@@ -277,6 +277,21 @@ inline SweepPlan make_sweep_plan(long long M, long long P, int precision, int sy
     return sp;
 }
 
+// Fewer targets to a warp of an FP32 far-field sweep while its items leave SMs idle: a warp's time is that of the
+// panels near any of its targets (some 900 cycles each), and a target's sums do not depend on the others. 21
+// targets x 2,100 panels (33 chunks): 41 us with 64 targets a warp, 28 with 2; filling the SMs more than once
+// over gained nothing (183 x 54,900: 62 either way).
+inline void spread_targets(BsJob& J, SweepPlan& sp, int sym, int sms) {
+    const int T = bs_targets_per_thread(sym);
+    auto tiles = [&](int w) { return (bs_slots(J) + kBsThreads / 32 * w - 1) / (kBsThreads / 32 * w); };
+    int w = 32 * T;
+    while (w > T && tiles(w / 2) * sp.n_chunks <= sms) w /= 2;
+    if (w == 32 * T) return;
+    J.warp_targets = w;
+    sp.n_ttiles = tiles(w);
+    sp.grid = static_cast<int>(sp.n_ttiles * sp.n_chunks);
+}
+
 // Device work space of one standalone call: stream-ordered allocations freed on exit.
 struct StreamBufs {
     cudaStream_t s = nullptr;
@@ -329,6 +344,7 @@ inline void panel_sweep_impl(int device, const double* corners, const double* st
         a.job0.p_end = P;
         a.job0.targets = dt;
         a.job0.M = M;
+        if (precision != 2) spread_targets(a.job0, sp, symmetry, num_sms(device));
         a.job0.chunk_panels = sp.chunk;
         a.job0.n_chunks = sp.n_chunks;
         a.job0.n_ttiles = sp.n_ttiles;
@@ -824,6 +840,7 @@ struct sb_sim {
             a.job0.targets = targets;
             a.job0.target_wing = twing;
             a.job0.M = M;
+            if (precision != 2 && !d.chain && !neglect) spread_targets(a.job0, sp, sym, sms);
             a.job0.chunk_panels = sp.chunk;
             a.job0.n_chunks = sp.n_chunks;
             a.job0.n_ttiles = sp.n_ttiles;

@@ -48,3 +48,19 @@ def test_runs(gpu_lib, oracle_mod, panels, zeros, symmetry):
         m = oracle_mod.bs_sweep(corners, core, g, 1.5, mirrored, nthreads=4)
         ref = ref + m * [1.0, 1.0, -1.0]
     assert rel_inf(ours, ref) <= 1e-5
+
+
+@pytest.mark.parametrize("symmetry", [0, 3])
+@pytest.mark.parametrize("targets", [1, 2, 3, 7, 8, 9, 31, 33, 64, 65, 130, 255, 256])
+def test_few_targets(gpu_lib, targets, symmetry):
+    """With few targets a warp takes 32 down to 1 or 2 of them: a target's velocity stays the one it has among
+    256, bit for bit (its sums run over the same panels in the same order)."""
+    rng = np.random.default_rng(8)
+    panels = 150
+    k = np.arange(panels)
+    quad = np.array([[0, 0, 0], [1, 0, 0], [1, 1, 0], [0, 1, 0]], dtype=float)
+    corners = quad + np.stack([k // 5, k % 5, 5.0 + 0 * k], axis=1)[:, None, :] + rng.normal(0, 0.05, (panels, 4, 3))
+    g, core = rng.normal(0, 1, panels), np.full(panels, 0.05)
+    x = rng.uniform([0, 0, 5.2], [30, 5, 8], (256, 3))
+    every = panel_sweep(corners, g, core, x, far_field_ratio=3.0, symmetry=symmetry)
+    assert np.array_equal(panel_sweep(corners, g, core, x[:targets], far_field_ratio=3.0, symmetry=symmetry), every[:targets])

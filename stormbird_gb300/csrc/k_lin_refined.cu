@@ -16,6 +16,8 @@
 //      the FP32 inverse is good for);
 //   4. induced velocities, viscous correction, residual and outputs (linearized.rs:141-213), each CTA
 //      its rows.
+// Steps 1 and 4 are FP64 work of N^2 entries. One large case alone has them done by all SMs before and after
+// the cluster (k_lin_build, k_lin_finish; kSplitLines).
 // No pivoting across blocks: the diagonal dominates (2 / (c u) plus the line's own trailing pair
 // against its neighbours'), and a system where that fails shows in step 3. Where a pivot is below
 // 1e-6 (the reference calls 1e-12 singular), a correction does not shrink or a value is not finite,
@@ -89,6 +91,82 @@ __device__ __forceinline__ double residual_of(const DevModel& m, int i, double g
     return fabs(clg - cl_pre);
 }
 
+// lin_work: scaled rows [2][16][n] floats, the f64 matrix [N][N], and for a split solve its FP32 copy [n][n], the
+// right-hand side [n], the solution [n], the circulation [n] after the viscous correction, the residual terms [n]
+// and a counter.
+struct Work {
+    float* Pg;
+    double* A64;
+    float* A32;
+    double *rhs, *x, *g, *terms;
+    unsigned* counter;
+    __device__ Work(double* p, int N) {
+        const size_t n = padded(N);
+        Pg = reinterpret_cast<float*>(p);
+        A64 = p + kBlk * n;
+        double* q = A64 + (static_cast<size_t>(N) * N + 1) / 2 * 2;
+        A32 = reinterpret_cast<float*>(q);
+        rhs = q + n * n / 2;
+        x = rhs + n;
+        g = x + n;
+        terms = g + n;
+        counter = reinterpret_cast<unsigned*>(terms + n);
+    }
+    static size_t doubles(int N) {
+        const size_t n = padded(N);
+        return kBlk * n + (static_cast<size_t>(N) * N + 1) / 2 * 2 + n * n / 2 + 4 * n + 2;
+    }
+};
+
+// Row i of the system (linearized.rs:61-136): dot(factors[i][c], w) + diagonal, with w = -cl slope / u_t x the
+// normal of the row's in-plane velocity.
+struct SystemRow {
+    d3 w;
+    double rhs, diag;
+};
+__device__ __noinline__ SystemRow system_row(const DevModel& m, const SolveBuffers& b, int i, const double* tab) {
+    SystemRow r;
+    const d3 sd = normalize(m.span_e[i] - m.span_s[i]);
+    d3 v = m.felt_ctrl[i] + b.fixed[i];
+    v = v - sd * dot(v, sd);
+    const d3 un = normalize(v);
+    const double iut = rcp_any(dot(v, un));
+    const FoilP& f = m.foils[m.wing_of_line[i]];
+    r.w = cross(un, sd) * (-f.cl_initial_slope * iut);
+    r.rhs = -line_lift(f, m.chord_global[i], v, sd, tab).cl_linear;
+    r.diag = 2.0 * iut * rcp_any(m.chord_len[i]);
+    return r;
+}
+__device__ __noinline__ LineLift lift_at(const DevModel& m, int i, d3 v, const double* tab) {
+    return line_lift(m.foils[m.wing_of_line[i]], m.chord_global[i], v, normalize(m.span_e[i] - m.span_s[i]), tab);
+}
+// The viscous correction of line i's circulation (linearized.rs:178-202)
+__device__ __forceinline__ double corrected_circulation(const LineLift& o, double x) {
+    return fabs(o.cl_linear) > kMinPositive ? x * (o.cl_pre / o.cl_linear) : x;
+}
+__device__ __forceinline__ void write_line(const SolveBuffers& b, int i, double gi, d3 v) {
+    b.gamma_prev[i] = gi;
+    b.vel_out[i] = v;
+    if (b.wake_str_row0) b.wake_str_row0[i] = gi;
+    if (b.rec32_row0) b.rec32_row0[i].v[kRec32Gamma] = static_cast<float>(gi);
+    if (b.rec64_row0) b.rec64_row0[i].v[kRec64Gamma] = gi;
+}
+// Mean of the residual terms and the solve's flags, by one warp.
+__device__ __forceinline__ void write_scalars(const SolveBuffers& b, const double* terms, int N, int lane) {
+    double s = 0.0;
+    for (int i = lane; i < N; i += 32) s += terms[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+        b.scalars[0] = s / static_cast<double>(N);
+        b.scalars[1] = 1.0;
+        b.scalars[2] = 1.0;
+        b.scalars[5] = 1.0;
+    }
+}
+
+// SPLIT: the system comes from k_lin_build, and the solution goes to k_lin_finish (scalars[5] = 2).
+template <bool SPLIT>
 __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuffers& b, unsigned char* dyn) {
     cg::cluster_group cl = cg::this_cluster();
     const int C = static_cast<int>(cl.num_blocks()), rank = static_cast<int>(cl.block_rank());
@@ -108,8 +186,9 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
     double* rhs = reinterpret_cast<double*>(dyn + L.rhs);
     double* diag = rhs + R;
     double* tab = reinterpret_cast<double*>(dyn + L.tab);
-    float* Pg = reinterpret_cast<float*>(b.lin_work);          // [2][16][n] (lin_work_doubles)
-    double* A64 = b.lin_work + static_cast<size_t>(kBlk) * n;  // [N][N]
+    const Work W(b.lin_work, N);
+    float* Pg = W.Pg;
+    double* A64 = W.A64;
     __shared__ __align__(16) float s_inv[kBlk][kBlk];
     __shared__ float s_red[kWarps][2];
     __shared__ int s_bad;
@@ -121,42 +200,41 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
         else __syncthreads();
     };
 
-    load_f64_tables(tab, tid, kThreads);
     if (tid == 0) s_bad = 0;
-    __syncthreads();
-    // 1. the system (linearized.rs:61-136): row i is dot(factors[i][c], w_i) + diagonal, with
-    // w_i = -cl slope / u_t x the normal of the row's in-plane velocity
-    for (int l = tid; l < R; l += kThreads) {
-        const int i = row_of(l);
-        roww[l] = mk(0, 0, 0);
-        rhs[l] = 0.0;
-        diag[l] = 1.0;  // rows past the end: the identity
-        if (i < N) {
-            const d3 sd = normalize(m.span_e[i] - m.span_s[i]);
-            d3 v = m.felt_ctrl[i] + b.fixed[i];
-            v = v - sd * dot(v, sd);
-            const d3 un = normalize(v);
-            const double iut = rcp_any(dot(v, un));
-            const FoilP& f = m.foils[m.wing_of_line[i]];
-            roww[l] = cross(un, sd) * (-f.cl_initial_slope * iut);
-            rhs[l] = -line_lift(f, m.chord_global[i], v, sd, tab).cl_linear;
-            diag[l] = 2.0 * iut * rcp_any(m.chord_len[i]);
+    // 1. the system; rows past the end: the identity
+    if constexpr (SPLIT) {
+        for (int l = tid; l < R; l += kThreads) rhs[l] = row_of(l) < n ? W.rhs[row_of(l)] : 0.0;
+        for (int t = tid; t < R * n / 4; t += kThreads) {
+            const int l = t / (n / 4), c = t % (n / 4) * 4, i = row_of(l);
+            reinterpret_cast<float4*>(A)[t] = i < n ? __ldcg(reinterpret_cast<const float4*>(W.A32 + static_cast<long long>(i) * n + c))
+                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-    }
-    __syncthreads();
-    for (int l = warp; l < R; l += kWarps) {
-        const int i = row_of(l);
-        const d3 w = roww[l];
-        const double dg = diag[l];
-        for (int c = lane; c < n; c += 32) {
-            float a = i == c && i >= N ? 1.f : 0.f;
-            if (i < N && c < N) {
-                double v = dot(b.factors[static_cast<long long>(i) * N + c], w);
-                if (i == c) v += dg;
-                A64[static_cast<long long>(i) * N + c] = v;
-                a = static_cast<float>(v);
+    } else {
+        load_f64_tables(tab, tid, kThreads);
+        __syncthreads();
+        for (int l = tid; l < R; l += kThreads) {
+            const int i = row_of(l);
+            SystemRow r = {mk(0, 0, 0), 0.0, 1.0};
+            if (i < N) r = system_row(m, b, i, tab);
+            roww[l] = r.w;
+            rhs[l] = r.rhs;
+            diag[l] = r.diag;
+        }
+        __syncthreads();
+        for (int l = warp; l < R; l += kWarps) {
+            const int i = row_of(l);
+            const d3 w = roww[l];
+            const double dg = diag[l];
+            for (int c = lane; c < n; c += 32) {
+                float a = i == c && i >= N ? 1.f : 0.f;
+                if (i < N && c < N) {
+                    double v = dot(b.factors[static_cast<long long>(i) * N + c], w);
+                    if (i == c) v += dg;
+                    A64[static_cast<long long>(i) * N + c] = v;
+                    a = f64_to_f32(v);
+                }
+                A[static_cast<long long>(l) * n + c] = a;
             }
-            A[static_cast<long long>(l) * n + c] = a;
         }
     }
     __syncthreads();
@@ -396,6 +474,13 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
         return;
     }
 
+    if constexpr (SPLIT) {
+        for (int l = tid; l < R; l += kThreads)
+            if (row_of(l) < N) W.x[row_of(l)] = x[row_of(l)];
+        if (rank == 0 && tid == 0) b.scalars[5] = 2.0;
+        barrier();
+        return;
+    }
     // 4. induced velocity, total velocity, viscous correction (linearized.rs:141-202)
     auto total_velocities = [&](const double* gam) {
         for (int l = 4 * warp + (lane >> 3); l < R; l += 4 * kWarps) {
@@ -427,9 +512,7 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
         for (int l = tid; l < R; l += kThreads) {
             const int i = row_of(l);
             if (i >= N) break;
-            const LineLift o = line_lift(m.foils[m.wing_of_line[i]], m.chord_global[i], vel[l],
-                                         normalize(m.span_e[i] - m.span_s[i]), tab);
-            store_all(g, i, fabs(o.cl_linear) > kMinPositive ? x[i] * (o.cl_pre / o.cl_linear) : x[i]);
+            store_all(g, i, corrected_circulation(lift_at(m, i, vel[l], tab), x[i]));
         }
         barrier();
         gam = g;
@@ -444,40 +527,118 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
         if (i >= N) break;
         const double gi = gam[i];
         const d3 v = vel[l];
-        const LineLift o = line_lift(m.foils[m.wing_of_line[i]], m.chord_global[i], v,
-                                     normalize(m.span_e[i] - m.span_s[i]), tab);
-        *(cl.map_shared_rank(terms, 0) + i) = residual_of(m, i, gi, v, o.cl_pre);
-        b.gamma_prev[i] = gi;
-        b.vel_out[i] = v;
-        if (b.wake_str_row0) b.wake_str_row0[i] = gi;
-        if (b.rec32_row0) b.rec32_row0[i].v[kRec32Gamma] = static_cast<float>(gi);
-        if (b.rec64_row0) b.rec64_row0[i].v[kRec64Gamma] = gi;
+        *(cl.map_shared_rank(terms, 0) + i) = residual_of(m, i, gi, v, lift_at(m, i, v, tab).cl_pre);
+        write_line(b, i, gi, v);
     }
     barrier();
-    if (rank == 0 && warp == 0) {
-        double s = 0.0;
-        for (int i = lane; i < N; i += 32) s += terms[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0) {
-            b.scalars[0] = s / static_cast<double>(N);
-            b.scalars[1] = 1.0;
-            b.scalars[2] = 1.0;
-            b.scalars[5] = 1.0;
-        }
+    if (rank == 0 && warp == 0) write_scalars(b, terms, N, lane);
+}
+
+// Lines from which a case alone has its system built and its results evaluated by all SMs. Solve in us, one
+// kernel / split: 256 lines 121 / 131, 384 193 / 191, 570 347 / 318, 768 516 / 479 (two or three launches of
+// some 20 us, of which the chain of a line's lift is 10, against N^2 / 16 entries of FP64 work a CTA).
+constexpr int kSplitLines = 448;
+constexpr int kRowThreads = 128;  // a warp to a row, four rows a CTA
+constexpr int kRowWarps = kRowThreads / 32;
+
+// Step 1 for four rows: one warp's lanes evaluate the rows' vectors side by side, then a warp takes each
+// row's entries. FP64-bound: 4 instructions an entry.
+__global__ void __launch_bounds__(kRowThreads) k_lin_build(DevModel m, SolveBuffers b) {
+    __shared__ __align__(16) double tab[kF64TableDoubles + 1];
+    __shared__ SystemRow rows[kRowWarps];
+    const int N = m.N, n = padded(N), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Work W(b.lin_work, N);
+    load_f64_tables(tab, tid, kRowThreads);
+    __syncthreads();
+    if (tid < kRowWarps) {
+        const int i = blockIdx.x * kRowWarps + tid;
+        SystemRow r = {mk(0, 0, 0), 0.0, 1.0};
+        if (i < N) r = system_row(m, b, i, tab);
+        rows[tid] = r;
+        if (i < n) W.rhs[i] = r.rhs;
+        if (i == 0) *W.counter = 0;
     }
+    __syncthreads();
+    const int i = blockIdx.x * kRowWarps + warp;
+    if (i >= n) return;
+    const SystemRow r = rows[warp];
+#pragma unroll 4
+    for (int c = lane; c < n; c += 32) {
+        float a = i == c && i >= N ? 1.f : 0.f;
+        if (i < N && c < N) {
+            double v = dot(b.factors[static_cast<long long>(i) * N + c], r.w);
+            if (i == c) v += r.diag;
+            W.A64[static_cast<long long>(i) * N + c] = v;
+            a = f64_to_f32(v);
+        }
+        W.A32[static_cast<long long>(i) * n + c] = a;
+    }
+}
+
+// Step 4 for four rows, eight lanes a row as in the one-kernel form (the same bits alone and in a batch), a
+// warp to each component (a lone warp issues an FP64 instruction per 65 cycles, three of them on an SM as well).
+// pass 0: the velocity from the solution and the corrected circulation; it
+// is the last one unless the correction's own induced velocities are wanted (pass 1). The last CTA of the
+// last pass sums the residual.
+constexpr int kFinishThreads = 96;
+__global__ void __launch_bounds__(kFinishThreads) k_lin_finish(DevModel m, SolveSettings st, SolveBuffers b, int pass, int last) {
+    __shared__ __align__(16) double tab[kF64TableDoubles + 1];
+    __shared__ double ind[kRowWarps][3];
+    if (b.scalars[5] != 2.0) return;  // the elimination kernels take the case
+    const int N = m.N, lane = threadIdx.x & 31, comp = threadIdx.x >> 5;
+    const Work W(b.lin_work, N);
+    load_f64_tables(tab, threadIdx.x, kFinishThreads);
+    const double* gam = pass == 0 ? W.x : W.g;
+    int i = blockIdx.x * kRowWarps + (lane >> 3);
+    double s = 0.0;
+    if (i < N) {
+        const double* f = reinterpret_cast<const double*>(b.factors + static_cast<long long>(i) * N) + comp;
+#pragma unroll 4
+        for (int c = lane & 7; c < N; c += 8) s = fma(f[3 * c], gam[c], s);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((lane & 7) == 0) ind[lane >> 3][comp] = s;
+    __syncthreads();
+    if (comp > 0) return;
+    i = blockIdx.x * kRowWarps + lane;
+    if (lane < kRowWarps && i < N) {
+        const d3 u = b.fixed[i] + mk(ind[lane][0], ind[lane][1], ind[lane][2]), fs = m.felt_ctrl[i];
+        const d3 v = st.velocity_correction == 0 ? fs + u : corrected_velocity(st, fs, u);
+        const LineLift o = lift_at(m, i, v, tab);
+        double gi = gam[i];
+        if (pass == 0 && !st.disable_viscous_corrections) gi = corrected_circulation(o, gi);
+        if (last) {
+            W.terms[i] = residual_of(m, i, gi, v, o.cl_pre);
+            write_line(b, i, gi, v);
+        } else {
+            W.g[i] = gi;
+        }
+        __threadfence();
+    }
+    if (!last) return;
+    __syncwarp();
+    unsigned before = 0;
+    if (lane == 0) before = atomicAdd(W.counter, 1u);
+    if (__shfl_sync(0xffffffffu, before, 0) != gridDim.x - 1) return;
+    __threadfence();
+    write_scalars(b, W.terms, N, lane);
 }
 
 __global__ void __launch_bounds__(kThreads, 1) k_lin_refined(DevModel m, SolveSettings st, SolveBuffers b) {
     extern __shared__ __align__(16) unsigned char refined_dyn[];
-    solve(m, st, b, refined_dyn);
+    solve<false>(m, st, b, refined_dyn);
+}
+__global__ void __launch_bounds__(kThreads, 1) k_lin_refined_split(DevModel m, SolveSettings st, SolveBuffers b) {
+    extern __shared__ __align__(16) unsigned char refined_dyn[];
+    solve<true>(m, st, b, refined_dyn);
 }
 
 // Every case of a batch whose cluster size is this launch's: cluster i solves jobs[i].
 __global__ void __launch_bounds__(kThreads, 1) k_lin_refined_jobs(const SolveJob* jobs) {
     extern __shared__ __align__(16) unsigned char refined_dyn[];
     const SolveJob& j = jobs[blockIdx.x / cg::this_cluster().num_blocks()];
-    solve(j.m, j.st, j.b, refined_dyn);
+    solve<false>(j.m, j.st, j.b, refined_dyn);
 }
 
 void config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, int clusters, int C, size_t smem, cudaStream_t s) {
@@ -510,7 +671,7 @@ int largest_cluster() {
                    cudaSuccess &&
                cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     };
-    int c = prepare(k_lin_refined) && prepare(k_lin_refined_jobs) ? 16 : 0;
+    int c = prepare(k_lin_refined) && prepare(k_lin_refined_split) && prepare(k_lin_refined_jobs) ? 16 : 0;
     for (; c > 8; c /= 2) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr;
@@ -526,8 +687,7 @@ int largest_cluster() {
 }  // namespace
 
 size_t lin_work_doubles(int N) {
-    // the elimination's [N][N + 1], or the f64 matrix [N][N] and two buffers of scaled rows [16][padded] floats
-    return std::max(static_cast<size_t>(N) * (N + 1), static_cast<size_t>(N) * N + static_cast<size_t>(kBlk) * padded(N));
+    return std::max(static_cast<size_t>(N) * (N + 1), Work::doubles(N));  // the elimination's [N][N + 1], or Work
 }
 
 LinPlan linearized_refined_plan(int N, int crowding) {
@@ -543,7 +703,16 @@ cudaError_t launch_solve_linearized_refined(const DevModel& m, const SolveSettin
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr;
     config(cfg, attr, 1, p.cluster, p.smem, s);
-    return cudaLaunchKernelEx(&cfg, k_lin_refined, m, st, b);
+    if (m.N < kSplitLines) return cudaLaunchKernelEx(&cfg, k_lin_refined, m, st, b);
+    k_lin_build<<<(padded(m.N) + kRowWarps - 1) / kRowWarps, kRowThreads, 0, s>>>(m, b);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, k_lin_refined_split, m, st, b);
+    const int passes = st.full_induced_correction && !st.disable_viscous_corrections ? 2 : 1;
+    for (int k = 0; k < passes && e == cudaSuccess; ++k) {
+        k_lin_finish<<<(m.N + kRowWarps - 1) / kRowWarps, kFinishThreads, 0, s>>>(m, st, b, k, k + 1 == passes);
+        e = cudaGetLastError();
+    }
+    return e;
 }
 
 cudaError_t launch_solve_linearized_refined_jobs(const SolveJob* jobs, int n, const LinPlan& p, cudaStream_t s) {

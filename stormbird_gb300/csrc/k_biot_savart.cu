@@ -87,7 +87,10 @@ __device__ __noinline__ d3 ring_f64(const double* v, d3 x) {
 __device__ __forceinline__ void add_panel_f64(const double* v, d3 x, double g, d3& u) {
     const d3 t = x - mk(v[16], v[17], v[18]);
     const double d2 = len2(t);
-    if (d2 <= v[19]) {
+    // d2 <= v[19], as integers (the FP64 pipe, which bounds the sweep, takes a compare like an add): neither is
+    // negative, and a NaN on the right is no bound
+    const long long ff = __double_as_longlong(v[19]);
+    if (__double_as_longlong(d2) <= ff && ff <= 0x7FF0000000000000ll) {
         const d3 w = ring_f64(v, x);
         const double f = g * kFourPiInv;
         u.x = fma(f, w.x, u.x);

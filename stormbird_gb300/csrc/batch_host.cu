@@ -461,7 +461,7 @@ struct sb_batch {
         for (auto& g : groups) {
             const int tile = bs_tile_panels(precision, g.sym, g.chain, t.tile);
             g.tile = tile;
-            const int T = bs_targets_per_thread(g.sym);
+            const int T = bs_targets_per_thread(g.sym, precision);
             const long long TM = static_cast<long long>(kBsThreads) * T;
             const int occ = bs_occupancy_blocks_per_sm(precision, g.sym, g.neglect, g.chain ? 0 : t.tile);
             const int bps = t.blocks_per_sm > 0 ? std::min(t.blocks_per_sm, occ) : occ;
@@ -526,7 +526,7 @@ struct sb_batch {
     void fill_jobs() {
         last_pairs = 0;
         for (auto& g : groups) {
-            const int T = bs_targets_per_thread(g.sym);
+            const int T = bs_targets_per_thread(g.sym, precision);
             const long long TM = static_cast<long long>(kBsThreads) * T;
             long long item = 0;
             for (size_t k = 0; k < g.cases.size(); ++k) {

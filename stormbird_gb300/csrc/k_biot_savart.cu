@@ -1237,23 +1237,26 @@ static cudaError_t launch_sym(const BsArgs& a, int grid, cudaStream_t s) {
             return a.neglect ? launch_t<R, 2, KAHAN, 0, true, false, 96>(a, grid, s)
                              : launch_t<R, 2, KAHAN, 0, false, false, 96>(a, grid, s);
     }
+    // FP32: two targets a thread, one packed pair. FP64 (bound by its pipe, which four warps fill): one, so that
+    // the last items are half as long (9,900 panels x 1,501 targets: 906 us with two, 874 with one).
+    constexpr int T = sizeof(R) == 4 ? 2 : 1;
     if (a.neglect) {
         switch (a.symmetry) {
-            case 0: return launch_t<R, 2, KAHAN, 0, true>(a, grid, s);
+            case 0: return launch_t<R, T, KAHAN, 0, true>(a, grid, s);
             case 1: return launch_t<R, 1, KAHAN, 1, true>(a, grid, s);
             case 2: return launch_t<R, 1, KAHAN, 2, true>(a, grid, s);
             default: return launch_t<R, 1, KAHAN, 3, true>(a, grid, s);
         }
     }
     switch (a.symmetry) {
-        case 0: return launch_t<R, 2, KAHAN, 0, false>(a, grid, s);
+        case 0: return launch_t<R, T, KAHAN, 0, false>(a, grid, s);
         case 1: return launch_t<R, 1, KAHAN, 1, false>(a, grid, s);
         case 2: return launch_t<R, 1, KAHAN, 2, false>(a, grid, s);
         default: return launch_t<R, 1, KAHAN, 3, false>(a, grid, s);
     }
 }
 
-int bs_targets_per_thread(int symmetry) { return symmetry == 0 ? 2 : 1; }
+int bs_targets_per_thread(int symmetry, int precision) { return symmetry == 0 && precision != 2 ? 2 : 1; }
 int bs_tile_panels(int precision) { return precision == 2 ? TileSize<double>::value : TileSize<float>::value; }
 int bs_tile_panels(int precision, int symmetry, int chain, int tile) {
     return tuned_tile_variant(precision, symmetry, chain, tile) ? tile : bs_tile_panels(precision);
@@ -1296,7 +1299,7 @@ int bs_occupancy_blocks_per_sm(int precision, int symmetry, int neglect, int til
 #define SB_OCC(R, T, K, S, NG) \
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_bs_sweep<R, T, K, S, NG, false>, kBsThreads, 0)
     if (precision == 2) {
-        if (symmetry == 0) { if (neglect) SB_OCC(double, 2, false, 0, true); else SB_OCC(double, 2, false, 0, false); }
+        if (symmetry == 0) { if (neglect) SB_OCC(double, 1, false, 0, true); else SB_OCC(double, 1, false, 0, false); }
         else { if (neglect) SB_OCC(double, 1, false, 1, true); else SB_OCC(double, 1, false, 1, false); }
     } else if (precision == 1) {
         if (symmetry == 0) { if (neglect) SB_OCC(float, 2, false, 0, true); else SB_OCC(float, 2, false, 0, false); }

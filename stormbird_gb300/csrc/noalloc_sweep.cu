@@ -157,7 +157,7 @@ extern "C" int sb_panel_sweep_no_alloc(int device, const double* corners, const 
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (sms < 1) sms = 1;
-    const int T = bs_targets_per_thread(symmetry);
+    const int T = bs_targets_per_thread(symmetry, 0);
     const long long TM = static_cast<long long>(kBsThreads) * T;
     const long long n_ttiles = (M + TM - 1) / TM;
     const int tile = bs_tile_panels(0);

@@ -83,7 +83,7 @@ cudaError_t launch_wait_probe(int polls, int* err, cudaStream_t s);
 
 constexpr int kBsReduceThreads = 256;
 
-int bs_targets_per_thread(int symmetry);
+int bs_targets_per_thread(int symmetry, int precision);
 int bs_tile_panels(int precision);
 // Panels per stage a launch with BsArgs::tile = `tile` uses: the tuned shape where a variant
 // exists (compensated FP32, no symmetry, panel records), else the default.

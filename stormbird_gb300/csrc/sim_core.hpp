@@ -254,7 +254,7 @@ struct SweepPlan {
 
 inline SweepPlan make_sweep_plan(long long M, long long P, int precision, int sym, int neglect, int sms) {
     SweepPlan sp;
-    int T = bs_targets_per_thread(sym);
+    int T = bs_targets_per_thread(sym, precision);
     long long TM = static_cast<long long>(kBsThreads) * T;
     sp.n_ttiles = (M + TM - 1) / TM;
     int tile = bs_tile_panels(precision);
@@ -282,7 +282,7 @@ inline SweepPlan make_sweep_plan(long long M, long long P, int precision, int sy
 // targets x 2,100 panels (33 chunks): 41 us with 64 targets a warp, 28 with 2; filling the SMs more than once
 // over gained nothing (183 x 54,900: 62 either way).
 inline void spread_targets(BsJob& J, SweepPlan& sp, int sym, int sms) {
-    const int T = bs_targets_per_thread(sym);
+    const int T = bs_targets_per_thread(sym, 0);
     auto tiles = [&](int w) { return (bs_slots(J) + kBsThreads / 32 * w - 1) / (kBsThreads / 32 * w); };
     int w = 32 * T;
     while (w > T && tiles(w / 2) * sp.n_chunks <= sms) w /= 2;

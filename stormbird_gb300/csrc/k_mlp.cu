@@ -286,14 +286,16 @@ __global__ void __launch_bounds__(kGemmThreads) k_mlp_gemm(const __grid_constant
             }
             // transposed: with row 8 t + 2 m + e as row 2 t + e of matrix m, lane 4 c + t of a transposed
             // ldmatrix gets rows 8 t .. 8 t + 7 of column c, 16 bytes of a row of the transpose
-            const int lr = 8 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);
+            if (g.hT_out) {
+                const int lr = 8 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                uint4 w;
-                asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(smem_u32(chunk(lr, q))) : "memory");
-                *reinterpret_cast<uint4*>(g.hT_out + static_cast<long long>(c0 + 8 * q + (lane >> 2)) * g.ldt + m0 + quad * 32 +
-                                          (lane & 3) * 8) = w;
+                for (int q = 0; q < 4; ++q) {
+                    uint4 w;
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(smem_u32(chunk(lr, q))) : "memory");
+                    *reinterpret_cast<uint4*>(g.hT_out + static_cast<long long>(c0 + 8 * q + (lane >> 2)) * g.ldt + m0 + quad * 32 +
+                                              (lane & 3) * 8) = w;
+                }
             }
             __syncwarp();
         }
@@ -322,9 +324,11 @@ constexpr int kFwdThreads = 32 * (kFwdWarps + 2);
 constexpr int kFwdRing = 5;
 constexpr uint32_t kFwdSub = 128 * kKStep * 2;   // a 128 x 64 BF16 sub-tile (A quarter or half slab)
 constexpr uint32_t kFwdTile = 4 * kFwdSub;       // activations of a tile
+constexpr int kFwdTurnLd = 20;                   // floats of a row of a warp's 32 x 16 turning tile
 constexpr int kFwdPartLd = 33;                   // row pitch of the output layer's partial sums
 constexpr uint32_t kFwdSmem = 2 * kFwdTile + kFwdRing * kFwdSub + (kMlpHidden * kMlpWidth + kMlpWidth + 4) * 4 + 1024;
 static_assert(128 * kFwdPartLd * 4 <= kFwdTile, "partial sums fit a tile's activations");
+static_assert(kFwdWarps * 32 * kFwdTurnLd * 4 <= kFwdTile, "the turning tiles fit the second slot");
 
 struct FwdMaps {
     CUtensorMap w[kMlpHidden];
@@ -334,6 +338,11 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// TRAIN: every layer's pre-activations, activations and their transposes go out as well (FwdArgs::z, h, hT)
+// and the output layer is left to k_mlp_head. One tile a CTA: the second slot's shared memory turns the
+// stores, and activations go out under the next layer's MMAs. 16,384 rows: 46 us, against four GEMM launches of 13 to 16
+// and the gaps between them (with activations stored before the next layer may start 53).
+template <bool TRAIN>
 __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const __grid_constant__ FwdMaps maps, FwdArgs g) {
     extern __shared__ unsigned char dyn[];
     unsigned char* act = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
@@ -460,6 +469,33 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const __grid_con
                     *reinterpret_cast<uint4*>(chunk(c)) = *reinterpret_cast<uint4*>(p);
                 }
             }
+            // TRAIN: what the warp has written of layer l's activations, by rows and by columns
+            auto publish = [&](int l) {
+                const long long row0 = static_cast<long long>(tile_of(k, q)) * 128 + quad * 32;
+                auto at = [&](int rr, int col) {
+                    const int w = quad * 32 + rr;
+                    return a + (col >> 6) * kFwdSub + w * 128 + ((((col & 63) >> 3) ^ (w & 7)) << 4);
+                };
+                __syncwarp();
+#pragma unroll 1
+                for (int c0 = part * width; c0 < (part + 1) * width; c0 += 32) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 8) {
+                        const int rr = i + (lane >> 2), col = c0 + (lane & 3) * 8;
+                        *reinterpret_cast<uint4*>(g.h[l] + (row0 + rr) * kMlpWidth + col) = *reinterpret_cast<const uint4*>(at(rr, col));
+                    }
+                    if (!g.hT[l]) continue;
+                    const int lr = 8 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);  // as in k_mlp_gemm
+#pragma unroll
+                    for (int i = 0; i < 32; i += 8) {
+                        uint4 w;
+                        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                                     : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(smem_u32(at(lr, c0 + i))) : "memory");
+                        *reinterpret_cast<uint4*>(g.hT[l] + static_cast<long long>(c0 + i + (lane >> 2)) * g.ldt + row0 + (lane & 3) * 8) = w;
+                    }
+                }
+                __syncwarp();
+            };
 #pragma unroll 1
             for (int l = 0; l < kMlpHidden; ++l, ++layer) {
                 // the operand is written (and the accumulator read): the tensor cores may start
@@ -467,6 +503,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const __grid_con
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&act_ready[q]);
+                if (TRAIN && l > 0) publish(l - 1);  // under this layer's MMAs
                 if (ok && !mbar_wait_bounded(&acc_full[q], layer & 1, g.err)) ok = false;
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) continue;
@@ -476,20 +513,50 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const __grid_con
                 for (int c0 = part * width; c0 < (part + 1) * width; c0 += 32) {
                     float v[32];
                     tmem_ld32(lane_addr + static_cast<uint32_t>(q * 256 + c0), v);
+                    const long long row0 = static_cast<long long>(tile_of(k, q)) * 128 + quad * 32;  // the warp's rows
+                    if constexpr (TRAIN) {
 #pragma unroll
-                    for (int j = 0; j < 32; j += 4) {
-                        const float4 b4 = *reinterpret_cast<const float4*>(bl + c0 + j);
-                        v[j] = gelu(v[j] + b4.x);
-                        v[j + 1] = gelu(v[j + 1] + b4.y);
-                        v[j + 2] = gelu(v[j + 2] + b4.z);
-                        v[j + 3] = gelu(v[j + 3] + b4.w);
+                        for (int j = 0; j < 32; j += 4) {
+                            const float4 b4 = *reinterpret_cast<const float4*>(bl + c0 + j);
+                            v[j] += b4.x;
+                            v[j + 1] += b4.y;
+                            v[j + 2] += b4.z;
+                            v[j + 3] += b4.w;
+                        }
+                        // sixteen columns at a time, rows of 20 floats: stores of 64 bytes a row
+                        float* turn = reinterpret_cast<float*>(act + kFwdTile) + warp * (32 * kFwdTurnLd);
+#pragma unroll
+                        for (int j = 0; j < 32; j += 16) {
+#pragma unroll
+                            for (int i = 0; i < 16; i += 4)
+                                *reinterpret_cast<float4*>(turn + lane * kFwdTurnLd + i) = make_float4(v[j + i], v[j + i + 1], v[j + i + 2], v[j + i + 3]);
+                            __syncwarp();
+#pragma unroll
+                            for (int i = 0; i < 32; i += 8) {
+                                const int rr = i + (lane >> 2);
+                                *reinterpret_cast<float4*>(g.z[l] + (row0 + rr) * kMlpWidth + c0 + j + (lane & 3) * 4) =
+                                    *reinterpret_cast<const float4*>(turn + rr * kFwdTurnLd + (lane & 3) * 4);
+                            }
+                            __syncwarp();
+                        }
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = gelu(v[j]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; j += 4) {
+                            const float4 b4 = *reinterpret_cast<const float4*>(bl + c0 + j);
+                            v[j] = gelu(v[j] + b4.x);
+                            v[j + 1] = gelu(v[j + 1] + b4.y);
+                            v[j + 2] = gelu(v[j + 2] + b4.z);
+                            v[j + 3] = gelu(v[j + 3] + b4.w);
+                        }
                     }
 #pragma unroll
                     for (int j = 0; j < 32; j += 8) {
                         __nv_bfloat162 p[4];
 #pragma unroll
                         for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(v[j + 2 * i], v[j + 2 * i + 1]);
-                        if (l + 1 < kMlpHidden) {
+                        if (TRAIN || l + 1 < kMlpHidden) {
                             *reinterpret_cast<uint4*>(chunk(c0 + j)) = *reinterpret_cast<uint4*>(p);
                         } else {  // output layer: the partial sum of these 8 columns
                             float s = 0.f;
@@ -503,6 +570,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const __grid_con
                         }
                     }
                 }
+            }
+            if constexpr (TRAIN) {
+                publish(kMlpHidden - 1);
+                break;  // the one tile
             }
             // a row's 32 partial sums in the order of a butterfly over 32 lanes
             asm volatile("bar.sync %0, %1;" ::"r"(1 + q), "r"(meet) : "memory");
@@ -660,7 +731,7 @@ __global__ void __launch_bounds__(256) k_mlp_pack(const float* x, int rows, int 
     __syncthreads();
     for (int i = tid; i < kPackRows * kMlpInPad / 8; i += 256) {
         const int r = i / (kMlpInPad / 8), c = i % (kMlpInPad / 8) * 8;
-        *reinterpret_cast<uint4*>(X + static_cast<long long>(r0 + r) * kMlpInPad + c) = *reinterpret_cast<const uint4*>(&t[r][c]);
+        if (X) *reinterpret_cast<uint4*>(X + static_cast<long long>(r0 + r) * kMlpInPad + c) = *reinterpret_cast<const uint4*>(&t[r][c]);
         __align__(16) bf16 w[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) w[j] = t[c + j][r];  // here r is a column and c a row
@@ -813,9 +884,10 @@ unsigned blocks_for(long long n, int t) { return static_cast<unsigned>((n + t - 
 size_t mlp_gemm_smem_bytes() { return kStages * static_cast<size_t>(kStage) + 1024; }
 
 cudaError_t configure_mlp_gemm() {
-    const cudaError_t e = cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(kFwdSmem));
-    if (e != cudaSuccess) return e;
+    for (auto kernel : {k_mlp_forward<false>, k_mlp_forward<true>}) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kFwdSmem));
+        if (e != cudaSuccess) return e;
+    }
     return cudaFuncSetAttribute(k_mlp_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(mlp_gemm_smem_bytes()));
 }
@@ -877,7 +949,12 @@ cudaError_t launch_mlp_forward(const FwdArgs& args, cudaStream_t s) {
         if (!encode_bf16_map(&maps.w[l], g.w[l], kMlpWidth, in, in, 128)) return cudaErrorInvalidValue;
     }
     const int tiles = (g.rows + 127) / 128;
-    k_mlp_forward<<<std::min(tiles, std::max(1, g.sms)), kFwdThreads, kFwdSmem, s>>>(maps, g);
+    if (g.z[0]) {
+        if (tiles > g.sms) return cudaErrorInvalidValue;
+        k_mlp_forward<true><<<tiles, kFwdThreads, kFwdSmem, s>>>(maps, g);
+    } else {
+        k_mlp_forward<false><<<std::min(tiles, std::max(1, g.sms)), kFwdThreads, kFwdSmem, s>>>(maps, g);
+    }
     return cudaGetLastError();
 }
 

@@ -24,7 +24,7 @@ struct sb_mlp {
     cudaStream_t stream = nullptr;
     // Beside the chain of input gradients: weight and bias gradients; the output layer's.
     cudaStream_t side[2] = {nullptr, nullptr};
-    cudaEvent_t ev_dz[kMlpHidden] = {nullptr}, ev_side[2] = {nullptr, nullptr};
+    cudaEvent_t ev_dz[kMlpHidden] = {nullptr}, ev_side[2] = {nullptr, nullptr}, ev_in = nullptr;
     long long off_W[kMlpHidden] = {0}, off_b[kMlpHidden] = {0}, off_out = 0, n_params = 0;
     int in_dim[kMlpHidden] = {0};
     DevBuf<float> params, grads, adam_m, adam_v;
@@ -42,6 +42,7 @@ struct sb_mlp {
     ~sb_mlp() {
         for (auto& e : ev_dz) if (e) cudaEventDestroy(e);
         for (auto& e : ev_side) if (e) cudaEventDestroy(e);
+        if (ev_in) cudaEventDestroy(ev_in);
         for (auto& q : side) if (q) cudaStreamDestroy(q);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -56,6 +57,7 @@ struct sb_mlp {
         for (auto& q : side) ck(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking), "cudaStreamCreate");
         for (auto& e : ev_dz) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         for (auto& e : ev_side) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+        ck(cudaEventCreateWithFlags(&ev_in, cudaEventDisableTiming), "cudaEventCreate");
         long long at = 0;
         for (int l = 0; l < kMlpHidden; ++l) {
             in_dim[l] = l == 0 ? kMlpInPad : kMlpWidth;
@@ -166,10 +168,8 @@ struct sb_mlp {
         return g;
     }
 
-    // Inference over rows of x [rows][n_in] (device) into y [rows].
-    void forward(const float* x, long long rows, float* y, cudaStream_t s) {
+    FwdArgs fwd_args() const {
         FwdArgs g;
-        g.x = x;
         g.n_in = n_in;
         for (int l = 0; l < kMlpHidden; ++l) {
             g.w[l] = Wb[l].p;
@@ -178,6 +178,12 @@ struct sb_mlp {
         g.w_out = params.p + off_out;
         g.sms = sms;
         g.err = err.p;
+        return g;
+    }
+
+    // Inference over rows of x [rows][n_in] (device) into y [rows].
+    void forward(const float* x, long long rows, float* y, cudaStream_t s) {
+        FwdArgs g = fwd_args();
         constexpr long long kPass = 1 << 30;  // rows per launch (row numbers of a launch are int)
         for (long long r0 = 0; r0 < rows; r0 += kPass) {
             g.x = x + r0 * n_in;
@@ -187,22 +193,40 @@ struct sb_mlp {
         }
     }
 
-    // Forward pass of a training step: keeps what the backward pass needs.
+    // Forward pass of a training step: keeps what the backward pass needs. Up to a tile of 128 rows per SM
+    // the hidden layers are one launch, and the packed inputs (for the first layer's weight gradients alone) are
+    // made beside it.
     void forward_train(const float* x, long long rows, const float* target, cudaStream_t s) {
         const int R = pad_rows(rows);
-        ck(launch_mlp_pack(x, static_cast<int>(rows), n_in, R, X0.p, X0T.p, s), "pack inputs");
-        const bf16* in = X0.p;
-        long long ld = kMlpInPad;
-        for (int l = 0; l < kMlpHidden; ++l) {
-            GemmArgs g = gemm(in, ld, Wb[l].p, in_dim[l], R, kMlpWidth, in_dim[l], kGemmForward);
-            g.bias = params.p + off_b[l];
-            g.z_out = Z[l].p;
-            g.h_out = H[l].p;
-            g.hT_out = HT[l].p;
+        if (R / kMlpRowTile <= sms) {
+            ck(cudaEventRecord(ev_in, s), "event");
+            ck(cudaStreamWaitEvent(side[0], ev_in, 0), "side stream");
+            ck(launch_mlp_pack(x, static_cast<int>(rows), n_in, R, nullptr, X0T.p, side[0]), "pack inputs");
+            FwdArgs g = fwd_args();
+            g.x = x;
+            g.rows = static_cast<int>(rows);
             g.ldt = R;
-            ck(launch_mlp_gemm(g, s), "forward GEMM");
-            in = H[l].p;
-            ld = kMlpWidth;
+            for (int l = 0; l < kMlpHidden; ++l) {
+                g.z[l] = Z[l].p;
+                g.h[l] = H[l].p;
+                g.hT[l] = l + 1 < kMlpHidden ? HT[l].p : nullptr;
+            }
+            ck(launch_mlp_forward(g, s), "hidden layers");
+        } else {
+            ck(launch_mlp_pack(x, static_cast<int>(rows), n_in, R, X0.p, X0T.p, s), "pack inputs");
+            const bf16* in = X0.p;
+            long long ld = kMlpInPad;
+            for (int l = 0; l < kMlpHidden; ++l) {
+                GemmArgs g = gemm(in, ld, Wb[l].p, in_dim[l], R, kMlpWidth, in_dim[l], kGemmForward);
+                g.bias = params.p + off_b[l];
+                g.z_out = Z[l].p;
+                g.h_out = H[l].p;
+                g.hT_out = l + 1 < kMlpHidden ? HT[l].p : nullptr;
+                g.ldt = R;
+                ck(launch_mlp_gemm(g, s), "forward GEMM");
+                in = H[l].p;
+                ld = kMlpWidth;
+            }
         }
         HeadArgs h;
         h.h = H[kMlpHidden - 1].p;

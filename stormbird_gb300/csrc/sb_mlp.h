@@ -56,6 +56,12 @@ struct FwdArgs {
     const float* bias[kMlpHidden] = {nullptr};
     const float* w_out = nullptr;             // [257]
     float* y = nullptr;
+    // training (z[0] not null; at most sms tiles of 128 rows): pre-activations [rows_pad][256], activations
+    // [rows_pad][256] and [256][ldt] (null: not wanted) of every layer instead of y
+    float* z[kMlpHidden] = {nullptr};
+    bf16* h[kMlpHidden] = {nullptr};
+    bf16* hT[kMlpHidden] = {nullptr};
+    long long ldt = 0;
     int sms = 1;
     int* err = nullptr;
 };
@@ -80,7 +86,8 @@ constexpr int kHeadGroups = 4;      // partial sums a CTA makes
 cudaError_t launch_mlp_head_sums(const float* part, int groups, float* grad, float* loss, cudaStream_t s);
 cudaError_t launch_mlp_head(const HeadArgs& a, cudaStream_t s);
 
-// Input packing: x [rows][n_in] f32 -> X [rows_pad][64] BF16 (zero padded) and its transpose XT [64][rows_pad].
+// Input packing: x [rows][n_in] f32 -> X [rows_pad][64] BF16 (zero padded; null: not wanted) and its transpose XT
+// [64][rows_pad].
 cudaError_t launch_mlp_pack(const float* x, int rows, int n_in, int rows_pad, bf16* X, bf16* XT, cudaStream_t s);
 // gw[i] = sum over s < splits of part[s * n + i] in split order; gb[o] = sum over r < rows_pad of dzT[o][r].
 cudaError_t launch_mlp_grads(const float* part, int splits, int n, float* gw, const bf16* dzT, int rows_pad, float* gb, cudaStream_t s);

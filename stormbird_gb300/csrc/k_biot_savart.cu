@@ -9,7 +9,7 @@
 // k_bs_sweep: an N-body sweep over (target tile x source chunk) work items, taken from an
 // atomic work counter by a persistent grid. Panel records of a chunk are streamed into
 // shared memory in tiles by one thread with bulk asynchronous copies (cp.async.bulk,
-// completion on an mbarrier), double-buffered. Each thread holds T targets in registers.
+// completion on an mbarrier), in two or three stages. Each thread holds T targets in registers.
 // Near/far classification follows panel.rs:53-57 per pair; a warp evaluates the vortex
 // ring only if one of its lanes needs it and the point doublet only if one needs that.
 // Sums: FP32 within a tile, then an error-free TwoSum fold across tiles (compensated

@@ -4,9 +4,8 @@
 //
 // A CTA per wing: a thread per line evaluates the line's forces (about 200 FP64 instructions,
 // sb_line.cuh), then a warp per force component sums the wing's forces and moments over the lines; the
-// CTA that finishes last adds up the wings. Bound by the FP64 instructions of one line (a warp
-// instruction takes 62-65 cycles whatever the active lanes; four warps of lines run side by side on the
-// SM's four FP64 pipes). One CTA for all wings with CUDA's f64 functions inlined (160 KB of code,
+// CTA that finishes last adds up the wings. Bound by the FP64 instructions of one line (a lone warp issues
+// one per 65 cycles whatever the active lanes; three warps run side by side on the SM's FP64 pipe). One CTA for all wings with CUDA's f64 functions inlined (160 KB of code,
 // most of it fetched once per launch) and sums by one thread per (wing, component) took 68 us at
 // 21 lines, 118 at 4 x 64, 359 at 8 x 128; this takes 18, 22 and 25 us (CUDA events).
 #include "sb_device.cuh"

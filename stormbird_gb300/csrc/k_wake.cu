@@ -297,51 +297,54 @@ cudaError_t launch_wake_advect(const DevModel& m, const WakeBuffers& w, double d
 // |e_hi - e| <= d = sqrt(3) 2^-24 (2 |c|_inf + 2 r) and ||e_hi|^2 - r^2| <= 2 r d + d^2, plus
 // the FP32 rounding of |e_hi|^2 and of ff2 (below 2^-21 ff2). The band is twice that sum.
 __device__ inline void far_field_fields(double ff2, d3 c, float* hi, float* lo, float* band) {
-    const float h = static_cast<float>(ff2);
+    const float h = f64_to_f32_rn(ff2);
     *hi = h;
     if (isinf(h)) {
         *lo = 0.f;
         *band = 0.f;
         return;
     }
-    *lo = static_cast<float>(ff2 - static_cast<double>(h));
+    *lo = f64_to_f32_rn(ff2 - f32_to_f64_exact(h));
     const float r = __fsqrt_ru(h);
-    const float cm = fmaxf(fmaxf(fabsf(static_cast<float>(c.x)), fabsf(static_cast<float>(c.y))),
-                           fabsf(static_cast<float>(c.z)));
+    const float cm = fmaxf(fmaxf(fabsf(f64_to_f32_rn(c.x)), fabsf(f64_to_f32_rn(c.y))),
+                           fabsf(f64_to_f32_rn(c.z)));
     const float d = 1.7320509f * 0x1p-24f * (2.f * cm + 2.f * r);
     *band = 2.f * ((2.f * r * d + d * d) + 0x1p-21f * h);
 }
 
+// FP64-bound (19 cycles a warp instruction on the SM's pipe): the 45 conversions a panel go through the integer
+// pipe, with the conversion's own results (409,600 panels: 119 us with conversions, 84; 49,152 chain
+// records 20 -> 16).
 __device__ void write_panel_records(const d3 (&pp)[4], double rc, double g, double far_field_ratio, int wing,
                                     PanelRec<float>* r32, PanelRec<double>* r64) {
     const d3 c = 0.25 * (((pp[0] + pp[1]) + pp[2]) + pp[3]);
     PanelRec<float> r;
     auto split = [](double x, float* hi, float* lo) {
-        float h = static_cast<float>(x);
+        const float h = f64_to_f32_rn(x);
         *hi = h;
-        *lo = static_cast<float>(x - static_cast<double>(h));
+        *lo = f64_to_f32_rn(x - f32_to_f64_exact(h));
     };
     double l2[4];
     for (int k = 0; k < 4; ++k) {
         const d3 ok = pp[k] - c;
-        r.v[3 * k] = static_cast<float>(ok.x);
-        r.v[3 * k + 1] = static_cast<float>(ok.y);
-        r.v[3 * k + 2] = static_cast<float>(ok.z);
+        r.v[3 * k] = f64_to_f32_rn(ok.x);
+        r.v[3 * k + 1] = f64_to_f32_rn(ok.y);
+        r.v[3 * k + 2] = f64_to_f32_rn(ok.z);
         const d3 dk = pp[(k + 1) & 3] - pp[k];
-        r.v[12 + 3 * k] = static_cast<float>(dk.x);
-        r.v[12 + 3 * k + 1] = static_cast<float>(dk.y);
-        r.v[12 + 3 * k + 2] = static_cast<float>(dk.z);
+        r.v[12 + 3 * k] = f64_to_f32_rn(dk.x);
+        r.v[12 + 3 * k + 1] = f64_to_f32_rn(dk.y);
+        r.v[12 + 3 * k + 2] = f64_to_f32_rn(dk.z);
         l2[k] = len2(dk);
-        r.v[kRec32DD + k] = static_cast<float>(l2[k]);
+        r.v[kRec32DD + k] = f64_to_f32_rn(l2[k]);
     }
     split(c.x, &r.v[28], &r.v[32]);
     split(c.y, &r.v[29], &r.v[33]);
     split(c.z, &r.v[30], &r.v[34]);
-    r.v[kRec32Gamma] = static_cast<float>(g);
+    r.v[kRec32Gamma] = f64_to_f32_rn(g);
     // core length^4; a zero core (reference: factor 1) only occurs in the horseshoe path, which
     // runs in FP64, so the FP32 sweep always evaluates d^2 / sqrt(d^4 + rc^4)
     const double rc2 = rc * rc;
-    r.v[40] = static_cast<float>(rc2 * rc2);
+    r.v[40] = f64_to_f32_rn(rc2 * rc2);
     r.v[41] = static_cast<float>(wing);
     for (int k = kRec32DD + 4; k < 48; ++k) r.v[k] = 0.f;
     if (r64) {
@@ -353,12 +356,12 @@ __device__ void write_panel_records(const d3 (&pp)[4], double rc, double g, doub
         const double ff2 = t * t;
         double il2[4];
         for (int k = 0; k < 4; ++k) il2[k] = rcp_any(l2[k]);
-        for (int k = 0; k < 4; ++k) r.v[24 + k] = l2[k] > 0.0 ? static_cast<float>(il2[k]) : 0.f;
+        for (int k = 0; k < 4; ++k) r.v[24 + k] = l2[k] > 0.0 ? f64_to_f32_rn(il2[k]) : 0.f;
         far_field_fields(ff2, c, &r.v[31], &r.v[kRec32FF2Lo], &r.v[kRec32FF2Band]);
-        r.v[35] = static_cast<float>(area * kFourPiInv * kInv3Sqrt3);
-        r.v[36] = static_cast<float>(n.x);
-        r.v[37] = static_cast<float>(n.y);
-        r.v[38] = static_cast<float>(n.z);
+        r.v[35] = f64_to_f32_rn(area * kFourPiInv * kInv3Sqrt3);
+        r.v[36] = f64_to_f32_rn(n.x);
+        r.v[37] = f64_to_f32_rn(n.y);
+        r.v[38] = f64_to_f32_rn(n.z);
         PanelRec<double> q;
         for (int k = 0; k < 4; ++k) {
             q.v[3 * k] = pp[k].x;
@@ -382,7 +385,7 @@ __device__ void write_panel_records(const d3 (&pp)[4], double rc, double g, doub
     } else {
         float lf[4];
         for (int k = 0; k < 4; ++k) {
-            const float q = static_cast<float>(l2[k]);
+            const float q = f64_to_f32_rn(l2[k]);
             r.v[24 + k] = q > 0.f ? __frcp_rn(q) : 0.f;
             lf[k] = __fsqrt_rn(q);
         }
@@ -391,8 +394,8 @@ __device__ void write_panel_records(const d3 (&pp)[4], double rc, double g, doub
         const float prod = fmaxf((sp - lf[0]) * (sp - lf[1]) * (sp - lf[2]) * (sp - lf[3]), 0.f);
         r.v[35] = __fsqrt_rn(prod) * static_cast<float>(kFourPiInv * kInv3Sqrt3);
         const d3 a = pp[2] - pp[0], b = pp[3] - pp[1];
-        const float ax = static_cast<float>(a.x), ay = static_cast<float>(a.y), az = static_cast<float>(a.z);
-        const float bx = static_cast<float>(b.x), by = static_cast<float>(b.y), bz = static_cast<float>(b.z);
+        const float ax = f64_to_f32_rn(a.x), ay = f64_to_f32_rn(a.y), az = f64_to_f32_rn(a.z);
+        const float bx = f64_to_f32_rn(b.x), by = f64_to_f32_rn(b.y), bz = f64_to_f32_rn(b.z);
         const float nx = ay * bz - az * by, ny = az * bx - ax * bz, nz = ax * by - ay * bx;
         const float nl = __fsqrt_rn(nx * nx + ny * ny + nz * nz);
         const float inl = nl > 0.f ? __frcp_rn(nl) : 0.f;
@@ -491,35 +494,35 @@ __device__ inline void chain_record_elem(const ChainArgs& a, long long n_build, 
         for (int k = npts; k <= kChainSegs; ++k) pt[k] = pt[npts - 1];  // empty segments
         const d3 anchor = pt[2 < npts ? 2 : npts - 1];
         auto split = [](double x, float* hi, float* lo) {
-            const float h = static_cast<float>(x);
+            const float h = f64_to_f32_rn(x);
             *hi = h;
-            *lo = static_cast<float>(x - static_cast<double>(h));
+            *lo = f64_to_f32_rn(x - f32_to_f64_exact(h));
         };
         split(anchor.x, &rec.v[0], &rec.v[3]);
         split(anchor.y, &rec.v[1], &rec.v[4]);
         split(anchor.z, &rec.v[2], &rec.v[5]);
         for (int k = 0; k <= kChainSegs; ++k) {
             const d3 o = pt[k] - anchor;
-            rec.v[kChainOff + 3 * k] = static_cast<float>(o.x);
-            rec.v[kChainOff + 3 * k + 1] = static_cast<float>(o.y);
-            rec.v[kChainOff + 3 * k + 2] = static_cast<float>(o.z);
+            rec.v[kChainOff + 3 * k] = f64_to_f32_rn(o.x);
+            rec.v[kChainOff + 3 * k + 1] = f64_to_f32_rn(o.y);
+            rec.v[kChainOff + 3 * k + 2] = f64_to_f32_rn(o.z);
         }
         double any = 0.0;
         for (int k = 0; k < kChainSegs; ++k) {
             const d3 dk = pt[k + 1] - pt[k];
-            rec.v[kChainD + 3 * k] = static_cast<float>(dk.x);
-            rec.v[kChainD + 3 * k + 1] = static_cast<float>(dk.y);
-            rec.v[kChainD + 3 * k + 2] = static_cast<float>(dk.z);
-            const float l2 = static_cast<float>(len2(dk));
+            rec.v[kChainD + 3 * k] = f64_to_f32_rn(dk.x);
+            rec.v[kChainD + 3 * k + 1] = f64_to_f32_rn(dk.y);
+            rec.v[kChainD + 3 * k + 2] = f64_to_f32_rn(dk.z);
+            const float l2 = f64_to_f32_rn(len2(dk));
             rec.v[kChainIl + k] = l2 > 0.f ? __frcp_rn(l2) : 0.f;  // FP32: an f64 division costs ~10 FP64 instructions here
             rec.v[kChainDD + k] = l2;
-            rec.v[kChainG + k] = static_cast<float>(g[k] * kFourPiInv);
+            rec.v[kChainG + k] = f64_to_f32_rn(g[k] * kFourPiInv);
             any += fabs(g[k]);
         }
         const double rc2 = a.rc * a.rc;
-        rec.v[kChainRc4] = static_cast<float>(rc2 * rc2);
+        rec.v[kChainRc4] = f64_to_f32_rn(rc2 * rc2);
         rec.v[kChainWing] = static_cast<float>(wing);
-        rec.v[kChainAny] = static_cast<float>(any);
+        rec.v[kChainAny] = f64_to_f32_rn(any);
     }
     a.out[id] = rec;
 }

@@ -1,7 +1,7 @@
 // f64 elementary functions for the per-line math (sm_103a), made for few FP64 instructions.
 //
-// This part's FP64 pipe takes a warp instruction every 62 to 65 cycles per SM sub-partition,
-// whatever the active lanes, independent or not (four independent DFMAs: 261 cycles), and a
+// A warp issues an FP64 instruction every 62 to 65 cycles, whatever the active lanes, independent or
+// not (four independent DFMAs: 261 cycles; the SM's one pipe takes one per 19 from four or more warps), and a
 // conversion between f64 and FP32 as long as a DFMA; CUDA's f64 division, square root, acos, sin and
 // exp are chains of 9 to 22 of them (574 to 1,425 cycles measured, one warp). The functions here
 // reach the same accuracy (an ulp or two) in 3 to 8 FP64 instructions:
@@ -49,6 +49,16 @@ __device__ __forceinline__ float f64_to_f32(double v) {
     const unsigned bits = __funnelshift_l(lo, mag, 3) + ((lo >> 28) & 1u);
     return __uint_as_float((mag - 0x00100000u < 0x0FE00000u ? bits : 0u) | (hi & 0x80000000u));
 }
+// The nearest float of v, ties to even (the conversion's own result), by integer arithmetic for 0 and
+// |v| in [2^-126, 2^127); others through the conversion.
+static __device__ __noinline__ float f64_to_f32_slow(double v) { return __double2float_rn(v); }
+__device__ __forceinline__ float f64_to_f32_rn(double v) {
+    const unsigned hi = static_cast<unsigned>(__double2hiint(v)), lo = static_cast<unsigned>(__double2loint(v));
+    const unsigned mag = (hi & 0x7FFFFFFFu) - 0x38000000u;
+    if (mag - 0x00100000u >= 0x0FE00000u) return ((hi & 0x7FFFFFFFu) | lo) == 0u ? __uint_as_float(hi) : f64_to_f32_slow(v);
+    const unsigned bits = __funnelshift_l(lo, mag, 3);
+    return __uint_as_float((bits + (((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (bits & 1u)) >> 29)) | (hi & 0x80000000u));
+}
 // v exactly, by integer arithmetic, for v finite; magnitudes below 2^-126 give a value below 2^-126.
 __device__ __forceinline__ double f32_to_f64(float v) {
     const unsigned u = __float_as_uint(v), mag = u & 0x7FFFFFFFu;
@@ -57,6 +67,13 @@ __device__ __forceinline__ double f32_to_f64(float v) {
 // the same with infinities and NaNs kept
 __device__ __forceinline__ double f32_to_f64_any(float v) {
     if ((__float_as_uint(v) & 0x7F800000u) == 0x7F800000u) return static_cast<double>(v);
+    return f32_to_f64(v);
+}
+// v exactly, whatever it is
+static __device__ __noinline__ double f32_to_f64_slow(float v) { return static_cast<double>(v); }
+__device__ __forceinline__ double f32_to_f64_exact(float v) {
+    const unsigned u = __float_as_uint(v), mag = u & 0x7FFFFFFFu;
+    if (mag - 0x00800000u >= 0x7F000000u) return mag == 0u ? __hiloint2double(static_cast<int>(u), 0) : f32_to_f64_slow(v);
     return f32_to_f64(v);
 }
 // f64 value as a pair of floats: hi = the nearest float, lo = the nearest float of v - hi

@@ -439,8 +439,10 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
         int tw[TT];
         // with the far-field fast path a warp's targets are consecutive points (a compact box), T adjacent ones
         // to a thread; else a thread's targets are T rows of the tile apart
-        const int wt = FAST_FAR && J.warp_targets > 0 ? J.warp_targets : 32 * T;
-        const bool mine = lane * T < wt;
+        int wt = 32 * T;
+        if constexpr (FAST_FAR)
+            if (J.warp_targets > 0) wt = J.warp_targets;
+        const bool mine = !FAST_FAR || lane * T < wt;
         auto target_slot = [&](int t) {
             return FAST_FAR ? (s_ttile * kWarps + (tid >> 5)) * wt + lane * T + t
                             : s_ttile * TM + static_cast<long long>(t) * kBsThreads + tid;
@@ -466,10 +468,13 @@ __global__ void __launch_bounds__(kBsThreads, (sizeof(R) == 4 && !CHAIN) ? 5 : 1
                 tw[u] = tw[t];
             }
         }
-        bool some = false;
+        bool busy = true;  // the warp has a target (FAST_FAR)
+        if constexpr (FAST_FAR) {
+            bool some = false;
 #pragma unroll
-        for (int t = 0; t < T; ++t) some = some || valid[t];
-        const bool busy = __any_sync(0xffffffffu, some);
+            for (int t = 0; t < T; ++t) some = some || valid[t];
+            busy = __any_sync(0xffffffffu, some);
+        }
         // running sums and compensations; for FP32 lane j of a float2 is target j (s_acc)
         R sx[TT], sy[TT], sz[TT], cx[TT], cy[TT], cz[TT];
         if constexpr (SMEM_ACC) {

@@ -19,7 +19,7 @@ LIB = os.path.join(OUT_DIR, "libstormbird_gb300.so")
 UNITS = ["k_biot_savart.cu", "k_wake.cu", "k_solve.cu", "k_lin_refined.cu", "k_forces.cu", "k_probe.cu", "sim_host.cu", "batch_host.cu", "noalloc_sweep.cu", "k_mlp.cu",
          "mlp_host.cu", "k_wind.cu", "csm_host.cu",
          "result_io.cu"]
-HEADERS = ["sb_device.cuh", "sb_f64.cuh", "sb_f64_tables.inc", "sb_line.cuh", "sb_kernels.h", "sb_setup.hpp", "json_min.hpp", "sim_core.hpp", "sb_ptx.cuh", "sb_mlp.h", "sb_wind_setup.hpp",
+HEADERS = ["sb_device.cuh", "sb_f64.cuh", "sb_f64_tables.inc", "sb_line.cuh", "sb_lin_layout.h", "sb_kernels.h", "sb_setup.hpp", "json_min.hpp", "sim_core.hpp", "sb_ptx.cuh", "sb_mlp.h", "sb_wind_setup.hpp",
            "sb_controller_setup.hpp", "batch_access.hpp", "result_io.hpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

@@ -31,6 +31,7 @@
 
 #include "sb_device.cuh"
 #include "sb_kernels.h"
+#include "sb_lin_layout.h"
 #include "sb_line.cuh"
 
 namespace cg = cooperative_groups;
@@ -40,34 +41,7 @@ namespace sbgpu {
 namespace {
 
 constexpr int kThreads = 512;
-constexpr int kBlk = 16;  // rows of a block
 constexpr int kMaxRefine = 20;
-
-__host__ __device__ inline int padded(int N) { return (N + kBlk - 1) / kBlk * kBlk; }
-__host__ __device__ inline int local_rows(int N, int C) { return (padded(N) / kBlk + C - 1) / C * kBlk; }
-
-// Shared memory of a CTA, in order (all multiples of 16 bytes)
-struct Layout {
-    size_t A, P, M, x, g, rv, dx, vel, w, rhs, tab, total;
-    __host__ __device__ static Layout make(int N, int C) {
-        const size_t n = padded(N), R = local_rows(N, C);
-        Layout l{};
-        size_t at = 0;
-        l.A = at; at += R * n * 4;         // own rows, FP32
-        l.P = at; at += kBlk * n * 4;      // scaled pivot rows
-        l.M = at; at += kBlk * R * 4;      // multipliers, [16][R]
-        l.x = at; at += n * 8;             // solution
-        l.g = at; at += n * 8;             // corrected circulation, then residual terms (CTA 0)
-        l.rv = at; at += n * 4;            // residual
-        l.dx = at; at += n * 4;            // correction
-        l.vel = at; at += R * sizeof(d3);  // velocity of the own rows
-        l.w = at; at += R * sizeof(d3);    // row vectors of the matrix
-        l.rhs = at; at += 2 * R * 8;       // right-hand side, diagonal term
-        l.tab = at; at += (kF64TableDoubles + 1) / 2 * 16;
-        l.total = at;
-        return l;
-    }
-};
 
 // velocity_corrections.rs:28-100 (returns freestream + induced, corrected)
 __device__ __noinline__ d3 corrected_velocity(const SolveSettings& st, d3 fs, d3 ind) {
@@ -101,9 +75,9 @@ struct Work {
     double *rhs, *x, *g, *terms;
     unsigned* counter;
     __device__ Work(double* p, int N) {
-        const size_t n = padded(N);
+        const size_t n = lin_padded(N);
         Pg = reinterpret_cast<float*>(p);
-        A64 = p + kBlk * n;
+        A64 = p + kLinBlk * n;
         double* q = A64 + (static_cast<size_t>(N) * N + 1) / 2 * 2;
         A32 = reinterpret_cast<float*>(q);
         rhs = q + n * n / 2;
@@ -113,8 +87,8 @@ struct Work {
         counter = reinterpret_cast<unsigned*>(terms + n);
     }
     static size_t doubles(int N) {
-        const size_t n = padded(N);
-        return kBlk * n + (static_cast<size_t>(N) * N + 1) / 2 * 2 + n * n / 2 + 4 * n + 2;
+        const size_t n = lin_padded(N);
+        return kLinBlk * n + (static_cast<size_t>(N) * N + 1) / 2 * 2 + n * n / 2 + 4 * n + 2;
     }
 };
 
@@ -170,10 +144,10 @@ template <bool SPLIT>
 __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuffers& b, unsigned char* dyn) {
     cg::cluster_group cl = cg::this_cluster();
     const int C = static_cast<int>(cl.num_blocks()), rank = static_cast<int>(cl.block_rank());
-    const int N = m.N, n = padded(N), R = local_rows(N, C), blocks = n / kBlk;
+    const int N = m.N, n = lin_padded(N), R = lin_local_rows(N, C), blocks = n / kLinBlk;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int kWarps = kThreads / 32;
-    const Layout L = Layout::make(N, C);
+    const LinLayout L = LinLayout::make(N, C);
     float* A = reinterpret_cast<float*>(dyn + L.A);
     float* P = reinterpret_cast<float*>(dyn + L.P);
     float* M = reinterpret_cast<float*>(dyn + L.M);
@@ -189,12 +163,12 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
     const Work W(b.lin_work, N);
     float* Pg = W.Pg;
     double* A64 = W.A64;
-    __shared__ __align__(16) float s_inv[kBlk][kBlk];
+    __shared__ __align__(16) float s_inv[kLinBlk][kLinBlk];
     __shared__ float s_red[kWarps][2];
     __shared__ int s_bad;
 
-    // row l of the CTA is row (rank + (l / 16) C) 16 + l % 16 of the system
-    auto row_of = [&](int l) { return (rank + l / kBlk * C) * kBlk + l % kBlk; };
+    auto row_of = [&](int l) { return lin_row(l, rank, C); };
+    const int here = lin_own_rows(N, C, rank);  // of the R local rows, those of the system
     auto barrier = [&]() {
         if (C > 1) cl.sync();
         else __syncthreads();
@@ -244,16 +218,16 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
     // columns a lane), its rows scaled into P and the global buffer: outside the block's
     // columns inverse x row, inside the inverse.
     auto publish = [&](int k, int lk) {
-        float* Pk = Pg + (k & 1) * kBlk * n;
+        float* Pk = Pg + (k & 1) * kLinBlk * n;
         if (warp == 0) {
             const int row = lane & 15, half = lane >> 4;
-            float* a = A + static_cast<long long>(lk + row) * n + k * kBlk + 8 * half;
+            float* a = A + static_cast<long long>(lk + row) * n + k * kLinBlk + 8 * half;
             float v[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c) v[c] = a[c];
             float least = 3e38f;
 #pragma unroll
-            for (int q = 0; q < kBlk; ++q) {
+            for (int q = 0; q < kLinBlk; ++q) {
                 const int holder = q & 8 ? 16 : 0;  // lanes holding column q
                 const float f = __shfl_sync(0xffffffffu, v[q & 7], holder + row);  // column q of the own row
                 const float p = __shfl_sync(0xffffffffu, v[q & 7], holder + q);    // the pivot
@@ -274,16 +248,16 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
         for (int t = tid; t < n / 2; t += kThreads) {
             const int j = t % (n / 4) * 4, r0 = t / (n / 4) * 8;
             float4 o[8];
-            if (j / kBlk == k) {
+            if (j / kLinBlk == k) {
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
-                    o[q] = make_float4(s_inv[j % kBlk][r0 + q], s_inv[j % kBlk + 1][r0 + q], s_inv[j % kBlk + 2][r0 + q],
-                                       s_inv[j % kBlk + 3][r0 + q]);
+                    o[q] = make_float4(s_inv[j % kLinBlk][r0 + q], s_inv[j % kLinBlk + 1][r0 + q], s_inv[j % kLinBlk + 2][r0 + q],
+                                       s_inv[j % kLinBlk + 3][r0 + q]);
             } else {
 #pragma unroll
                 for (int q = 0; q < 8; ++q) o[q] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-                for (int e = 0; e < kBlk; ++e) {
+                for (int e = 0; e < kLinBlk; ++e) {
                     const float4 a = *reinterpret_cast<const float4*>(A + static_cast<long long>(lk + e) * n + j);
                     const float4 f0 = *reinterpret_cast<const float4*>(&s_inv[e][r0]);
                     const float4 f1 = *reinterpret_cast<const float4*>(&s_inv[e][r0 + 4]);
@@ -309,14 +283,14 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
             const int l = l0 + t / quads * 8, j = t % quads * 4;
             float* a = A + static_cast<long long>(l) * n + j;
             float4 o[8];
-            if (l >= own && l < own + kBlk) {
+            if (l >= own && l < own + kLinBlk) {
 #pragma unroll
                 for (int q = 0; q < 8; ++q) o[q] = *reinterpret_cast<const float4*>(P + (l - own + q) * n + j);
             } else {
 #pragma unroll
                 for (int q = 0; q < 8; ++q) o[q] = *reinterpret_cast<const float4*>(a + static_cast<long long>(q) * n);
 #pragma unroll 2
-                for (int e = 0; e < kBlk; ++e) {
+                for (int e = 0; e < kLinBlk; ++e) {
                     const float4 p = *reinterpret_cast<const float4*>(P + e * n + j);
                     const float4 m0 = *reinterpret_cast<const float4*>(M + e * R + l);
                     const float4 m1 = *reinterpret_cast<const float4*>(M + e * R + l + 4);
@@ -348,25 +322,25 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
     arrive();
 #pragma unroll 1
     for (int k = 0; k < blocks; ++k) {
-        const float* Pk = Pg + (k & 1) * kBlk * n;
-        const int lk = k % C == rank ? k / C * kBlk : -kBlk;  // the block's first row where it is this CTA's
-        const int nx = (k + 1 < blocks && (k + 1) % C == rank) ? (k + 1) / C * kBlk : -1;  // the next block's
+        const float* Pk = Pg + (k & 1) * kLinBlk * n;
+        const int lk = k % C == rank ? k / C * kLinBlk : -kLinBlk;  // the block's first row where it is this CTA's
+        const int nx = (k + 1 < blocks && (k + 1) % C == rank) ? (k + 1) / C * kLinBlk : -1;  // the next block's
         // the rows of block k are published; the buffer of block k - 1, which the owner of block k + 1
         // writes next, has been read by every CTA
         wait();
 #pragma unroll 4
-        for (int t = tid; t < kBlk * n / 4; t += kThreads)
+        for (int t = tid; t < kLinBlk * n / 4; t += kThreads)
             reinterpret_cast<float4*>(P)[t] = __ldcg(reinterpret_cast<const float4*>(Pk) + t);
         // multipliers of the own rows; the block's columns then start from 0
-        for (int t = tid; t < R * kBlk; t += kThreads) {
-            const int l = t >> 4, e = t & (kBlk - 1);
-            float* a = A + static_cast<long long>(l) * n + k * kBlk + e;
+        for (int t = tid; t < R * kLinBlk; t += kThreads) {
+            const int l = t >> 4, e = t & (kLinBlk - 1);
+            float* a = A + static_cast<long long>(l) * n + k * kLinBlk + e;
             M[e * R + l] = *a;
             *a = 0.f;
         }
         __syncthreads();
         if (nx >= 0) {
-            update(nx, nx + kBlk, lk);
+            update(nx, nx + kLinBlk, lk);
             __syncthreads();
             publish(k + 1, nx);
         }
@@ -374,7 +348,7 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
         if (k + 1 < blocks) arrive();
         if (nx >= 0) {
             update(0, nx, lk);
-            update(nx + kBlk, R, lk);
+            update(nx + kLinBlk, R, lk);
         } else {
             update(0, R, lk);
         }
@@ -388,6 +362,8 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
             for (int q = 0; q < C; ++q) cl.map_shared_rank(arr, q)[i] = v;
     };
     // 3. refinement. A bad pivot of any CTA makes its first residual NaN, so that all of them stop.
+    // Only rows of the system (l < here) are stored into the other CTAs: rv and dx hold n values each, and a
+    // store past rv would land in dx, which a CTA behind may still be reading (no barrier between the two).
     for (int i = tid; i < n; i += kThreads) x[i] = 0.0;
     const float poison = s_bad ? __int_as_float(0x7FC00000) : 0.f;
     barrier();
@@ -397,7 +373,7 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
     for (int it = 0; it < kMaxRefine; ++it) {
         // residual of the own rows, to every CTA: eight lanes a row (the FP64 pipe takes a warp
         // instruction as long for one row's tree as for four rows')
-        for (int l = 4 * warp + (lane >> 3); l < R; l += 4 * kWarps) {
+        for (int l = 4 * warp + (lane >> 3); l < here; l += 4 * kWarps) {
             const int i = row_of(l);
             double s = 0.0;
             if (it > 0 && i < N)
@@ -413,7 +389,7 @@ __device__ void solve(const DevModel& m, const SolveSettings& st, const SolveBuf
         }
         barrier();
         // correction of the own rows, to every CTA
-        for (int l = warp; l < R; l += kWarps) {
+        for (int l = warp; l < here; l += kWarps) {
             const int i = row_of(l);
             float s = 0.f;
             for (int c = 4 * lane; c < n; c += 128) {
@@ -546,7 +522,7 @@ constexpr int kRowWarps = kRowThreads / 32;
 __global__ void __launch_bounds__(kRowThreads) k_lin_build(DevModel m, SolveBuffers b) {
     __shared__ __align__(16) double tab[kF64TableDoubles + 1];
     __shared__ SystemRow rows[kRowWarps];
-    const int N = m.N, n = padded(N), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int N = m.N, n = lin_padded(N), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const Work W(b.lin_work, N);
     load_f64_tables(tab, tid, kRowThreads);
     __syncthreads();
@@ -692,10 +668,10 @@ size_t lin_work_doubles(int N) {
 
 LinPlan linearized_refined_plan(int N, int crowding) {
     int C = largest_cluster();
-    while (C > 1 && C > padded(N) / kBlk) C /= 2;
-    if (C < 1 || Layout::make(N, C).total > kSmemLimit) return {0, 0};
-    for (; crowding > 0 && C > 1 && Layout::make(N, C / 2).total <= kSmemLimit; --crowding) C /= 2;
-    return {C, Layout::make(N, C).total};
+    while (C > 1 && C > lin_padded(N) / kLinBlk) C /= 2;
+    if (C < 1 || LinLayout::make(N, C).total > kSmemLimit) return {0, 0};
+    for (; crowding > 0 && C > 1 && LinLayout::make(N, C / 2).total <= kSmemLimit; --crowding) C /= 2;
+    return {C, LinLayout::make(N, C).total};
 }
 
 cudaError_t launch_solve_linearized_refined(const DevModel& m, const SolveSettings& st, const SolveBuffers& b,
@@ -704,7 +680,7 @@ cudaError_t launch_solve_linearized_refined(const DevModel& m, const SolveSettin
     cudaLaunchAttribute attr;
     config(cfg, attr, 1, p.cluster, p.smem, s);
     if (m.N < kSplitLines) return cudaLaunchKernelEx(&cfg, k_lin_refined, m, st, b);
-    k_lin_build<<<(padded(m.N) + kRowWarps - 1) / kRowWarps, kRowThreads, 0, s>>>(m, b);
+    k_lin_build<<<(lin_padded(m.N) + kRowWarps - 1) / kRowWarps, kRowThreads, 0, s>>>(m, b);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, k_lin_refined_split, m, st, b);
     const int passes = st.full_induced_correction && !st.disable_viscous_corrections ? 2 : 1;

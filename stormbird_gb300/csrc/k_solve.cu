@@ -160,7 +160,11 @@ __device__ __noinline__ void solve_line(const DevModel& m, int i, d3 fixed, Solv
     L.fslope = static_cast<float>(L.exp_slope);
     L.fpos = static_cast<float>(L.exp_pos);
     L.fneg = static_cast<float>(L.exp_neg);
-    L.any = !(L.kappa > 0.0) || f.cl_high_order_power > 0.0;
+    // The exponent's FP32 copy, which picks its integer part and decides that it is beyond -32768, has to be
+    // good to a few hundred: its terms are off by some 1e-6 of the slope (the angle in FP32) and 6e-8 of the
+    // stall angles' part. A stall range of 0 has an infinite slope.
+    const bool fits = fabsf(L.fslope) < 1e8f && fabsf(L.fpos) < 1e9f && fabsf(L.fneg) < 1e9f && fabsf(L.fcd) < 4.f;
+    L.any = !(L.kappa > 0.0) || f.cl_high_order_power > 0.0 || !fits;
     L.skew = L.k2 != 0.0;
     L.even = L.exp_pos == L.exp_neg;
     out = L;
@@ -175,7 +179,8 @@ struct LineFlow {
 
 // The same by CUDA's f64 functions, for what lies outside the ranges of line_flow's
 // arithmetic: |u| = 0, infinite or beyond 2^(+-50), a chord along the span or of no length, a
-// high-order lift term, a stall range so narrow that its exponential overflows.
+// high-order lift term, a stall range so narrow that FP32 cannot tell the exponent (below 2e-3
+// degrees; 0: a step), an exponent above 32000.
 __device__ __noinline__ LineFlow line_flow_any(double kappa, const FoilP& f, double a, double c, bool post) {
     LineFlow o;
     o.ul = sqrt(a * a + c * c);

@@ -23,9 +23,10 @@ static __device__ __noinline__ double stall_slow(const FoilP& f, double e) {
 __device__ __forceinline__ double stall_f64(const FoilP& f, double e, const double* tab) {
     const double mean = fabs(__double2hiint(e) >= 0 ? f.mean_positive_stall_angle : f.mean_negative_stall_angle);
     const double w = (f.stall_slope * 738.6598609351493) * (mean - fabs(e));  // 512 / ln 2
-    const float wf = f64_to_f32(w);
-    if (!(fabsf(wf) < 32000.f)) return wf < 0.f ? 1.0 : stall_slow(f, e);
-    const float n = rintf(wf);
+    // |w| >= 32000, infinite or no number, from the high word: the FP32 copy is good only below 2^127 (a stall
+    // range of 0 has an infinite slope)
+    if ((static_cast<unsigned>(__double2hiint(w)) & 0x7FFFFFFFu) >= 0x40DF4000u) return w < 0.0 ? 1.0 : stall_slow(f, e);
+    const float n = rintf(f64_to_f32(w));
     return rcp_f64(1.0 + exp2_512_f64(static_cast<int>(n), w - f32_to_f64(n), tab));
 }
 

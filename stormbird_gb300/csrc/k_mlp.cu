@@ -925,11 +925,7 @@ bool encode_bf16_map(CUtensorMap* map, const bf16* ptr, long long rows, long lon
 }  // namespace
 
 cudaError_t launch_mlp_gemm(const GemmArgs& g, cudaStream_t s) {
-    // TMA: 16-byte aligned bases and row strides; every box lies inside its matrix
-    if (g.M <= 0 || g.M % kMlpRowTile || g.K <= 0 || g.K % kKStep || g.k_split <= 0 || g.k_split % kKStep ||
-        (g.N != 64 && g.N != 128 && g.N != 256) || g.lda % 8 || g.ldb % 8 || g.lda < g.K || g.ldb < g.K ||
-        reinterpret_cast<uintptr_t>(g.A) % 16 || reinterpret_cast<uintptr_t>(g.B) % 16)
-        return cudaErrorInvalidValue;
+    if (!mlp_gemm_args_ok(g)) return cudaErrorInvalidValue;
     CUtensorMap ma, mb;
     const int splits = (g.K + g.k_split - 1) / g.k_split, tiles = g.M / kMlpRowTile;
     const int z = g.N >= 128 && tiles * splits <= g.sms ? 2 : 1;
@@ -951,8 +947,11 @@ cudaError_t launch_mlp_forward(const FwdArgs& args, cudaStream_t s) {
     const int tiles = (g.rows + 127) / 128;
     if (g.z[0]) {
         if (tiles > g.sms) return cudaErrorInvalidValue;
+        for (int l = 0; l < kMlpHidden; ++l)
+            if (!g.z[l] || !g.h[l]) return cudaErrorInvalidValue;
         k_mlp_forward<true><<<tiles, kFwdThreads, kFwdSmem, s>>>(maps, g);
     } else {
+        if (!g.y) return cudaErrorInvalidValue;
         k_mlp_forward<false><<<std::min(tiles, std::max(1, g.sms)), kFwdThreads, kFwdSmem, s>>>(maps, g);
     }
     return cudaGetLastError();

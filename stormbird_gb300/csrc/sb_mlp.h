@@ -34,15 +34,26 @@ struct GemmArgs {
     int M = 0, N = 0, K = 0, k_split = 0;
     int mode = 0;
     const float* bias = nullptr;
-    float* z_out = nullptr;   // [M][N] or nullptr
-    bf16* h_out = nullptr;    // [M][N] or nullptr
-    bf16* hT_out = nullptr;   // [N][ldt] or nullptr
+    float* z_out = nullptr;   // [M][N] (forward)
+    bf16* h_out = nullptr;    // [M][N] (forward, backward)
+    bf16* hT_out = nullptr;   // [N][ldt] or nullptr (forward, backward)
     long long ldt = 0;
-    const float* z_in = nullptr;
-    float* part_out = nullptr;
+    const float* z_in = nullptr;  // [M][N] (backward)
+    float* part_out = nullptr;    // partial
     int sms = 1;
     int* err = nullptr;
 };
+// Shapes the kernel takes (TMA: 16-byte aligned bases and row strides; every box lies inside its matrix) and
+// every array that its mode reads or writes.
+inline bool mlp_gemm_args_ok(const GemmArgs& g) {
+    if (g.M <= 0 || g.M % kMlpRowTile || g.K <= 0 || g.K % 64 || g.k_split <= 0 || g.k_split % 64 ||
+        (g.N != 64 && g.N != 128 && g.N != 256) || g.lda % 8 || g.ldb % 8 || g.lda < g.K || g.ldb < g.K || !g.A || !g.B ||
+        reinterpret_cast<uintptr_t>(g.A) % 16 || reinterpret_cast<uintptr_t>(g.B) % 16)
+        return false;
+    if (g.mode == kGemmPartial) return g.part_out != nullptr;
+    if (!g.h_out || (g.hT_out && g.ldt < g.M)) return false;
+    return g.mode == kGemmForward ? g.bias && g.z_out : g.mode == kGemmBackward && g.z_in;
+}
 size_t mlp_gemm_smem_bytes();
 // Raises the GEMM kernel's dynamic shared-memory limit (once, before any stream capture).
 cudaError_t configure_mlp_gemm();
@@ -57,7 +68,7 @@ struct FwdArgs {
     const float* w_out = nullptr;             // [257]
     float* y = nullptr;
     // training (z[0] not null; at most sms tiles of 128 rows): pre-activations [rows_pad][256], activations
-    // [rows_pad][256] and [256][ldt] (null: not wanted) of every layer instead of y
+    // [rows_pad][256] and their transposes [256][ldt] (these null: not wanted) of every layer instead of y
     float* z[kMlpHidden] = {nullptr};
     bf16* h[kMlpHidden] = {nullptr};
     bf16* hT[kMlpHidden] = {nullptr};

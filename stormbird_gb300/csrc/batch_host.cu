@@ -514,11 +514,9 @@ struct sb_batch {
             g.job_off = job_entries;
             job_entries += static_cast<long long>(n) + 1;  // + sentinel
         }
-        if (partial.n < static_cast<size_t>(std::max<long long>(part_total, 1))) partial.alloc(std::max<long long>(part_total, 1));
-        if (h_jobs.n < static_cast<size_t>(std::max<long long>(job_entries, 1))) {
-            h_jobs.alloc(std::max<long long>(job_entries, 1));
-            d_jobs.alloc(std::max<long long>(job_entries, 1));
-        }
+        partial.grow(std::max<long long>(part_total, 1));
+        h_jobs.grow(std::max<long long>(job_entries, 1));
+        d_jobs.grow(std::max<long long>(job_entries, 1));
         tuning = t;
     }
 
@@ -734,7 +732,7 @@ struct sb_batch {
             if (mode != 0 && c->solver_kind != 0) raise(SB_ERR_UNSUPPORTED, "the warm start needs SimpleIterative solvers");
         ck(cudaStreamSynchronize(main), "sync");
         drop_graphs();
-        if (mode != 0 && w_feat.n == 0) {
+        if (mode != 0 && d_feat.n == 0) {  // the last one below: all of them, or again from the first
             w_feat.alloc(static_cast<size_t>(N_total) * kMlpFeatures);
             w_y.alloc(N_total);
             w_target.alloc(N_total);
@@ -1021,12 +1019,10 @@ struct sb_batch {
     void set_wind(const char* env_json, const char* const* cond_jsons) {
         ck(cudaStreamSynchronize(main), "sync");
         drop_graphs();
-        if (wind_steps.n == 0) {
-            h_wind_jobs.alloc(cases.size());
-            d_wind_jobs.alloc(cases.size());
-            wind_steps.alloc(cases.size() * 2);
-            h_wind_steps.alloc(cases.size() * 2);
-        }
+        h_wind_jobs.grow(cases.size());
+        d_wind_jobs.grow(cases.size());
+        wind_steps.grow(cases.size() * 2);
+        h_wind_steps.grow(cases.size() * 2);
         std::vector<WindPack> packs;
         packs.reserve(cases.size());
         sbsetup::WindEnvironment env;
@@ -1068,10 +1064,8 @@ struct sb_batch {
             h_wind_steps.p[2 * i] = time;
             h_wind_steps.p[2 * i + 1] = ship_velocities[i];
         }
-        if (ctrl_in.n == 0) {
-            ctrl_in.alloc(static_cast<size_t>(N_total) * 3);
-            h_ctrl_in.alloc(static_cast<size_t>(N_total) * 3);
-        }
+        ctrl_in.grow(static_cast<size_t>(N_total) * 3);
+        h_ctrl_in.grow(static_cast<size_t>(N_total) * 3);
         ck(cudaMemcpyAsync(wind_steps.p, h_wind_steps.p, cases.size() * 2 * sizeof(double), cudaMemcpyHostToDevice, main),
            "H2D wind steps");
         fill_wind_jobs(ctrl_in.p);
@@ -1090,10 +1084,8 @@ struct sb_batch {
     const double* wing_totals() {
         size_t total = 0;
         for (const auto& c : cases) total += static_cast<size_t>(c->S) * 36;
-        if (h_wing_totals.n < total) {
-            h_wing_totals.alloc(total);
-            wing_totals_dev.alloc(total);
-        }
+        h_wing_totals.grow(total);
+        wing_totals_dev.grow(total);
         k_gather_totals<<<static_cast<unsigned>(cases.size()), 128, 0, main>>>(gather_jobs.p, wing_totals_dev.p);
         ck(cudaGetLastError(), "wing totals");
         ck(cudaMemcpyAsync(h_wing_totals.p, wing_totals_dev.p, total * sizeof(double), cudaMemcpyDeviceToHost, main),

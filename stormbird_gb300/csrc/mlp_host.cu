@@ -135,6 +135,7 @@ struct sb_mlp {
     void ensure(long long rows) {
         const int need = pad_rows(std::max<long long>(rows, 1));
         if (need <= cap) return;
+        cap = 0;  // until all of them are there
         const size_t w = static_cast<size_t>(need) * kMlpWidth;
         X0.alloc(static_cast<size_t>(need) * kMlpInPad);
         X0T.alloc(static_cast<size_t>(need) * kMlpInPad);

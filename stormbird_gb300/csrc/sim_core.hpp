@@ -72,8 +72,13 @@ struct DevBuf {
     ~DevBuf() { if (p) cudaFree(p); }
     void alloc(size_t count) {
         if (p) { cudaFree(p); p = nullptr; }
-        n = count;
+        n = 0;  // until there is memory: a failed allocation leaves an empty buffer
         if (count) ck(cudaMalloc(&p, count * sizeof(T)), "cudaMalloc");
+        n = count;
+    }
+    // Room for count values (the old ones are not kept).
+    void grow(size_t count) {
+        if (n < count) alloc(count);
     }
     void upload(const std::vector<T>& h) {
         alloc(h.size());
@@ -102,8 +107,12 @@ struct PinnedBuf {
     ~PinnedBuf() { if (p) cudaFreeHost(p); }
     void alloc(size_t count) {
         if (p) { cudaFreeHost(p); p = nullptr; }
-        n = count;
+        n = 0;
         if (count) ck(cudaMallocHost(&p, count * sizeof(T)), "cudaMallocHost");
+        n = count;
+    }
+    void grow(size_t count) {
+        if (n < count) alloc(count);
     }
 };
 
@@ -130,10 +139,14 @@ struct WindArena {
         size_t n = 0;
         for (const auto& p : packs) n += p.data.size() + p.ranges.size() + (p.ints.size() + 1) / 2;
         n = std::max<size_t>(n, 1);
+        // a larger buffer before the old one goes: where there is no room, the models keep their tables
+        DevBuf<double> larger;
+        if (dev.n < n) larger.alloc(n);
         ck(cudaStreamSynchronize(s), "wind tables");
+        host.grow(n);
         if (dev.n < n) {
-            dev.alloc(n);
-            host.alloc(n);
+            std::swap(dev.p, larger.p);
+            std::swap(dev.n, larger.n);
         }
         size_t at = 0;
         for (auto& p : packs) {
@@ -832,7 +845,7 @@ struct sb_sim {
             target_layout(d, a.job0);
             SweepPlan sp = plan_sweep(bs_slots(a.job0), P, sym, neglect);
             size_t need = static_cast<size_t>(sp.n_chunks) * static_cast<size_t>(M) * 3;
-            if (partial.n < need) partial.alloc(need);
+            partial.grow(need);
             a.job0.panels = d.src ? d.src : precision == 2 ? static_cast<const void*>(rec64.p) : static_cast<const void*>(rec32.p);
             a.chain = d.chain ? 1 : 0;
             a.job0.p_begin = p0;
@@ -1469,10 +1482,8 @@ struct sb_sim {
         } catch (const sbsetup::SetupError& e) {
             raise(SB_ERR_BAD_JSON, e.what());
         }
-        if (wind_step_own.n == 0) {
-            wind_step_own.alloc(2);
-            h_wind_step.alloc(2);
-        }
+        wind_step_own.grow(2);
+        h_wind_step.grow(2);
         wind_arena.upload(packs, stream);
         use_wind(packs[0].w, has_wind && wind.step ? wind.step : wind_step_own.p);
     }
@@ -1524,7 +1535,8 @@ struct sb_sim {
         if (!dynamic) raise(SB_ERR_STATE, "Induced velocities not implemented for pure quasi-steady simulations yet");
         if (n == 0) return;
         ensure_rec64();
-        if (aux_targets.n < n) { aux_targets.alloc(n); aux_out.alloc(n); }
+        aux_targets.grow(n);
+        aux_out.grow(n);
         ck(cudaMemcpyAsync(aux_targets.p, p, n * sizeof(d3), cudaMemcpyHostToDevice, stream), "H2D points");
         sweep({aux_targets.p, static_cast<long long>(n), 0, P_pan, nullptr, nullptr, static_cast<long long>(n), aux_out.p},
               2);

@@ -395,10 +395,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const __grid_con
                             mbar_expect_tx(&full[s], kFwdSub);
                             tma_load_2d(ring + s * kFwdSub, &maps.w[l], (h >> 1) * kKStep, (h & 1) * 128, &full[s]);
                         }
-            // every copy has landed before the CTA leaves (those of a finished pass were waited for)
-            if (!ok)
-                for (int k = n - kFwdRing > 0 ? n - kFwdRing : 0; k < n; ++k)
-                    mbar_wait_bounded(&full[k % kFwdRing], (k / kFwdRing) & 1, g.err);
+            // every copy has landed before the CTA leaves: the MMA thread waits for them as it reads them, but
+            // reads no more after a wait of its own that ran out
+            for (int k = n - kFwdRing > 0 ? n - kFwdRing : 0; k < n; ++k)
+                mbar_wait_bounded(&full[k % kFwdRing], (k / kFwdRing) & 1, g.err);
         }
     } else if (warp == kFwdWarps + 1) {
         if (lane == 0) {  // MMAs

@@ -152,9 +152,6 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 sub2s(float2 a, float b) { return __ffma2_rn(make_float2(b, b), make_float2(-1.f, -1.f), a); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 sel2(bool cx, float2 a, bool cy, float2 b) {
-    return make_float2(cx ? a.x : b.x, cy ? a.y : b.y);
-}
 // The hardware reciprocal square root (PTX rsqrt.approx.ftz.f32). Every argument below is
 // first clamped to a normal float, where this is the same approximation rsqrtf returns,
 // without the handling of subnormal arguments around it.

@@ -63,8 +63,6 @@ __host__ __device__ inline long long si_slab_offset(int N, int cluster) {
 struct RowGeom {
     d3 felt, span_dir, chord, span_rel_out;  // span_dir = normalize(span end - span start)
     double chord_len, area;
-    double chord_norm;  // |chord vector|
-    double cl_gamma;    // 2 |span_rel| / area (0 if the area or density is 0): see residual_of_row
     int wing;
 };
 
@@ -77,8 +75,6 @@ __device__ inline RowGeom row_geom(const DevModel& m, int i) {
     g.span_rel_out = m.output_body ? (m.span_e_local[i] - m.span_s_local[i]) : span_rel;
     g.chord_len = m.chord_len[i];
     g.area = m.chord_len[i] * m.span_len_local[i];
-    g.chord_norm = len(g.chord);
-    g.cl_gamma = (g.area == 0.0 || m.density == 0.0) ? 0.0 : 2.0 * len(span_rel) / g.area;
     g.wing = m.wing_of_line[i];
     return g;
 }
@@ -93,12 +89,6 @@ __device__ inline d3 total_velocity(const SolveSettings& st, d3 fs, d3 ind) {
     }
     if (st.velocity_correction == 2) return normalize(fs + ind) * len(fs);
     return fs + ind;
-}
-
-__device__ inline double circulation_cl(const DevModel& m, const FoilP& f, double aoa) {
-    double cl = foil_cl_pre_stall(f, aoa);
-    if (m.include_viscous_lift) cl += foil_cl_post_stall(f, aoa);
-    return cl;
 }
 
 // |cl_gamma - cl_direct| of force_calculations.rs:552-607, given cl_direct = the foil's
@@ -696,7 +686,7 @@ __device__ void si_solve(const DevModel& m, const SolveSettings& st, const Solve
             const double gold = src ? src[i] : gown[RPT == 1 ? 0 : k];
             double r = residual_of_line(m, L, i, gold, a, c, o);
             if (start == 3) {
-                // circulation_cl: the pre-stall lift serves the estimate and the residual alike
+                // the pre-stall lift serves the estimate and the residual alike
                 const double est = L.half_chord * o.ul * (m.include_viscous_lift ? o.cl_pre + o.cl_post : o.cl_pre);
                 const double d = est - gold;
                 const double gnew = fma(st.damping, d, gold);

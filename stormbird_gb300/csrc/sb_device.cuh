@@ -173,23 +173,6 @@ __device__ inline double foil_cl_post_stall(const FoilP& f, double a) {
     double raw = f.cl_max_after_stall * sin(2.0 * stall_angle(a));
     return raw * foil_amount_of_stall(f, a);
 }
-// foil.rs:212-243
-__device__ inline double foil_cd(const FoilP& f, double a) {
-    double sa = stall_angle(a);
-    double eff = fabs(a + f.angle_cd_min);
-    double pre = f.cd_min + f.cd_second_order_factor * (eff * eff);
-    double post = f.cd_max_after_stall * pow(fabs(sin(sa)), f.cd_power_after_stall);
-    double at = a + f.cd_stall_angle_offset * signum(a);
-    double s = foil_amount_of_stall(f, at);
-    double raw = pre * (1.0 - s) + s * post;
-    double during = f.cd_bump_during_stall * ((1.0 - cos(s * kTau)) * 0.5);
-    if (f.cdi_correction_factor != 0.0) {
-        double cl = fabs(foil_cl_post_stall(f, a) + foil_cl_pre_stall(f, a));
-        return raw + f.cdi_correction_factor * (cl * cl) + during;
-    }
-    return raw + during;
-}
-
 // Job that block b of a launch over a job list belongs to: the last one whose first block of the kind is
 // at or before it (jobs [n] ascending in each kind's first block).
 template <class Job, long long Job::*First>
@@ -294,8 +277,6 @@ struct DevModel {
     const FoilP* foils = nullptr;
     const int* sp_line = nullptr;    // [Np] line whose start (or end, sp_end) is span point k
     const unsigned char* sp_end = nullptr;
-    const int* sp_val_a = nullptr;   // [Np] value mapping control -> span points
-    const int* sp_val_b = nullptr;   //       value = (c[a] + c[b]) * 0.5, or c[a] if a == b
     const double* panel_core = nullptr;  // [W*N]
     // per-step geometry
     d3* chord_local = nullptr;

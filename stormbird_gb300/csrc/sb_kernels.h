@@ -250,10 +250,9 @@ struct SolveBuffers {
     // other entry is an FP32 value, lo = 0)
     const float* factors_split = nullptr;
     int split_full = 1;
-    // components per entry: 2 in the rows' in-plane bases (basis, [2N]: the velocity's span
+    // components per entry: 2 in the rows' in-plane bases (DevModel::solve_basis: the velocity's span
     // component is projected out anyway; no velocity correction), else 3 (x, y, z)
     int split_comps = 3;
-    const d3* basis = nullptr;
     double* gamma_prev = nullptr;   // [N] in: initial solution, out: solution
     d3* vel_out = nullptr;          // [N] output control-point velocity
     double* scalars = nullptr;      // [8]: residual, iterations, converged, singular, start (below),

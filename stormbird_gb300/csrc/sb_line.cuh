@@ -87,7 +87,7 @@ __device__ __forceinline__ LineLift line_lift(const FoilP& f, d3 chord, d3 v, d3
     return o;
 }
 
-// foil_cd (foil.rs:212-243) at the lift's angle
+// The foil's drag coefficient (foil.rs:212-243) at the lift's angle
 static __device__ __noinline__ double cd_bump(double amount, double s) { return amount * ((1.0 - cos(s * kTau)) * 0.5); }
 __device__ __forceinline__ double line_drag(const FoilP& f, const LineLift& o, const double* tab) {
     const double eff = fabs(o.aoa + f.angle_cd_min);

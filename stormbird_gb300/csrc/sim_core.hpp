@@ -410,7 +410,7 @@ struct sb_sim {
     // constants
     DevBuf<d3> span_s_local, span_e_local, chord_nr;
     DevBuf<double> chord_len, span_len_local, panel_core;
-    DevBuf<int> wing_of_line, wing_start, wing_end, sp_line, sp_a, sp_b;
+    DevBuf<int> wing_of_line, wing_start, wing_end, sp_line;
     DevBuf<unsigned char> is_virtual, sp_end;
     DevBuf<FoilP> foils;
     // geometry
@@ -545,14 +545,14 @@ struct sb_sim {
         if (S > kMaxWings) raise(SB_ERR_UNSUPPORTED, "more than 64 wings");
         Np = N + S;
         chord_lengths_h = cl;
-        // span points and control -> span value mapping (data_update.rs:41-55, value_mapping.rs:87-137)
-        std::vector<int> spl, spa, spb;
+        // span points (data_update.rs:41-55)
+        std::vector<int> spl;
         std::vector<unsigned char> spe;
         for (int w = 0; w < S; ++w) {
-            spl.push_back(ws[w]); spe.push_back(0); spa.push_back(ws[w]); spb.push_back(ws[w]);
+            spl.push_back(ws[w]); spe.push_back(0);
             for (int i = ws[w]; i < we[w]; ++i) {
-                if (i == we[w] - 1) { spl.push_back(i); spe.push_back(1); spa.push_back(i); spb.push_back(i); }
-                else { spl.push_back(i + 1); spe.push_back(0); spa.push_back(i); spb.push_back(i + 1); }
+                if (i == we[w] - 1) { spl.push_back(i); spe.push_back(1); }
+                else { spl.push_back(i + 1); spe.push_back(0); }
             }
         }
         span_s_local.upload(ss); span_e_local.upload(se); chord_nr.upload(cn);
@@ -561,7 +561,7 @@ struct sb_sim {
         wing_of_line_h = wol;
         wing_start_h = ws;
         is_virtual.upload(virt); foils.upload(fo);
-        sp_line.upload(spl); sp_end.upload(spe); sp_a.upload(spa); sp_b.upload(spb);
+        sp_line.upload(spl); sp_end.upload(spe);
 
         // step parameters from the builder (builder/mod.rs:97-108)
         for (int w = 0; w < S; ++w) params.local_wing_angles[w] = b.local_wing_angles.empty() ? 0.0 : b.local_wing_angles[w];
@@ -578,7 +578,7 @@ struct sb_sim {
         dm.span_s_local = span_s_local.p; dm.span_e_local = span_e_local.p; dm.chord_not_rotated = chord_nr.p;
         dm.chord_len = chord_len.p; dm.span_len_local = span_len_local.p; dm.wing_of_line = wing_of_line.p;
         dm.wing_start = wing_start.p; dm.wing_end = wing_end.p; dm.is_virtual = is_virtual.p; dm.foils = foils.p;
-        dm.sp_line = sp_line.p; dm.sp_end = sp_end.p; dm.sp_val_a = sp_a.p; dm.sp_val_b = sp_b.p;
+        dm.sp_line = sp_line.p; dm.sp_end = sp_end.p;
         if (dynamic) {
             const auto& w = setup.dynamic_wake;
             W = static_cast<int>(w.nr_panels_per_line_element);
@@ -1082,8 +1082,7 @@ struct sb_sim {
         sb.factors_split = factors_split.p;
         // off-diagonal lo parts are zero when the unit matrix came from the FP32 records
         sb.split_full = (dynamic && precision != 2) ? 0 : 1;
-        sb.basis = split_basis();
-        sb.split_comps = sb.basis ? 2 : 3;
+        sb.split_comps = split_basis() ? 2 : 3;
         sb.gamma_prev = gamma_p;
         sb.vel_out = vel_out.p;
         sb.scalars = scalars.p;

@@ -674,6 +674,10 @@ LinPlan linearized_refined_plan(int N, int crowding) {
     return {C, LinLayout::make(N, C).total};
 }
 
+static int finish_passes(const SolveSettings& st) { return st.full_induced_correction && !st.disable_viscous_corrections ? 2 : 1; }
+
+int linearized_refined_launches(int N, const SolveSettings& st) { return N < kSplitLines ? 1 : 2 + finish_passes(st); }
+
 cudaError_t launch_solve_linearized_refined(const DevModel& m, const SolveSettings& st, const SolveBuffers& b,
                                             const LinPlan& p, cudaStream_t s) {
     cudaLaunchConfig_t cfg;
@@ -683,7 +687,7 @@ cudaError_t launch_solve_linearized_refined(const DevModel& m, const SolveSettin
     k_lin_build<<<(lin_padded(m.N) + kRowWarps - 1) / kRowWarps, kRowThreads, 0, s>>>(m, b);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, k_lin_refined_split, m, st, b);
-    const int passes = st.full_induced_correction && !st.disable_viscous_corrections ? 2 : 1;
+    const int passes = finish_passes(st);
     for (int k = 0; k < passes && e == cudaSuccess; ++k) {
         k_lin_finish<<<(m.N + kRowWarps - 1) / kRowWarps, kFinishThreads, 0, s>>>(m, st, b, k, k + 1 == passes);
         e = cudaGetLastError();

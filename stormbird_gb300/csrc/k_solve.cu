@@ -475,7 +475,7 @@ __device__ void si_solve(const DevModel& m, const SolveSettings& st, const Solve
     const long long buf_floats = static_cast<long long>(slab_rows) * rowf * (LO ? 2 : 1);
     const long long lo_plane = static_cast<long long>(C) * N * S;
     const int lp = b.lanes_log2;  // log2 of the lanes per row of the product
-   if (tid == 0) {
+    if (tid == 0) {
         mbar_init(&s_mbar[0], 1);
         mbar_init(&s_mbar[1], 1);
         fence_mbar_init();
@@ -1338,6 +1338,10 @@ LinPlan linearized_plan(int N) {
         if (bytes <= kLinSmemLimit && cluster_fits(C, bytes)) return {C, bytes};
     }
     return {1, v};  // matrix in the case's global scratch
+}
+
+int linearized_launches(int N, const SolveSettings& st) {
+    return 1 + (linearized_refined_plan(N, 0).cluster > 0 ? linearized_refined_launches(N, st) : 0);
 }
 
 cudaError_t launch_solve_linearized(const DevModel& m, const SolveSettings& st, const SolveBuffers& b, cudaStream_t s) {

@@ -282,6 +282,7 @@ constexpr int kMaxCrowding = 4;
 int solve_cluster_size(int N, int crowding);
 cudaError_t launch_solve_simple_iterative(const DevModel& m, const SolveSettings& st, const SolveBuffers& b, cudaStream_t s);
 cudaError_t launch_solve_linearized(const DevModel& m, const SolveSettings& st, const SolveBuffers& b, cudaStream_t s);
+int linearized_launches(int N, const SolveSettings& st);  // kernels that it launches
 
 // One solve of a batch (k_solve_lin_jobs, k_solve_lin_cluster_jobs, k_solve_si_jobs).
 struct SolveJob {
@@ -307,6 +308,7 @@ LinPlan linearized_refined_plan(int N, int crowding);
 size_t lin_work_doubles(int N);  // SolveBuffers::lin_work
 cudaError_t launch_solve_linearized_refined(const DevModel& m, const SolveSettings& st, const SolveBuffers& b,
                                             const LinPlan& plan, cudaStream_t s);
+int linearized_refined_launches(int N, const SolveSettings& st);
 // n solves of one plan shape in one launch (smem: the largest of the jobs' plans).
 cudaError_t launch_solve_linearized_jobs(const SolveJob* jobs, int n, const LinPlan& plan, cudaStream_t s);
 cudaError_t launch_solve_linearized_refined_jobs(const SolveJob* jobs, int n, const LinPlan& plan, cudaStream_t s);

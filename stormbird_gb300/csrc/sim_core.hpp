@@ -1122,15 +1122,16 @@ struct sb_sim {
                 lb.rec64_row0 = nullptr;
                 SolveSettings ls;  // Linearized::default()
                 ck(launch_solve_linearized(dm, ls, lb, stream), "linearized start");
-                launches += 1;
+                launches += linearized_launches(N, ls);
                 ck(cudaMemcpyAsync(gamma_p, gamma_tmp.p, N * sizeof(double), cudaMemcpyDeviceToDevice, stream), "copy");
                 st.correction_factor_initial = 1.0;
             }
             ck(launch_solve_simple_iterative(dm, st, sb, stream), "simple iterative solve");
+            launches += 1;
         } else {
             ck(launch_solve_linearized(dm, solve, sb, stream), "linearized solve");
+            launches += linearized_launches(N, solve);
         }
-        launches += 1;
     }
 
     void step_after_solve() {

@@ -40,8 +40,8 @@ __device__ __forceinline__ void load_f64_tables(double* t, int tid, int nt) {
 __device__ __forceinline__ bool f64_seed_range(double v) {
     return static_cast<unsigned>(__double2hiint(v)) - 0x39B00000u < 0x0C800000u;
 }
-// The nearest float of v (ties away from zero) by integer arithmetic, for |v| in [2^-126, 2^127);
-// smaller magnitudes give 0.
+// The nearest float of v (ties away from zero) by integer arithmetic, for |v| in [2^-126, 2^128);
+// all others give 0, infinities and no numbers too.
 __device__ __forceinline__ float f64_to_f32(double v) {
     const unsigned hi = static_cast<unsigned>(__double2hiint(v));
     const unsigned lo = static_cast<unsigned>(__double2loint(v));
@@ -50,7 +50,7 @@ __device__ __forceinline__ float f64_to_f32(double v) {
     return __uint_as_float((mag - 0x00100000u < 0x0FE00000u ? bits : 0u) | (hi & 0x80000000u));
 }
 // The nearest float of v, ties to even (the conversion's own result), by integer arithmetic for 0 and
-// |v| in [2^-126, 2^127); others through the conversion.
+// |v| in [2^-126, 2^128); others through the conversion.
 static __device__ __noinline__ float f64_to_f32_slow(double v) { return __double2float_rn(v); }
 __device__ __forceinline__ float f64_to_f32_rn(double v) {
     const unsigned hi = static_cast<unsigned>(__double2hiint(v)), lo = static_cast<unsigned>(__double2loint(v));
@@ -160,7 +160,8 @@ __device__ __forceinline__ double arcsin_f64(double d) {
     return fma(d * d * d, p, d);
 }
 
-// 2^((n + f) / 512) for |f| <= 0.6 and n in [-512 * 900, 512 * 99]; t: the tables. 5 FP64 instructions.
+// 2^((n + f) / 512) for |f| <= 0.6 and n in [-512 * 1021, 512 * 1022] (the result a normal number: its exponent is
+// shifted in place); t: the tables. 5 FP64 instructions.
 __device__ __forceinline__ double exp2_512_f64(int n, double f, const double* t) {
     constexpr double kC = 0.0013538030870311431;  // ln 2 / 512
     const float ff = f64_to_f32(f);

@@ -23,7 +23,7 @@ static __device__ __noinline__ double stall_slow(const FoilP& f, double e) {
 __device__ __forceinline__ double stall_f64(const FoilP& f, double e, const double* tab) {
     const double mean = fabs(__double2hiint(e) >= 0 ? f.mean_positive_stall_angle : f.mean_negative_stall_angle);
     const double w = (f.stall_slope * 738.6598609351493) * (mean - fabs(e));  // 512 / ln 2
-    // |w| >= 32000, infinite or no number, from the high word: the FP32 copy is good only below 2^127 (a stall
+    // |w| >= 32000, infinite or no number, from the high word: the FP32 copy is good only below 2^128 (a stall
     // range of 0 has an infinite slope)
     if ((static_cast<unsigned>(__double2hiint(w)) & 0x7FFFFFFFu) >= 0x40DF4000u) return w < 0.0 ? 1.0 : stall_slow(f, e);
     const float n = rintf(f64_to_f32(w));
@@ -31,7 +31,7 @@ __device__ __forceinline__ double stall_f64(const FoilP& f, double e, const doub
 }
 
 // x^p for x in [0, 1]: log2 x from 2^(j/512), j the nearest, and the series of the rest
-// (|r| <= 6.8e-4, next term below 3e-17), then exp2_512_f64.
+// (|r| <= 6.8e-4, next term below 3e-17), then exp2_512_f64 (n >= -512 * 960: x >= 2^-60, p <= 16).
 static __device__ __noinline__ double pow_slow(double x, double p) { return pow(x, p); }
 __device__ __forceinline__ double pow_f64(double x, double p, const double* tab) {
     const int hi = __double2hiint(x), k = (hi >> 20) - 1023;

@@ -743,7 +743,7 @@ struct sb_batch {
             w_cand_ex.alloc(N_total);
             w_gamma_old.alloc(N_total);
             w_fs_old.alloc(N_total);
-            ck(cudaMemset(w_target.p, 0, N_total * sizeof(float)), "memset");
+            ck(cudaMemsetAsync(w_target.p, 0, N_total * sizeof(float), main), "memset");
             h_feat.alloc(cases.size());
             d_feat.alloc(cases.size());
         }
@@ -883,14 +883,14 @@ struct sb_batch {
             for (auto& h : warm_hist) h = std::min(h + 1, 2);
         if (mlp) mlp_check(mlp);
         if (h_err.p[0] != kDevOk) {
-            ck(cudaMemset(err.p, 0, sizeof(int)), "memset");
+            ck(cudaMemsetAsync(err.p, 0, sizeof(int), main), "memset");
             raise(SB_ERR_TIMEOUT, "a bounded device-side wait ran out in a batched sweep");
         }
         for (size_t i = 0; i < cases.size(); ++i) {
             const double st = h_compact.p[N_total + static_cast<long long>(i) * SB_BATCH_SUMMARY + 9];
             if (st != 0.0) {
                 sb_sim& c = *cases[i];
-                ck(cudaMemset(c.err.p, 0, sizeof(int)), "memset");
+                ck(cudaMemsetAsync(c.err.p, 0, sizeof(int), main), "memset");
                 if (st == kDevTimeout) raise(SB_ERR_TIMEOUT, "case " + std::to_string(i) + ": a bounded device-side wait ran out");
                 if (st == kDevSingular) raise(SB_ERR_STATE, "case " + std::to_string(i) + ": Matrix is singular or nearly singular");
                 raise(SB_ERR_CUDA, "case " + std::to_string(i) + ": device error word " + std::to_string(st));
@@ -1167,7 +1167,7 @@ struct sb_batch {
         ck(cudaMemcpyAsync(h_err.p, err.p, sizeof(int), cudaMemcpyDeviceToHost, main), "D2H status");
         ck(cudaStreamSynchronize(main), "tuning");
         if (h_err.p[0] != kDevOk) {
-            ck(cudaMemset(err.p, 0, sizeof(int)), "memset");
+            ck(cudaMemsetAsync(err.p, 0, sizeof(int), main), "memset");
             raise(SB_ERR_TIMEOUT, "a bounded device-side wait ran out in a batched sweep");
         }
         tuned = true;

@@ -97,16 +97,16 @@ struct sb_mlp {
         grads.alloc(n_params);
         adam_m.alloc(n_params);
         adam_v.alloc(n_params);
-        ck(cudaMemset(grads.p, 0, n_params * sizeof(float)), "memset");
-        ck(cudaMemset(adam_m.p, 0, n_params * sizeof(float)), "memset");
-        ck(cudaMemset(adam_v.p, 0, n_params * sizeof(float)), "memset");
+        ck(cudaMemsetAsync(grads.p, 0, n_params * sizeof(float), stream), "memset");
+        ck(cudaMemsetAsync(adam_m.p, 0, n_params * sizeof(float), stream), "memset");
+        ck(cudaMemsetAsync(adam_v.p, 0, n_params * sizeof(float), stream), "memset");
         for (int l = 0; l < kMlpHidden; ++l) {
             Wb[l].alloc(static_cast<size_t>(kMlpWidth) * in_dim[l]);
             if (l > 0) WbT[l].alloc(static_cast<size_t>(kMlpWidth) * in_dim[l]);
         }
         loss.alloc(1);
         err.alloc(1);
-        ck(cudaMemset(err.p, 0, sizeof(int)), "memset");
+        ck(cudaMemsetAsync(err.p, 0, sizeof(int), stream), "memset");
         h_loss.alloc(1);
         h_err.alloc(1);
         ck(configure_mlp_gemm(), "GEMM shared-memory limit");
@@ -287,7 +287,7 @@ struct sb_mlp {
         ck(cudaMemcpyAsync(h_err.p, err.p, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H status");
         ck(cudaStreamSynchronize(s), "mlp");
         if (h_err.p[0] != kDevOk) {
-            ck(cudaMemset(err.p, 0, sizeof(int)), "memset");
+            ck(cudaMemsetAsync(err.p, 0, sizeof(int), s), "memset");
             raise(SB_ERR_TIMEOUT, "a bounded device-side wait ran out in the network kernels");
         }
     }

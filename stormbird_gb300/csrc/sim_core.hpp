@@ -620,6 +620,7 @@ struct sb_sim {
         }
     }
 
+    // Zeroes go in on the case's own stream, which does not wait for the default one.
     void allocate() {
         chord_local.alloc(N); chord_global.alloc(N); chord_span_pts.alloc(Np); span_s.alloc(N); span_e.alloc(N);
         solve_basis.alloc(2 * static_cast<size_t>(N));
@@ -634,23 +635,23 @@ struct sb_sim {
         if (solver_kind == 1 || solve.start_with_linearized) factors.alloc(static_cast<size_t>(N) * N);
         if (solver_kind == 0) {  // two planes of N rows x 3 x stride; the padding columns stay 0
             factors_split.alloc(static_cast<size_t>(N) * si_matrix_stride(N) * 6);
-            ck(cudaMemset(factors_split.p, 0, factors_split.n * sizeof(float)), "memset");
+            ck(cudaMemsetAsync(factors_split.p, 0, factors_split.n * sizeof(float), stream), "memset");
         }
-        ck(cudaMemset(fixed.p, 0, N * sizeof(d3)), "memset");
+        ck(cudaMemsetAsync(fixed.p, 0, N * sizeof(d3), stream), "memset");
         counters.alloc(4); err.alloc(4);
-        ck(cudaMemset(counters.p, 0, 4 * sizeof(unsigned long long)), "memset");
-        ck(cudaMemset(err.p, 0, 4 * sizeof(int)), "memset");
+        ck(cudaMemsetAsync(counters.p, 0, 4 * sizeof(unsigned long long), stream), "memset");
+        ck(cudaMemsetAsync(err.p, 0, 4 * sizeof(int), stream), "memset");
         gamma_prev.alloc(N); gamma_tmp.alloc(N); scalars.alloc(8);
-        ck(cudaMemset(gamma_prev.p, 0, N * sizeof(double)), "memset");
+        ck(cudaMemsetAsync(gamma_prev.p, 0, N * sizeof(double), stream), "memset");
         gamma_p = gamma_prev.p;
-        ck(cudaMemset(scalars.p, 0, 8 * sizeof(double)), "memset");
+        ck(cudaMemsetAsync(scalars.p, 0, 8 * sizeof(double), stream), "memset");
         if (solver_kind == 1 || solve.start_with_linearized) lin_work.alloc(lin_work_doubles(N));
         vel_out.alloc(N); hist0.alloc(N); hist1.alloc(N);
-        ck(cudaMemset(hist0.p, 0, N * sizeof(d3)), "memset");
-        ck(cudaMemset(hist1.p, 0, N * sizeof(d3)), "memset");
+        ck(cudaMemsetAsync(hist0.p, 0, N * sizeof(d3), stream), "memset");
+        ck(cudaMemsetAsync(hist1.p, 0, N * sizeof(d3), stream), "memset");
         L = OutLayout::make(N, S);
         out.alloc(L.total);
-        ck(cudaMemset(out.p, 0, L.total * sizeof(double)), "memset");
+        ck(cudaMemsetAsync(out.p, 0, L.total * sizeof(double), stream), "memset");
         h_out.alloc(L.total);
         h_err.alloc(4);
         fs.alloc(nfs);

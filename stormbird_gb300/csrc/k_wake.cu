@@ -413,9 +413,6 @@ __device__ inline void wake_panel_elem(const DevModel& m, const WakeBuffers& w, 
     const int N = m.N;
     const long long Np = m.Np;
     const int s = static_cast<int>(id / N), j = static_cast<int>(id % N);
-    const int wg = m.wing_of_line[j];
-    const d3* P = w.pts_new;
-    const d3 pp[4] = {P[s * Np + j + wg], P[s * Np + j + 1 + wg], P[(s + 1) * Np + j + 1 + wg], P[(s + 1) * Np + j + wg]};
     double g;
     if (shift) g = (s == 0) ? w.str_old[j] : w.str_old[id - N];
     else g = w.str_old[id];
@@ -428,6 +425,9 @@ __device__ inline void wake_panel_elem(const DevModel& m, const WakeBuffers& w, 
         w.rec32[id].v[kRec32Gamma] = 0.f;
         return;
     }
+    const int wg = m.wing_of_line[j];
+    const d3* P = w.pts_new;
+    const d3 pp[4] = {P[s * Np + j + wg], P[s * Np + j + 1 + wg], P[(s + 1) * Np + j + 1 + wg], P[(s + 1) * Np + j + wg]};
     PanelRec<double> q;
     const bool need64 = (s == 0) || w.rec64;
     write_panel_records(pp, m.panel_core[id], g, m.far_field_ratio, wg, &w.rec32[id], need64 ? &q : nullptr);
@@ -577,7 +577,11 @@ __global__ void k_wake_advect_jobs(const CaseStepJob* jobs, int n) {
     wake_advect_elem(J.m, J.w, J.p.dt, J.steps_done, id);
 }
 
-__global__ void k_wake_panels_jobs(const CaseStepJob* jobs, int n) {
+// Five blocks an SM: while wakes fill, most panels are of zero strength and their threads only wait for it. With the
+// 130 registers of the integer conversions three blocks fit (512 filling wakes, 23.5M panels: 1.18 ms; 0.83
+// with five and the points loaded after the test). In full wakes the spills are lost among the FP64 work (24
+// cases, 1.05M panels: 210 us, 213 with five).
+__global__ void __launch_bounds__(kPanelThreads, 5) k_wake_panels_jobs(const CaseStepJob* jobs, int n) {
     const CaseStepJob& J = jobs[job_of_block<CaseStepJob, &CaseStepJob::blk_panels>(jobs, n, blockIdx.x)];
     const long long id = (blockIdx.x - J.blk_panels) * static_cast<long long>(kPanelThreads) + threadIdx.x;
     wake_panel_elem(J.m, J.w, 1, id);

@@ -616,8 +616,9 @@ __device__ void si_solve(const DevModel& m, const SolveSettings& st, const Solve
         if (C == 2) {
             fa = L.fa0 + o[0];
             fc = L.fc0 + o[2];
-            a = L.a0 + (f32_to_f64_any(o[0]) + f32_to_f64_any(o[1]));
-            c = L.c0 + (f32_to_f64_any(o[2]) + f32_to_f64_any(o[3]));
+            // exactly: in calm air at rest the sums are 0, and so have to be the velocity and its angle
+            a = L.a0 + (f32_to_f64_exact(o[0]) + f32_to_f64_exact(o[1]));
+            c = L.c0 + (f32_to_f64_exact(o[2]) + f32_to_f64_exact(o[3]));
             return;
         }
         const d3 fx = b.fixed[i];

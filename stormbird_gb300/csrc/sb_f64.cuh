@@ -59,15 +59,11 @@ __device__ __forceinline__ float f64_to_f32_rn(double v) {
     const unsigned bits = __funnelshift_l(lo, mag, 3);
     return __uint_as_float((bits + (((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (bits & 1u)) >> 29)) | (hi & 0x80000000u));
 }
-// v exactly, by integer arithmetic, for v finite; magnitudes below 2^-126 give a value below 2^-126.
+// v exactly, by integer arithmetic, for v finite; magnitudes below 2^-126 give a value below 2^-126, 0 too: not
+// where a result of 0 counts.
 __device__ __forceinline__ double f32_to_f64(float v) {
     const unsigned u = __float_as_uint(v), mag = u & 0x7FFFFFFFu;
     return __hiloint2double(static_cast<int>(((mag >> 3) + 0x38000000u) | (u & 0x80000000u)), static_cast<int>(u << 29));
-}
-// the same with infinities and NaNs kept
-__device__ __forceinline__ double f32_to_f64_any(float v) {
-    if ((__float_as_uint(v) & 0x7F800000u) == 0x7F800000u) return static_cast<double>(v);
-    return f32_to_f64(v);
 }
 // v exactly, whatever it is
 static __device__ __noinline__ double f32_to_f64_slow(float v) { return static_cast<double>(v); }

@@ -88,7 +88,7 @@ __device__ void wing_forces(const DevModel& m, const StepParams& p, const ForceA
         const d3 circ = q == 0.0 ? mk(0, 0, 0) : (g * cross(fv, sl_out)) * m.density;
         d3 visc = mk(0, 0, 0);
         if (!m.include_viscous_lift) visc = normalize(cross(sl_local, fv)) * (lift.cl_post * ff);
-        const d3 drag = q > 0.0 ? fv * (rsqrt_any(q) * line_drag(fo, lift, tab) * ff) : mk(0, 0, 0);
+        const d3 drag = q == 0.0 ? mk(0, 0, 0) : fv * (rsqrt_any(q) * line_drag(fo, lift, tab) * ff);  // a NaN stays
         d3 am = mk(0, 0, 0);
         if (fo.added_mass_factor != 0.0)
             am = added_mass(fo.added_mass_factor, m.density, m.chord_len[i], sl_out,

@@ -44,3 +44,16 @@ def test_batch(gpu_lib):
     for k in range(5):
         b.do_step(time=0.1 * k, time_step=0.1, freestream_velocity=np.zeros((3 * 34, 3)))
         assert not np.any(b.circulation()) and not np.any(b.summary()[:, :7])
+
+
+@pytest.mark.parametrize("panels", [17, 100, 240])
+def test_linearized(gpu_lib, oracle_mod, panels):
+    """Calm air has no Linearized solution: no number in all that follows from it, the drag included."""
+    js = setup(None, panels)
+    g, o = Simulation(js), oracle_mod.OracleSimulation(js)
+    for _ in range(2):
+        fs = np.zeros((g.nr_freestream_points, 3))
+        a = outputs(g.do_step(time=0.0, time_step=0.1, freestream_velocity=fs))
+        b = outputs(o.do_step(time=0.0, time_step=0.1, freestream_velocity=fs))
+        for name in a:
+            assert np.array_equal(a[name], b[name], equal_nan=True), name

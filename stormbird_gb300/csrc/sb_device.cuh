@@ -61,8 +61,11 @@ __host__ __device__ inline d3 normalize(d3 a) {
 #ifdef __CUDA_ARCH__
     const double q = len2(a);
     if (q > 0.0) {
-        const double r = rsqrt_any(q);
-        return {a.x * r, a.y * r, a.z * r};
+        // one Newton step to unit length: exactly 1 for a vector along an axis, so that what is taken out along a
+        // vertical span (a velocity along it, the chord) leaves 0 and not rounding
+        const double r = rsqrt_any(q), x = a.x * r, y = a.y * r, z = a.z * r;
+        const double h = 0.5 * fma(-x, x, fma(-y, y, fma(-z, z, 1.0)));
+        return {fma(x, h, x), fma(y, h, y), fma(z, h, z)};
     }
     return {0.0, 0.0, 0.0};
 #else

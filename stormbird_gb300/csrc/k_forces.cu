@@ -89,7 +89,8 @@ __device__ void wing_forces(const DevModel& m, const StepParams& p, const ForceA
         d3 visc = mk(0, 0, 0);
         if (!m.include_viscous_lift) visc = normalize(cross(sl_local, fv)) * (lift.cl_post * ff);
         const d3 drag = q == 0.0 ? mk(0, 0, 0) : fv * (rsqrt_any(q) * line_drag(fo, lift, tab) * ff);  // a NaN stays
-        d3 am = mk(0, 0, 0);
+        const double none = 0.0 * (fa.x + fa.y + fa.z);  // no number where the acceleration is none
+        d3 am = mk(none, none, none);
         if (fo.added_mass_factor != 0.0)
             am = added_mass(fo.added_mass_factor, m.density, m.chord_len[i], sl_out,
                             body ? m.chord_local[i] : m.chord_global[i], fa);

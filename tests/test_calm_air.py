@@ -20,7 +20,7 @@ def outputs(r):
     s = r.sectional_forces
     return {"circulation": r.circulation_strength, "velocity": r.force_input.velocity, "angles": r.force_input.angles_of_attack,
             "circulatory": s.circulatory, "viscous": s.viscous_lift, "drag": s.sectional_drag, "total": s.total,
-            "force": r.force_sum, "moment": r.moment_sum, "residual": np.array([r.residual])}
+            "added": s.added_mass, "force": r.force_sum, "moment": r.moment_sum, "residual": np.array([r.residual])}
 
 
 @pytest.mark.parametrize("wind", [(0.0, 0.0, 0.0), (0.0, 0.0, 5.0)])
@@ -53,9 +53,22 @@ def test_linearized(gpu_lib, oracle_mod, panels, wind):
     included, and no error (which rounding beside the 0 would give: a singular matrix)."""
     js = setup(None, panels)
     g, o = Simulation(js), oracle_mod.OracleSimulation(js)
-    for _ in range(2):
+    for _ in range(3):  # accelerations from the third step
         fs = np.tile(wind, (g.nr_freestream_points, 1))
         a = outputs(g.do_step(time=0.0, time_step=0.1, freestream_velocity=fs))
         b = outputs(o.do_step(time=0.0, time_step=0.1, freestream_velocity=fs))
         for name in a:
             assert np.array_equal(a[name], b[name], equal_nan=True), name
+
+
+def test_no_time(gpu_lib, oracle_mod):
+    """Steps of no length have no acceleration: no added mass, not even of a foil without one."""
+    js = setup(S.simple_iterative(5, 0.05, 0.0, 0.0))
+    g, o = Simulation(js), oracle_mod.OracleSimulation(js)
+    for k in range(4):
+        fs = np.tile([8.0 + 0.3 * k * k, 5.0, 0.0], (g.nr_freestream_points, 1))
+        a = outputs(g.do_step(time=0.0, time_step=0.0, freestream_velocity=fs))
+        b = outputs(o.do_step(time=0.0, time_step=0.0, freestream_velocity=fs))
+        for name in ("added", "total", "force"):
+            assert np.array_equal(np.isnan(a[name]), np.isnan(b[name])), name
+    assert np.all(np.isnan(b["added"]))

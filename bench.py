@@ -750,8 +750,8 @@ def qs_sweep(args, device):
     """Solves/s of a quasi-steady sweep (the shape of CompleteSailModel wind-angle sweeps):
     seeded cases of 1-6 sails x 16-96 panels at AWA 20-180 deg, 5-20 m/s, quasi-steady
     defaults (Linearized solver, horseshoe wake). plain = one Simulation per case; batched =
-    one Batch (horseshoe matrices per case on the pool streams, all Linearized solves in one
-    k_solve_lin_jobs launch, graph replay). Host clock around the public calls, host
+    one Batch (horseshoe matrices by one job list, the Linearized solves in one
+    k_lin_refined_jobs launch per cluster size, graph replay). Host clock around the public calls, host
     freestream in, results out; steps 0-3 untimed, then `steps` timed."""
     import torch
 
@@ -771,9 +771,9 @@ def qs_sweep(args, device):
         if k >= warm:
             t_plain += time.perf_counter() - t0
     g_plain = np.concatenate([r.circulation_strength for r in rs])
-    # the largest case alone: its Linearized solve (Gaussian elimination, 2N^3/3 FLOP in f64)
-    # timed with CUDA events on the library's stream, against the measured FP64 peak
-    from stormbird_gb300.simulation import measure_fp64_peak
+    # the largest case alone: its Linearized solve (FP32 block inverse, f64 refinement) timed with CUDA
+    # events on the library's stream, the inverse's 2N^3 operations against the measured FP32 peak
+    from stormbird_gb300.simulation import measure_fp32_peak
 
     ib = max(range(n), key=lambda i: sims[i].nr_span_lines)
     big, (_, ub) = sims[ib], cases[ib]
@@ -783,13 +783,14 @@ def qs_sweep(args, device):
         big.do_step(time=0.0, time_step=0.1, freestream_velocity=np.tile(ub * (1.0 + 0.01 * k), (big.nr_freestream_points, 1)))
         solve_ms.append(big.last_step_timing()["solve"])
     nb = big.nr_span_lines
-    ge_flop = 2.0 * nb ** 3 / 3.0
-    fp64 = measure_fp64_peak(device, 3)
+    refined = nb <= 768  # more lines are eliminated in f64
+    flop = 2.0 * nb ** 3
+    fp32 = measure_fp32_peak(device, 3)
     largest = {"span_lines": nb, "solve_ms": min(solve_ms),
-               "elimination_gflops": ge_flop / (min(solve_ms) * 1e-3) / 1e9, "fp64_peak_tflops": fp64,
-               "frac_of_fp64_peak": ge_flop / (min(solve_ms) * 1e-3) / (fp64 * 1e12) if fp64 > 0 else None,
-               "note": "solve phase = matrix elimination, back substitution and the Linearized epilogue; "
-                       "FLOP counts the elimination only"}
+               "inverse_gflops": flop / (min(solve_ms) * 1e-3) / 1e9 if refined else None, "fp32_peak_tflops": fp32,
+               "frac_of_fp32_peak": flop / (min(solve_ms) * 1e-3) / (fp32 * 1e12) if refined and fp32 > 0 else None,
+               "note": "solve phase = system, FP32 inverse, f64 refinement and the Linearized epilogue; the operations "
+                       "counted are the inverse's alone"}
     for s in sims:
         s.close()
     del sims
@@ -960,9 +961,10 @@ def run_profile_wake(args):
 
 
 def run_profile_mlp(args):
-    """Warm-start network forward passes over 131,072 rows (1,024 GEMM tiles of 128 rows),
-    three times, then one training step on 16,384 rows: 4 tensor-core GEMMs per forward pass
-    (K = 64, 256, 256, 256), so -k regex:k_mlp_gemm -s 4 -c 4 captures the second pass.
+    """Warm-start network forward passes over 131,072 rows (1,024 tiles of 128 rows), three
+    times, then one training step on 16,384 rows: a forward pass is one k_mlp_forward launch, so
+    -k regex:k_mlp_forward -s 1 -c 1 captures the second pass, -s 3 -c 1 the training step's, and
+    -k regex:k_mlp_gemm its input- and weight-gradient GEMMs.
     Prints the forward time per pass (CUDA events) and the GEMM rate it implies."""
     import torch
 
@@ -985,7 +987,7 @@ def run_profile_mlp(args):
     flops = 2.0 * rows * 256 * (64 + 3 * 256)
     print(json.dumps({"mode": "profile-mlp", "rows": rows, "forward_ms": ms,
                       "gemm_tflops_best_pass": flops / (min(ms) * 1e-3) / 1e12,
-                      "note": "host-launched forward incl. input packing and the output layer"}), flush=True)
+                      "note": "host-launched forward incl. the output layer and the status read back"}), flush=True)
 
 
 # --------------------------------------------------------------------------------------
